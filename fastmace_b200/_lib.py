@@ -62,6 +62,7 @@ class LayerStruct(ctypes.Structure):
         ("sc_coef", c_void_p), ("w_readout", c_void_p), ("tc", c_void_p * 9), ("first", c_void_p * 4),
         ("rad_img", c_void_p), ("tc_img", c_void_p * 9), ("first_img", c_void_p * 2),
         ("mlp_img", c_void_p),
+        ("rad_tab", c_void_p), ("rad_tab_intervals", c_int32), ("rad_tab_per_angstrom", c_float),
     ]
 
 

@@ -54,6 +54,9 @@ struct EdgeParams {
     double cell[9];
     const float* rad_w[FMB_MAX_LAYERS][3];
     const float* mlp_img[FMB_MAX_LAYERS];     // the same three layers as tensor-core operand images (or null)
+    const float* table[FMB_MAX_LAYERS];       // or the third layer's features as polynomials of the edge length
+    int table_intervals[FMB_MAX_LAYERS];
+    float table_per_angstrom[FMB_MAX_LAYERS];
     uint32_t* error_word;
 };
 
@@ -512,6 +515,86 @@ k_edge_features_tc(const __grid_constant__ EdgeParams p, const double* __restric
     }
 }
 
+// ------------------------------------------------------------------------------------------------ tabulated MLP
+// The hidden features of an edge are a function of its length alone, fixed by the model's weights: instead of running
+// three layers per edge, interaction and direction (209 kFLOP on the tensor cores and 384 SiLUs, a chain of six
+// MMA -> SiLU round trips), look the function up as a piecewise polynomial of degree 5 (value and exact derivative
+// from the same six coefficients). The table (295 KB per interaction at 32 intervals per Å) lives in L2 and, for the
+// distances a crystal has, largely in L1.
+//
+// A warp takes 16 edges: both halves form the edge vectors (lane i and lane 16 + i the same one; the lower half goes on
+// to the interval, the upper half to the harmonics), then the lower half evaluates interaction 0 and the upper half
+// interaction 1 of one edge after the other, four features per lane, so that every load and store is a whole 256-byte
+// row. The position inside the interval is exact in fp32 (the interval is a power of two).
+//
+// Bound by the 1.1 KB written per edge and 3 KB of table rows read.
+constexpr int kTabCoefs = 6;
+constexpr int kTabEdges = 16;                 // per warp
+constexpr int kTabWarps = 8;
+
+__device__ __forceinline__ void horner(float c0, float c1, float c2, float c3, float c4, float c5, float u, float& value,
+                                       float& slope) {
+    float b = c5, d = c5;
+    b = fmaf(b, u, c4);
+    d = fmaf(d, u, b);
+    b = fmaf(b, u, c3);
+    d = fmaf(d, u, b);
+    b = fmaf(b, u, c2);
+    d = fmaf(d, u, b);
+    b = fmaf(b, u, c1);
+    d = fmaf(d, u, b);
+    value = fmaf(b, u, c0);
+    slope = d;
+}
+
+__global__ void __launch_bounds__(kTabWarps * 32)
+k_edge_features_table(const __grid_constant__ EdgeParams p, const double* __restrict__ x,
+                      const int32_t* __restrict__ edge_index, const float* __restrict__ unit_shifts,
+                      const long long* __restrict__ count_ptr, float* __restrict__ edge_vec, float* __restrict__ edge_sh,
+                      float* __restrict__ edge_hidden) {
+    const int lane = threadIdx.x & 31, half = lane >> 4, sub = lane & 15;
+    const long long count = *count_ptr;
+    const long long e0 = ((long long)blockIdx.x * kTabWarps + (threadIdx.x >> 5)) * kTabEdges;
+    if (e0 >= count) return;
+    const int live = (int)min((long long)kTabEdges, count - e0);
+    float len = 0.0f;
+    if (sub < live) {
+        const EdgeGeometry g = edge_geometry(p, x, edge_index, unit_shifts, e0 + sub);
+        len = g.len;
+        if (half) store_harmonics(g, edge_vec, edge_sh, e0 + sub);
+    }
+    for (int layer = half; layer < p.n_layers; layer += 2) {
+        const float4* __restrict__ table = reinterpret_cast<const float4*>(p.table[layer]) + sub;
+        const float per = p.table_per_angstrom[layer], slope_scale = 2.0f * per;
+        const int last = p.table_intervals[layer] - 1;
+        float4* hv = reinterpret_cast<float4*>(edge_hidden + ((long long)(2 * layer) * p.capacity + e0) * kRadial) + sub;
+        float4* ht = reinterpret_cast<float4*>(edge_hidden + ((long long)(2 * layer + 1) * p.capacity + e0) * kRadial) + sub;
+        const unsigned mask = half ? 0xffff0000u : 0x0000ffffu;
+#pragma unroll 4
+        for (int s = 0; s < kTabEdges; ++s) {
+            const float r = __shfl_sync(mask, len, (half << 4) + s);
+            if (s >= live) break;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f), t = v;
+            if (r < p.r_cut) {
+                const float at = r * per;
+                const int i = min((int)at, last);
+                // a pair of atoms in one place has no radial features: not a number, as 1 / r makes it
+                const float u = r > 0.0f ? fmaf(2.0f, at - (float)i, -1.0f) : __int_as_float(0x7fffffff);
+                const float4* row = table + (long long)i * (kTabCoefs * kRadial / 4);
+                const float4 c0 = __ldg(row), c1 = __ldg(row + 16), c2 = __ldg(row + 32), c3 = __ldg(row + 48),
+                             c4 = __ldg(row + 64), c5 = __ldg(row + 80);
+                horner(c0.x, c1.x, c2.x, c3.x, c4.x, c5.x, u, v.x, t.x);
+                horner(c0.y, c1.y, c2.y, c3.y, c4.y, c5.y, u, v.y, t.y);
+                horner(c0.z, c1.z, c2.z, c3.z, c4.z, c5.z, u, v.z, t.z);
+                horner(c0.w, c1.w, c2.w, c3.w, c4.w, c5.w, u, v.w, t.w);
+                t.x *= slope_scale; t.y *= slope_scale; t.z *= slope_scale; t.w *= slope_scale;
+            }
+            hv[s * (kRadial / 4)] = v;
+            ht[s * (kRadial / 4)] = t;
+        }
+    }
+}
+
 // The harmonics and their gradient exactly as the edge and adjoint kernels evaluate them, on plain vectors.
 __global__ void k_harmonics_probe(const float* __restrict__ vectors, const float* __restrict__ grad_sh,
                                   float* __restrict__ sh, float* __restrict__ grad_vectors, int n) {
@@ -546,10 +629,22 @@ int edge_features(const fmb_model_t* model, const fmb_nl_t* nl, const fmb_work_t
     for (int t = 0; t < model->n_layers; ++t)
         for (int k = 0; k < 3; ++k) p.rad_w[t][k] = model->layer[t].rad_w[k];
     p.error_word = work->status;
-    bool images = model->n_layers > 0;
+    bool images = model->n_layers > 0, tables = model->n_layers > 0;
     for (int t = 0; t < model->n_layers; ++t) {
         p.mlp_img[t] = model->layer[t].mlp_img;
         images = images && p.mlp_img[t] != nullptr;
+        const fmb_layer_t& layer = model->layer[t];
+        p.table[t] = layer.rad_tab;
+        p.table_intervals[t] = layer.rad_tab_intervals;
+        p.table_per_angstrom[t] = layer.rad_tab_per_angstrom;
+        tables = tables && layer.rad_tab != nullptr && layer.rad_tab_intervals > 0 &&
+                 layer.rad_tab_intervals >= layer.rad_tab_per_angstrom * model->r_cut;
+    }
+    if (tables) {
+        k_edge_features_table<<<ceil_div(nl->capacity, kTabWarps * kTabEdges), kTabWarps * 32, 0, stream>>>(
+            p, positions, nl->edge_index, nl->unit_shifts, count, work->edge_vec, work->edge_sh, work->edge_hidden);
+        FMB_LAUNCH_CHECK();
+        return FMB_OK;
     }
     if (images) {
         // operand images packed: the tcgen05 kernel, 64 edges per CTA

@@ -10,6 +10,7 @@ into W, species skip restricted to present species: ``fastmace/config.py:208-219
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 
 import numpy as np
@@ -58,6 +59,8 @@ def tensor_core_image(blocks) -> torch.Tensor:
     of the transposed block as 4,096 tf32 values followed by their 4,096 remainders, both in the swizzled operand
     layout. Blocks with N % 128 != 0 or K % 32 != 0 stay zero."""
     index = _swizzled_tile_index()
+    source_of = torch.empty_like(index)
+    source_of[index] = torch.arange(len(index))          # where each float of a tile comes from
     out = []
     for block in blocks:
         k, n = block.shape
@@ -67,11 +70,9 @@ def tensor_core_image(blocks) -> torch.Tensor:
             hi = tf32_round(bt)
             lo = tf32_round(bt - hi)
             view = image.view(n // 128, k // 32, 2, 4096)
-            for nt in range(n // 128):
-                for kc in range(k // 32):
-                    rows, cols = slice(nt * 128, nt * 128 + 128), slice(kc * 32, kc * 32 + 32)
-                    view[nt, kc, 0, index] = hi[rows, cols].reshape(-1)
-                    view[nt, kc, 1, index] = lo[rows, cols].reshape(-1)
+            for part, source in enumerate((hi, lo)):
+                tiles = source.view(n // 128, 128, k // 32, 32).transpose(1, 2).reshape(n // 128, k // 32, 4096)
+                view[:, :, part] = tiles[:, :, source_of]
         out.append(image)
     return torch.cat(out)
 
@@ -130,32 +131,95 @@ def mlp_image(w0: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor) -> torch.Ten
     return image
 
 
-def contraction_terms(spec: MaceSpec, weights, layer: int, species_z):
-    """(terms int32 [T, 4], coef float64 [n_species, T, C]) of one layer's symmetric contraction, sorted by output."""
-    c = spec.channels
-    merged: dict[tuple, np.ndarray] = {}
-    for big_l in range(spec.l_out_max(layer) + 1):
-        for nu in range(1, spec.correlation + 1):
-            mono, m_out, weight, coef, _ = so3.contraction_polynomial(nu, big_l, spec.sh_lmax)
-            w = _f64(weights[f"l{layer}.sc.{big_l}.{nu}"]).numpy()[[z - 1 for z in species_z]]  # [nz, k, C]
-            for t in range(len(coef)):
-                key = (big_l * big_l + int(m_out[t]), nu, tuple(int(i) for i in mono[t]))
-                value = coef[t] * w[:, weight[t], :]
-                if key in merged:
-                    merged[key] = merged[key] + value
-                else:
-                    merged[key] = value
-    keys = sorted(merged)
-    if tuple(keys) != so3.contraction_keys(spec.l_out_max(layer), spec.correlation, spec.sh_lmax):
-        raise RuntimeError("contraction terms are not in the order the generated kernels expect")
+RADIAL_DEGREE = 5
+
+
+def radial_hidden_float64(w0, w1, w2, r: torch.Tensor, r_cut: float, with_tangent: bool = True):
+    """Third hidden layer of a radial MLP (scaled fp32 weights [8][64], [64][64], [64][64]) and its d/dr (or None) at
+    lengths ``r``, [n, 64] float64 each. The envelope polynomial is continued beyond the cutoff (the caller cuts there)."""
+    x = (r / r_cut)[:, None]
+    x2 = x * x
+    x5 = x2 * x2 * x
+    envelope = 1 + x5 * (-21 + 35 * x - 15 * x2)
+    k = torch.arange(1, 9, dtype=torch.float64) * (math.pi / r_cut)
+    a = r[:, None] * k
+    bessel = k * torch.sinc(a / math.pi)                  # sin(k r) / r
+    value, tangent = math.sqrt(2 / r_cut) * bessel * envelope, None
+    if with_tangent:
+        d_envelope = x2 * x2 * (-105 + 210 * x - 105 * x2) / r_cut
+        # smooth at r = 0, where the quotient loses its digits to cancellation
+        d_bessel = torch.where(a < 0.02, k * k * a * (-1 / 3 + a * a / 30), (k * torch.cos(a) - bessel) / r[:, None])
+        tangent = math.sqrt(2 / r_cut) * (d_bessel * envelope + bessel * d_envelope)
+    for w in (w0, w1, w2):
+        w = w.to(torch.float64)
+        z = value @ w
+        s = torch.sigmoid(z)
+        if with_tangent:
+            tangent = SILU_NORM * s * (1 + z * (1 - s)) * (tangent @ w)
+        value = SILU_NORM * z * s
+    return value, tangent
+
+
+def radial_table(w0, w1, w2, r_cut: float):
+    """The hidden radial features as piecewise polynomials of the length: (coefficients [intervals, 6, 64] fp32,
+    intervals per Å), or None where 512 intervals per Å are not enough.
+
+    The features of an edge depend on its length only, through a smooth function fixed by the weights. Polynomials of
+    degree 5 through the Chebyshev nodes of intervals of 1/32 Å reproduce it below fp32 rounding for the benchmark's
+    models (4e-8 of the norm in the value and 5e-8 in d/dr, rounding of the coefficients included; the 3xTF32 chain of
+    three layers they replace is off by 3e-7 to 1e-6). The interval is halved until value and d/dr, checked between the
+    nodes, are within 2e-7 and 4e-7 of their largest magnitude, so a model with a steeper radial function gets a finer
+    table and one that no table serves keeps the MLP kernel."""
+    n_c = RADIAL_DEGREE + 1
+    w0, w1, w2 = (w.cpu() for w in (w0, w1, w2))
+    nodes = torch.cos(math.pi * (torch.arange(n_c, dtype=torch.float64) + 0.5) / n_c)
+    fit = torch.linalg.inv(torch.stack([nodes ** k for k in range(n_c)], dim=1))
+    probes = torch.tensor([-1.0, 0.5], dtype=torch.float64)        # d/dr is worst at the ends
+    powers = torch.stack([probes ** k for k in range(n_c)], dim=1)
+    slopes = torch.stack([k * probes ** max(k - 1, 0) for k in range(n_c)], dim=1)
+    for per in (32, 64, 128, 256, 512):
+        n = int(math.ceil(r_cut * per))
+        middle = (torch.arange(n, dtype=torch.float64)[:, None] + 0.5) / per
+        at_nodes = radial_hidden_float64(w0, w1, w2, (middle + nodes / (2 * per)).reshape(-1), r_cut, False)[0]
+        table = (fit @ at_nodes.reshape(n, n_c, -1)).to(torch.float32)
+        r = (middle + probes / (2 * per)).reshape(-1)
+        value, tangent = radial_hidden_float64(w0, w1, w2, r, r_cut)
+        inside = (r < r_cut)[:, None]
+        got = (powers @ table.double()).reshape(value.shape)
+        d_got = (slopes @ table.double()).reshape(value.shape) * (2 * per)
+        if bool((((got - value) * inside).abs().max() <= 2e-7 * value.abs().max())
+                & (((d_got - tangent) * inside).abs().max() <= 4e-7 * tangent.abs().max())):
+            return table.contiguous(), per
+    return None
+
+
+@functools.lru_cache(maxsize=None)
+def _contraction_layout(l_out_max: int, correlation: int, sh_lmax: int):
+    """(terms int32 [T, 4], per (l_out, degree) block the row of the coefficient table each polynomial term adds to)."""
+    keys = so3.contraction_keys(l_out_max, correlation, sh_lmax)
     terms = np.full((len(keys), 4), -1, dtype=np.int32)
-    coefs = np.zeros((len(species_z), len(keys), c), dtype=np.float64)
-    for t, key in enumerate(keys):
-        m_out, _, mono = key
+    for t, (m_out, _, mono) in enumerate(keys):
         terms[t, :len(mono)] = mono
         terms[t, 3] = m_out
-        coefs[:, t, :] = merged[key]
-    return terms, coefs
+    row_of = {key: t for t, key in enumerate(keys)}
+    rows = {}
+    for big_l in range(l_out_max + 1):
+        for nu in range(1, correlation + 1):
+            mono, m_out, _, _, _ = so3.contraction_polynomial(nu, big_l, sh_lmax)
+            rows[big_l, nu] = np.array([row_of[big_l * big_l + int(m), nu, tuple(int(i) for i in q)]
+                                        for m, q in zip(m_out, mono)])
+    return terms, rows
+
+
+def contraction_terms(spec: MaceSpec, weights, layer: int, species_z):
+    """(terms int32 [T, 4], coef float64 [n_species, T, C]) of one layer's symmetric contraction, sorted by output."""
+    terms, rows = _contraction_layout(spec.l_out_max(layer), spec.correlation, spec.sh_lmax)
+    coefs = np.zeros((len(terms), len(species_z), spec.channels), dtype=np.float64)
+    for (big_l, nu), row in rows.items():
+        _, _, weight, coef, _ = so3.contraction_polynomial(nu, big_l, spec.sh_lmax)
+        w = _f64(weights[f"l{layer}.sc.{big_l}.{nu}"]).numpy()[[z - 1 for z in species_z]]  # [nz, k, C]
+        np.add.at(coefs, row, coef[:, None, None] * w[:, weight, :].transpose(1, 0, 2))
+    return terms.copy(), coefs.transpose(1, 0, 2)
 
 
 class PackedModel:
@@ -213,6 +277,11 @@ class PackedModel:
             if spec.num_bessel == 8 and tuple(spec.radial_hidden) == (64, 64, 64):
                 layer.mlp_img = self._put(f"l{t}.rad.mlp_img",
                                           mlp_image(*(self.tensors[f"l{t}.rad.{i}"].cpu() for i in range(3))))
+                if spec.cutoff_p == 5:
+                    found = radial_table(*(self.tensors[f"l{t}.rad.{i}"] for i in range(3)), spec.r_cut)
+                    if found is not None:
+                        layer.rad_tab = self._put(f"l{t}.rad.table", found[0])
+                        layer.rad_tab_intervals, layer.rad_tab_per_angstrom = int(found[0].shape[0]), float(found[1])
             if t == 0:
                 x_species = h0 @ (w["l0.up.0"] / math.sqrt(c))
                 sc = torch.zeros(len(idx), spec.out_dim(0), c, dtype=torch.float64)

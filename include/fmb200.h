@@ -168,6 +168,13 @@ typedef struct {
      * 0 / 2,048 (first), 4,096 / 8,192 (second), 12,288 / 16,384 (third), 20,480 floats in all. Null on any layer =
      * the warp-level tensor-core kernel evaluates the MLPs from rad_w. */
     const float* mlp_img;
+    /* The third hidden layer of the radial MLP as a function of the edge length alone: rad_tab_intervals intervals of
+     * 1 / rad_tab_per_angstrom (a power of two) from length 0 to beyond the cutoff, per interval the six coefficients
+     * [6][64] of a polynomial in u in [-1, 1), constant term first. Null on any layer = the kernels above evaluate
+     * the MLPs edge by edge. */
+    const float* rad_tab;
+    int32_t rad_tab_intervals;
+    float rad_tab_per_angstrom;
 } fmb_layer_t;
 
 typedef struct {
