@@ -243,6 +243,7 @@ void block_linear(LinearBatch& batch, const Ctx& c, int rows, const float* in, l
                   long long out_off, int n_out, int l, int accumulate, const int32_t* batch_species = nullptr,
                   int select = -1) {
     GemmArgs& g = batch.list[batch.count++];
+    g = GemmArgs{};
     const int nm = 2 * l + 1;
     g.a = in + in_off;
     g.a_nm = nm; g.a_bs = in_atom; g.a_rs = k;
@@ -259,6 +260,12 @@ void block_linear(LinearBatch& batch, const Ctx& c, int rows, const float* in, l
     g.accumulate = accumulate;
     g.batch_species = batch_species;
     g.select = select;
+    if (batch_species && c.w->symcon_groups && c.w->n_symcon_groups > 0) {
+        // the contraction's groups hold every atom that gets rows, sorted by species
+        g.batch_list = c.w->symcon_groups;
+        g.batch_limit = rows;
+        g.list_m = 4 * c.w->n_symcon_groups * nm;
+    }
 }
 
 int run_linears(const Ctx& c, LinearBatch& batch) {

@@ -31,6 +31,12 @@ struct GemmArgs {
     // optional: only batches whose species equals `select` are written (species-dependent linear)
     const int32_t* batch_species = nullptr;
     int select = -1;
+    // optional, read by gemm_ws only: the batches of the rows are batch_list[0 ..] instead of 0, 1, 2, ... (`list_m` rows
+    // in all) -- atoms listed by species, so that a species-dependent linear visits the tiles of its own species;
+    // entries that are negative or not below batch_limit have no rows
+    const int32_t* batch_list = nullptr;
+    int batch_limit = 0;
+    int list_m = 0;
 };
 
 int gemm_simt(const GemmArgs& args, cudaStream_t stream);

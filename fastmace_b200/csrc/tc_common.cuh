@@ -37,7 +37,7 @@ __device__ __forceinline__ uint64_t k_step(int k8) {
 
 // instruction descriptor: D fp32, A and B tf32, both K-major, M = 128, N = TN
 template <int TN>
-__device__ __forceinline__ uint32_t make_idesc() {
+__host__ __device__ __forceinline__ constexpr uint32_t make_idesc() {
     return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
@@ -46,6 +46,42 @@ __device__ __forceinline__ float tf32_rna(float x) {
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
     return __uint_as_float(r);
 }
+
+// v = hi + lo with both parts representable in tf32 (hi rounds half away from zero, lo to nearest): six full-rate
+// instructions, where cvt.rna.tf32 runs at an eighth of the rate (splitting a 128 x 32 operand chunk with eight warps
+// took 1,000 cycles by conversions, 330 like this). A value that is not finite leaves lo not a number.
+__device__ __forceinline__ void split_tf32(float v, float& hi, float& lo) {
+    hi = __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u);
+    const float rest = v - hi;
+    const float scaled = rest * 8193.0f;                    // 2^13 + 1: keeps the upper 11 of 24 significant bits
+    lo = __fsub_rn(scaled, __fsub_rn(scaled, rest));
+}
+
+__device__ __forceinline__ void split_tf32(const float4& v, float4& hi, float4& lo) {
+    split_tf32(v.x, hi.x, lo.x);
+    split_tf32(v.y, hi.y, lo.y);
+    split_tf32(v.z, hi.z, lo.z);
+    split_tf32(v.w, hi.w, lo.w);
+}
+
+// One lane of a converged warp, the same one every time. Code that issues tcgen05 or bulk-copy instructions runs with
+// the whole warp on the same path and puts only the issue under this predicate: descriptors and addresses then stay in
+// uniform registers, where code under `lane == 0` moves each of them over per instruction (60 to 80 cycles per MMA and
+// 350 per bulk copy, measured, against 64 that an N = 128 MMA takes to execute).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t chosen;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "elect.sync _|p, 0xffffffff;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(chosen));
+    return chosen != 0;
+}
+
+// the warp's index as a value the compiler knows to be the same for all its lanes
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 
 __device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, int accumulate) {
     asm volatile(
