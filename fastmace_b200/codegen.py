@@ -72,24 +72,6 @@ def _emit(lin: int) -> str:
                               for mi, me, c in terms)
             out.append(f"    acc[{slots[(p, mo)]}] = fmaf(w[{p}], {expr}, acc[{slots[(p, mo)]}]);")
     out += ["}", ""]
-    # forward, two channels per thread on the packed FP32 pipe (fma.rn.f32x2): the per-channel quantities are pairs,
-    # a harmonic times its coupling coefficient is one scalar product shared by the pair
-    out += [f"template <> __device__ __forceinline__ void tp_forward_pair<{lin}>(const float2 (&x)[{in_dim}], "
-            f"const float (&Y)[16], const float2 (&w)[{len(paths)}], float2 (&acc)[{mid}]) {{"]
-    for p, path in enumerate(paths):
-        out.append(f"    // path {p}: {path['l_in']} x {path['l_edge']} -> {path['l_out']}")
-        by_out = {}
-        for mi, me, mo, c in path["terms"]:
-            by_out.setdefault(mo, []).append((mi, me, c))
-        for mo, terms in sorted(by_out.items()):
-            lines = []
-            for k, (mi, me, c) in enumerate(terms):
-                pair = f"pair_of({_lit(c)} * Y[{path['edge_off'] + me}])"
-                xin = f"x[{path['in_off'] + mi}]"
-                lines.append(f"float2 e = __fmul2_rn({xin}, {pair});" if k == 0 else f"e = __ffma2_rn({xin}, {pair}, e);")
-            slot = slots[(p, mo)]
-            out.append(f"    {{ {' '.join(lines)} acc[{slot}] = __ffma2_rn(w[{p}], e, acc[{slot}]); }}")
-    out += ["}", ""]
     # backward
     out += [f"template <bool FLIP, bool NEED_DX> __device__ __forceinline__ void tp_backward_{lin}("
             f"const float (&x)[{in_dim}], const float (&Y)[16], const float (&w)[{len(paths)}], "
@@ -119,44 +101,6 @@ def _emit(lin: int) -> str:
         out.append("        }")
         out.append("    }")
     out += ["}", ""]
-    # backward, two channels per thread (packed FP32): x, w, wp, g, dx and the partial sums dY, dr are pairs, the
-    # harmonics scalars; a coupling coefficient enters as a constant pair
-    out += [f"template <bool FLIP, bool NEED_DX> __device__ __forceinline__ void tp_backward_pair_{lin}("
-            f"const float2 (&x)[{in_dim}], const float (&Y)[16], const float2 (&w)[{len(paths)}], "
-            f"const float2 (&wp)[{len(paths)}], const float2 (&g)[{mid}], float2 (&dY)[16], float2& dr, "
-            f"float2 (&dx)[{in_dim}]) {{"]
-    for p, path in enumerate(paths):
-        sign = -1.0 if path["l_edge"] % 2 else 1.0
-        out.append(f"    {{  // path {p}: {path['l_in']} x {path['l_edge']} -> {path['l_out']}")
-        out.append(f"        constexpr float sg = FLIP ? {_lit(sign)} : 1.0f;")
-        by_edge = {}
-        by_in = {}
-        for mi, me, mo, c in path["terms"]:
-            by_edge.setdefault(me, []).append((mi, mo, c))
-            by_in.setdefault(mi, []).append((me, mo, c))
-        out.append("        float2 dw = make_float2(0.0f, 0.0f);")
-        for me, terms in sorted(by_edge.items()):
-            lines = []
-            for k, (mi, mo, c) in enumerate(terms):
-                prod = f"__fmul2_rn(x[{path['in_off'] + mi}], g[{slots[(p, mo)]}])"
-                coef = f"pair_of(sg * {_lit(c)})"
-                lines.append(f"float2 s = __fmul2_rn({prod}, {coef});" if k == 0 else f"s = __ffma2_rn({prod}, {coef}, s);")
-            ye = path["edge_off"] + me
-            out.append(f"        {{ {' '.join(lines)} dw = __ffma2_rn(s, pair_of(Y[{ye}]), dw); "
-                       f"dY[{ye}] = __ffma2_rn(w[{p}], s, dY[{ye}]); }}")
-        out.append(f"        dr = __ffma2_rn(wp[{p}], dw, dr);")
-        out.append("        if (NEED_DX) {")
-        for mi, terms in sorted(by_in.items()):
-            lines = []
-            for k, (me, mo, c) in enumerate(terms):
-                prod = f"__fmul2_rn(g[{slots[(p, mo)]}], pair_of(Y[{path['edge_off'] + me}]))"
-                coef = f"pair_of(sg * {_lit(c)})"
-                lines.append(f"float2 u = __fmul2_rn({prod}, {coef});" if k == 0 else f"u = __ffma2_rn({prod}, {coef}, u);")
-            xi = path["in_off"] + mi
-            out.append(f"            {{ {' '.join(lines)} dx[{xi}] = __ffma2_rn(w[{p}], u, dx[{xi}]); }}")
-        out.append("        }")
-        out.append("    }")
-    out += ["}", ""]
     # per-l blocks of the message layout for the host (base component, segments)
     out.append(f"template <> struct TpBlocks<{lin}> {{")
     out.append("    static constexpr int kBase[4] = {" + ", ".join(str(blocks[l][0]) for l in range(4)) + "};")
@@ -179,10 +123,6 @@ def render() -> str:
             "template <int LIN> __device__ __forceinline__ void tp_forward(const float (&x)[(LIN + 1) * (LIN + 1)], "
             "const float (&Y)[16], const float (&w)[LIN == 0 ? 4 : LIN == 1 ? 10 : 17], "
             "float (&acc)[LIN == 0 ? 16 : LIN == 1 ? 40 : 71]);",
-            "template <int LIN> __device__ __forceinline__ void tp_forward_pair(const float2 (&x)[(LIN + 1) * (LIN + 1)], "
-            "const float (&Y)[16], const float2 (&w)[LIN == 0 ? 4 : LIN == 1 ? 10 : 17], "
-            "float2 (&acc)[LIN == 0 ? 16 : LIN == 1 ? 40 : 71]);",
-            "__device__ __forceinline__ float2 pair_of(float v) { return make_float2(v, v); }",
             ""]
     body = [_emit(lin) for lin in (0, 1, 2)]
     tail = ["}  // namespace fmb", ""]
@@ -395,6 +335,141 @@ def render_paths() -> str:
     return "\n".join(head + [_emit_paths(lin) for lin in (1, 2)] + ["}  // namespace fmb", ""])
 
 
+# --------------------------------------------------------------------------------------------- coupled bodies
+COUPLED_OUT = os.path.join(HERE, "csrc", "generated", "tp_coupled_generated.cuh")
+COUPLE_PARTS = {0: (4,), 1: (4, 8), 2: (8, 16)}      # threads an edge's couplings are spread over
+
+
+def coupled_layout(paths):
+    """Where the couplings of an edge stand: T[path][m_out][m_in] = sum_me coef * Y[me], structural zeros left out, every
+    path on a 16-byte boundary. Returns ({(path, m_out, m_in): offset}, {offset: [(edge component, coef)]}, floats); the
+    row stride is 4 mod 32 floats so that the rows of neighbouring edges start in different banks."""
+    offset, sums, at = {}, {}, 0
+    for p, path in enumerate(paths):
+        for mi, me, mo, c in sorted(path["terms"], key=lambda t: (t[2], t[0], t[1])):
+            if (p, mo, mi) not in offset:
+                offset[p, mo, mi] = at
+                sums[at] = []
+                at += 1
+            sums[offset[p, mo, mi]].append((path["edge_off"] + me, c))
+        at = -(-at // 4) * 4
+    stride = at
+    while stride % 32 != 4:
+        stride += 4
+    return offset, sums, stride
+
+
+def _emit_coupled(lin: int) -> str:
+    """Bodies for two channels per thread (packed FP32, fma.rn.f32x2) that take the harmonics already coupled: what an edge
+    needs of them is the small matrix T of every path, the same for all channels."""
+    paths = so3.tp_paths(lin)
+    slots, _ = message_slots(paths)
+    in_dim, mid = (lin + 1) ** 2, so3.mid_dim(paths)
+    offset, sums, stride = coupled_layout(paths)
+    out = [f"// ---- node l_max = {lin}",
+           f"template <> struct TpCoupled<{lin}> {{ static constexpr int kFloats = {stride}; }};", ""]
+    order = sorted(sums)
+    for parts in COUPLE_PARTS[lin]:
+        # thread `part` of `parts` computes a run of the couplings of one edge
+        out.append(f"template <> __device__ __forceinline__ void tp_couple<{lin}, {parts}>(int part, const float* Y, float* T) {{")
+        per = -(-len(order) // parts)
+        for q in range(parts):
+            body = " ".join(f"T[{k}] = " + " + ".join(f"{_lit(c)} * Y[{e}]" for e, c in sums[k]) + ";"
+                            for k in order[q * per:(q + 1) * per])
+            out.append(f"    {'else ' if q else ''}if (part == {q}) {{ {body} }}")
+        out += ["}", ""]
+
+    def t_loads(p):
+        ks = [k for (pp, _, _), k in offset.items() if pp == p]
+        first, last = min(ks) // 4, max(ks) // 4
+        lines = [f"const float4 t{k} = T[{k}];" for k in range(first, last + 1)]
+        return lines, lambda mo, mi: f"t{offset[p, mo, mi] // 4}.{'xyzw'[offset[p, mo, mi] % 4]}"
+
+    fwd = [f"template <> __device__ __forceinline__ void tp_forward_coupled<{lin}>(const float2* x, const float4* T, "
+           f"const float2* w, float2 (&acc)[{mid}]) {{"]
+    fwd += [f"    const float2 x{k} = x[{k * 64}];" for k in range(in_dim)]
+    for p, path in enumerate(paths):
+        l_in, l_out, off = path["l_in"], path["l_out"], path["in_off"]
+        n_in, n_out = 2 * l_in + 1, 2 * l_out + 1
+        loads, t = t_loads(p)
+        fwd.append(f"    {{  // path {p}: {l_in} x {path['l_edge']} -> {l_out}")
+        fwd.append(f"        const float2 wp = w[{p * 64}]; {' '.join(loads)}")
+        if n_in <= n_out:
+            fwd.append("        " + " ".join(f"const float2 a{mi} = __fmul2_rn(wp, x{off + mi});" for mi in range(n_in)))
+        for mo in range(n_out):
+            ins = [mi for mi in range(n_in) if (p, mo, mi) in offset]
+            slot = slots[p, mo]
+            if n_in <= n_out:
+                fwd += [f"        acc[{slot}] = __ffma2_rn(a{mi}, pair_of({t(mo, mi)}), acc[{slot}]);" for mi in ins]
+            else:
+                lines = [f"float2 s = __fmul2_rn(x{off + ins[0]}, pair_of({t(mo, ins[0])}));"]
+                lines += [f"s = __ffma2_rn(x{off + mi}, pair_of({t(mo, mi)}), s);" for mi in ins[1:]]
+                fwd.append(f"        {{ {' '.join(lines)} acc[{slot}] = __ffma2_rn(wp, s, acc[{slot}]); }}")
+        fwd.append("    }")
+    fwd += ["}", ""]
+
+    bwd = [f"template <> __device__ __forceinline__ void tp_backward_coupled<{lin}>(const float2* xp, const float4* T, "
+           f"const float2* w, const float2* wd, const float2 (&g)[{mid}], float2 (&dY)[16], float2& dr, float2 (&dx)[{in_dim}]) {{"]
+    bwd += [f"    const float2 x{k} = xp[{k * 64}];" for k in range(in_dim)]
+    for p, path in enumerate(paths):
+        l_in, l_out, off = path["l_in"], path["l_out"], path["in_off"]
+        n_in, n_out = 2 * l_in + 1, 2 * l_out + 1
+        loads, t = t_loads(p)
+        bwd.append(f"    {{  // path {p}: {l_in} x {path['l_edge']} -> {l_out}")
+        bwd.append(f"        const float2 wp = w[{p * 64}]; {' '.join(loads)}")
+        # gradient of the weighted sender features, shared by dx and by the derivative of the weight
+        for mi in range(n_in):
+            outs = [mo for mo in range(n_out) if (p, mo, mi) in offset]
+            lines = [f"float2 u{mi} = __fmul2_rn(g[{slots[p, outs[0]]}], pair_of({t(outs[0], mi)}));"]
+            lines += [f"u{mi} = __ffma2_rn(g[{slots[p, mo]}], pair_of({t(mo, mi)}), u{mi});" for mo in outs[1:]]
+            bwd.append("        " + " ".join(lines))
+        bwd.append("        float2 dw = __fmul2_rn(" + f"x{off}, u0); "
+                   + " ".join(f"dw = __ffma2_rn(x{off + mi}, u{mi}, dw);" for mi in range(1, n_in))
+                   + f" dr = __ffma2_rn(wd[{p * 64}], dw, dr);")
+        bwd.append("        " + " ".join(f"dx[{off + mi}] = __ffma2_rn(wp, u{mi}, dx[{off + mi}]);" for mi in range(n_in)))
+        # products of weighted features and message gradient, coupled into the harmonics' gradient
+        by_pair: dict[tuple, list] = {}
+        for mi, me, mo, c in path["terms"]:
+            by_pair.setdefault((mi, mo), []).append((path["edge_off"] + me, c))
+        weigh_in = n_in <= n_out
+        if weigh_in:
+            bwd.append("        " + " ".join(f"const float2 a{mi} = __fmul2_rn(wp, x{off + mi});" for mi in range(n_in)))
+        else:
+            bwd.append("        " + " ".join(f"const float2 a{mo} = __fmul2_rn(wp, g[{slots[p, mo]}]);" for mo in range(n_out)))
+        for (mi, mo), terms in sorted(by_pair.items()):
+            prod = (f"a{mi}, g[{slots[p, mo]}]" if weigh_in else f"x{off + mi}, a{mo}")
+            if len(terms) == 1 and abs(terms[0][1] - 1.0) < 1e-12:
+                e = terms[0][0]
+                bwd.append(f"        dY[{e}] = __ffma2_rn({prod}, dY[{e}]);")
+            else:
+                bwd.append(f"        {{ const float2 s = __fmul2_rn({prod}); "
+                           + " ".join(f"dY[{e}] = __ffma2_rn(s, pair_of({_lit(c)}), dY[{e}]);" for e, c in terms) + " }")
+        bwd.append("    }")
+    bwd += ["}", ""]
+    return "\n".join(out + fwd + bwd)
+
+
+def render_coupled() -> str:
+    head = ["// GENERATED by fastmace_b200/codegen.py from fastmace_b200/so3.py -- do not edit.",
+            "// The channelwise tensor product for two channels per thread on harmonics coupled once per edge (same",
+            "// coefficients and message layout as tp_generated.cuh). x, w, wd: this thread's channel pair of the rows in",
+            "// shared memory, 64 pairs from one component or path to the next; T: the edge's couplings, 16-byte aligned.",
+            "#pragma once",
+            "",
+            "namespace fmb {",
+            "",
+            "__device__ __forceinline__ float2 pair_of(float v) { return make_float2(v, v); }",
+            "template <int LIN> struct TpCoupled;",
+            "template <int LIN, int PARTS> __device__ __forceinline__ void tp_couple(int part, const float* Y, float* T);",
+            "template <int LIN> __device__ __forceinline__ void tp_forward_coupled(const float2* x, const float4* T, const float2* w, "
+            "float2 (&acc)[LIN == 0 ? 16 : LIN == 1 ? 40 : 71]);",
+            "template <int LIN> __device__ __forceinline__ void tp_backward_coupled(const float2* xp, const float4* T, "
+            "const float2* w, const float2* wd, const float2 (&g)[LIN == 0 ? 16 : LIN == 1 ? 40 : 71], float2 (&dY)[16], "
+            "float2& dr, float2 (&dx)[(LIN + 1) * (LIN + 1)]);",
+            ""]
+    return "\n".join(head + [_emit_coupled(lin) for lin in (0, 1, 2)] + ["}  // namespace fmb", ""])
+
+
 _tp_main = main
 
 
@@ -402,6 +477,7 @@ def main() -> str:  # noqa: F811  (both generated headers)
     out = _tp_main()
     _write(SYMCON_OUT, render_symcon())
     _write(PATHS_OUT, render_paths())
+    _write(COUPLED_OUT, render_coupled())
     return out
 
 

@@ -168,12 +168,12 @@ const long long* edge_limit(const Ctx& c, int which) {
 }
 
 // One row of radial weights per pair of opposite edges (they have the same length): the whole list is one chunk whose
-// weights are kept, the per-edge adjoint's mirror map exists, and the kernels that read the rows by slot are the ones
-// that run (node l_max 1, tensor-core producer).
+// weights are kept, the per-edge adjoint's mirror map exists, and the tensor-core producer applies (the kernels of a
+// whole list read the rows by slot).
 bool pair_rows(const Ctx& c) {
     const int last = c.m->n_layers - 1;
     return last > 0 && keeps_forward_weights(c, last) && edge_local_adjoint(c) && c.w->edge_slot && c.w->canon_list &&
-           c.w->canon_count && c.m->layer[last].l_in_max == 1 && c.m->layer[last].rad_img != nullptr;
+           c.w->canon_count && c.m->layer[last].rad_img != nullptr;
 }
 
 // rows of each half of tp_w (values, then d/dr)

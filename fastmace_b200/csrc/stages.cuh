@@ -38,6 +38,8 @@ struct TpArgs {
 };
 int tp_forward_launch(const TpArgs& t, cudaStream_t stream);
 int tp_backward_launch(const TpArgs& t, cudaStream_t stream);
+// whole list, weights of every edge in tp_w (tp_coupled.cu)
+int tp_forward_coupled_launch(const TpArgs& t, cudaStream_t stream);
 
 // Tensor product of an interaction after the first with the last radial layer fused in (tp_fused.cu): no per-edge
 // weight matrix; one launch covers all rows.
@@ -123,6 +125,8 @@ int mirror_map(const fmb_nl_t* nl, int32_t* mirror, uint32_t* status, const long
 // per-edge adjoint of an interaction after the first for one chunk of edges; after the last chunk the gather of the
 // sender-side gradients into d_x
 int tp_adjoint_edges(const EdgeAdjointArgs& t, cudaStream_t stream);
+// its form for a whole list of which every row carries a gradient (tp_coupled.cu)
+int tp_adjoint_coupled_launch(const EdgeAdjointArgs& t, cudaStream_t stream);
 int gather_sender_gradient(const EdgeAdjointArgs& t, cudaStream_t stream);
 // first interaction: adds its edge-vector gradients to qe (rows below n_add) or stores them
 int first_adjoint_edges(const FirstArgs& f, int n_add, float* qe, cudaStream_t stream);

@@ -1,0 +1,429 @@
+// Channelwise tensor product of the interactions after the first over a whole edge list whose radial weights are in
+// memory, forward and per-edge adjoint: every per-edge operand streamed through shared memory, two channels per thread on
+// the packed FP32 pipe (fma.rn.f32x2), the harmonics coupled once per edge.
+//
+// An edge's harmonics enter every channel in the same few combinations, T[path][m_out][m_in] = sum_me C Y[me]. The
+// threads of a CTA compute them for a batch of edges at a time (a sixteenth to a quarter of an edge per thread, from
+// harmonics that a bulk copy brought) and read them back as broadcasts: per channel pair the forward pass is then 110
+// packed FMAs for node l_max 1 and the adjoint 330, where coupling inside each thread took 126 + 86 scalar products and
+// 456. In the adjoint the gradient of the weighted sender features serves dE/dx and the derivative of the weights, and
+// the products of weighted features and message gradient are formed once for all the harmonics they couple to.
+//
+// Streaming: a group of 64 threads walks a contiguous range of edges; one thread keeps STAGES - 1 edges ahead of the
+// group with bulk copies that complete on mbarriers (weights, in the adjoint their d/dr, the sender's feature rows), a
+// stage is handed back by one arrival per warp. Weights and rows are read from the stage where a path needs them and
+// not copied to registers first, which is what lets node l_max 2 (71 message components) run in this form.
+//
+// Bound: the weights from HBM (4 P C bytes per edge and direction of the pass) for node l_max 0 and 1, the FMA pipe with
+// two warps per scheduler for l_max 2 (860 packed FMAs, two cycles each, 255 registers); below a few hundred receivers the
+// chain of a row's edges. Forward / adjoint with its gather, before (scalar or in-thread coupling) and after: 62 k
+// edges of l_max 1 118 -> 75 and 250 -> 188 us; 748 k edges of l_max 2 2.29 -> 1.41 and 7.21 -> 4.43 ms; 88 k edges of
+// l_max 0 92 -> 64 and 205 -> 135 us.
+
+#include "stages.cuh"
+#include "generated/tp_generated.cuh"
+#include "generated/tp_coupled_generated.cuh"
+#include "edge_gradient.cuh"
+#include "tc_common.cuh"
+
+namespace fmb {
+
+namespace {
+
+constexpr int kGroup = kC / 2;                 // threads of a group: channels 2 c and 2 c + 1
+constexpr unsigned kSpin = 1u << 20;
+
+__device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, %1;" :: "r"(id), "r"(kGroup) : "memory"); }
+
+// What a group knows of a range of edges ahead of their use: the couplings of the next batch (Y and T double buffered, Y
+// by bulk copy two batches ahead), and the senders and weight rows of the next two (four-byte asynchronous copies), so
+// that the thread that requests an edge's rows never waits for an index.
+template <int LIN, int BATCH>
+struct Ahead {
+    static constexpr int kT = TpCoupled<LIN>::kFloats;
+    static constexpr int kFloats = 2 * BATCH * (kT + 16) + 8 * BATCH;
+    static constexpr int kParts = kGroup / BATCH;
+    float* t;                                  // [2][BATCH][kT]
+    float* y;                                  // [2][BATCH][16]
+    int32_t* index;                            // [4][senders BATCH, weight rows BATCH]
+    uint32_t bar;                              // two barriers
+    const float* edge_sh;
+    const int32_t* senders;
+    const int32_t* slot;
+    long long eb, ee;
+    int c, sync_id;
+    volatile int* abort_flag;
+
+    __device__ __forceinline__ Ahead(float* memory, uint32_t bar_, const float* edge_sh_, const int32_t* senders_,
+                                     const int32_t* slot_, long long eb_, long long ee_, int c_, int sync_id_, volatile int* abort_)
+        : t(memory), y(memory + 2 * BATCH * kT), index(reinterpret_cast<int32_t*>(memory + 2 * BATCH * (kT + 16))), bar(bar_),
+          edge_sh(edge_sh_), senders(senders_), slot(slot_), eb(eb_), ee(ee_), c(c_), sync_id(sync_id_), abort_flag(abort_) {}
+
+    // thread c < BATCH: the indices of its edge of batch b
+    __device__ __forceinline__ void look_up(int b) const {
+        const long long e = eb + (long long)b * BATCH + c;
+        if (c < BATCH && e < ee) {
+            const uint32_t dst = tc::smem_u32(index + (b & 3) * 2 * BATCH + c);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(dst), "l"(senders + e) : "memory");
+            if (slot) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(dst + 4 * BATCH), "l"(slot + e) : "memory");
+        }
+    }
+    __device__ __forceinline__ int sender(long long e) const {
+        const int k = (int)(e - eb);
+        return index[((k / BATCH) & 3) * 2 * BATCH + k % BATCH];
+    }
+    // the row of tp_w that holds an edge's weights: its own, or with one row per pair of opposite edges the pair's
+    __device__ __forceinline__ long long weight_row(long long e) const {
+        const int k = (int)(e - eb);
+        return slot ? (long long)index[((k / BATCH) & 3) * 2 * BATCH + BATCH + k % BATCH] : e;
+    }
+
+    __device__ __forceinline__ void request(int b) const {
+        const long long first = eb + (long long)b * BATCH;
+        if (c == 0 && first < ee) {
+            const uint32_t bytes = (uint32_t)min((long long)BATCH, ee - first) * 64u, full = bar + 8u * (b & 1);
+            tc::mbar_expect_tx(full, bytes);
+            tc::bulk_load(tc::smem_u32(y + (b & 1) * BATCH * 16), edge_sh + 16 * first, bytes, full);
+        }
+    }
+    __device__ __forceinline__ void compute(int b) const {
+        if (eb + (long long)b * BATCH >= ee) return;
+        tc::mbar_wait(bar + 8u * (b & 1), (uint32_t)(b >> 1) & 1u, abort_flag, kSpin);
+        const int el = c % BATCH;
+        if (eb + (long long)b * BATCH + el < ee)
+            tp_couple<LIN, kParts>(c / BATCH, y + ((b & 1) * BATCH + el) * 16, t + ((b & 1) * BATCH + el) * kT);
+    }
+    __device__ __forceinline__ void start() const {
+        look_up(0);
+        look_up(1);
+        request(0);
+        request(1);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        group_sync(sync_id);
+    }
+    // before the first edge of batch b: its couplings become visible and the indices of batch b + 1, and it is certain that
+    // the harmonics of batch b and the couplings of batch b - 1 have been read
+    __device__ __forceinline__ void enter(int b) const {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        group_sync(sync_id);
+        look_up(b + 2);
+        request(b + 2);
+        compute(b + 1);
+    }
+    __device__ __forceinline__ const float4* row(int b, int el) const {
+        return reinterpret_cast<const float4*>(t + ((b & 1) * BATCH + el) * kT);
+    }
+};
+
+// One thread's requests for the edges' rows.
+template <int LIN, int STAGES, bool TANGENT>
+struct Rows {
+    static constexpr int P = TpShape<LIN>::kPaths, IN = TpShape<LIN>::kInDim;
+    static constexpr int kW = P * kC;
+    static constexpr int kX = (TANGENT ? 2 : 1) * kW;           // float offset of the sender rows in a stage
+    static constexpr int kStage = kX + IN * kC;
+    float* ring;
+    uint32_t bar;                              // full[STAGES], empty[STAGES]
+    const float* tp_w;
+    long long tangent_offset;
+    const float* x;
+    long long ee, issued;
+    volatile int* abort_flag;
+    int stage = 0;
+    uint32_t parity = 1;
+
+    template <typename AheadT>
+    __device__ __forceinline__ void issue(const AheadT& ahead) {
+        tc::mbar_wait(bar + 8u * (STAGES + stage), parity, abort_flag, kSpin);
+        const uint32_t full = bar + 8u * stage, dst = tc::smem_u32(ring + stage * kStage);
+        const long long weight_row = ahead.weight_row(issued);
+        tc::mbar_expect_tx(full, kStage * 4);
+        tc::bulk_load(dst, tp_w + weight_row * kW, kW * 4, full);
+        if (TANGENT) tc::bulk_load(dst + kW * 4, tp_w + tangent_offset + weight_row * kW, kW * 4, full);
+        tc::bulk_load(dst + kX * 4, x + (long long)ahead.sender(issued) * (IN * kC), IN * kC * 4, full);
+        ++issued;
+        if (++stage == STAGES) { stage = 0; parity ^= 1u; }
+    }
+};
+
+template <int LIN, int STAGES, int BATCH>
+constexpr int forward_group_floats() { return STAGES * Rows<LIN, STAGES, false>::kStage + Ahead<LIN, BATCH>::kFloats; }
+
+// GROUPS = 1: a CTA owns a contiguous block of receivers. GROUPS > 1 (few receivers): a CTA owns one, its groups take
+// runs of the row's edges and meet in shared memory at the end.
+template <int LIN, int STAGES, int BATCH, int GROUPS, int MINB>
+__global__ void __launch_bounds__(kGroup * GROUPS, MINB)
+k_tp_forward_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ senders,
+                     const float* __restrict__ x, const float* __restrict__ edge_sh, const float* __restrict__ tp_w,
+                     float* __restrict__ mid, uint32_t* __restrict__ error_word, const int32_t* __restrict__ slot) {
+    constexpr int MID = TpShape<LIN>::kMidDim;
+    extern __shared__ __align__(128) float smem[];
+    __shared__ uint64_t bars[GROUPS * (2 * STAGES + 2)];
+    __shared__ int abort_sh;
+    const int group = threadIdx.x / kGroup, c = threadIdx.x % kGroup, lane = c & 31;
+    const int r0 = (int)((long long)blockIdx.x * n_rows / gridDim.x), r1 = (int)((long long)(blockIdx.x + 1) * n_rows / gridDim.x);
+    if (r0 >= r1) return;
+    long long eb = row_ptr[r0], ee = row_ptr[r1];
+    if (GROUPS > 1) {
+        const long long len = ee - eb;
+        ee = eb + len * (group + 1) / GROUPS;
+        eb = eb + len * group / GROUPS;
+    }
+    const uint32_t bar = tc::smem_u32(bars) + 8u * group * (2 * STAGES + 2);
+    if (c == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            tc::mbar_init(bar + 8 * s, 1);                            // full
+            tc::mbar_init(bar + 8 * (STAGES + s), kGroup / 32);       // empty: one arrival per warp
+        }
+        tc::mbar_init(bar + 8 * (2 * STAGES), 1);
+        tc::mbar_init(bar + 8 * (2 * STAGES + 1), 1);
+        abort_sh = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    float* const own = smem + group * forward_group_floats<LIN, STAGES, BATCH>();
+    float* const tail = own + STAGES * Rows<LIN, STAGES, false>::kStage;
+    const Ahead<LIN, BATCH> ahead(tail, bar + 8 * (2 * STAGES), edge_sh, senders, slot, eb, ee, c, 1 + group, &abort_sh);
+    Rows<LIN, STAGES, false> rows{own, bar, tp_w, 0, x, ee, eb, &abort_sh};
+    ahead.start();
+    if (c == 0)
+        while (rows.issued < ee && rows.issued < eb + STAGES - 1) rows.issue(ahead);
+    ahead.compute(0);
+    int stage = 0, batch = -1, el = BATCH;
+    uint32_t parity = 0;
+    long long e = eb;
+    for (int i = r0; i < r1; ++i) {
+        const long long re = GROUPS > 1 ? ee : (long long)row_ptr[i + 1];
+        float2 acc[MID];
+#pragma unroll
+        for (int k = 0; k < MID; ++k) acc[k] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+        for (; e < re; ++e) {
+            if (el == BATCH) {
+                ahead.enter(++batch);
+                el = 0;
+            }
+            if (c == 0 && rows.issued < ee && rows.issued < e + STAGES) rows.issue(ahead);
+            tc::mbar_wait(bar + 8 * stage, parity, &abort_sh, kSpin);
+            const float* st = own + stage * Rows<LIN, STAGES, false>::kStage;
+            tp_forward_coupled<LIN>(reinterpret_cast<const float2*>(st + Rows<LIN, STAGES, false>::kX) + c, ahead.row(batch, el),
+                                    reinterpret_cast<const float2*>(st) + c, acc);
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(bar + 8 * (STAGES + stage));
+            if (++stage == STAGES) { stage = 0; parity ^= 1u; }
+            ++el;
+        }
+        if (GROUPS == 1) {
+            float2* out = reinterpret_cast<float2*>(mid + ((long long)i * MID) * kC) + c;
+#pragma unroll
+            for (int k = 0; k < MID; ++k) out[(long long)k * (kC / 2)] = acc[k];
+        } else {
+            __syncthreads();                                          // every group is done with its stages
+            float2* const part = reinterpret_cast<float2*>(smem);     // [GROUPS - 1][MID][64]
+            if (group > 0) {
+#pragma unroll
+                for (int k = 0; k < MID; ++k) part[((group - 1) * MID + k) * kGroup + c] = acc[k];
+            }
+            __syncthreads();
+            if (group == 0) {
+                float2* out = reinterpret_cast<float2*>(mid + ((long long)i * MID) * kC) + c;
+#pragma unroll
+                for (int k = 0; k < MID; ++k) {
+                    float2 v = acc[k];
+#pragma unroll
+                    for (int q = 0; q < GROUPS - 1; ++q) {
+                        const float2 o = part[(q * MID + k) * kGroup + c];
+                        v.x += o.x;
+                        v.y += o.y;
+                    }
+                    out[(long long)k * (kC / 2)] = v;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && abort_sh && error_word) atomicOr(error_word, FMB_STATUS_TENSOR_TIMEOUT);
+}
+
+// Every CTA takes the same number of edges (an edge is independent of the others of its row). The gradients of the
+// harmonics and of the length are summed over the channels by shuffles and across the two warps in shared memory, where a
+// batch's edge-vector gradients are finished while the next batch is under way.
+template <int LIN, int STAGES, int BATCH>
+constexpr int adjoint_floats() { return STAGES * Rows<LIN, STAGES, true>::kStage + Ahead<LIN, BATCH>::kFloats; }
+
+template <int LIN, int STAGES, int BATCH, int MINB>
+__global__ void __launch_bounds__(kGroup, MINB)
+k_tp_adjoint_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ senders,
+                     const float* __restrict__ x, const float* __restrict__ edge_sh, const float* __restrict__ edge_vec,
+                     const float* __restrict__ tp_w, long long tangent_offset, const float* __restrict__ d_mid,
+                     float* __restrict__ dxe, float4* __restrict__ qe, uint32_t* __restrict__ error_word,
+                     const int32_t* __restrict__ slot) {
+    constexpr int IN = TpShape<LIN>::kInDim, MID = TpShape<LIN>::kMidDim;
+    using RowsT = Rows<LIN, STAGES, true>;
+    extern __shared__ __align__(128) float smem[];
+    __shared__ uint64_t bars[2 * STAGES + 2];
+    __shared__ int abort_sh, first_row_sh;
+    __shared__ float red[2][BATCH][2][18];
+    const int c = threadIdx.x, warp = c >> 5, lane = c & 31;
+    const long long total = row_ptr[n_rows];
+    const long long per_cta = (total + gridDim.x - 1) / gridDim.x;
+    const long long eb = (long long)blockIdx.x * per_cta, ee = min(total, eb + per_cta);
+    if (eb >= ee) return;
+    const uint32_t bar = tc::smem_u32(bars);
+    if (c == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            tc::mbar_init(bar + 8 * s, 1);                            // full
+            tc::mbar_init(bar + 8 * (STAGES + s), kGroup / 32);       // empty: one arrival per warp
+        }
+        tc::mbar_init(bar + 8 * (2 * STAGES), 1);
+        tc::mbar_init(bar + 8 * (2 * STAGES + 1), 1);
+        abort_sh = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    float* const tail = smem + STAGES * RowsT::kStage;
+    const Ahead<LIN, BATCH> ahead(tail, bar + 8 * (2 * STAGES), edge_sh, senders, slot, eb, ee, c, 1, &abort_sh);
+    RowsT rows{smem, bar, tp_w, tangent_offset, x, ee, eb, &abort_sh};
+    ahead.start();
+    if (c == 0) {
+        while (rows.issued < ee && rows.issued < eb + STAGES - 1) rows.issue(ahead);
+        int lo = 0, hi = n_rows - 1;
+        while (lo < hi) {
+            const int at = (lo + hi + 1) >> 1;
+            if (row_ptr[at] <= eb) lo = at; else hi = at - 1;
+        }
+        first_row_sh = lo;
+    }
+    __syncthreads();
+    int a = first_row_sh;
+    long long row_end = row_ptr[a + 1];
+    float2 g[MID];
+#pragma unroll
+    for (int k = 0; k < MID; ++k) g[k] = __ldg(reinterpret_cast<const float2*>(d_mid + ((long long)a * MID + k) * kC) + c);
+    ahead.compute(0);
+    auto finish = [&](int b) {
+        const long long e = eb + (long long)b * BATCH + c;
+        if (c >= BATCH || e >= ee) return;
+        const float (&r)[2][18] = red[b & 1][c];
+        float gy[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) gy[q] = r[0][q] + r[1][q];
+        const float4 uv = __ldg(reinterpret_cast<const float4*>(edge_vec) + e);
+        float q3[3];
+        edge_vector_gradient(gy, r[0][16] + r[1][16], uv.x, uv.y, uv.z, uv.w, q3);
+        qe[e] = make_float4(q3[0], q3[1], q3[2], 0.0f);
+    };
+    int stage = 0, batch = -1, el = BATCH;
+    uint32_t parity = 0;
+#pragma unroll 1
+    for (long long e = eb; e < ee; ++e) {
+        if (el == BATCH) {
+            ahead.enter(++batch);
+            el = 0;
+            if (batch > 0) finish(batch - 1);
+        }
+        if (e >= row_end) {
+            do { ++a; row_end = row_ptr[a + 1]; } while (e >= row_end);
+#pragma unroll
+            for (int k = 0; k < MID; ++k) g[k] = __ldg(reinterpret_cast<const float2*>(d_mid + ((long long)a * MID + k) * kC) + c);
+        }
+        if (c == 0 && rows.issued < ee && rows.issued < e + STAGES) rows.issue(ahead);
+        float2 dY2[16], dx[IN], dr2 = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) dY2[q] = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int q = 0; q < IN; ++q) dx[q] = make_float2(0.0f, 0.0f);
+        tc::mbar_wait(bar + 8 * stage, parity, &abort_sh, kSpin);
+        const float* st = smem + stage * RowsT::kStage;
+        tp_backward_coupled<LIN>(reinterpret_cast<const float2*>(st + RowsT::kX) + c, ahead.row(batch, el),
+                                 reinterpret_cast<const float2*>(st) + c, reinterpret_cast<const float2*>(st + RowsT::kW) + c, g, dY2,
+                                 dr2, dx);
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(bar + 8 * (STAGES + stage));
+        if (++stage == STAGES) { stage = 0; parity ^= 1u; }
+#pragma unroll
+        for (int q = 0; q < IN; ++q) reinterpret_cast<float2*>(dxe + (e * IN + q) * kC)[c] = dx[q];
+        // 16 + 1 sums over the channels: transpose-reduce inside the warp, the two warps meet in shared memory
+        float dY[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) dY[q] = dY2[q].x + dY2[q].y;
+#pragma unroll
+        for (int half = 8, bit = 16; half >= 1; half >>= 1, bit >>= 1) {
+            const bool upper = (lane & bit) != 0;
+#pragma unroll
+            for (int i = 0; i < half; ++i) {
+                const float keep = upper ? dY[i + half] : dY[i];
+                const float send = upper ? dY[i] : dY[i + half];
+                dY[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+            }
+        }
+        dY[0] += __shfl_xor_sync(0xffffffffu, dY[0], 1);
+        const float dr = warp_sum(dr2.x + dr2.y);
+        if ((lane & 1) == 0) red[batch & 1][el][warp][lane >> 1] = dY[0];
+        if (lane == 0) red[batch & 1][el][warp][16] = dr;
+        ++el;
+    }
+    __syncthreads();
+    finish(batch);
+    if (c == 0 && abort_sh && error_word) atomicOr(error_word, FMB_STATUS_TENSOR_TIMEOUT);
+}
+
+// CTAs that fill the device once
+int resident(const void* kernel, int threads, int smem) {
+    int per_sm = 0, sms = 148, dev = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, (size_t)smem) != cudaSuccess || per_sm < 1) per_sm = 1;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return per_sm * sms;
+}
+
+template <int LIN, int STAGES, int BATCH, int GROUPS, int MINB>
+int launch_forward(const TpArgs& t, cudaStream_t stream) {
+    constexpr int smem = GROUPS * forward_group_floats<LIN, STAGES, BATCH>() * 4;
+    auto kernel = k_tp_forward_coupled<LIN, STAGES, BATCH, GROUPS, MINB>;
+    FMB_CUDA_CHECK(opt_in_shared_memory((const void*)kernel, smem));
+    static const int cap = resident((const void*)kernel, kGroup * GROUPS, smem);
+    const int grid = GROUPS > 1 || t.n_rows < cap ? t.n_rows : cap;
+    kernel<<<grid, kGroup * GROUPS, smem, stream>>>(t.n_rows, t.row_ptr, t.senders, t.x, t.edge_sh, t.tp_w, t.mid, t.error_word,
+                                                    t.slot);
+    FMB_LAUNCH_CHECK();
+    return FMB_OK;
+}
+
+template <int LIN, int STAGES, int BATCH, int MINB>
+int launch_adjoint(const EdgeAdjointArgs& t, cudaStream_t stream) {
+    constexpr int smem = adjoint_floats<LIN, STAGES, BATCH>() * 4;
+    auto kernel = k_tp_adjoint_coupled<LIN, STAGES, BATCH, MINB>;
+    FMB_CUDA_CHECK(opt_in_shared_memory((const void*)kernel, smem));
+    static const int cap = resident((const void*)kernel, kGroup, smem);
+    kernel<<<cap, kGroup, smem, stream>>>(t.n_rows, t.row_ptr, t.senders, t.x, t.edge_sh, t.edge_vec, t.tp_w, t.tangent_offset,
+                                          t.d_mid, t.dxe, reinterpret_cast<float4*>(t.qe), t.error_word, t.slot);
+    FMB_LAUNCH_CHECK();
+    return FMB_OK;
+}
+
+}  // namespace
+
+int tp_forward_coupled_launch(const TpArgs& t, cudaStream_t stream) {
+    // Few receivers leave SMs idle and a receiver's edges are a serial chain: four groups (two where the stages of node
+    // l_max 2 do not fit four times) share a receiver while one CTA of that size per SM and two waves of them suffice.
+    // 64 atoms: 31 -> 11 us (l_max 0); 249 atoms of 59 neighbours: 64 -> 31 us (l_max 1).
+    const bool few = t.n_rows <= 296;
+    // otherwise the shape (stages, batch, CTAs per SM) measured best: warps in flight count for more than stages. l_max 1,
+    // 62 k edges: 75 us at 3 / 8 / 8, 86 at 3 / 16 / 6, 91 at 4 / 8 / 6; l_max 2, 748 k edges: 1.41 ms at 3 / 8 / 3, 1.46 at
+    // 2 / 8 / 4, 1.70 at 3 / 4 / 4
+    if (t.lin == 0) return few ? launch_forward<0, 4, 16, 4, 1>(t, stream) : launch_forward<0, 6, 16, 1, 8>(t, stream);
+    if (t.lin == 1) return few ? launch_forward<1, 4, 16, 4, 1>(t, stream) : launch_forward<1, 3, 8, 1, 8>(t, stream);
+    if (t.lin == 2) return few ? launch_forward<2, 3, 8, 2, 1>(t, stream) : launch_forward<2, 3, 8, 1, 3>(t, stream);
+    return FMB_ERR_UNSUPPORTED;
+}
+
+int tp_adjoint_coupled_launch(const EdgeAdjointArgs& t, cudaStream_t stream) {
+    // shapes (stages, batch, CTAs per SM) measured with the gather behind them, 62 k edges of l_max 1: 188 us at 2 / 8 / 6,
+    // 207 at 2 / 16 / 5, 208 at 3 / 8 / 5; 748 k edges of l_max 2: 4.43 ms at 2 / 4 / 4, 5.08 at 2 / 8 / 3, 5.55 at 3 / 4 / 3
+    if (t.lin == 0) return launch_adjoint<0, 4, 16, 8>(t, stream);
+    if (t.lin == 1) return launch_adjoint<1, 2, 8, 6>(t, stream);
+    if (t.lin == 2) return launch_adjoint<2, 2, 4, 4>(t, stream);
+    return FMB_ERR_UNSUPPORTED;
+}
+
+}  // namespace fmb

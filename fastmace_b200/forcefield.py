@@ -208,7 +208,7 @@ class B200ForceField:
             others = 16 + 64 + spec.num_interactions * 2 * 64 * 4 + hid * c * 4 + 28
             row = 2 * max_paths * c * 4
             layers = self.packed.struct.layer
-            pair_rows = (self.edge_adjoint is not False and spec.num_interactions == 2 and spec.l_in_max(1) == 1
+            pair_rows = (self.edge_adjoint is not False and spec.num_interactions == 2
                          and bool(layers[1].rad_img) and bool(layers[0].first[0]))
             pairs = cap // 2 + cap // 16
             if pair_rows and cap * others + pairs * row <= 0.85 * free:
