@@ -99,9 +99,43 @@ __global__ void k_bin_fill(int n, const int32_t* __restrict__ atom_bin, const in
 
 constexpr int kWarpsPerBlock = 4;
 
+// The bins a receiver looks at are runs of the bin-ordered atom list (neighbouring bins along the last axis, one run per
+// periodic image and per pair of bins along the other two): a warp works out up to 32 runs at a time, one per lane, and
+// then walks the atoms of all of them as one sequence, 32 at a time. Walking bin by bin (12 atoms in the benchmark's
+// cells) left two thirds of the lanes without an atom and paid three dependent loads 27 times per receiver instead of two
+// ten times. Consecutive receivers of a warp that share a bin share the runs.
+struct RowRuns {
+    double image[32][3];       // what is added to receiver minus sender
+    int offset[32];            // index into bin_atoms minus position in the sequence
+    int end[32];               // position after the run
+    int key[32];               // the image as sort key
+    unsigned char home[32];    // the receiver's own image
+    int total;                 // length of the sequence
+    int bin;                   // the bin whose runs these are, or -1 (more than 32 runs: never kept)
+};
+
+__device__ __forceinline__ int floor_div(int v, int n) { return v >= 0 ? v / n : -((-v + n - 1) / n); }
+
+// position of `key` among the distinct keys[0 .. count)
+template <int PER_LANE>
+__device__ __forceinline__ void rank_keys(const unsigned long long* keys, int count, int lane, unsigned long long (&mine)[PER_LANE],
+                                          int (&rank)[PER_LANE]) {
+#pragma unroll
+    for (int q = 0; q < PER_LANE; ++q) {
+        mine[q] = lane + 32 * q < count ? keys[lane + 32 * q] : ~0ull;
+        rank[q] = 0;
+    }
+#pragma unroll 4
+    for (int j = 0; j < count; ++j) {
+        const unsigned long long other = keys[j];
+#pragma unroll
+        for (int q = 0; q < PER_LANE; ++q) rank[q] += other < mine[q] ? 1 : 0;
+    }
+}
+
 // One warp per receiver. MODE 0: count the candidates; MODE 1: collect, sort by (sender, image) and write them.
 template <int MODE>
-__device__ __forceinline__ void rows_receiver(const NlConst& c, int r, int lane, unsigned long long* keys, int capacity,
+__device__ __forceinline__ void rows_receiver(const NlConst& c, int r, int lane, unsigned long long* keys, RowRuns& runs, int capacity,
                                               const double* __restrict__ wrapped, const double* __restrict__ offsets,
                                               const int32_t* __restrict__ atom_bin, const int32_t* __restrict__ bin_start,
                                               const int32_t* __restrict__ bin_atoms, int32_t* __restrict__ row_count,
@@ -110,54 +144,76 @@ __device__ __forceinline__ void rows_receiver(const NlConst& c, int r, int lane,
     const double rx = wrapped[3 * r], ry = wrapped[3 * r + 1], rz = wrapped[3 * r + 2];
     const int bin = atom_bin[r];
     const int b2 = bin % c.nbins[2], b1 = (bin / c.nbins[2]) % c.nbins[1], b0 = bin / (c.nbins[2] * c.nbins[1]);
+    const int n2_first = floor_div(b2 - c.reach[2], c.nbins[2]);
+    const int images2 = floor_div(b2 + c.reach[2], c.nbins[2]) - n2_first + 1, width1 = 2 * c.reach[1] + 1;
+    const int all_runs = (2 * c.reach[0] + 1) * width1 * images2;
     int found = 0;
-    for (int d0 = -c.reach[0]; d0 <= c.reach[0]; ++d0) {
-        const int B0 = b0 + d0;
-        const int n0 = (B0 >= 0) ? B0 / c.nbins[0] : -((-B0 + c.nbins[0] - 1) / c.nbins[0]);
-        const int s0 = B0 - n0 * c.nbins[0];
-        for (int d1 = -c.reach[1]; d1 <= c.reach[1]; ++d1) {
-            const int B1 = b1 + d1;
-            const int n1 = (B1 >= 0) ? B1 / c.nbins[1] : -((-B1 + c.nbins[1] - 1) / c.nbins[1]);
-            const int s1 = B1 - n1 * c.nbins[1];
-            for (int d2 = -c.reach[2]; d2 <= c.reach[2]; ++d2) {
-                const int B2 = b2 + d2;
-                const int n2 = (B2 >= 0) ? B2 / c.nbins[2] : -((-B2 + c.nbins[2] - 1) / c.nbins[2]);
-                const int s2 = B2 - n2 * c.nbins[2];
-                // the sender's image sits n cells away, so the reference's image (added to r - s) is -n
-                const double i0 = (double)(-n0), i1 = (double)(-n1), i2 = (double)(-n2);
-                double iv[3];
-                times_3x3(i0, i1, i2, c.cell, iv);
-                const int sbin = (s0 * c.nbins[1] + s1) * c.nbins[2] + s2;
-                const int begin = bin_start[sbin], end = bin_start[sbin + 1];
-                for (int base = begin; base < end; base += 32) {
-                    const int k = base + lane;
-                    bool hit = false;
-                    int s = 0;
-                    if (k < end) {
-                        s = bin_atoms[k];
-                        const double vx = add(sub(rx, wrapped[3 * s]), iv[0]);
-                        const double vy = add(sub(ry, wrapped[3 * s + 1]), iv[1]);
-                        const double vz = add(sub(rz, wrapped[3 * s + 2]), iv[2]);
-                        hit = norm2(vx, vy, vz) < c.reach2;
-                        if (hit && s == r) {
-                            // self pair: dropped only when the unit shift is zero (skin.py:462-463)
-                            hit = !(n0 == 0 && n1 == 0 && n2 == 0);
-                        }
-                    }
-                    const unsigned mask = __ballot_sync(0xffffffffu, hit);
-                    if (MODE == 1 && hit) {
-                        const int slot = found + __popc(mask & ((1u << lane) - 1u));
-                        if (slot < FMB_MAX_ROW) {
-                            const unsigned long long image_key =
-                                ((unsigned long long)(-n0 + 128) << 16) | ((unsigned long long)(-n1 + 128) << 8) |
-                                (unsigned long long)(-n2 + 128);
-                            keys[slot] = ((unsigned long long)(unsigned)s << 24) | image_key;
-                        }
-                    }
-                    found += __popc(mask);
-                }
-            }
+    for (int first = 0; first < all_runs; first += 32) {
+        int begin = 0, length = 0;
+        const bool kept = runs.bin == bin;
+        if (!kept && first + lane < all_runs) {
+            const int pair = (first + lane) / images2, n2 = n2_first + (first + lane) % images2;
+            const int B0 = b0 + pair / width1 - c.reach[0], B1 = b1 + pair % width1 - c.reach[1];
+            const int n0 = floor_div(B0, c.nbins[0]), n1 = floor_div(B1, c.nbins[1]);
+            const int row = ((B0 - n0 * c.nbins[0]) * c.nbins[1] + (B1 - n1 * c.nbins[1])) * c.nbins[2];
+            const int low = n2 * c.nbins[2];
+            begin = bin_start[row + max(b2 - c.reach[2], low) - low];
+            length = bin_start[row + min(b2 + c.reach[2], low + c.nbins[2] - 1) - low + 1] - begin;
+            // the sender's image sits n cells away, so the reference's image (added to r - s) is -n
+            double iv[3];
+            times_3x3((double)(-n0), (double)(-n1), (double)(-n2), c.cell, iv);
+            runs.image[lane][0] = iv[0]; runs.image[lane][1] = iv[1]; runs.image[lane][2] = iv[2];
+            runs.key[lane] = ((-n0 + 128) << 16) | ((-n1 + 128) << 8) | (-n2 + 128);
+            runs.home[lane] = n0 == 0 && n1 == 0 && n2 == 0;
         }
+        __syncwarp();
+        if (!kept) {
+            int end = length;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, end, o);
+                if (lane >= o) end += t;
+            }
+            runs.end[lane] = end;
+            runs.offset[lane] = begin - (end - length);
+            if (lane == 31) {
+                runs.total = end;
+                runs.bin = all_runs <= 32 ? bin : -1;
+            }
+            __syncwarp();
+        }
+        const int total = runs.total;
+        int run = 0, s_next = 0, run_next = 0;
+        auto look = [&](int at) {
+            if (at < total) {
+                while (at >= runs.end[run]) ++run;
+                run_next = run;
+                s_next = bin_atoms[runs.offset[run] + at];
+            }
+        };
+        look(lane);
+        for (int base = 0; base < total; base += 32) {
+            const bool live = base + lane < total;
+            const int s = s_next, q = run_next;
+            look(base + 32 + lane);                                   // the next atom's index travels during this one's test
+            bool hit = false;
+            if (live) {
+                const double vx = add(sub(rx, wrapped[3 * s]), runs.image[q][0]);
+                const double vy = add(sub(ry, wrapped[3 * s + 1]), runs.image[q][1]);
+                const double vz = add(sub(rz, wrapped[3 * s + 2]), runs.image[q][2]);
+                hit = norm2(vx, vy, vz) < c.reach2;
+                // self pair: dropped only when the unit shift is zero (skin.py:462-463)
+                if (hit && s == r) hit = !runs.home[q];
+            }
+            const unsigned mask = __ballot_sync(0xffffffffu, hit);
+            if (MODE == 1 && hit) {
+                const int slot = found + __popc(mask & ((1u << lane) - 1u));
+                if (slot < FMB_MAX_ROW)
+                    keys[slot] = ((unsigned long long)(unsigned)s << 24) | (unsigned long long)(unsigned)runs.key[q];
+            }
+            found += __popc(mask);
+        }
+        __syncwarp();                                                 // the table is free for the next runs
     }
     if (MODE == 0) {
         if (lane == 0) row_count[r] = found;
@@ -167,15 +223,51 @@ __device__ __forceinline__ void rows_receiver(const NlConst& c, int r, int lane,
         if (lane == 0) atomicOr(status, FMB_STATUS_ROW_OVERFLOW);
         found = FMB_MAX_ROW;
     }
+    const int start = row_ptr[r];
+    const double or0 = offsets[3 * r], or1 = offsets[3 * r + 1], or2 = offsets[3 * r + 2];
+    auto write = [&](unsigned long long key, int position) {
+        const int dst = start + position;
+        if (dst >= capacity) return;
+        const int s = (int)(key >> 24);
+        const double i0 = (double)((int)((key >> 16) & 0xff) - 128);
+        const double i1 = (double)((int)((key >> 8) & 0xff) - 128);
+        const double i2 = (double)((int)(key & 0xff) - 128);
+        cand_index[dst] = s;
+        cand_index[capacity + dst] = r;
+        cand_shift[3 * dst + 0] = (float)add(sub(i0, or0), offsets[3 * s]);
+        cand_shift[3 * dst + 1] = (float)add(sub(i1, or1), offsets[3 * s + 1]);
+        cand_shift[3 * dst + 2] = (float)add(sub(i2, or2), offsets[3 * s + 2]);
+    };
+    __syncwarp();
+    // the keys of a row are distinct, so a key's place is the number of smaller ones: up to 64 or 128 keys two or four
+    // per lane are compared with all (330 instructions for 47 keys, the bitonic network below takes 2,000)
+    if (found <= 64) {
+        unsigned long long mine[2];
+        int rank[2];
+        rank_keys<2>(keys, found, lane, mine, rank);
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+            if (lane + 32 * q < found) write(mine[q], rank[q]);
+        return;
+    }
+    if (found <= 128) {
+        unsigned long long mine[4];
+        int rank[4];
+        rank_keys<4>(keys, found, lane, mine, rank);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (lane + 32 * q < found) write(mine[q], rank[q]);
+        return;
+    }
     // bitonic sort of keys[0..found) padded to a power of two
-    int padded = 32;
+    int padded = 256;
     while (padded < found) padded <<= 1;
     for (int k = found + lane; k < padded; k += 32) keys[k] = ~0ull;
     __syncwarp();
     for (int size = 2; size <= padded; size <<= 1) {
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+        for (int stride = size >> 1, shift = __ffs(size) - 2; stride > 0; stride >>= 1, --shift) {
             for (int t = lane; t < (padded >> 1); t += 32) {
-                const int lo = ((t / stride) * (stride << 1)) + (t % stride);
+                const int lo = ((t >> shift) << (shift + 1)) + (t & (stride - 1));
                 const int hi = lo + stride;
                 const bool ascending = ((lo & size) == 0);
                 const unsigned long long a = keys[lo], b = keys[hi];
@@ -187,22 +279,7 @@ __device__ __forceinline__ void rows_receiver(const NlConst& c, int r, int lane,
             __syncwarp();
         }
     }
-    const int start = row_ptr[r];
-    const double or0 = offsets[3 * r], or1 = offsets[3 * r + 1], or2 = offsets[3 * r + 2];
-    for (int k = lane; k < found; k += 32) {
-        const int dst = start + k;
-        if (dst >= capacity) break;
-        const unsigned long long key = keys[k];
-        const int s = (int)(key >> 24);
-        const double i0 = (double)((int)((key >> 16) & 0xff) - 128);
-        const double i1 = (double)((int)((key >> 8) & 0xff) - 128);
-        const double i2 = (double)((int)(key & 0xff) - 128);
-        cand_index[dst] = s;
-        cand_index[capacity + dst] = r;
-        cand_shift[3 * dst + 0] = (float)add(sub(i0, or0), offsets[3 * s]);
-        cand_shift[3 * dst + 1] = (float)add(sub(i1, or1), offsets[3 * s + 1]);
-        cand_shift[3 * dst + 2] = (float)add(sub(i2, or2), offsets[3 * s + 2]);
-    }
+    for (int k = lane; k < found; k += 32) write(keys[k], k);
 }
 
 template <int MODE>
@@ -210,15 +287,21 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 k_rows(NlConst c, int n, int capacity, const double* __restrict__ wrapped, const double* __restrict__ offsets,
        const int32_t* __restrict__ atom_bin, const int32_t* __restrict__ bin_start, const int32_t* __restrict__ bin_atoms,
        int32_t* __restrict__ row_count, const int32_t* __restrict__ row_ptr, int32_t* __restrict__ cand_index,
-       float* __restrict__ cand_shift, uint32_t* __restrict__ status, const int32_t* flag) {
+       float* __restrict__ cand_shift, uint32_t* __restrict__ status, const int32_t* flag, int rows_per_warp) {
     if (flag && *flag == 0) return;
     extern __shared__ unsigned long long s_keys[];   // MODE 1: [kWarpsPerBlock][FMB_MAX_ROW]
+    __shared__ RowRuns runs[kWarpsPerBlock];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = blockIdx.x * kWarpsPerBlock + warp;
-    if (r >= n) return;
     unsigned long long* keys = MODE == 1 ? s_keys + (size_t)warp * FMB_MAX_ROW : nullptr;
-    rows_receiver<MODE>(c, r, lane, keys, capacity, wrapped, offsets, atom_bin, bin_start, bin_atoms, row_count, row_ptr,
-                        cand_index, cand_shift, status);
+    if (lane == 0) runs[warp].bin = -1;
+    __syncwarp();
+    // receivers in bin order
+    const int first = (blockIdx.x * kWarpsPerBlock + warp) * rows_per_warp;
+    for (int k = first; k < first + rows_per_warp && k < n; ++k) {
+        rows_receiver<MODE>(c, bin_atoms[k], lane, keys, runs[warp], capacity, wrapped, offsets, atom_bin, bin_start, bin_atoms,
+                            row_count, row_ptr, cand_index, cand_shift, status);
+        __syncwarp();
+    }
 }
 
 struct FinishArgs {
@@ -520,6 +603,7 @@ __global__ void __launch_bounds__(kCoopThreads)
 k_build_small(const __grid_constant__ SmallBuildArgs a) {
     if (a.flag && *a.flag == 0) return;                 // the same answer in every CTA: nobody reaches a grid barrier
     extern __shared__ unsigned long long s_keys[];      // [warps of the CTA][FMB_MAX_ROW]
+    __shared__ RowRuns runs[kCoopThreads / 32];
     cooperative_groups::grid_group grid = cooperative_groups::this_grid();
     const int tid = blockIdx.x * kCoopThreads + threadIdx.x, stride = gridDim.x * kCoopThreads;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -531,15 +615,16 @@ k_build_small(const __grid_constant__ SmallBuildArgs a) {
     if (blockIdx.x == 0) scan_by_one_cta(a.bin_count, a.bin_start, a.total_bins);
     grid.sync();
     for (int i = tid; i < a.n; i += stride) bin_fill_item(i, a.atom_bin, a.bin_start, a.bin_fill, a.bin_atoms);
+    if (lane == 0) runs[warp].bin = -1;
     grid.sync();
     for (int r = first_row; r < a.n; r += row_stride)
-        rows_receiver<0>(a.c, r, lane, nullptr, a.capacity, a.wrapped, a.offsets, a.atom_bin, a.bin_start, a.bin_atoms,
+        rows_receiver<0>(a.c, r, lane, nullptr, runs[warp], a.capacity, a.wrapped, a.offsets, a.atom_bin, a.bin_start, a.bin_atoms,
                          a.cand_row_count, nullptr, nullptr, nullptr, a.finish.status);
     grid.sync();
     if (blockIdx.x == 0) scan_by_one_cta(a.cand_row_count, a.cand_row_ptr, a.n);
     grid.sync();
     for (int r = first_row; r < a.n; r += row_stride) {
-        rows_receiver<1>(a.c, r, lane, s_keys + (size_t)warp * FMB_MAX_ROW, a.capacity, a.wrapped, a.offsets, a.atom_bin,
+        rows_receiver<1>(a.c, r, lane, s_keys + (size_t)warp * FMB_MAX_ROW, runs[warp], a.capacity, a.wrapped, a.offsets, a.atom_bin,
                          a.bin_start, a.bin_atoms, nullptr, a.cand_row_ptr, a.finish.cand_index, a.finish.cand_shift,
                          a.finish.status);
         __syncwarp();
@@ -597,7 +682,7 @@ FinishArgs finish_args(const fmb_nl_t* nl) {
     return f;
 }
 
-// the gated build of a small list as one cooperative launch; FMB_ERR_UNSUPPORTED when the device cannot hold the grid
+// the build of a small list as one cooperative launch; FMB_ERR_UNSUPPORTED when the device cannot hold the grid
 int build_small(const fmb_nl_t* nl, const double* positions, const int32_t* flag, cudaStream_t stream) {
     const size_t smem = (size_t)(kCoopThreads / 32) * FMB_MAX_ROW * sizeof(unsigned long long);
     FMB_CUDA_CHECK(opt_in_shared_memory((const void*)k_build_small, (int)smem));
@@ -640,7 +725,7 @@ extern "C" FMB_API int fmb_nl_build(const fmb_nl_t* nl, const double* positions,
     const int n = nl->n_atoms;
     const int total_bins = nl->nbins[0] * nl->nbins[1] * nl->nbins[2];
     const int32_t* flag = only_if_flag ? nl->rebuild_flag : nullptr;
-    if (only_if_flag && n <= kSmallBuild && total_bins < kSmallBuild) {
+    if (n <= kSmallBuild && total_bins < kSmallBuild) {
         const int rc = build_small(nl, positions, flag, stream);
         if (rc != FMB_ERR_UNSUPPORTED) return rc;
     }
@@ -653,10 +738,12 @@ extern "C" FMB_API int fmb_nl_build(const fmb_nl_t* nl, const double* positions,
     if (rc) return rc;
     k_bin_fill<<<ceil_div(n, 256), 256, 0, stream>>>(n, nl->atom_bin, nl->bin_start, nl->bin_fill, nl->bin_atoms, flag);
     FMB_LAUNCH_CHECK();
-    const int row_blocks = ceil_div(n, kWarpsPerBlock);
+    // receivers of a warp one after the other, sharing the runs of their bin, once that leaves every SM 32 warps
+    const int rows_per_warp = n >= 4 * 32 * 148 ? 4 : 1;
+    const int row_blocks = ceil_div(n, kWarpsPerBlock * rows_per_warp);
     k_rows<0><<<row_blocks, kWarpsPerBlock * 32, 0, stream>>>(c, n, nl->capacity, nl->wrapped, nl->offsets, nl->atom_bin,
                                                                nl->bin_start, nl->bin_atoms, nl->cand_row_count, nullptr,
-                                                               nullptr, nullptr, nl->status, flag);
+                                                               nullptr, nullptr, nl->status, flag, rows_per_warp);
     FMB_LAUNCH_CHECK();
     rc = exclusive_scan(nl->cand_row_count, nl->cand_row_ptr, n, nl->scan_scratch, flag, stream);
     if (rc) return rc;
@@ -664,7 +751,7 @@ extern "C" FMB_API int fmb_nl_build(const fmb_nl_t* nl, const double* positions,
     k_rows<1><<<row_blocks, kWarpsPerBlock * 32, smem, stream>>>(c, n, nl->capacity, nl->wrapped, nl->offsets,
                                                                   nl->atom_bin, nl->bin_start, nl->bin_atoms, nullptr,
                                                                   nl->cand_row_ptr, nl->candidate_index,
-                                                                  nl->candidate_unit_shifts, nl->status, flag);
+                                                                  nl->candidate_unit_shifts, nl->status, flag, rows_per_warp);
     FMB_LAUNCH_CHECK();
     k_finish_build<<<148 * 2, 256, 0, stream>>>(c, n, nl->capacity, nl->cand_row_ptr, positions, finish_args(nl), flag);
     FMB_LAUNCH_CHECK();
