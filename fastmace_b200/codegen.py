@@ -202,9 +202,13 @@ def _emit_symcon(l_out_max: int) -> str:
     return "\n".join(fwd + bwd)
 
 
+SYMCON_PARTS = (1, 2)
+
+
 def _emit_symcon_group(l_out_max: int) -> str:
-    """The same polynomial for R atoms of one species at once: every coefficient is loaded once and used R times
-    (the single-atom bodies are bound by their coefficient loads: 410 per atom and channel for outputs 0e + 1o)."""
+    """The same polynomial for the four atoms of a group at once, two pairs on the packed FP32 pipe: every coefficient is
+    loaded once and used four times. ``part`` of ``parts`` evaluates a run of the monomials only (the parts' results are
+    added afterwards), so that several warps share a (group, channel block)."""
     keys = so3.contraction_keys(l_out_max)
     n_out = (l_out_max + 1) ** 2
     index = {key: t for t, key in enumerate(keys)}
@@ -215,48 +219,64 @@ def _emit_symcon_group(l_out_max: int) -> str:
     deg2 = sorted(m for m in by_mono if len(m) == 2)
     deg3 = sorted(m for m in by_mono if len(m) == 3)
     prefixes = sorted({m[:2] for m in deg3} | set(deg2))
-    loop = "_Pragma(\"unroll\") for (int r = 0; r < R; ++r)"
-    fwd = [f"template <int R> __device__ __forceinline__ void symcon_forward_group_{l_out_max}(const float (&x)[R][16], "
-           f"const float* __restrict__ cf, float (&y)[R][{n_out}]) {{"]
+    loop = "_Pragma(\"unroll\") for (int r = 0; r < 2; ++r)"
 
-    def consume(mono, expr, lines):
-        for m_out, t in sorted(by_mono.get(mono, ())):
-            lines.append(f"    {{ const float w = __ldg(cf + {t * 128}); {loop} y[r][{m_out}] = fmaf(w, {expr}, y[r][{m_out}]); }}")
+    def weight(t):
+        return f"const float2 w = symcon_pair(__ldg(cf + {t * 128}));"
 
+    def fwd_terms(mono, value):
+        return [f"      {{ {weight(t)} {loop} y[r][{m_out}] = __ffma2_rn(w, {value}, y[r][{m_out}]); }}"
+                for m_out, t in sorted(by_mono.get(mono, ()))]
+
+    def bwd_terms(mono, target):
+        return [f"      {{ {weight(t)} {loop} {target}[r] = __ffma2_rn(w, g[r][{m_out}], {target}[r]); }}"
+                for m_out, t in sorted(by_mono[mono])]
+
+    zero = "make_float2(0.0f, 0.0f)"
+    fwd_blocks, bwd_blocks = [], []                                   # (terms, lines)
     for mono in deg1:
-        consume(mono, f"x[r][{mono[0]}]", fwd)
-    for pre in prefixes:
-        fwd.append(f"    {{ float p[R]; {loop} p[r] = x[r][{pre[0]}] * x[r][{pre[1]}];")
-        consume(pre, "p[r]", fwd)
-        for mono in (m for m in deg3 if m[:2] == pre):
-            consume(mono, f"(p[r] * x[r][{mono[2]}])", fwd)
-        fwd.append("    }")
-    fwd += ["}", ""]
-    bwd = [f"template <int R> __device__ __forceinline__ void symcon_backward_group_{l_out_max}(const float (&x)[R][16], "
-           f"const float* __restrict__ cf, const float (&g)[R][{n_out}], float (&dx)[R][16]) {{"]
-
-    def adjoint_into(mono, target, lines):
-        for m_out, t in sorted(by_mono[mono]):
-            lines.append(f"      {{ const float w = __ldg(cf + {t * 128}); {loop} {target}[r] = fmaf(w, g[r][{m_out}], {target}[r]); }}")
-
-    for mono in deg1:
-        bwd.append(f"    {{ float h[R]; {loop} h[r] = 0.0f;")
-        adjoint_into(mono, "h", bwd)
-        bwd.append(f"      {loop} dx[r][{mono[0]}] += h[r]; }}")
+        n = len(by_mono[mono])
+        fwd_blocks.append((n, fwd_terms(mono, f"x[r][{mono[0]}]")))
+        bwd_blocks.append((n, [f"    {{ float2 h[2]; {loop} h[r] = {zero};", *bwd_terms(mono, "h"),
+                               f"      {loop} dx[r][{mono[0]}] = __fadd2_rn(dx[r][{mono[0]}], h[r]); }}"]))
     for pre in prefixes:
         i, j = pre
-        bwd.append(f"    {{ float p[R], hp[R]; {loop} {{ p[r] = x[r][{i}] * x[r][{j}]; hp[r] = 0.0f; }}")
+        longer = [m for m in deg3 if m[:2] == pre]
+        n = len(by_mono.get(pre, ())) + sum(len(by_mono[m]) for m in longer)
+        lines = [f"    {{ float2 p[2]; {loop} p[r] = __fmul2_rn(x[r][{i}], x[r][{j}]);", *fwd_terms(pre, "p[r]")]
+        for mono in longer:
+            lines += [f"      {{ float2 q[2]; {loop} q[r] = __fmul2_rn(p[r], x[r][{mono[2]}]);", *fwd_terms(mono, "q[r]"), "      }"]
+        fwd_blocks.append((n, lines + ["    }"]))
+        lines = [f"    {{ float2 p[2], hp[2]; {loop} {{ p[r] = __fmul2_rn(x[r][{i}], x[r][{j}]); hp[r] = {zero}; }}"]
         if pre in by_mono:
-            adjoint_into(pre, "hp", bwd)
-        for mono in (m for m in deg3 if m[:2] == pre):
+            lines += bwd_terms(pre, "hp")
+        for mono in longer:
             k = mono[2]
-            bwd.append(f"      {{ float h[R]; {loop} h[r] = 0.0f;")
-            adjoint_into(mono, "h", bwd)
-            bwd.append(f"        {loop} {{ dx[r][{k}] = fmaf(h[r], p[r], dx[r][{k}]); hp[r] = fmaf(h[r], x[r][{k}], hp[r]); }} }}")
-        bwd.append(f"      {loop} {{ dx[r][{i}] = fmaf(hp[r], x[r][{j}], dx[r][{i}]); dx[r][{j}] = fmaf(hp[r], x[r][{i}], dx[r][{j}]); }}")
-        bwd.append("    }")
-    bwd += ["}", ""]
-    return "\n".join(fwd + bwd)
+            lines += [f"      {{ float2 h[2]; {loop} h[r] = {zero};", *bwd_terms(mono, "h"),
+                      f"        {loop} {{ dx[r][{k}] = __ffma2_rn(h[r], p[r], dx[r][{k}]); hp[r] = __ffma2_rn(h[r], x[r][{k}], hp[r]); }} }}"]
+        lines += [f"      {loop} {{ dx[r][{i}] = __ffma2_rn(hp[r], x[r][{j}], dx[r][{i}]); "
+                  f"dx[r][{j}] = __ffma2_rn(hp[r], x[r][{i}], dx[r][{j}]); }}", "    }"]
+        bwd_blocks.append((n, lines))
+
+    def split(blocks, parts):
+        total, out, done = sum(n for n, _ in blocks), [[] for _ in range(parts)], 0
+        for n, lines in blocks:
+            out[min(parts - 1, (2 * done + n) * parts // (2 * total))] += lines
+            done += n
+        return out
+
+    text = []
+    for parts in SYMCON_PARTS:
+        for head, blocks in (
+                (f"template <> __device__ __forceinline__ void symcon_forward_group<{l_out_max}, {parts}>(int part, const float2 (&x)[2][16], "
+                 f"const float* __restrict__ cf, float2 (&y)[2][{n_out}]) {{", fwd_blocks),
+                (f"template <> __device__ __forceinline__ void symcon_backward_group<{l_out_max}, {parts}>(int part, const float2 (&x)[2][16], "
+                 f"const float* __restrict__ cf, const float2 (&g)[2][{n_out}], float2 (&dx)[2][16]) {{", bwd_blocks)):
+            text.append(head)
+            for q, lines in enumerate(split(blocks, parts)):
+                text += [f"    {'else ' if q else ''}if (part == {q}) {{", *lines, "    }"]
+            text += ["}", ""]
+    return "\n".join(text)
 
 
 def render_symcon() -> str:
@@ -272,6 +292,11 @@ def render_symcon() -> str:
             "const float* __restrict__ cf, float (&y)[(LOUT + 1) * (LOUT + 1)]);",
             "template <int LOUT> __device__ __forceinline__ void symcon_backward_body(const float (&x)[16], "
             "const float* __restrict__ cf, const float (&g)[(LOUT + 1) * (LOUT + 1)], float (&dx)[16]);",
+            "__device__ __forceinline__ float2 symcon_pair(float v) { return make_float2(v, v); }",
+            "template <int LOUT, int PARTS> __device__ __forceinline__ void symcon_forward_group(int part, const float2 (&x)[2][16], "
+            "const float* __restrict__ cf, float2 (&y)[2][(LOUT + 1) * (LOUT + 1)]);",
+            "template <int LOUT, int PARTS> __device__ __forceinline__ void symcon_backward_group(int part, const float2 (&x)[2][16], "
+            "const float* __restrict__ cf, const float2 (&g)[2][(LOUT + 1) * (LOUT + 1)], float2 (&dx)[2][16]);",
             ""]
     return "\n".join(head + [_emit_symcon(l) for l in (0, 1, 2)] + [_emit_symcon_group(l) for l in (0, 1, 2)] +
                      ["}  // namespace fmb", ""])

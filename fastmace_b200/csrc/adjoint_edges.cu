@@ -233,9 +233,23 @@ k_gather_dx(int n_rows, int n_source, const int32_t* __restrict__ row_ptr, const
 // shared memory -- and only the four threads of an edge meet at the end, by shuffles inside a group of four lanes. (A
 // thread per (feature, eight harmonics) spent 137 instructions per warp and edge on 16 FMAs per thread: channel
 // reductions by shuffle and two barriers per eight edges; 72 -> 45 us.)
+// The features of 16 edges arrive by asynchronous copies a pass ahead, and features and gradient block are read four
+// values at a time: with single values the six shared-memory reads per nine FMAs bounded the kernel (42 -> 35 us at 62 k
+// edges, 217 -> 197 us at 615 k, 431 -> 330 us at 748 k edges and five species).
 constexpr int kFaPass = 16;                       // edges per pass
 constexpr int kFaThreads = 4 * kFaPass;
-constexpr int kFaLd = kRadial + 1;                // row stride of the staged features (conflict-free across edges)
+constexpr int kFaLd = kRadial + 4;                // row stride: 16-byte rows, neighbouring rows start four banks apart
+
+// Floats from one group of four harmonics to the next in the gradient block: 8 mod 32, so that the four groups and two
+// neighbouring species are read from different banks.
+__host__ __device__ constexpr int fa_group(int n_species) {
+    const int rows = 4 * n_species * kFaLd;
+    return rows + (8 - rows % 32 + 32) % 32;
+}
+
+__device__ __forceinline__ void copy_row_part(float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(tc::smem_u32(dst)), "l"(src) : "memory");
+}
 
 __global__ void __launch_bounds__(kFaThreads)
 k_first_adjoint_rows(int n_rows, int n_valid, int n_add, int n_species, const int32_t* __restrict__ row_ptr,
@@ -243,12 +257,21 @@ k_first_adjoint_rows(int n_rows, int n_valid, int n_add, int n_species, const in
                      const float* __restrict__ edge_sh, const float* __restrict__ edge_vec,
                      const float* __restrict__ hidden, const float* __restrict__ hidden_tangent,
                      const float* __restrict__ d_s, float4* __restrict__ qe) {
-    __shared__ float hs[kFaPass][kFaLd], hps[kFaPass][kFaLd];
-    extern __shared__ float own[];                        // [16][n_species][kFaLd]: the four harmonics groups and the
-                                                          // species of a warp's edges fall into different banks
+    extern __shared__ __align__(16) float staged[];       // [2 buffers][values, tangents][kFaPass][kFaLd]
+    float* const own = staged + 4 * kFaPass * kFaLd;      // [4 groups][4][n_species][kFaLd]
     const int c = threadIdx.x, slot = c >> 2, grp = c & 3, lane = c & 31;
-    const long long row_floats = (long long)kNSH * n_species * kRadial;
-    const int lm_stride = n_species * kFaLd;
+    const int row_floats = kNSH * n_species * kRadial;
+    const int lm_stride = n_species * kFaLd, group = fa_group(n_species);
+    auto stage = [&](long long first, long long re, int buf) {
+        const int nb = (int)min((long long)kFaPass, re - first);
+        float* const to = staged + buf * 2 * kFaPass * kFaLd;
+        for (int q = c; q < nb * (kRadial / 4); q += kFaThreads) {
+            const int el = q >> 4, k = 4 * (q & 15);
+            copy_row_part(to + el * kFaLd + k, hidden + (first + el) * kRadial + k);
+            copy_row_part(to + (kFaPass + el) * kFaLd + k, hidden_tangent + (first + el) * kRadial + k);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
     for (int a = blockIdx.x; a < n_rows; a += gridDim.x) {
         const long long rb = row_ptr[a], re = row_ptr[a + 1];
         if (a >= n_valid) {
@@ -256,31 +279,46 @@ k_first_adjoint_rows(int n_rows, int n_valid, int n_add, int n_species, const in
                 for (long long e = rb + c; e < re; e += kFaThreads) qe[e] = make_float4(0.f, 0.f, 0.f, 0.f);
             continue;
         }
-        __syncthreads();                                  // the previous row's block is no longer read
-        for (int q = c; q < (int)row_floats; q += kFaThreads) own[(q >> 6) * kFaLd + (q & 63)] = __ldg(d_s + a * row_floats + q);
-        for (long long batch = rb; batch < re; batch += kFaPass) {
+        if (rb >= re) continue;
+        // the previous row's last barrier freed its block and both buffers
+        for (int q = c; q < row_floats / 4; q += kFaThreads)
+            copy_row_part(own + (q >> 4) * kFaLd + ((q >> 4) / (4 * n_species)) * (group - 4 * lm_stride) + 4 * (q & 15),
+                          d_s + (long long)a * row_floats + 4 * q);
+        stage(rb, re, 0);
+        int z_next = rb + slot < re ? species[senders[rb + slot]] : 0;
+        int buf = 0;
+        for (long long batch = rb; batch < re; batch += kFaPass, buf ^= 1) {
             const int nb = (int)min((long long)kFaPass, re - batch);
-            __syncthreads();                              // the previous pass is done with the staged features
-            for (int q = c; q < nb * kRadial; q += kFaThreads) {
-                const int el = q >> 6, k = q & 63;
-                hs[el][k] = __ldg(hidden + (batch + el) * kRadial + k);
-                hps[el][k] = __ldg(hidden_tangent + (batch + el) * kRadial + k);
+            const int zj = z_next;
+            if (batch + kFaPass < re) {
+                stage(batch + kFaPass, re, buf ^ 1);
+                const long long e = batch + kFaPass + slot;
+                z_next = e < re ? species[senders[e]] : 0;
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
             }
             __syncthreads();
             const bool live = slot < nb;
             const long long e = batch + (live ? slot : 0);
             float g[4] = {0.f, 0.f, 0.f, 0.f}, dr = 0.0f;
             if (live) {
-                const int zj = species[senders[e]];
                 const float4 y = __ldg(reinterpret_cast<const float4*>(edge_sh + 16 * e) + grp);
-                const float* ds = own + (4 * grp * n_species + zj) * kFaLd;       // harmonics 4 grp .. 4 grp + 3
-#pragma unroll 8
-                for (int k = 0; k < kRadial; ++k) {
-                    const float h = hs[slot][k], hp = hps[slot][k];
-                    const float d0 = ds[k], d1 = ds[lm_stride + k], d2 = ds[2 * lm_stride + k], d3 = ds[3 * lm_stride + k];
+                const float4* hs = reinterpret_cast<const float4*>(staged + (buf * 2 * kFaPass + slot) * kFaLd);
+                const float4* hps = hs + kFaPass * kFaLd / 4;
+                const float4* ds = reinterpret_cast<const float4*>(own + grp * group + zj * kFaLd);     // harmonics 4 grp ..
+                const int next = lm_stride / 4;
+                auto term = [&](float h, float hp, float d0, float d1, float d2, float d3) {
                     g[0] = fmaf(d0, h, g[0]); g[1] = fmaf(d1, h, g[1]); g[2] = fmaf(d2, h, g[2]); g[3] = fmaf(d3, h, g[3]);
-                    const float dh = fmaf(d0, y.x, fmaf(d1, y.y, fmaf(d2, y.z, d3 * y.w)));
-                    dr = fmaf(dh, hp, dr);
+                    dr = fmaf(fmaf(d0, y.x, fmaf(d1, y.y, fmaf(d2, y.z, d3 * y.w))), hp, dr);
+                };
+#pragma unroll 4
+                for (int k = 0; k < kRadial / 4; ++k) {
+                    const float4 h = hs[k], hp = hps[k], d0 = ds[k], d1 = ds[next + k], d2 = ds[2 * next + k], d3 = ds[3 * next + k];
+                    term(h.x, hp.x, d0.x, d1.x, d2.x, d3.x);
+                    term(h.y, hp.y, d0.y, d1.y, d2.y, d3.y);
+                    term(h.z, hp.z, d0.z, d1.z, d2.z, d3.z);
+                    term(h.w, hp.w, d0.w, d1.w, d2.w, d3.w);
                 }
             }
             // the four threads of an edge exchange their harmonics' gradients and add up the radial one
@@ -303,6 +341,7 @@ k_first_adjoint_rows(int n_rows, int n_valid, int n_add, int n_species, const in
                 }
                 qe[e] = out;
             }
+            __syncthreads();                              // the pass is done with its buffer (and, at the end, with the block)
         }
     }
 }
@@ -417,9 +456,10 @@ int gather_sender_gradient(const EdgeAdjointArgs& t, cudaStream_t stream) {
 
 int first_adjoint_edges(const FirstArgs& f, int n_add, float* qe, cudaStream_t stream) {
     if (f.n_rows <= 0) return FMB_OK;
-    const size_t smem = (size_t)f.n_species * kNSH * kFaLd * sizeof(float);
-    static int grid_cap = 0;
-    if (grid_cap == 0) grid_cap = grid_for((const void*)k_first_adjoint_rows, 1 << 30, kFaThreads, smem);
+    const size_t smem = (size_t)(4 * fa_group(f.n_species) + 4 * kFaPass * kFaLd) * sizeof(float);
+    FMB_CUDA_CHECK(opt_in_shared_memory((const void*)k_first_adjoint_rows,
+                                        (4 * fa_group(FMB_MAX_SPECIES) + 4 * kFaPass * kFaLd) * (int)sizeof(float)));
+    const int grid_cap = grid_for((const void*)k_first_adjoint_rows, 1 << 30, kFaThreads, smem);
     k_first_adjoint_rows<<<f.n_rows < grid_cap ? f.n_rows : grid_cap, kFaThreads, smem, stream>>>(
         f.n_rows, f.n_valid, n_add, f.n_species, f.row_ptr, f.senders, f.species, f.edge_sh, f.edge_vec, f.hidden,
         f.hidden_tangent, f.d_s, reinterpret_cast<float4*>(qe));

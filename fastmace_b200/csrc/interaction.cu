@@ -251,16 +251,18 @@ k_tp_backward(int n_atoms, int n_rows, int n_valid, int fresh_from, long long ch
 constexpr int kFirstZ = FMB_MAX_SPECIES;
 
 // CTA per receiver, thread = (k = tid & 63, half = tid >> 6 -> harmonics 8 * half .. 8 * half + 7). The sums live in
-// registers, one set per sender species (an edge adds into the set of its sender's species through a 0 / 1 factor, so
-// that no index depends on data), and the operands of four edges are requested together: the chain sender -> species
-// -> features is three dependent loads, which a loop over single edges pays in full for every edge (11 warps stalled
-// on loads per issued instruction in the version that accumulated in shared memory).
+// registers, one set per sender species: the species of the row's senders are looked up first, a block of 128 edges at a
+// time, so that the chain sender -> species is paid once per block and not per edge, and an edge then branches (the
+// whole CTA the same way) to the set of its species. Adding into every set through a factor of 0 or 1 cost Z times the
+// FMAs: 30 -> 25 us at 62 k edges of two species, 269 -> 189 us at 615 k of two, 536 -> 300 us at 748 k of five. (Harmonics
+// staged in shared memory, features eight edges ahead in registers: 249 us, the chain of shared-memory reads bounds it.)
 template <int Z>
 __global__ void __launch_bounds__(kC)
 k_first_accumulate(int n_rows, const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ senders,
                    const int32_t* __restrict__ species, const float* __restrict__ edge_sh,
                    const float* __restrict__ hidden, float* __restrict__ s_out) {
-    constexpr int kAhead = 4;
+    constexpr int kAhead = 8;
+    __shared__ int32_t zs[kC];
     const int k = threadIdx.x & 63, half = threadIdx.x >> 6;
     for (int i = blockIdx.x; i < n_rows; i += gridDim.x) {
         float acc[Z][8];
@@ -269,34 +271,41 @@ k_first_accumulate(int n_rows, const int32_t* __restrict__ row_ptr, const int32_
 #pragma unroll
             for (int m = 0; m < 8; ++m) acc[z][m] = 0.0f;
         const long long rb = row_ptr[i], re = row_ptr[i + 1];
-        for (long long e0 = rb; e0 < re; e0 += kAhead) {
-            int zs[kAhead];
-            float h[kAhead];
-            float4 y0[kAhead], y1[kAhead];
+        for (long long block = rb; block < re; block += kC) {
+            const int len = (int)min((long long)kC, re - block);
+            __syncthreads();                                   // the previous block's species have been read
+            if (threadIdx.x < len) zs[threadIdx.x] = species[senders[block + threadIdx.x]];
+            __syncthreads();
+            const float* hp = hidden + block * kRadial + k;
+            const float4* yp = reinterpret_cast<const float4*>(edge_sh + 16 * block + 8 * half);
+            for (int e0 = 0; e0 < len; e0 += kAhead) {
+                float h[kAhead];
+                float4 y0[kAhead], y1[kAhead];
 #pragma unroll
-            for (int q = 0; q < kAhead; ++q) {
-                const bool live = e0 + q < re;
-                const long long e = live ? e0 + q : rb;
-                zs[q] = species[senders[e]];
-                h[q] = live ? __ldg(hidden + e * kRadial + k) : 0.0f;
-                const float4* yp = reinterpret_cast<const float4*>(edge_sh + 16 * e + 8 * half);
-                y0[q] = __ldg(yp);
-                y1[q] = __ldg(yp + 1);
-            }
-#pragma unroll
-            for (int q = 0; q < kAhead; ++q)
-#pragma unroll
-                for (int z = 0; z < Z; ++z) {
-                    const float hz = zs[q] == z ? h[q] : 0.0f;
-                    acc[z][0] = fmaf(y0[q].x, hz, acc[z][0]);
-                    acc[z][1] = fmaf(y0[q].y, hz, acc[z][1]);
-                    acc[z][2] = fmaf(y0[q].z, hz, acc[z][2]);
-                    acc[z][3] = fmaf(y0[q].w, hz, acc[z][3]);
-                    acc[z][4] = fmaf(y1[q].x, hz, acc[z][4]);
-                    acc[z][5] = fmaf(y1[q].y, hz, acc[z][5]);
-                    acc[z][6] = fmaf(y1[q].z, hz, acc[z][6]);
-                    acc[z][7] = fmaf(y1[q].w, hz, acc[z][7]);
+                for (int q = 0; q < kAhead; ++q) {
+                    const int e = min(e0 + q, len - 1);
+                    h[q] = __ldg(hp + e * kRadial);
+                    y0[q] = __ldg(yp + 4 * e);
+                    y1[q] = __ldg(yp + 4 * e + 1);
                 }
+#pragma unroll
+                for (int q = 0; q < kAhead; ++q) {
+                    if (e0 + q >= len) break;
+                    const int ze = zs[e0 + q];
+#pragma unroll
+                    for (int z = 0; z < Z; ++z)
+                        if (ze == z) {
+                            acc[z][0] = fmaf(y0[q].x, h[q], acc[z][0]);
+                            acc[z][1] = fmaf(y0[q].y, h[q], acc[z][1]);
+                            acc[z][2] = fmaf(y0[q].z, h[q], acc[z][2]);
+                            acc[z][3] = fmaf(y0[q].w, h[q], acc[z][3]);
+                            acc[z][4] = fmaf(y1[q].x, h[q], acc[z][4]);
+                            acc[z][5] = fmaf(y1[q].y, h[q], acc[z][5]);
+                            acc[z][6] = fmaf(y1[q].z, h[q], acc[z][6]);
+                            acc[z][7] = fmaf(y1[q].w, h[q], acc[z][7]);
+                        }
+                }
+            }
         }
         // global layout [i][lm][z][k]: the K = n_species * 64 values of one (atom, harmonic) row are contiguous
         float* out = s_out + (long long)i * kNSH * Z * kRadial + k;
