@@ -382,7 +382,8 @@ k_tp_fused(const __grid_constant__ FusedArgs a) {
 // consumers only move accumulator columns to global memory -- lane = channel, so a warp writes 128 contiguous bytes of
 // one edge row per store (a path-major layout [path][edge][128], contiguous per tile, measured slower both for this
 // kernel and for its readers). The hidden features of a tile are split and staged once for all paths, the accumulator of
-// path p is stored while the tensor cores work on path p + 1. HBM-write bound: 4 * paths * 128 bytes per edge.
+// path p is stored while the tensor cores work on path p + 1 (or on the next tile's first). Bound by the stores: 4 * paths *
+// 128 bytes per edge leave an SM at 25 bytes a cycle, 5,150 of the 5,400 cycles a path of 256 edges takes.
 struct WeightArgs {
     const float* hidden;          // [edges][64]
     const float* image;           // fmb_layer_t.rad_img
@@ -390,7 +391,6 @@ struct WeightArgs {
     const long long* limit;       // device scalar: rows at or beyond *limit - limit_offset are skipped
     long long limit_offset;
     int rows;                     // host bound on the rows of this launch
-    int n_paths;
     uint32_t* error_word;
     const int32_t* row_index;     // or null: output row r comes from hidden row row_index[r]
 };
@@ -401,6 +401,7 @@ constexpr int kWeightRing = 2 * kWeightTile * 256;                    // after t
 constexpr int kWeightBars = kWeightRing + kWeightStages * kStageBytes;
 constexpr int kWeightBytes = kWeightBars + 256 + 16 + 1024;
 
+template <int P>
 __global__ void __launch_bounds__(kFusedThreads, 1)
 k_radial_weights(const __grid_constant__ WeightArgs a) {
     constexpr int TN = kWeightTile, NST = kWeightStages;
@@ -436,7 +437,6 @@ k_radial_weights(const __grid_constant__ WeightArgs a) {
     long long rows = a.rows;
     if (a.limit) rows = min(rows, max(*a.limit - a.limit_offset, 0LL));
     const int n_tiles = (int)((rows + TN - 1) / TN);
-    const int P = a.n_paths;
 
     if (warp == 8) {
         if (lane == 0) {
@@ -456,45 +456,70 @@ k_radial_weights(const __grid_constant__ WeightArgs a) {
         const int wg = tid >> 7, c = tid & 127, quadrant = warp & 3;
         const uint32_t lane_base = (uint32_t)(quadrant * 32) << 16;
         const int ld_row = warp * 8 + (lane & 7), ld_q = lane >> 3;
-        const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        const long long ld = (long long)P * kC;
-        uint32_t gpath = 0;
-        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-            const long long e0 = (long long)t * TN;
+        constexpr int ld = P * kC;
+        // the hidden features of the CTA's next tile are on their way while the last paths of this one are stored
+        float4 held[TN / 64][4];
+        auto fetch = [&](int t) {
 #pragma unroll
             for (int sweep = 0; sweep < TN / 64; ++sweep) {
-                const int row = ld_row + 64 * sweep;
-                const bool ok = e0 + row < rows;
-                const long long source = a.row_index ? (ok ? (long long)a.row_index[e0 + row] : 0) : e0 + row;
-                const float* src = a.hidden + source * kRadial;
+                const long long r = (long long)t * TN + ld_row + 64 * sweep;
+                const bool ok = t < n_tiles && r < rows;
+                const long long source = a.row_index ? (ok ? (long long)a.row_index[r] : 0) : r;
+                const float4* src = reinterpret_cast<const float4*>(a.hidden + source * kRadial) + ld_q;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) held[sweep][j] = ok ? __ldg(src + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        };
+        auto stage = [&]() {
+#pragma unroll
+            for (int sweep = 0; sweep < TN / 64; ++sweep)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const float4 v = ok ? __ldg(reinterpret_cast<const float4*>(src) + ld_q + 4 * j) : zero4;
-                    const float4 hi = make_float4(tf32_rna(v.x), tf32_rna(v.y), tf32_rna(v.z), tf32_rna(v.w));
-                    const float4 lo = make_float4(tf32_rna(v.x - hi.x), tf32_rna(v.y - hi.y), tf32_rna(v.z - hi.z),
-                                                  tf32_rna(v.w - hi.w));
-                    const uint32_t off = tile_offset<TN>(row, (ld_q + 4 * j) * 4);
+                    float4 hi, lo;
+                    split_tf32(held[sweep][j], hi, lo);
+                    const uint32_t off = tile_offset<TN>(ld_row + 64 * sweep, (ld_q + 4 * j) * 4);
                     *reinterpret_cast<float4*>(b_hi + off) = hi;
                     *reinterpret_cast<float4*>(b_lo + off) = lo;
                 }
-            }
             fence_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(kBarB));
+        };
+        uint32_t gpath = 0;
+        fetch(blockIdx.x);
+        if ((int)blockIdx.x < n_tiles) stage();
+        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+            const long long e0 = (long long)t * TN;
             const long long eg = e0 + 128 * wg;                        // first edge of this group's 128 columns
             const int live = (int)min(128LL, max(rows - eg, 0LL));
             for (int p = 0; p < P; ++p) {
                 const uint32_t buf = gpath & 1u;
                 const uint32_t t0 = tmem_base + lane_base + buf * TN + 128u * (uint32_t)wg;
+                if (p == P - 2) fetch(t + gridDim.x);
                 mbar_wait(bar(kBarTFull + buf), (gpath >> 1) & 1u, abort_flag, kSpin);
                 fence_after_sync();
-                float* dst = a.out + eg * ld + (long long)p * kC + c;
-                for (int sb = 0; sb < live; sb += 16) {
-                    float w[16];
-                    tmem_load<16>(t0 + sb, w);
+                // the last path's MMAs are the last to read the operand: the next tile's replaces it before this path is
+                // stored, so that the next tile's first MMAs run meanwhile
+                if (p == P - 1 && t + (int)gridDim.x < n_tiles) stage();
+                float* dst = a.out + eg * ld + p * kC + c;
+                if (live == 128) {
+#pragma unroll 1
+                    for (int sb = 0; sb < 128; sb += 32, dst += 32 * ld) {
+                        float w[16], v[16];
+                        tmem_load_16x2(t0 + sb, t0 + sb + 16, w, v);
 #pragma unroll
-                    for (int q = 0; q < 16; ++q)
-                        if (sb + q < live) dst[(long long)(sb + q) * ld] = w[q];
+                        for (int q = 0; q < 16; ++q) dst[q * ld] = w[q];
+#pragma unroll
+                        for (int q = 0; q < 16; ++q) dst[(16 + q) * ld] = v[q];
+                    }
+                } else {
+                    for (int sb = 0; sb < live; sb += 16) {
+                        float w[16];
+                        tmem_load<16>(t0 + sb, w);
+#pragma unroll
+                        for (int q = 0; q < 16; ++q)
+                            if (sb + q < live) dst[(sb + q) * ld] = w[q];
+                    }
                 }
                 fence_before_sync();
                 __syncwarp();
@@ -531,25 +556,39 @@ int launch_fused(const FusedArgs& f, cudaStream_t stream) {
 
 }  // namespace
 
-int radial_weights_tc(const float* hidden, const float* image, float* out, int rows, int n_paths, const long long* limit,
-                      long long limit_offset, const int32_t* row_index, uint32_t* error_word, int max_ctas,
-                      cudaStream_t stream) {
-    if (!image || n_paths < 1) return FMB_ERR_UNSUPPORTED;
-    if (rows <= 0) return FMB_OK;
+namespace {
+
+template <int P>
+int launch_weights(const WeightArgs& a, int max_ctas, cudaStream_t stream) {
     static int sms = 0;
-    FMB_CUDA_CHECK(opt_in_shared_memory((const void*)k_radial_weights, kWeightBytes));
+    FMB_CUDA_CHECK(opt_in_shared_memory((const void*)k_radial_weights<P>, kWeightBytes));
     if (sms == 0) {
         int dev = 0, count = 148;
         FMB_CUDA_CHECK(cudaGetDevice(&dev));
         FMB_CUDA_CHECK(cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev));
         sms = count;
     }
-    WeightArgs a{hidden, image, out, limit, limit_offset, rows, n_paths, error_word, row_index};
-    const int tiles = (rows + kWeightTile - 1) / kWeightTile;
+    const int tiles = (a.rows + kWeightTile - 1) / kWeightTile;
     const int ctas = max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
-    k_radial_weights<<<tiles < ctas ? tiles : ctas, kFusedThreads, kWeightBytes, stream>>>(a);
+    k_radial_weights<P><<<tiles < ctas ? tiles : ctas, kFusedThreads, kWeightBytes, stream>>>(a);
     FMB_LAUNCH_CHECK();
     return FMB_OK;
+}
+
+}  // namespace
+
+int radial_weights_tc(const float* hidden, const float* image, float* out, int rows, int n_paths, const long long* limit,
+                      long long limit_offset, const int32_t* row_index, uint32_t* error_word, int max_ctas,
+                      cudaStream_t stream) {
+    if (!image) return FMB_ERR_UNSUPPORTED;
+    if (rows <= 0) return FMB_OK;
+    const WeightArgs a{hidden, image, out, limit, limit_offset, rows, error_word, row_index};
+    switch (n_paths) {                       // a compile-time row length makes every store's offset an immediate
+        case TpShape<0>::kPaths: return launch_weights<TpShape<0>::kPaths>(a, max_ctas, stream);
+        case TpShape<1>::kPaths: return launch_weights<TpShape<1>::kPaths>(a, max_ctas, stream);
+        case TpShape<2>::kPaths: return launch_weights<TpShape<2>::kPaths>(a, max_ctas, stream);
+        default: return FMB_ERR_UNSUPPORTED;
+    }
 }
 
 int tp_fused_forward(const FusedArgs& f, cudaStream_t stream) {
