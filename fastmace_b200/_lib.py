@@ -87,7 +87,7 @@ class WorkStruct(ctypes.Structure):
         ("mirror", c_void_p), ("edge_q", c_void_p), ("edge_dx", c_void_p),
         ("edge_slot", c_void_p), ("canon_list", c_void_p), ("canon_count", c_void_p),
         ("symcon_groups", c_void_p), ("n_symcon_groups", c_int32), ("halo_exchange", c_int32),
-        ("pair_capacity", c_int32), ("pad_", c_int32),
+        ("pair_capacity", c_int32), ("dx_edges", c_int32),
     ]
 
 

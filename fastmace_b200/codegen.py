@@ -310,56 +310,6 @@ def _write(path: str, text: str) -> None:
             handle.write(text)
 
 
-# --------------------------------------------------------------------------------------------- path-major bodies
-PATHS_OUT = os.path.join(HERE, "csrc", "generated", "tp_paths_generated.cuh")
-
-
-def _emit_paths(lin: int) -> str:
-    """One ``TpPath<LIN, P>`` per path: shape constants and the forward of that path alone, for the kernel that takes
-    the radial weights of one path at a time from tensor memory."""
-    paths = so3.tp_paths(lin)
-    slots, blocks = message_slots(paths)
-    out = [f"// ---- node l_max = {lin}"]
-    seen_in: set[int] = set()
-    for p, path in enumerate(paths):
-        l_in, l_edge, l_out = path["l_in"], path["l_edge"], path["l_out"]
-        n_in, n_e, n_o = 2 * l_in + 1, 2 * l_edge + 1, 2 * l_out + 1
-        base, n_seg = blocks[l_out]
-        seg = slots[(p, 0)] - base
-        first_for_in = l_in not in seen_in
-        seen_in.add(l_in)
-        out += [f"template <> struct TpPath<{lin}, {p}> {{  // {l_in} x {l_edge} -> {l_out}",
-                f"    static constexpr int kNin = {n_in}, kNe = {n_e}, kNo = {n_o};",
-                f"    static constexpr int kInOff = {path['in_off']}, kEdgeOff = {path['edge_off']};",
-                f"    static constexpr int kSlotBase = {base + seg}, kSlotStride = {n_seg};",
-                f"    static constexpr bool kFirstForIn = {'true' if first_for_in else 'false'};",
-                f"    static __device__ __forceinline__ void forward(const float (&x)[{n_in}], const float (&Y)[{n_e}], "
-                f"float w, float (&acc)[{n_o}]) {{"]
-        by_out: dict[int, list] = {}
-        for mi, me, mo, c in path["terms"]:
-            by_out.setdefault(mo, []).append((mi, me, c))
-        for mo, terms in sorted(by_out.items()):
-            expr = " + ".join(f"{_lit(c)} * x[{mi}] * Y[{me}]" for mi, me, c in terms)
-            out.append(f"        acc[{mo}] = fmaf(w, {expr}, acc[{mo}]);")
-        out += ["    }", "};"]
-    out.append(f"#define FMB_FOR_EACH_PATH_{lin}(X) " + " ".join(f"X({p})" for p in range(len(paths))))
-    out.append("")
-    return "\n".join(out)
-
-
-def render_paths() -> str:
-    head = ["// GENERATED by fastmace_b200/codegen.py from fastmace_b200/so3.py -- do not edit.",
-            "// The channelwise tensor product one path at a time (same coefficients and message layout as",
-            "// tp_generated.cuh): message component of output m is kSlotBase + m * kSlotStride.",
-            "#pragma once",
-            "",
-            "namespace fmb {",
-            "",
-            "template <int LIN, int P> struct TpPath;",
-            ""]
-    return "\n".join(head + [_emit_paths(lin) for lin in (1, 2)] + ["}  // namespace fmb", ""])
-
-
 # --------------------------------------------------------------------------------------------- coupled bodies
 COUPLED_OUT = os.path.join(HERE, "csrc", "generated", "tp_coupled_generated.cuh")
 COUPLE_PARTS = {0: (4,), 1: (4, 8), 2: (8, 16)}      # threads an edge's couplings are spread over
@@ -501,7 +451,6 @@ _tp_main = main
 def main() -> str:  # noqa: F811  (both generated headers)
     out = _tp_main()
     _write(SYMCON_OUT, render_symcon())
-    _write(PATHS_OUT, render_paths())
     _write(COUPLED_OUT, render_coupled())
     return out
 

@@ -1,5 +1,5 @@
-// Adjoint of the interactions with per-edge hand-over instead of the mirror evaluation (used when the edge list is a
-// single chunk, so that per-edge buffers of the whole list fit).
+// Adjoint of the interactions with per-edge hand-over instead of the mirror evaluation (buffers for the whole list where
+// they fit, for one chunk of it otherwise).
 //
 // The mirror kernels (interaction.cu) make every receiver's CTA evaluate each of its edges twice -- as stored and in
 // the opposite direction -- because that yields the sender-side gradient and the force without a scatter; the price is
@@ -93,7 +93,7 @@ k_tp_adjoint_edges(int n_atoms, int n_rows, int n_valid, long long chunk_e0, lon
                    const long long* __restrict__ count_ptr, const int32_t* __restrict__ row_ptr,
                    const int32_t* __restrict__ senders, const float* __restrict__ x, const float* __restrict__ edge_sh,
                    const float* __restrict__ edge_vec, const float* __restrict__ tp_w, long long tangent_offset,
-                   const float* __restrict__ d_mid, float* __restrict__ dxe, float4* __restrict__ qe) {
+                   const float* __restrict__ d_mid, float* __restrict__ dxe, float4* __restrict__ qe, long long dx0) {
     constexpr int P = TpShape<LIN>::kPaths, IN = TpShape<LIN>::kInDim, MID = TpShape<LIN>::kMidDim;
     __shared__ float red[kBatch][4][18];
     const int c = threadIdx.x, warp = c >> 5, lane = c & 31;
@@ -118,7 +118,7 @@ k_tp_adjoint_edges(int n_atoms, int n_rows, int n_valid, long long chunk_e0, lon
             // no message gradient on this receiver: its edges hand over zeros
             for (long long e = rb; e < re; ++e) {
 #pragma unroll
-                for (int k = 0; k < IN; ++k) dxe[(e * IN + k) * kC + c] = 0.0f;
+                for (int k = 0; k < IN; ++k) dxe[((e - dx0) * IN + k) * kC + c] = 0.0f;
                 if (c == 0) qe[e] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
             continue;
@@ -154,7 +154,7 @@ k_tp_adjoint_edges(int n_atoms, int n_rows, int n_valid, long long chunk_e0, lon
                 float dr = 0.0f;
                 TpBackwardSel<LIN, false, true>::run(x_j, Y, w, wp, g_a, dY, dr, dxj);
 #pragma unroll
-                for (int q = 0; q < IN; ++q) dxe[(e * IN + q) * kC + c] = dxj[q];
+                for (int q = 0; q < IN; ++q) dxe[((e - dx0) * IN + q) * kC + c] = dxj[q];
                 // 16 + 1 sums over the channels: transpose-reduce inside the warp, the four warps meet in shared memory
                 {
 #pragma unroll
@@ -190,16 +190,19 @@ k_tp_adjoint_edges(int n_atoms, int n_rows, int n_valid, long long chunk_e0, lon
     }
 }
 
-// dE/dx_a = sum over the row of a of the hand-over of the mirror edges (rows at or beyond n_source hand over nothing)
+// dE/dx_a = sum over the row of a of the hand-over of the mirror edges (rows at or beyond n_source hand over nothing); of
+// those in [first, end) where the buffer holds a chunk of the list, added to what the chunks before gave
 template <int IN>
 __global__ void __launch_bounds__(kC)
 k_gather_dx(int n_rows, int n_source, const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ senders,
-            const int32_t* __restrict__ mirror, const float* __restrict__ dxe, float* __restrict__ d_x) {
+            const int32_t* __restrict__ mirror, const float* __restrict__ dxe, float* __restrict__ d_x, long long first,
+            long long end, bool add) {
     const int c = threadIdx.x;
+    if (add && first >= row_ptr[n_source]) return;
     for (int a = blockIdx.x; a < n_rows; a += gridDim.x) {
         float acc[IN];
 #pragma unroll
-        for (int k = 0; k < IN; ++k) acc[k] = 0.0f;
+        for (int k = 0; k < IN; ++k) acc[k] = add ? d_x[((long long)a * IN + k) * kC + c] : 0.0f;
         const long long rb = row_ptr[a], re = row_ptr[a + 1];
         // four edges at a time: their mirror indices first, then all the rows, so that the loads overlap
         for (long long e = rb; e < re; e += 4) {
@@ -209,13 +212,14 @@ k_gather_dx(int n_rows, int n_source, const int32_t* __restrict__ row_ptr, const
                 const bool live = e + q < re;
                 m[q] = live ? mirror[e + q] : -1;
                 if (live && senders[e + q] >= n_source) m[q] = -1;
+                if (m[q] < first || m[q] >= end) m[q] = -1;
             }
             float v[4][IN];
 #pragma unroll
             for (int q = 0; q < 4; ++q)
 #pragma unroll
                 for (int k = 0; k < IN; ++k)
-                    v[q][k] = m[q] >= 0 ? __ldg(dxe + ((long long)m[q] * IN + k) * kC + c) : 0.0f;
+                    v[q][k] = m[q] >= 0 ? __ldg(dxe + ((m[q] - first) * IN + k) * kC + c) : 0.0f;
 #pragma unroll
             for (int q = 0; q < 4; ++q)
 #pragma unroll
@@ -410,25 +414,23 @@ int mirror_map(const fmb_nl_t* nl, int32_t* mirror, uint32_t* status, const long
 
 int tp_adjoint_edges(const EdgeAdjointArgs& t, cudaStream_t stream) {
     if (t.n_rows <= 0) return FMB_OK;
-    if (t.whole_list && t.n_valid >= t.n_rows && t.chunk_e0 == 0) return tp_adjoint_coupled_launch(t, stream);
+    if (t.n_valid >= t.n_rows) return tp_adjoint_coupled_launch(t, stream);
     if (t.lin == 0) {
         static const int grid_cap = grid_for((const void*)k_tp_adjoint_edges<0, 2>, 1 << 30, kC, 0);
         k_tp_adjoint_edges<0, 2><<<t.n_rows < grid_cap ? t.n_rows : grid_cap, kC, 0, stream>>>(
             t.n_atoms, t.n_rows, t.n_valid, t.chunk_e0, t.chunk_edges, t.count, t.row_ptr, t.senders, t.x, t.edge_sh, t.edge_vec,
-            t.tp_w, t.tangent_offset, t.d_mid, t.dxe,
-            reinterpret_cast<float4*>(t.qe));
+            t.tp_w, t.tangent_offset, t.d_mid, t.dxe, reinterpret_cast<float4*>(t.qe), t.dx_e0);
     } else if (t.lin == 1) {
         // four CTAs per SM (127 registers): measured best on the 1,944-atom cell among 2 .. 6
         static const int grid_cap = grid_for((const void*)k_tp_adjoint_edges<1, 4>, 1 << 30, kC, 0);
         k_tp_adjoint_edges<1, 4><<<t.n_rows < grid_cap ? t.n_rows : grid_cap, kC, 0, stream>>>(
             t.n_atoms, t.n_rows, t.n_valid, t.chunk_e0, t.chunk_edges, t.count, t.row_ptr, t.senders, t.x, t.edge_sh,
-            t.edge_vec, t.tp_w, t.tangent_offset, t.d_mid, t.dxe, reinterpret_cast<float4*>(t.qe));
+            t.edge_vec, t.tp_w, t.tangent_offset, t.d_mid, t.dxe, reinterpret_cast<float4*>(t.qe), t.dx_e0);
     } else if (t.lin == 2) {
         static const int grid_cap = grid_for((const void*)k_tp_adjoint_edges<2, 2>, 1 << 30, kC, 0);
         k_tp_adjoint_edges<2, 2><<<t.n_rows < grid_cap ? t.n_rows : grid_cap, kC, 0, stream>>>(
             t.n_atoms, t.n_rows, t.n_valid, t.chunk_e0, t.chunk_edges, t.count, t.row_ptr, t.senders, t.x, t.edge_sh, t.edge_vec,
-            t.tp_w, t.tangent_offset, t.d_mid, t.dxe,
-            reinterpret_cast<float4*>(t.qe));
+            t.tp_w, t.tangent_offset, t.d_mid, t.dxe, reinterpret_cast<float4*>(t.qe), t.dx_e0);
     } else {
         return FMB_ERR_UNSUPPORTED;
     }
@@ -436,17 +438,20 @@ int tp_adjoint_edges(const EdgeAdjointArgs& t, cudaStream_t stream) {
     return FMB_OK;
 }
 
-int gather_sender_gradient(const EdgeAdjointArgs& t, cudaStream_t stream) {
+int gather_sender_gradient(const EdgeAdjointArgs& t, long long first, long long count, bool add, cudaStream_t stream) {
     const int rows = t.n_gather > 0 ? t.n_gather : t.n_rows;     // atoms that collect; the edges of [0, n_rows) hand over
     if (rows <= 0) return FMB_OK;
     const int in_dim = (t.lin + 1) * (t.lin + 1);
     const int grid = rows < 1184 ? rows : 1184;
     if (in_dim == 1) {
-        k_gather_dx<1><<<grid, kC, 0, stream>>>(rows, t.n_rows, t.row_ptr, t.senders, t.mirror, t.dxe, t.d_x);
+        k_gather_dx<1><<<grid, kC, 0, stream>>>(rows, t.n_rows, t.row_ptr, t.senders, t.mirror, t.dxe, t.d_x, first,
+                                                first + count, add);
     } else if (in_dim == 4) {
-        k_gather_dx<4><<<grid, kC, 0, stream>>>(rows, t.n_rows, t.row_ptr, t.senders, t.mirror, t.dxe, t.d_x);
+        k_gather_dx<4><<<grid, kC, 0, stream>>>(rows, t.n_rows, t.row_ptr, t.senders, t.mirror, t.dxe, t.d_x, first,
+                                                first + count, add);
     } else if (in_dim == 9) {
-        k_gather_dx<9><<<grid, kC, 0, stream>>>(rows, t.n_rows, t.row_ptr, t.senders, t.mirror, t.dxe, t.d_x);
+        k_gather_dx<9><<<grid, kC, 0, stream>>>(rows, t.n_rows, t.row_ptr, t.senders, t.mirror, t.dxe, t.d_x, first,
+                                                first + count, add);
     } else {
         return FMB_ERR_UNSUPPORTED;
     }

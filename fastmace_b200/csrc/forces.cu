@@ -129,9 +129,8 @@ struct Ctx {
 };
 
 // When the whole edge list is one chunk, the last interaction's radial weights written by the forward pass are still
-// in tp_w when its adjoint runs (the reassociated first layer never touches tp_w), so the adjoint only adds their d/dr.
-// The forward pass then takes the unfused route (GEMM + tensor-product kernel) so that the weights exist; with more
-// than one chunk the fused kernel runs instead and the adjoint recomputes both per chunk. The rows of the forward pass
+// in tp_w when its adjoint runs (the reassociated first layer never touches tp_w), so the adjoint only adds their d/dr;
+// with more than one chunk the adjoint recomputes both per chunk. The rows of the forward pass
 // (n1) and of the adjoint (n0) must be the same prefix of the list: true without decomposition and for a rank of a
 // halo-exchange run, not for the ghost-shell scheme (n1 < n0).
 bool keeps_forward_weights(const Ctx& c, int layer) {
@@ -144,6 +143,9 @@ bool keeps_forward_weights(const Ctx& c, int layer) {
 bool edge_local_adjoint(const Ctx& c) {
     return c.w->mirror && c.w->edge_q && c.w->edge_dx && c.m->n_layers == 2 && c.m->layer[0].first[0] != nullptr;
 }
+
+// edges the hand-over buffer of the sender gradients holds: the whole list or one chunk
+long long dx_rows(const Ctx& c) { return c.w->dx_edges > 0 ? (long long)c.w->dx_edges : c.count_cap; }
 
 float* h_of(const Ctx& c, int layer) {
     return layer == 0 ? c.w->h : c.w->h + (long long)c.n * c.hidden_dim * kC;
@@ -344,21 +346,7 @@ int forward_layer(const Ctx& c, int layer, bool with_up = true) {
                          (long long)l * l * kC, kC, l, 0);
         FMB_TRY(run_linears(c, lb));
     } else {
-    bool fused = false;
-    if (layer > 0 && L.rad_img && tensor_cores_enabled() && !keeps_forward_weights(c, layer)) {
-        // last radial layer inside the tensor-product kernel: no per-edge weight matrix, one launch for all rows
-        FusedArgs f{};
-        f.lin = L.l_in_max; f.n_rows = rows; f.row_ptr = c.nl->edge_row_ptr; f.senders = c.nl->edge_index;
-        f.x = x; f.edge_sh = c.w->edge_sh; f.hidden = hidden_of(c, layer, 0); f.image = L.rad_img; f.mid = c.w->mid;
-        f.error_word = c.w->status;
-        StageScope scope(c.stream, kStTpFwd1);
-        const int rc = tp_fused_forward(f, c.stream);
-        if (rc != FMB_ERR_UNSUPPORTED) {
-            if (rc) return rc;
-            fused = true;
-        }
-    }
-    for (int k = 0; k < c.n_chunks && !fused; ++k) {
+    for (int k = 0; k < c.n_chunks; ++k) {
         const long long e0 = (long long)k * c.chunk;
         if (c.radial_ready && layer > 0) {
             FMB_CUDA_CHECK(cudaStreamWaitEvent(c.stream, c.radial_ready, 0));     // produced beside the first interaction
@@ -469,7 +457,7 @@ int backward_layer(const Ctx& c, int layer, const float* d_h_out, float* d_h_in,
         t.row_ptr = c.nl->edge_row_ptr; t.senders = c.nl->edge_index; t.mirror = c.w->mirror; t.x = c.w->x;
         t.edge_sh = c.w->edge_sh; t.edge_vec = c.w->edge_vec; t.tp_w = c.w->tp_w;
         t.tangent_offset = weight_rows(c) * L.n_paths * kC; t.d_mid = c.w->d_mid; t.dxe = c.w->edge_dx; t.qe = c.w->edge_q;
-        t.d_x = c.w->d_x; t.whole_list = c.n_chunks == 1; t.error_word = c.w->status;
+        t.d_x = c.w->d_x; t.error_word = c.w->status;
         if (layer == c.m->n_layers - 1 && pair_rows(c)) t.slot = c.w->edge_slot;
         for (int k = 0; k < c.n_chunks; ++k) {
             const long long e0 = (long long)k * c.chunk;
@@ -479,12 +467,13 @@ int backward_layer(const Ctx& c, int layer, const float* d_h_out, float* d_h_in,
                 FMB_TRY(radial_weights(c, layer, e0, keeps_forward_weights(c, layer) ? 1 : 0, 1, edge_limit(c, 0)));
             }
             t.chunk_e0 = e0; t.chunk_edges = c.chunk;
+            // the sender gradients of the whole list are kept and collected at the end, or those of this chunk only
+            const bool by_chunk = dx_rows(c) < c.count_cap;
+            t.dx_e0 = by_chunk ? e0 : 0;
             StageScope scope(c.stream, kStTpBwd1);
             FMB_TRY(tp_adjoint_edges(t, c.stream));
-        }
-        {
-            StageScope scope(c.stream, kStTpBwd1);
-            FMB_TRY(gather_sender_gradient(t, c.stream));
+            if (by_chunk) FMB_TRY(gather_sender_gradient(t, e0, c.chunk, k > 0, c.stream));
+            else if (k == c.n_chunks - 1) FMB_TRY(gather_sender_gradient(t, 0, c.count_cap, false, c.stream));
         }
         if (with_up) FMB_TRY(backward_linear_up(c, layer, d_h_in));
         return FMB_OK;
@@ -539,6 +528,7 @@ int make_ctx(Ctx& c, const fmb_model_t* m, const fmb_nl_t* nl, const fmb_work_t*
     c.count_cap = nl->capacity;
     c.chunk = std::min<long long>(w->chunk_edges, nl->capacity);
     c.n_chunks = ceil_div(nl->capacity, c.chunk);
+    if (w->edge_dx) FMB_REQUIRE(dx_rows(c) >= c.chunk, "forces: edge_dx holds less than a chunk (dx_edges)");
     return FMB_OK;
 }
 

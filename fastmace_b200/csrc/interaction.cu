@@ -56,13 +56,14 @@ __device__ __forceinline__ void load_sh(const float* __restrict__ edge_sh, long 
 }
 
 // ---------------------------------------------------------------------------------------------- forward
-template <int LIN, bool SPECIES_X>
+// First interaction of a model without the reassociated form (below): the senders are rows of a per-species table. The
+// interactions after the first are in tp_coupled.cu.
 __global__ void __launch_bounds__(kC)
-k_tp_forward(int n_atoms, int n_rows, long long chunk_e0, long long chunk_edges, const long long* __restrict__ count_ptr,
+k_tp_forward_species(int n_atoms, int n_rows, long long chunk_e0, long long chunk_edges, const long long* __restrict__ count_ptr,
              const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ senders,
              const int32_t* __restrict__ species, const float* __restrict__ x, const float* __restrict__ edge_sh,
              const float* __restrict__ tp_w, float* __restrict__ mid) {
-    constexpr int P = TpShape<LIN>::kPaths, IN = TpShape<LIN>::kInDim, MID = TpShape<LIN>::kMidDim;
+    constexpr int P = TpShape<0>::kPaths, MID = TpShape<0>::kMidDim;
     const long long count = *count_ptr;
     const long long e0 = chunk_e0, e1 = min(count, chunk_e0 + chunk_edges);
     if (e0 >= e1 && !(e0 == 0 && count == 0)) return;
@@ -85,18 +86,13 @@ k_tp_forward(int n_atoms, int n_rows, long long chunk_e0, long long chunk_edges,
 #pragma unroll 4
         for (long long e = b; e < en; ++e) {
             const int s = senders[e];
-            float xs[IN], Y[16], w[P];
-            if (SPECIES_X) {
-                xs[0] = __ldg(x + (long long)species[s] * kC + c);
-            } else {
-#pragma unroll
-                for (int k = 0; k < IN; ++k) xs[k] = __ldg(x + ((long long)s * IN + k) * kC + c);
-            }
+            const float xs[1] = {__ldg(x + (long long)species[s] * kC + c)};
+            float Y[16], w[P];
             load_sh(edge_sh, e, Y);
             const float* wr = tp_w + (e - chunk_e0) * (long long)(P * kC) + c;
 #pragma unroll
             for (int p = 0; p < P; ++p) w[p] = __ldg(wr + p * kC);
-            tp_forward<LIN>(xs, Y, w, acc);
+            tp_forward<0>(xs, Y, w, acc);
         }
 #pragma unroll
         for (int k = 0; k < MID; ++k) out[(long long)k * kC] = acc[k];
@@ -442,27 +438,11 @@ int persistent_grid(const void* kernel, int n_atoms) {
 
 int tp_forward_launch(const TpArgs& t, cudaStream_t stream) {
     if (t.n_rows <= 0) return FMB_OK;
-#define FMB_FWD(LIN_, SP_)                                                                                             \
-    {                                                                                                                  \
-        auto kernel = k_tp_forward<LIN_, SP_>;                                                                         \
-        const int grid = persistent_grid((const void*)kernel, t.n_rows);                                                           \
-        kernel<<<grid, kC, 0, stream>>>(t.n_atoms, t.n_rows, t.chunk_e0, t.chunk_edges, t.count, t.row_ptr, t.senders, \
-                                        t.species, t.x, t.edge_sh, t.tp_w, t.mid);                                     \
-    }
-    if (t.whole_list && !t.species_x) return tp_forward_coupled_launch(t, stream);
-    if (t.species_x) {
-        FMB_REQUIRE(t.lin == 0, "tp_forward: species table only for scalar senders");
-        FMB_FWD(0, true)
-    } else if (t.lin == 0) {
-        FMB_FWD(0, false)
-    } else if (t.lin == 1) {
-        FMB_FWD(1, false)
-    } else if (t.lin == 2) {
-        FMB_FWD(2, false)
-    } else {
-        FMB_REQUIRE(false, "tp_forward: unsupported node l_max");
-    }
-#undef FMB_FWD
+    if (!t.species_x) return tp_forward_coupled_launch(t, stream);
+    FMB_REQUIRE(t.lin == 0, "tp_forward: species table only for scalar senders");
+    const int grid = persistent_grid((const void*)k_tp_forward_species, t.n_rows);
+    k_tp_forward_species<<<grid, kC, 0, stream>>>(t.n_atoms, t.n_rows, t.chunk_e0, t.chunk_edges, t.count, t.row_ptr, t.senders,
+                                                  t.species, t.x, t.edge_sh, t.tp_w, t.mid);
     FMB_LAUNCH_CHECK();
     return FMB_OK;
 }

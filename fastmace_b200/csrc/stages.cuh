@@ -17,7 +17,7 @@ struct TpArgs {
     int n_valid;           // backward: atoms [0, n_valid) have a message gradient, the others read as zero
     int fresh_from;        // backward: atoms at or beyond this start their force / virial sums from zero
     long long chunk_e0, chunk_edges, tangent_offset;
-    bool whole_list;       // the launch covers the whole edge list (one chunk): the streaming forward kernel applies
+    bool whole_list;       // the launch covers the whole edge list (one chunk)
     const long long* count;
     const int32_t* row_ptr;
     const int32_t* senders;
@@ -38,37 +38,11 @@ struct TpArgs {
 };
 int tp_forward_launch(const TpArgs& t, cudaStream_t stream);
 int tp_backward_launch(const TpArgs& t, cudaStream_t stream);
-// whole list, weights of every edge in tp_w (tp_coupled.cu)
+// senders with rows of their own (tp_coupled.cu)
 int tp_forward_coupled_launch(const TpArgs& t, cudaStream_t stream);
 
-// Tensor product of an interaction after the first with the last radial layer fused in (tp_fused.cu): no per-edge
-// weight matrix; one launch covers all rows.
-struct FusedArgs {
-    int lin;
-    int n_rows;            // receivers [0, n_rows)
-    int n_valid;           // adjoint: atoms [0, n_valid) have a message gradient, the others read as zero
-    int fresh_from;        // adjoint: atoms at or beyond this start their force / virial sums from zero
-    int first_layer_of_pass;
-    const int32_t* row_ptr;
-    const int32_t* senders;
-    const float* x;                // [atoms][(lin + 1)^2][C]
-    const float* edge_sh;
-    const float* edge_vec;
-    const float* hidden;           // [edges][64] last hidden radial layer of this interaction
-    const float* hidden_tangent;   // its derivative with respect to the edge length (adjoint)
-    const float* image;            // fmb_layer_t.rad_img
-    float* mid;                    // forward output
-    const float* d_mid;            // adjoint input
-    float* d_x;
-    float* force_acc;
-    float* atom_virial;
-    uint32_t* error_word;
-};
-// FMB_ERR_UNSUPPORTED when the fused kernels do not apply (no weight image, lin outside 1..2)
-int tp_fused_forward(const FusedArgs& f, cudaStream_t stream);
-
-// Per-edge radial weights (or their d/dr) [rows][n_paths * 128] = hidden [rows][64] x last radial layer, through the
-// fused kernels' tensor-core pipeline (tp_fused.cu); FMB_ERR_UNSUPPORTED without the weight image.
+// Per-edge radial weights (or their d/dr) [rows][n_paths * 128] = hidden [rows][64] x last radial layer on the
+// tensor cores (radial_weights.cu); FMB_ERR_UNSUPPORTED without the weight image.
 // `row_index` (or null): output row r is computed from hidden row row_index[r]
 int radial_weights_tc(const float* hidden, const float* image, float* out, int rows, int n_paths, const long long* limit,
                       long long limit_offset, const int32_t* row_index, uint32_t* error_word, int max_ctas,
@@ -112,10 +86,10 @@ struct EdgeAdjointArgs {
     const float* tp_w;             // [chunk edges][paths * C] values, d/dr behind them at tangent_offset
     long long tangent_offset;
     const float* d_mid;
-    float* dxe;                    // [edges][(lin + 1)^2][C]
+    float* dxe;                    // [edges from dx_e0 on][(lin + 1)^2][C]
+    long long dx_e0;
     float* qe;                     // [edges][4]
     float* d_x;                    // [n_rows][(lin + 1)^2][C]
-    bool whole_list;               // the launch covers the whole edge list (tp_w holds every edge's weights)
     uint32_t* error_word;
     const int32_t* slot;           // or null: the weights of edge e are row slot[min(e, mirror[e])] of tp_w
 };
@@ -125,9 +99,10 @@ int mirror_map(const fmb_nl_t* nl, int32_t* mirror, uint32_t* status, const long
 // per-edge adjoint of an interaction after the first for one chunk of edges; after the last chunk the gather of the
 // sender-side gradients into d_x
 int tp_adjoint_edges(const EdgeAdjointArgs& t, cudaStream_t stream);
-// its form for a whole list of which every row carries a gradient (tp_coupled.cu)
+// its form where every row carries a gradient (tp_coupled.cu)
 int tp_adjoint_coupled_launch(const EdgeAdjointArgs& t, cudaStream_t stream);
-int gather_sender_gradient(const EdgeAdjointArgs& t, cudaStream_t stream);
+// over the mirror edges [first, first + count) only; `add`: onto d_x as it is
+int gather_sender_gradient(const EdgeAdjointArgs& t, long long first, long long count, bool add, cudaStream_t stream);
 // first interaction: adds its edge-vector gradients to qe (rows below n_add) or stores them
 int first_adjoint_edges(const FirstArgs& f, int n_add, float* qe, cudaStream_t stream);
 // forces (as gradients) and per-atom virials from the per-edge gradients; only the edges into atoms [0, n_valid) carry

@@ -1,5 +1,5 @@
-// Channelwise tensor product of the interactions after the first over a whole edge list whose radial weights are in
-// memory, forward and per-edge adjoint: every per-edge operand streamed through shared memory, two channels per thread on
+// Channelwise tensor product of the interactions after the first over a range of edges (the whole list, or a chunk of one
+// too long for its radial weights to be held) whose radial weights are in memory, forward and per-edge adjoint: every per-edge operand streamed through shared memory, two channels per thread on
 // the packed FP32 pipe (fma.rn.f32x2), the harmonics coupled once per edge.
 //
 // An edge's harmonics enter every channel in the same few combinations, T[path][m_out][m_in] = sum_me C Y[me]. The
@@ -50,14 +50,16 @@ struct Ahead {
     const float* edge_sh;
     const int32_t* senders;
     const int32_t* slot;
+    long long w0;                              // the edge whose weights are row 0 of tp_w
     long long eb, ee;
     int c, sync_id;
     volatile int* abort_flag;
 
     __device__ __forceinline__ Ahead(float* memory, uint32_t bar_, const float* edge_sh_, const int32_t* senders_,
-                                     const int32_t* slot_, long long eb_, long long ee_, int c_, int sync_id_, volatile int* abort_)
+                                     const int32_t* slot_, long long w0_, long long eb_, long long ee_, int c_, int sync_id_,
+                                     volatile int* abort_)
         : t(memory), y(memory + 2 * BATCH * kT), index(reinterpret_cast<int32_t*>(memory + 2 * BATCH * (kT + 16))), bar(bar_),
-          edge_sh(edge_sh_), senders(senders_), slot(slot_), eb(eb_), ee(ee_), c(c_), sync_id(sync_id_), abort_flag(abort_) {}
+          edge_sh(edge_sh_), senders(senders_), slot(slot_), w0(w0_), eb(eb_), ee(ee_), c(c_), sync_id(sync_id_), abort_flag(abort_) {}
 
     // thread c < BATCH: the indices of its edge of batch b
     __device__ __forceinline__ void look_up(int b) const {
@@ -75,7 +77,7 @@ struct Ahead {
     // the row of tp_w that holds an edge's weights: its own, or with one row per pair of opposite edges the pair's
     __device__ __forceinline__ long long weight_row(long long e) const {
         const int k = (int)(e - eb);
-        return slot ? (long long)index[((k / BATCH) & 3) * 2 * BATCH + BATCH + k % BATCH] : e;
+        return slot ? (long long)index[((k / BATCH) & 3) * 2 * BATCH + BATCH + k % BATCH] : e - w0;
     }
 
     __device__ __forceinline__ void request(int b) const {
@@ -146,24 +148,64 @@ struct Rows {
     }
 };
 
+// The receivers of the edges [e0, e1) of `total`: those whose row starts in the range (rows without edges among them, the
+// trailing ones with the last range) and the one that straddles its beginning.
+__device__ __forceinline__ void rows_of_range(const int32_t* __restrict__ row_ptr, int n_rows, long long e0, long long e1,
+                                              long long total, int& first, int& last) {
+    first = 0;
+    last = n_rows;
+    if (e0 > 0) {
+        int lo = 0, hi = n_rows;
+        while (lo < hi) {
+            const int at = (lo + hi) >> 1;
+            if (row_ptr[at + 1] > e0 || row_ptr[at] >= e0) hi = at; else lo = at + 1;
+        }
+        first = lo;
+    }
+    if (e1 < total) {
+        int lo = first, hi = n_rows;
+        while (lo < hi) {
+            const int at = (lo + hi) >> 1;
+            if (row_ptr[at] >= e1) hi = at; else lo = at + 1;
+        }
+        last = lo;
+    }
+}
+
 template <int LIN, int STAGES, int BATCH>
 constexpr int forward_group_floats() { return STAGES * Rows<LIN, STAGES, false>::kStage + Ahead<LIN, BATCH>::kFloats; }
 
 // GROUPS = 1: a CTA owns a contiguous block of receivers. GROUPS > 1 (few receivers): a CTA owns one, its groups take
 // runs of the row's edges and meet in shared memory at the end.
-template <int LIN, int STAGES, int BATCH, int GROUPS, int MINB>
+// RANGE: the launch covers [e0, e0 + e_span) of a list evaluated in chunks, else all of it (the extra state of a range
+// costs the 128-register form 9 %).
+template <int LIN, int STAGES, int BATCH, int GROUPS, int MINB, bool RANGE>
 __global__ void __launch_bounds__(kGroup * GROUPS, MINB)
 k_tp_forward_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ senders,
                      const float* __restrict__ x, const float* __restrict__ edge_sh, const float* __restrict__ tp_w,
-                     float* __restrict__ mid, uint32_t* __restrict__ error_word, const int32_t* __restrict__ slot) {
+                     float* __restrict__ mid, uint32_t* __restrict__ error_word, const int32_t* __restrict__ slot,
+                     long long e0, long long e_span) {
     constexpr int MID = TpShape<LIN>::kMidDim;
     extern __shared__ __align__(128) float smem[];
     __shared__ uint64_t bars[GROUPS * (2 * STAGES + 2)];
     __shared__ int abort_sh;
     const int group = threadIdx.x / kGroup, c = threadIdx.x % kGroup, lane = c & 31;
-    const int r0 = (int)((long long)blockIdx.x * n_rows / gridDim.x), r1 = (int)((long long)(blockIdx.x + 1) * n_rows / gridDim.x);
+    int first = 0, last = n_rows;
+    long long e1 = 0;
+    if (RANGE) {
+        const long long total = row_ptr[n_rows];
+        e1 = min(total, e0 + e_span);
+        if (e0 > 0 && e0 >= total) return;
+        rows_of_range(row_ptr, n_rows, e0, e1, total, first, last);
+    }
+    const int r0 = first + (int)((long long)blockIdx.x * (last - first) / gridDim.x),
+              r1 = first + (int)((long long)(blockIdx.x + 1) * (last - first) / gridDim.x);
     if (r0 >= r1) return;
     long long eb = row_ptr[r0], ee = row_ptr[r1];
+    if (RANGE) {
+        eb = max(eb, e0);
+        ee = min(ee, e1);
+    }
     if (GROUPS > 1) {
         const long long len = ee - eb;
         ee = eb + len * (group + 1) / GROUPS;
@@ -183,7 +225,7 @@ k_tp_forward_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
     __syncthreads();
     float* const own = smem + group * forward_group_floats<LIN, STAGES, BATCH>();
     float* const tail = own + STAGES * Rows<LIN, STAGES, false>::kStage;
-    const Ahead<LIN, BATCH> ahead(tail, bar + 8 * (2 * STAGES), edge_sh, senders, slot, eb, ee, c, 1 + group, &abort_sh);
+    const Ahead<LIN, BATCH> ahead(tail, bar + 8 * (2 * STAGES), edge_sh, senders, slot, RANGE ? e0 : 0, eb, ee, c, 1 + group, &abort_sh);
     Rows<LIN, STAGES, false> rows{own, bar, tp_w, 0, x, ee, eb, &abort_sh};
     ahead.start();
     if (c == 0)
@@ -193,10 +235,13 @@ k_tp_forward_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
     uint32_t parity = 0;
     long long e = eb;
     for (int i = r0; i < r1; ++i) {
-        const long long re = GROUPS > 1 ? ee : (long long)row_ptr[i + 1];
+        long long re = GROUPS > 1 ? ee : (long long)row_ptr[i + 1];
+        if (RANGE) re = min(re, e1);
+        float2* const out = reinterpret_cast<float2*>(mid + ((long long)i * MID) * kC) + c;
+        const bool begun = RANGE && row_ptr[i] < e0;                  // the range before holds the row's first edges
         float2 acc[MID];
 #pragma unroll
-        for (int k = 0; k < MID; ++k) acc[k] = make_float2(0.0f, 0.0f);
+        for (int k = 0; k < MID; ++k) acc[k] = begun ? out[(long long)k * (kC / 2)] : make_float2(0.0f, 0.0f);
 #pragma unroll 1
         for (; e < re; ++e) {
             if (el == BATCH) {
@@ -214,7 +259,6 @@ k_tp_forward_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
             ++el;
         }
         if (GROUPS == 1) {
-            float2* out = reinterpret_cast<float2*>(mid + ((long long)i * MID) * kC) + c;
 #pragma unroll
             for (int k = 0; k < MID; ++k) out[(long long)k * (kC / 2)] = acc[k];
         } else {
@@ -226,7 +270,6 @@ k_tp_forward_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
             }
             __syncthreads();
             if (group == 0) {
-                float2* out = reinterpret_cast<float2*>(mid + ((long long)i * MID) * kC) + c;
 #pragma unroll
                 for (int k = 0; k < MID; ++k) {
                     float2 v = acc[k];
@@ -257,7 +300,7 @@ k_tp_adjoint_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
                      const float* __restrict__ x, const float* __restrict__ edge_sh, const float* __restrict__ edge_vec,
                      const float* __restrict__ tp_w, long long tangent_offset, const float* __restrict__ d_mid,
                      float* __restrict__ dxe, float4* __restrict__ qe, uint32_t* __restrict__ error_word,
-                     const int32_t* __restrict__ slot) {
+                     const int32_t* __restrict__ slot, long long e0, long long e_span, long long dx0) {
     constexpr int IN = TpShape<LIN>::kInDim, MID = TpShape<LIN>::kMidDim;
     using RowsT = Rows<LIN, STAGES, true>;
     extern __shared__ __align__(128) float smem[];
@@ -265,9 +308,10 @@ k_tp_adjoint_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
     __shared__ int abort_sh, first_row_sh;
     __shared__ float red[2][BATCH][2][18];
     const int c = threadIdx.x, warp = c >> 5, lane = c & 31;
-    const long long total = row_ptr[n_rows];
-    const long long per_cta = (total + gridDim.x - 1) / gridDim.x;
-    const long long eb = (long long)blockIdx.x * per_cta, ee = min(total, eb + per_cta);
+    const long long e1 = min((long long)row_ptr[n_rows], e0 + e_span);
+    if (e0 >= e1) return;
+    const long long per_cta = (e1 - e0 + gridDim.x - 1) / gridDim.x;
+    const long long eb = e0 + (long long)blockIdx.x * per_cta, ee = min(e1, eb + per_cta);
     if (eb >= ee) return;
     const uint32_t bar = tc::smem_u32(bars);
     if (c == 0) {
@@ -282,7 +326,7 @@ k_tp_adjoint_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
     }
     __syncthreads();
     float* const tail = smem + STAGES * RowsT::kStage;
-    const Ahead<LIN, BATCH> ahead(tail, bar + 8 * (2 * STAGES), edge_sh, senders, slot, eb, ee, c, 1, &abort_sh);
+    const Ahead<LIN, BATCH> ahead(tail, bar + 8 * (2 * STAGES), edge_sh, senders, slot, e0, eb, ee, c, 1, &abort_sh);
     RowsT rows{smem, bar, tp_w, tangent_offset, x, ee, eb, &abort_sh};
     ahead.start();
     if (c == 0) {
@@ -342,7 +386,7 @@ k_tp_adjoint_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
         if (lane == 0) tc::mbar_arrive(bar + 8 * (STAGES + stage));
         if (++stage == STAGES) { stage = 0; parity ^= 1u; }
 #pragma unroll
-        for (int q = 0; q < IN; ++q) reinterpret_cast<float2*>(dxe + (e * IN + q) * kC)[c] = dx[q];
+        for (int q = 0; q < IN; ++q) reinterpret_cast<float2*>(dxe + ((e - dx0) * IN + q) * kC)[c] = dx[q];
         // 16 + 1 sums over the channels: transpose-reduce inside the warp, the two warps meet in shared memory
         float dY[16];
 #pragma unroll
@@ -376,15 +420,15 @@ int resident(const void* kernel, int threads, int smem) {
     return per_sm * sms;
 }
 
-template <int LIN, int STAGES, int BATCH, int GROUPS, int MINB>
+template <int LIN, int STAGES, int BATCH, int GROUPS, int MINB, bool RANGE = false>
 int launch_forward(const TpArgs& t, cudaStream_t stream) {
     constexpr int smem = GROUPS * forward_group_floats<LIN, STAGES, BATCH>() * 4;
-    auto kernel = k_tp_forward_coupled<LIN, STAGES, BATCH, GROUPS, MINB>;
+    auto kernel = k_tp_forward_coupled<LIN, STAGES, BATCH, GROUPS, MINB, RANGE>;
     FMB_CUDA_CHECK(opt_in_shared_memory((const void*)kernel, smem));
     static const int cap = resident((const void*)kernel, kGroup * GROUPS, smem);
     const int grid = GROUPS > 1 || t.n_rows < cap ? t.n_rows : cap;
     kernel<<<grid, kGroup * GROUPS, smem, stream>>>(t.n_rows, t.row_ptr, t.senders, t.x, t.edge_sh, t.tp_w, t.mid, t.error_word,
-                                                    t.slot);
+                                                    t.slot, t.chunk_e0, t.chunk_edges);
     FMB_LAUNCH_CHECK();
     return FMB_OK;
 }
@@ -396,7 +440,8 @@ int launch_adjoint(const EdgeAdjointArgs& t, cudaStream_t stream) {
     FMB_CUDA_CHECK(opt_in_shared_memory((const void*)kernel, smem));
     static const int cap = resident((const void*)kernel, kGroup, smem);
     kernel<<<cap, kGroup, smem, stream>>>(t.n_rows, t.row_ptr, t.senders, t.x, t.edge_sh, t.edge_vec, t.tp_w, t.tangent_offset,
-                                          t.d_mid, t.dxe, reinterpret_cast<float4*>(t.qe), t.error_word, t.slot);
+                                          t.d_mid, t.dxe, reinterpret_cast<float4*>(t.qe), t.error_word, t.slot, t.chunk_e0,
+                                          t.chunk_edges, t.dx_e0);
     FMB_LAUNCH_CHECK();
     return FMB_OK;
 }
@@ -411,6 +456,11 @@ int tp_forward_coupled_launch(const TpArgs& t, cudaStream_t stream) {
     // otherwise the shape (stages, batch, CTAs per SM) measured best: warps in flight count for more than stages. l_max 1,
     // 62 k edges: 75 us at 3 / 8 / 8, 86 at 3 / 16 / 6, 91 at 4 / 8 / 6; l_max 2, 748 k edges: 1.41 ms at 3 / 8 / 3, 1.46 at
     // 2 / 8 / 4, 1.70 at 3 / 4 / 4
+    if (!t.whole_list) {
+        if (t.lin == 0) return launch_forward<0, 6, 16, 1, 8, true>(t, stream);
+        if (t.lin == 1) return launch_forward<1, 3, 8, 1, 7, true>(t, stream);
+        if (t.lin == 2) return launch_forward<2, 3, 8, 1, 3, true>(t, stream);
+    }
     if (t.lin == 0) return few ? launch_forward<0, 4, 16, 4, 1>(t, stream) : launch_forward<0, 6, 16, 1, 8>(t, stream);
     if (t.lin == 1) return few ? launch_forward<1, 4, 16, 4, 1>(t, stream) : launch_forward<1, 3, 8, 1, 8>(t, stream);
     if (t.lin == 2) return few ? launch_forward<2, 3, 8, 2, 1>(t, stream) : launch_forward<2, 3, 8, 1, 3>(t, stream);

@@ -78,9 +78,9 @@ class B200ForceField:
         # and the adjoint, streamed kernels) whenever its buffers fit in the free device memory, else chunks of
         # DEFAULT_CHUNK_EDGES with the weights recomputed per chunk; a number sets the chunk size by hand
         self.chunk_edges = None if chunk_edges is None else int(chunk_edges)
-        # ``edge_adjoint``: None = the per-edge hand-over adjoint whenever its buffers fit in the free device memory,
-        # else the mirror evaluation; False = the mirror evaluation regardless (the path of lists too large for the
-        # buffers, selectable so that tests reach it on small cells); True = refuse to fall back
+        # ``edge_adjoint``: None = the per-edge hand-over adjoint with buffers for the whole list whenever they fit in the
+        # free device memory, else a chunk at a time; False = a chunk at a time regardless (the path of lists too large
+        # for the buffers, selectable so that tests reach it on small cells); True = refuse to fall back
         self.edge_adjoint = edge_adjoint
         self.num_edges = 0
         self.calls = 0
@@ -242,7 +242,7 @@ class B200ForceField:
             "partial": torch.zeros(1024 * 8, dtype=torch.float64, device=dev),
         }
         # per-edge hand-over buffers of the adjoint (2 KB per edge for the medium model): when they fit in the memory
-        # that is free now with a tenth of the device kept back, else the mirror-evaluation kernels run
+        # that is free now with a tenth of the device kept back; else the sender gradients of one chunk at a time
         free, total = torch.cuda.mem_get_info(dev)
         free += torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)   # blocks torch holds but does not use
         need = cap * (hid * c * 4 + 20)
@@ -250,6 +250,7 @@ class B200ForceField:
         if (self.halo_exchange or self.edge_adjoint) and not self.edge_local:
             raise _lib.Fmb200Error(f"halo-exchange mode needs {need / 2 ** 30:.1f} GiB for the per-edge hand-over "
                                    f"buffers, {max(0, free - total // 10) / 2 ** 30:.1f} GiB are free: use more ranks")
+        dx_edges = 0
         if self.edge_local:
             try:
                 buf["mirror"] = torch.zeros(cap, dtype=torch.int32, device=dev)
@@ -259,7 +260,7 @@ class B200ForceField:
                 buf["canon_list"] = torch.zeros(cap, dtype=torch.int32, device=dev)
                 buf["canon_count"] = torch.zeros(1, dtype=torch.int64, device=dev)
             except torch.OutOfMemoryError:
-                # the free memory was there but not in one piece: run the mirror-evaluation adjoint instead
+                # the free memory was there but not in one piece
                 for name in ("mirror", "edge_q", "edge_dx", "edge_slot", "canon_list", "canon_count"):
                     buf.pop(name, None)
                 torch.cuda.empty_cache()
@@ -271,10 +272,21 @@ class B200ForceField:
                     torch.cuda.empty_cache()
                     self._chunked_only = True
                     return self._allocate_work()
+        if not self.edge_local:
+            try:
+                buf["mirror"] = torch.zeros(cap, dtype=torch.int32, device=dev)
+                buf["edge_q"] = torch.zeros(cap, 4, **f32)
+                buf["edge_dx"] = torch.zeros(chunk, hid, c, **f32)
+                dx_edges = chunk
+            except torch.OutOfMemoryError:
+                # not even those: the kernels that evaluate every edge from both ends
+                for name in ("mirror", "edge_q", "edge_dx"):
+                    buf.pop(name, None)
+                torch.cuda.empty_cache()
         self.buf = buf
         w = _lib.WorkStruct()
         w.edge_capacity, w.chunk_edges, w.compute_stress = cap, chunk, int(self._compute_stress)
-        w.pair_capacity = pair_capacity
+        w.pair_capacity, w.dx_edges = pair_capacity, dx_edges
         for name, tensor in buf.items():
             setattr(w, name, tensor.data_ptr())
         w.energy, w.forces, w.stress = self.energy.data_ptr(), self._forces_all.data_ptr(), self.stress.data_ptr()

@@ -241,7 +241,7 @@ typedef struct {
     /* Optional, with the three above: an edge and its opposite edge have the same length, hence the same radial
      * weights, so the last interaction's weights are produced once per pair. canon_list [edge_capacity] int32 lists the
      * edges that stand for their pair (the lower index of the two), canon_count [1] int64 their number, edge_slot
-     * [edge_capacity] int32 holds, for a listed edge, its row in tp_w. Written by fmb_edge_features every call. Null =
+     * [edge_capacity] int32 holds, for both edges of a pair, its row in tp_w. Written by fmb_edge_features every call. Null =
      * one row of tp_w per edge. */
     int32_t* edge_slot;
     int32_t* canon_list;
@@ -262,7 +262,9 @@ typedef struct {
      * opposite edges (a little over edge_capacity / 2) instead of chunk_edges rows; 0 = chunk_edges rows. A list with
      * more pairs than that raises FMB_STATUS_PAIR_OVERFLOW and the rows beyond are not produced. */
     int32_t pair_capacity;
-    int32_t pad_;
+    /* Edges edge_dx holds: 0 = edge_capacity, else at least chunk_edges -- the sender gradients of one chunk at a time,
+     * collected behind each chunk (a list too long for those of all its edges). */
+    int32_t dx_edges;
 } fmb_work_t;
 
 /* MACEForceField.__call__ (fastmace/model/forces.py:1127-1136,1220-1240): energy (float64), forces and stress of the
