@@ -318,7 +318,7 @@ def time_single_gpu_cell(w, spec, weights, structure, device, steps: int, warmup
     stop.synchronize()
     ms = start.elapsed_time(stop) / steps
     note = (f"{steps} steps after {warmup}: plain periodic force field, checked engine, "
-            f"{'per-edge hand-over' if ff.edge_local else 'mirror-evaluation'} adjoint, "
+            f"{'per-edge hand-over' if ff.edge_local else 'chunk-wise hand-over'} adjoint, "
             f"{int(ff.edge_count.item())} edges")
     del engine, integrator, state, ff
     torch.cuda.empty_cache()

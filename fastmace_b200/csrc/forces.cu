@@ -196,7 +196,7 @@ int radial_weights(const Ctx& c, int layer, long long e0, int first, int last, c
     if (!stream) stream = c.stream;
     StageScope scope(stream, kStRadial);
     if (L.rad_img && tensor_cores_enabled()) {
-        // the fused kernels' tensor-core pipeline as a plain producer (one launch per matrix)
+        // on the tensor cores, one launch per matrix
         const bool pairs = layer == c.m->n_layers - 1 && pair_rows(c);
         if (pairs) limit = c.w->canon_count;              // the listed edges, one row each
         bool done = true;

@@ -78,7 +78,7 @@ def tensor_core_image(blocks) -> torch.Tensor:
 
 
 def radial_image(w4: torch.Tensor, channels: int = 128) -> torch.Tensor:
-    """The last radial layer [64][paths * channels] (fp32, already scaled) as the fused tensor-product kernels stream it:
+    """The last radial layer [64][paths * channels] (fp32, already scaled) as the radial-weight producer streams it:
     per path p, K half h and part (0 = tf32 remainder, 1 = tf32 value) one 16 KB tile [128 channels][32 features] of the
     transposed block in the K-major operand layout with 128-byte swizzle (8-row groups of 1024 bytes, the 16-byte
     chunk index XORed with row mod 8), at float offset ((p * 2 + h) * 2 + part) * 4096."""
