@@ -160,35 +160,51 @@ def radial_hidden_float64(w0, w1, w2, r: torch.Tensor, r_cut: float, with_tangen
     return value, tangent
 
 
+def _table_is_accurate(table, per: int, function, r_cut: float) -> bool:
+    """Is a table off by at most 2e-7 (value) and 4e-7 (d/dr) of the largest magnitude its function takes within the same
+    quarter of an Å (counted from the cutoff)? Checked between the nodes and at both ends of every interval, where d/dr is
+    worst. The features of a pair that nearly touches are a hundred times those of a bond and ten thousand times those
+    near the cutoff: one bound for all lengths would let errors of 1e-5 and more pass where a crystal has its neighbours."""
+    n = len(table)
+    ends, inner = torch.arange(n + 1, dtype=torch.float64) / per, (torch.arange(n, dtype=torch.float64) + 0.75) / per
+    r = torch.cat([ends, inner])
+    inside = r < r_cut                                              # nothing is looked up at the cutoff or beyond
+    windows = max(int(r_cut / 0.25), 1)                             # the one at zero holds the remainder
+    window = ((r_cut - r) / 0.25).long().clamp(0, windows - 1)
+    value, tangent = function(r)
+    largest = [torch.zeros(windows, dtype=torch.float64).scatter_reduce(0, window, f.abs().amax(1) * inside, "amax")
+               for f in (value, tangent)]
+    c = table.double()
+    for u, at in ((-1.0, slice(0, n)), (1.0, slice(1, n + 1)), (0.5, slice(n + 1, 2 * n + 1))):
+        powers = torch.tensor([u ** k for k in range(c.shape[1])], dtype=torch.float64)
+        slopes = torch.tensor([k * u ** max(k - 1, 0) for k in range(c.shape[1])], dtype=torch.float64) * (2 * per)
+        for weights, exact, bound, top in ((powers, value, 2e-7, largest[0]), (slopes, tangent, 4e-7, largest[1])):
+            error = (torch.einsum("k,nkf->nf", weights, c) - exact[at]).abs().amax(1) * inside[at]
+            if not bool((error <= bound * top[window[at]]).all()):
+                return False
+    return True
+
+
 def radial_table(w0, w1, w2, r_cut: float):
     """The hidden radial features as piecewise polynomials of the length: (coefficients [intervals, 6, 64] fp32,
     intervals per Å), or None where 512 intervals per Å are not enough.
 
     The features of an edge depend on its length only, through a smooth function fixed by the weights. Polynomials of
     degree 5 through the Chebyshev nodes of intervals of 1/32 Å reproduce it below fp32 rounding for the benchmark's
-    models (4e-8 of the norm in the value and 5e-8 in d/dr, rounding of the coefficients included; the 3xTF32 chain of
-    three layers they replace is off by 3e-7 to 1e-6). The interval is halved until value and d/dr, checked between the
-    nodes, are within 2e-7 and 4e-7 of their largest magnitude, so a model with a steeper radial function gets a finer
-    table and one that no table serves keeps the MLP kernel."""
+    models (5e-8 of the local magnitude in value and d/dr from 1 Å on, 3e-7 in d/dr below, rounding of the coefficients
+    included; the 3xTF32 chain of three layers they replace is off by 3e-7 to 1e-6). The interval is halved until the
+    table is accurate at every length, so a model with a steeper radial function gets a finer table and one that no table
+    serves keeps the MLP kernel."""
     n_c = RADIAL_DEGREE + 1
     w0, w1, w2 = (w.cpu() for w in (w0, w1, w2))
     nodes = torch.cos(math.pi * (torch.arange(n_c, dtype=torch.float64) + 0.5) / n_c)
     fit = torch.linalg.inv(torch.stack([nodes ** k for k in range(n_c)], dim=1))
-    probes = torch.tensor([-1.0, 0.5], dtype=torch.float64)        # d/dr is worst at the ends
-    powers = torch.stack([probes ** k for k in range(n_c)], dim=1)
-    slopes = torch.stack([k * probes ** max(k - 1, 0) for k in range(n_c)], dim=1)
     for per in (32, 64, 128, 256, 512):
         n = int(math.ceil(r_cut * per))
         middle = (torch.arange(n, dtype=torch.float64)[:, None] + 0.5) / per
         at_nodes = radial_hidden_float64(w0, w1, w2, (middle + nodes / (2 * per)).reshape(-1), r_cut, False)[0]
         table = (fit @ at_nodes.reshape(n, n_c, -1)).to(torch.float32)
-        r = (middle + probes / (2 * per)).reshape(-1)
-        value, tangent = radial_hidden_float64(w0, w1, w2, r, r_cut)
-        inside = (r < r_cut)[:, None]
-        got = (powers @ table.double()).reshape(value.shape)
-        d_got = (slopes @ table.double()).reshape(value.shape) * (2 * per)
-        if bool((((got - value) * inside).abs().max() <= 2e-7 * value.abs().max())
-                & (((d_got - tangent) * inside).abs().max() <= 4e-7 * tangent.abs().max())):
+        if _table_is_accurate(table, per, lambda r: radial_hidden_float64(w0, w1, w2, r, r_cut), r_cut):
             return table.contiguous(), per
     return None
 
