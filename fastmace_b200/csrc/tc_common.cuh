@@ -47,14 +47,14 @@ __device__ __forceinline__ float tf32_rna(float x) {
     return __uint_as_float(r);
 }
 
-// v = hi + lo with both parts representable in tf32 (hi rounds half away from zero, lo to nearest): six full-rate
-// instructions, where cvt.rna.tf32 runs at an eighth of the rate (splitting a 128 x 32 operand chunk with eight warps
-// took 1,000 cycles by conversions, 330 like this). A value that is not finite leaves lo not a number.
+// v = hi + lo with both parts representable in tf32, each rounded half away from zero as cvt.rna.tf32 does: six full-rate
+// instructions, where the conversion runs at an eighth of the rate (splitting a 128 x 32 operand chunk with eight warps
+// took 1,000 cycles by conversions, 330 like this). Good to the end of the fp32 range. A value that is not finite leaves
+// lo not a number: the carry can turn a NaN's bits into a zero, the product with zero brings it back.
 __device__ __forceinline__ void split_tf32(float v, float& hi, float& lo) {
     hi = __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u);
     const float rest = v - hi;
-    const float scaled = rest * 8193.0f;                    // 2^13 + 1: keeps the upper 11 of 24 significant bits
-    lo = __fsub_rn(scaled, __fsub_rn(scaled, rest));
+    lo = fmaf(0.0f, rest, __uint_as_float((__float_as_uint(rest) + 0x1000u) & 0xffffe000u));
 }
 
 __device__ __forceinline__ void split_tf32(const float4& v, float4& hi, float4& lo) {

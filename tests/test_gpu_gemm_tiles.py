@@ -35,3 +35,21 @@ def test_gemm_tiles(m, n, k):
         assert ((c[:m][keep].double() - ref).abs() <= (k / 8 + 8) * 2 ** -23 * size + 1e-30).all()
         assert c[bad].isnan().all() and (c[m:] == 7.0).all()
     assert int(status.item()) == 0
+
+
+@pytest.mark.parametrize("m", [77, 40000])
+def test_operands_up_to_the_end_of_fp32(m):
+    """Activations of 1e38 to 3e38 with a product that fits: every step of the split stays finite. Bound: 3xTF32 of sums
+    of one sign, K = 128."""
+    from fastmace_b200 import _lib
+    from fastmace_b200.packing import tensor_core_image
+    g = torch.Generator().manual_seed(m)
+    a = ((1 + 2 * torch.rand(m, 128, generator=g)) * 1e38).cuda()
+    b = ((0.5 + torch.rand(128, 128, generator=g)) * 1e-3).cuda()
+    image = tensor_core_image([b.cpu()]).cuda()
+    c, status = torch.zeros(m, 128, device="cuda"), torch.zeros((), dtype=torch.int32, device="cuda")
+    _lib.check(_lib.load().fmb_gemm(a.data_ptr(), b.data_ptr(), image.data_ptr(), None, c.data_ptr(), m, 128, 128, 0, 2,
+                                    status.data_ptr(), _lib.current_stream()), "gemm")
+    want = a.double() @ b.double()
+    assert bool(torch.isfinite(c).all()) and int(status) == 0
+    assert float(((c.double() - want) / want).abs().max()) <= 2e-6
