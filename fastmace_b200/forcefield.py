@@ -192,6 +192,9 @@ class B200ForceField:
         c = spec.channels
         max_paths = max(len(spec.paths(t)) for t in range(spec.num_interactions))
         hid = (spec.hidden_lmax + 1) ** 2
+        max_mid = max(self.packed.struct.layer[t].mid_dim for t in range(spec.num_interactions))
+        # the reassociated first layer keeps its per-species outer-product sums [16][n_species][64] in `mid` / `d_mid`
+        mid_floats = max(max_mid * c, 16 * len(self.packed.species_z) * 64)
         pair_capacity = 0
         if self.chunk_edges is not None:
             chunk = min(self.chunk_edges, cap)
@@ -202,24 +205,24 @@ class B200ForceField:
         else:
             # what this function allocates per edge with the whole list as one chunk: vector, harmonics, hidden
             # features, hand-over buffers with the pair map -- and the weights with their d/dr, one row per edge or,
-            # where the kernels that read one row per pair of opposite edges apply, a little over half a row
-            free, _ = torch.cuda.mem_get_info(dev)
+            # where the kernels that read one row per pair of opposite edges apply, a little over half a row. Those rows
+            # need the hand-over buffers, which are given up where they would cut into a tenth of the device (below), so
+            # that tenth and the per-atom buffers are counted
+            free, total = torch.cuda.mem_get_info(dev)
             free += torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
             others = 16 + 64 + spec.num_interactions * 2 * 64 * 4 + hid * c * 4 + 28
             row = 2 * max_paths * c * 4
+            atoms = 4 * n * (2 * mid_floats + (6 * hid + 1 + 16 * (spec.num_interactions + 1)) * c + 10)
             layers = self.packed.struct.layer
             pair_rows = (self.edge_adjoint is not False and spec.num_interactions == 2
                          and bool(layers[1].rad_img) and bool(layers[0].first[0]))
             pairs = cap // 2 + cap // 16
-            if pair_rows and cap * others + pairs * row <= 0.85 * free:
+            if pair_rows and cap * others + pairs * row <= min(0.85 * free, free - total // 10 - atoms):
                 chunk, pair_capacity = cap, pairs
             elif cap * (others + row) <= 0.85 * free:
                 chunk = cap
             else:
                 chunk = DEFAULT_CHUNK_EDGES
-        max_mid = max(self.packed.struct.layer[t].mid_dim for t in range(spec.num_interactions))
-        # the reassociated first layer keeps its per-species outer-product sums [16][n_species][64] in `mid` / `d_mid`
-        mid_floats = max(max_mid * c, 16 * len(self.packed.species_z) * 64)
         f32 = dict(dtype=torch.float32, device=dev)
         buf = {
             "edge_vec": torch.zeros(cap, 4, **f32),
@@ -247,6 +250,16 @@ class B200ForceField:
         free += torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)   # blocks torch holds but does not use
         need = cap * (hid * c * 4 + 20)
         self.edge_local = need <= free - total // 10 and self.edge_adjoint is not False
+
+        def in_chunks():
+            # the weight buffer was sized for the pair map, which cannot be had: size everything again, in chunks
+            buf.clear()
+            torch.cuda.empty_cache()
+            self._chunked_only = True
+            return self._allocate_work()
+
+        if pair_capacity and not self.edge_local:
+            return in_chunks()
         if (self.halo_exchange or self.edge_adjoint) and not self.edge_local:
             raise _lib.Fmb200Error(f"halo-exchange mode needs {need / 2 ** 30:.1f} GiB for the per-edge hand-over "
                                    f"buffers, {max(0, free - total // 10) / 2 ** 30:.1f} GiB are free: use more ranks")
@@ -266,12 +279,7 @@ class B200ForceField:
                 torch.cuda.empty_cache()
                 self.edge_local = False
                 if pair_capacity:
-                    # the weight buffer was sized for the pair map that now does not exist: size everything again,
-                    # in chunks
-                    del buf
-                    torch.cuda.empty_cache()
-                    self._chunked_only = True
-                    return self._allocate_work()
+                    return in_chunks()
         if not self.edge_local:
             try:
                 buf["mirror"] = torch.zeros(cap, dtype=torch.int32, device=dev)
