@@ -159,6 +159,8 @@ class B200ForceField:
                                             dtype=torch.int32, device=self._device)
             self.neighbours.set_atom_capacity(self.atom_capacity)
             self._outputs()
+            moved = True
+        if moved or (self.work is not None and self.work.pair_capacity and not self._same_rows()):
             self.work, self.buf = None, None
             moved = True
         self._upload_atoms()
@@ -166,6 +168,12 @@ class B200ForceField:
         if self.work is not None:
             self._fill_counts(self.work)
         return moved
+
+    def _same_rows(self) -> bool:
+        """Both interactions are evaluated for the same atoms (all of them, or the owned ones), so that the adjoint can use
+        the radial weights of the forward pass."""
+        owned, inner = (k if k >= 0 else self.natoms for k in (self.n_owned, self.n_inner))
+        return owned == inner
 
     def _fill_counts(self, w) -> None:
         w.n_atoms = self.natoms
@@ -214,7 +222,7 @@ class B200ForceField:
             row = 2 * max_paths * c * 4
             atoms = 4 * n * (2 * mid_floats + (6 * hid + 1 + 16 * (spec.num_interactions + 1)) * c + 10)
             layers = self.packed.struct.layer
-            pair_rows = (self.edge_adjoint is not False and spec.num_interactions == 2
+            pair_rows = (self.edge_adjoint is not False and spec.num_interactions == 2 and self._same_rows()
                          and bool(layers[1].rad_img) and bool(layers[0].first[0]))
             pairs = cap // 2 + cap // 16
             if pair_rows and cap * others + pairs * row <= min(0.85 * free, free - total // 10 - atoms):

@@ -73,3 +73,12 @@ def test_pair_rows_come_with_their_map(monkeypatch, model, share):
         assert ff.buf["tp_w"].shape[0] == 2 * (w.pair_capacity or w.chunk_edges)
         seen.add(bool(w.pair_capacity))
     assert seen == {False, True}
+
+
+@pytest.mark.parametrize("model", ["small", "medium", "large"])
+@pytest.mark.parametrize("n_owned,n_inner,same", [(10, 20, False), (10, -1, False), (10, 10, True), (ATOMS, -1, True)])
+def test_pair_rows_need_both_interactions_on_the_same_atoms(monkeypatch, model, n_owned, n_inner, same):
+    """With an inner halo the adjoint covers more atoms than the forward pass and cannot use its radial weights."""
+    free = _sweep(model)[-1]
+    ff, _ = _allocated(monkeypatch, model, free, free, n_owned=n_owned, n_inner=n_inner)
+    assert bool(ff.work.pair_capacity) == same
