@@ -79,8 +79,9 @@ class B200ForceField:
         # DEFAULT_CHUNK_EDGES with the weights recomputed per chunk; a number sets the chunk size by hand
         self.chunk_edges = None if chunk_edges is None else int(chunk_edges)
         # ``edge_adjoint``: None = the per-edge hand-over adjoint with buffers for the whole list whenever they fit in the
-        # free device memory, else a chunk at a time; False = a chunk at a time regardless (the path of lists too large
-        # for the buffers, selectable so that tests reach it on small cells); True = refuse to fall back
+        # free device memory, else a chunk at a time, or every edge from both ends where not even a chunk's fit; False = a
+        # chunk at a time regardless (the path of lists too large for the buffers, selectable so that tests reach it on
+        # small cells); True = refuse to fall back
         self.edge_adjoint = edge_adjoint
         self.num_edges = 0
         self.calls = 0
@@ -253,11 +254,13 @@ class B200ForceField:
             "partial": torch.zeros(1024 * 8, dtype=torch.float64, device=dev),
         }
         # per-edge hand-over buffers of the adjoint (2 KB per edge for the medium model): when they fit in the memory
-        # that is free now with a tenth of the device kept back; else the sender gradients of one chunk at a time
+        # that is free now with a tenth of the device kept back; else the sender gradients of one chunk at a time, if those
+        # fit; else none, and every edge is evaluated from both ends
         free, total = torch.cuda.mem_get_info(dev)
         free += torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)   # blocks torch holds but does not use
-        need = cap * (hid * c * 4 + 20)
-        self.edge_local = need <= free - total // 10 and self.edge_adjoint is not False
+        need = cap * (hid * c * 4 + 28)
+        room = free - total // 10
+        self.edge_local = need <= room and self.edge_adjoint is not False
 
         def in_chunks():
             # the weight buffer was sized for the pair map, which cannot be had: size everything again, in chunks
@@ -270,7 +273,7 @@ class B200ForceField:
             return in_chunks()
         if (self.halo_exchange or self.edge_adjoint) and not self.edge_local:
             raise _lib.Fmb200Error(f"halo-exchange mode needs {need / 2 ** 30:.1f} GiB for the per-edge hand-over "
-                                   f"buffers, {max(0, free - total // 10) / 2 ** 30:.1f} GiB are free: use more ranks")
+                                   f"buffers, {max(0, room) / 2 ** 30:.1f} GiB are free: use more ranks")
         dx_edges = 0
         if self.edge_local:
             try:
@@ -288,14 +291,13 @@ class B200ForceField:
                 self.edge_local = False
                 if pair_capacity:
                     return in_chunks()
-        if not self.edge_local:
+        if not self.edge_local and cap * 20 + chunk * hid * c * 4 <= room:
             try:
                 buf["mirror"] = torch.zeros(cap, dtype=torch.int32, device=dev)
                 buf["edge_q"] = torch.zeros(cap, 4, **f32)
                 buf["edge_dx"] = torch.zeros(chunk, hid, c, **f32)
                 dx_edges = chunk
             except torch.OutOfMemoryError:
-                # not even those: the kernels that evaluate every edge from both ends
                 for name in ("mirror", "edge_q", "edge_dx"):
                     buf.pop(name, None)
                 torch.cuda.empty_cache()

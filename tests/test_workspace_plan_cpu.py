@@ -82,3 +82,21 @@ def test_pair_rows_need_both_interactions_on_the_same_atoms(monkeypatch, model, 
     free = _sweep(model)[-1]
     ff, _ = _allocated(monkeypatch, model, free, free, n_owned=n_owned, n_inner=n_inner)
     assert bool(ff.work.pair_capacity) == same
+
+
+@pytest.mark.parametrize("model", ["small", "medium", "large"])
+@pytest.mark.parametrize("share", [1.0, 0.5])
+@pytest.mark.parametrize("edge_adjoint", [None, False])
+def test_hand_over_buffers_leave_a_tenth_of_the_device(monkeypatch, model, share, edge_adjoint):
+    """Those of the whole list and those of one chunk; both occur in the sweep, and so does going without."""
+    seen = set()
+    for free in _sweep(model, 0.2):
+        try:
+            ff, left = _allocated(monkeypatch, model, free, int(free / share), edge_adjoint=edge_adjoint)
+        except torch.OutOfMemoryError:
+            continue
+        handed = [name in ff.buf for name in ("mirror", "edge_q", "edge_dx")]
+        assert all(handed) or not any(handed)
+        assert not any(handed) or left >= int(free / share) // 10
+        seen.add(len(ff.buf["edge_dx"]) if all(handed) else 0)
+    assert seen >= {0, CAPACITY} and (edge_adjoint is False or 256 in seen or share == 0.5)
