@@ -455,6 +455,7 @@ int backward_layer(const Ctx& c, int layer, const float* d_h_out, float* d_h_in,
         t.lin = L.l_in_max; t.n_atoms = c.n; t.n_rows = c.n0; t.n_valid = rows; t.count = (const long long*)c.nl->count;
         t.n_gather = c.exchange ? c.n : c.n0;      // halo atoms collect their shares too: they go back to their owners
         t.row_ptr = c.nl->edge_row_ptr; t.senders = c.nl->edge_index; t.mirror = c.w->mirror; t.x = c.w->x;
+        t.receivers = c.nl->edge_index + c.count_cap;
         t.edge_sh = c.w->edge_sh; t.edge_vec = c.w->edge_vec; t.tp_w = c.w->tp_w;
         t.tangent_offset = weight_rows(c) * L.n_paths * kC; t.d_mid = c.w->d_mid; t.dxe = c.w->edge_dx; t.qe = c.w->edge_q;
         t.d_x = c.w->d_x; t.error_word = c.w->status;
@@ -472,8 +473,7 @@ int backward_layer(const Ctx& c, int layer, const float* d_h_out, float* d_h_in,
             t.dx_e0 = by_chunk ? e0 : 0;
             StageScope scope(c.stream, kStTpBwd1);
             FMB_TRY(tp_adjoint_edges(t, c.stream));
-            if (by_chunk) FMB_TRY(gather_sender_gradient(t, e0, c.chunk, k > 0, c.stream));
-            else if (k == c.n_chunks - 1) FMB_TRY(gather_sender_gradient(t, 0, c.count_cap, false, c.stream));
+            if (by_chunk || k == c.n_chunks - 1) FMB_TRY(gather_sender_gradient(t, by_chunk, c.stream));
         }
         if (with_up) FMB_TRY(backward_linear_up(c, layer, d_h_in));
         return FMB_OK;

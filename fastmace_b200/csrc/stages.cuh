@@ -79,6 +79,7 @@ struct EdgeAdjointArgs {
     const long long* count;
     const int32_t* row_ptr;
     const int32_t* senders;
+    const int32_t* receivers;
     const int32_t* mirror;
     const float* x;
     const float* edge_sh;
@@ -96,13 +97,13 @@ struct EdgeAdjointArgs {
 // `slot`, `list`, `list_count` (or null): the edges below *listed_below that stand for their pair
 int mirror_map(const fmb_nl_t* nl, int32_t* mirror, uint32_t* status, const long long* listed_below, int32_t* slot,
                int32_t* list, long long* list_count, int list_capacity, cudaStream_t stream);
-// per-edge adjoint of an interaction after the first for one chunk of edges; after the last chunk the gather of the
-// sender-side gradients into d_x
+// per-edge adjoint of an interaction after the first for one chunk of edges
 int tp_adjoint_edges(const EdgeAdjointArgs& t, cudaStream_t stream);
 // its form where every row carries a gradient (tp_coupled.cu)
 int tp_adjoint_coupled_launch(const EdgeAdjointArgs& t, cudaStream_t stream);
-// over the mirror edges [first, first + count) only; `add`: onto d_x as it is
-int gather_sender_gradient(const EdgeAdjointArgs& t, long long first, long long count, bool add, cudaStream_t stream);
+// the gather of the sender-side gradients into d_x: of the whole list after its last chunk, or (`chunk`: dxe holds one
+// chunk) behind every chunk, the first of which starts d_x from zero
+int gather_sender_gradient(const EdgeAdjointArgs& t, bool chunk, cudaStream_t stream);
 // first interaction: adds its edge-vector gradients to qe (rows below n_add) or stores them
 int first_adjoint_edges(const FirstArgs& f, int n_add, float* qe, cudaStream_t stream);
 // forces (as gradients) and per-atom virials from the per-edge gradients; only the edges into atoms [0, n_valid) carry

@@ -233,8 +233,8 @@ typedef struct {
     int32_t n_inner_atoms;
     /* Optional per-edge hand-over buffers of the adjoint (all three or none):
      * mirror [edge_capacity] int32 (index of the opposite edge), edge_q [edge_capacity][4] (gradient of the edge vector),
-     * edge_dx [edge_capacity][(hidden_lmax + 1)^2][C] (gradient of the sender's features from that edge). Null = the
-     * mirror-evaluation kernels. */
+     * edge_dx [edge_capacity, or dx_edges][(hidden_lmax + 1)^2][C] (gradient of the sender's features from that edge;
+     * 16-byte aligned like d_x). Null = the mirror-evaluation kernels. */
     int32_t* mirror;
     float* edge_q;
     float* edge_dx;

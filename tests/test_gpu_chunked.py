@@ -46,3 +46,22 @@ def test_evaluation_from_both_ends_without_hand_over_buffers(model):
     for a, b in zip(ff(x), whole):
         assert (a.double() - b.double()).norm() <= 1e-5 * b.double().norm()
     ff.check_status()
+
+
+@pytest.mark.parametrize("model", ["small", "medium", "large"])
+@pytest.mark.parametrize("chunk", [37, 200, 1000, 4096])
+def test_sender_gradients_of_one_chunk_at_a_time_are_the_bits_of_the_whole_list(model, chunk):
+    """A row's terms come in the same order whether they are collected behind each chunk or at the end."""
+    from fastmace_b200.forcefield import B200ForceField
+    spec, weights, x, numbers, cell = _case(model)
+    outputs = []
+    for edge_adjoint in (None, False):
+        ff = B200ForceField(spec, weights, numbers, cell, positions=x, compute_stress=True, chunk_edges=chunk,
+                            edge_adjoint=edge_adjoint)
+        assert int(ff.work.dx_edges) == (0 if edge_adjoint is None else min(chunk, ff.edge_capacity))
+        ff(x)
+        ff.buf["d_x"].fill_(float("nan"))                # every row is written anew
+        out = ff(x)
+        outputs.append([t.clone() for t in out] + [ff.buf["d_x"][:len(numbers)].clone()])
+        ff.check_status()
+    assert all(torch.equal(a, b) for a, b in zip(*outputs))
