@@ -104,6 +104,7 @@ class LangevinStruct(ctypes.Structure):
 STAGES = ("edge_features", "radial_gemm", "tp_forward_l0", "tp_forward_l1", "node_linears", "symcon_forward",
           "symcon_backward", "tp_backward_l1", "tp_backward_l0", "readout_reduce")
 
+VERSION = 101                        # of include/fmb200.h
 _LIB = None
 
 
@@ -119,6 +120,8 @@ def load() -> ctypes.CDLL:
     lib.fmb_last_error.restype = c_char_p
     lib.fmb_sizeof.argtypes = [c_int]
     lib.fmb_launch_count.restype = ctypes.c_longlong
+    if lib.fmb_version() != VERSION:
+        raise Fmb200Error(f"the library has version {lib.fmb_version()}, this binding {VERSION}: rebuild the library")
     for which, struct in enumerate((NlStruct, ModelStruct, WorkStruct, LangevinStruct)):
         if lib.fmb_sizeof(which) != ctypes.sizeof(struct):
             raise Fmb200Error(f"struct {struct.__name__} is {ctypes.sizeof(struct)} bytes here, "

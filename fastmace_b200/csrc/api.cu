@@ -43,7 +43,7 @@ void set_error_text(const char* text) {
 
 }  // namespace fmb
 
-extern "C" FMB_API int fmb_version(void) { return 100; }
+extern "C" FMB_API int fmb_version(void) { return FMB_VERSION; }
 
 extern "C" FMB_API const char* fmb_last_error(void) {
     static thread_local std::string copy;

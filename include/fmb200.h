@@ -45,6 +45,9 @@ extern "C" {
 
 typedef void* fmb_stream_t;           /* a cudaStream_t */
 
+/* Version of this header: raised whenever the layout of a struct below or the size of a buffer in one changes. A host built
+ * against another version must not call the library (101: radial table in fmb_layer_t, dx_edges in fmb_work_t). */
+#define FMB_VERSION 101
 FMB_API int fmb_version(void);
 FMB_API const char* fmb_last_error(void);
 /* sizeof of the structs below, for the host binding to verify its mirror: which = 0 fmb_nl_t, 1 fmb_model_t,

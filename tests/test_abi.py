@@ -17,6 +17,17 @@ def test_library_exports_every_declared_symbol():
     assert lib.fmb_version() >= 100
 
 
+def test_a_changed_struct_has_a_new_version():
+    """A host built against another layout finds out by ``fmb_version``, not by a wrong pointer."""
+    from fastmace_b200 import _lib, build
+    build.build()
+    lib = _lib.load()
+    header = open(os.path.join(ROOT, "include", "fmb200.h")).read()
+    assert lib.fmb_version() == _lib.VERSION == int(re.search(r"#define FMB_VERSION (\d+)", header).group(1))
+    sizes = {100: (400, 864, 280, 152), 101: (400, 896, 280, 152)}        # neighbour list, model, workspace, Langevin
+    assert sizes[lib.fmb_version()] == tuple(lib.fmb_sizeof(which) for which in range(4))
+
+
 def test_no_cpu_fallback():
     import pytest
     import torch
