@@ -211,8 +211,8 @@ def radial_table(w0, w1, w2, r_cut: float):
 
 @functools.lru_cache(maxsize=None)
 def _contraction_layout(l_out_max: int, correlation: int, sh_lmax: int):
-    """(terms int32 [T, 4], per (l_out, degree) block the first polynomial term of every row of the
-    coefficient table and that row)."""
+    """(terms int32 [T, 4], per (l_out, degree) block the polynomial terms ordered by their row of the coefficient table,
+    the first of every row and that row)."""
     keys = so3.contraction_keys(l_out_max, correlation, sh_lmax)
     terms = np.full((len(keys), 4), -1, dtype=np.int32)
     for t, (m_out, _, mono) in enumerate(keys):
@@ -224,8 +224,10 @@ def _contraction_layout(l_out_max: int, correlation: int, sh_lmax: int):
         for nu in range(1, correlation + 1):
             mono, m_out, _, _, _ = so3.contraction_polynomial(nu, big_l, sh_lmax)
             row = np.array([row_of[big_l * big_l + int(m), nu, tuple(int(i) for i in q)] for m, q in zip(m_out, mono)])
-            first = np.flatnonzero(np.concatenate([[True], row[1:] != row[:-1]]))     # a row's terms are neighbours
-            rows[big_l, nu] = first, row[first]
+            order = np.argsort(row, kind="stable")
+            row = row[order]
+            first = np.flatnonzero(np.concatenate([[True], row[1:] != row[:-1]]))
+            rows[big_l, nu] = order, first, row[first]
     return terms, rows
 
 
@@ -233,10 +235,10 @@ def contraction_terms(spec: MaceSpec, weights, layer: int, species_z):
     """(terms int32 [T, 4], coef float64 [n_species, T, C]) of one layer's symmetric contraction, sorted by output."""
     terms, rows = _contraction_layout(spec.l_out_max(layer), spec.correlation, spec.sh_lmax)
     coefs = np.zeros((len(terms), len(species_z), spec.channels), dtype=np.float64)
-    for (big_l, nu), (first, row) in rows.items():
+    for (big_l, nu), (order, first, row) in rows.items():
         _, _, weight, coef, _ = so3.contraction_polynomial(nu, big_l, spec.sh_lmax)
         w = _f64(weights[f"l{layer}.sc.{big_l}.{nu}"]).numpy()[[z - 1 for z in species_z]]  # [nz, k, C]
-        coefs[row] += np.add.reduceat(coef[:, None, None] * w.transpose(1, 0, 2)[weight], first, axis=0)
+        coefs[row] += np.add.reduceat(coef[order, None, None] * w.transpose(1, 0, 2)[weight[order]], first, axis=0)
     return terms.copy(), coefs.transpose(1, 0, 2)
 
 

@@ -102,3 +102,24 @@ def test_species_groups_cover_every_atom_once():
         live = row[row >= 0]
         assert len(set(species[live].tolist())) == 1          # one species per group
         assert np.all(np.diff(live) > 0)                      # in index order
+
+
+def test_contraction_terms_in_any_order(monkeypatch):
+    """The terms of a coefficient need not be neighbours in the polynomial."""
+    from fastmace_b200 import packing, so3
+    from fastmace_b200.model import SPECS, init_weights
+    spec, weights = SPECS["medium"], init_weights(SPECS["medium"], 1)
+    packing._contraction_layout.cache_clear()
+    terms, coefs = packing.contraction_terms(spec, weights, 0, [11, 17])
+    real = so3.contraction_polynomial
+
+    def shuffled(*args):
+        mono, m_out, weight, coef, rest = real(*args)
+        at = np.random.default_rng(0).permutation(len(coef))
+        return [mono[i] for i in at], np.asarray(m_out)[at], weight[at], coef[at], rest
+
+    packing._contraction_layout.cache_clear()
+    monkeypatch.setattr(so3, "contraction_polynomial", shuffled)
+    other_terms, other = packing.contraction_terms(spec, weights, 0, [11, 17])
+    packing._contraction_layout.cache_clear()
+    assert np.array_equal(terms, other_terms) and np.abs(other - coefs).max() <= 1e-13 * np.abs(coefs).max()
