@@ -4,7 +4,7 @@
 (0, 1, 2) entering the product:
 
 * ``TpShape<LIN>``: number of paths, input components, components of the scattered message;
-* ``tp_forward<LIN>(x, Y, w, acc)``: ``acc[slot] += w[path] * sum_terms coef * x[m_in] * Y[m_edge]``;
+* ``tp_forward<0>(x, Y, w, acc)``: ``acc[slot] += w[path] * sum_terms coef * x[m_in] * Y[m_edge]``;
 * ``tp_backward<LIN, FLIP, NEED_DX>(x, Y, w, wp, g, dY, dr, dx)``: the adjoint of the same expression for one edge and
   one channel given the gradient ``g`` of the receiver's scattered message. ``FLIP`` evaluates the edge in the opposite
   direction (``Y_l -> (-1)^l Y_l``, folded into the coefficients), which is how a receiver-owned walk also produces
@@ -59,19 +59,19 @@ def _emit(lin: int) -> str:
            f"    static constexpr int kMidDim = {mid};",
            "};",
            ""]
-    # forward
-    out += [f"template <> __device__ __forceinline__ void tp_forward<{lin}>(const float (&x)[{in_dim}], "
-            f"const float (&Y)[16], const float (&w)[{len(paths)}], float (&acc)[{mid}]) {{"]
-    for p, path in enumerate(paths):
-        out.append(f"    // path {p}: {path['l_in']} x {path['l_edge']} -> {path['l_out']}")
-        by_out: dict[int, list] = {}
-        for mi, me, mo, c in path["terms"]:
-            by_out.setdefault(mo, []).append((mi, me, c))
-        for mo, terms in sorted(by_out.items()):
-            expr = " + ".join(f"{_lit(c)} * x[{path['in_off'] + mi}] * Y[{path['edge_off'] + me}]"
-                              for mi, me, c in terms)
-            out.append(f"    acc[{slots[(p, mo)]}] = fmaf(w[{p}], {expr}, acc[{slots[(p, mo)]}]);")
-    out += ["}", ""]
+    if lin == 0:                          # forward (first interaction; later ones: the coupled bodies)
+        out += [f"template <> __device__ __forceinline__ void tp_forward<{lin}>(const float (&x)[{in_dim}], "
+                f"const float (&Y)[16], const float (&w)[{len(paths)}], float (&acc)[{mid}]) {{"]
+        for p, path in enumerate(paths):
+            out.append(f"    // path {p}: {path['l_in']} x {path['l_edge']} -> {path['l_out']}")
+            by_out: dict[int, list] = {}
+            for mi, me, mo, c in path["terms"]:
+                by_out.setdefault(mo, []).append((mi, me, c))
+            for mo, terms in sorted(by_out.items()):
+                expr = " + ".join(f"{_lit(c)} * x[{path['in_off'] + mi}] * Y[{path['edge_off'] + me}]"
+                                  for mi, me, c in terms)
+                out.append(f"    acc[{slots[(p, mo)]}] = fmaf(w[{p}], {expr}, acc[{slots[(p, mo)]}]);")
+        out += ["}", ""]
     # backward
     out += [f"template <bool FLIP, bool NEED_DX> __device__ __forceinline__ void tp_backward_{lin}("
             f"const float (&x)[{in_dim}], const float (&Y)[16], const float (&w)[{len(paths)}], "
@@ -120,9 +120,8 @@ def render() -> str:
             "",
             "template <int LIN> struct TpShape;",
             "template <int LIN> struct TpBlocks;",
-            "template <int LIN> __device__ __forceinline__ void tp_forward(const float (&x)[(LIN + 1) * (LIN + 1)], "
-            "const float (&Y)[16], const float (&w)[LIN == 0 ? 4 : LIN == 1 ? 10 : 17], "
-            "float (&acc)[LIN == 0 ? 16 : LIN == 1 ? 40 : 71]);",
+            "template <int LIN> __device__ __forceinline__ void tp_forward(const float (&x)[1], const float (&Y)[16], "
+            "const float (&w)[4], float (&acc)[16]);",
             ""]
     body = [_emit(lin) for lin in (0, 1, 2)]
     tail = ["}  // namespace fmb", ""]
@@ -247,7 +246,8 @@ def _emit_symcon_group(l_out_max: int) -> str:
         for mono in longer:
             lines += [f"      {{ float2 q[2]; {loop} q[r] = __fmul2_rn(p[r], x[r][{mono[2]}]);", *fwd_terms(mono, "q[r]"), "      }"]
         fwd_blocks.append((n, lines + ["    }"]))
-        lines = [f"    {{ float2 p[2], hp[2]; {loop} {{ p[r] = __fmul2_rn(x[r][{i}], x[r][{j}]); hp[r] = {zero}; }}"]
+        lines = [f"    {{ float2 p[2], hp[2]; {loop} {{ p[r] = __fmul2_rn(x[r][{i}], x[r][{j}]); hp[r] = {zero}; }}" if longer
+                 else f"    {{ float2 hp[2]; {loop} hp[r] = {zero};"]
         if pre in by_mono:
             lines += bwd_terms(pre, "hp")
         for mono in longer:

@@ -363,7 +363,7 @@ int forward_layer(const Ctx& c, int layer, bool with_up = true) {
         t.chunk_e0 = e0; t.chunk_edges = chunk; t.whole_list = chunk >= c.count_cap; t.error_word = c.w->status;
         t.count = (const long long*)c.nl->count; t.row_ptr = c.nl->edge_row_ptr; t.senders = c.nl->edge_index;
         t.species = c.w->species; t.x = x; t.edge_sh = c.w->edge_sh; t.tp_w = c.w->tp_w; t.mid = c.w->mid;
-        if (layer == c.m->n_layers - 1 && pair_rows(c)) { t.mirror = c.w->mirror; t.slot = c.w->edge_slot; }
+        if (layer == c.m->n_layers - 1 && pair_rows(c)) t.slot = c.w->edge_slot;
         StageScope scope(c.stream, layer == 0 ? kStTpFwd0 : kStTpFwd1);
         FMB_TRY(tp_forward_launch(t, c.stream));
     }

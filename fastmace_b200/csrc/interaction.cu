@@ -465,9 +465,9 @@ int tp_backward_launch(const TpArgs& t, cudaStream_t stream) {
     } else if (t.lin == 0) {
         FMB_BWD(0, false, true)
     } else if (t.lin == 1) {
-        // CTAs per SM the compiler targets (FMB_TP_OCCUPANCY = 2, 3 or 4; 168 / 128 registers at 3 / 4). Measured on
-        // the 1,944-atom cell: 0.47 / 0.51 / 0.56 ms -- the kernel is bound by the 37 KB per edge it pulls through L2
-        // (the mirror receiver's 20 KB gradient row, 10 KB of radial weights), not by issue slots, so 2 stays.
+        // CTAs per SM the compiler targets, 2, 3 or 4 (168 / 128 registers at 3 / 4): 0.47 / 0.51 / 0.56 ms on the
+        // 1,944-atom cell. The kernel is bound by the 37 KB per edge it pulls through L2 (the mirror receiver's 20 KB
+        // gradient row, 10 KB of radial weights), not by issue slots, so 2 stays.
         FMB_BWD_OCC(1, false, true, 2)
     } else if (t.lin == 2) {
         FMB_BWD(2, false, true)

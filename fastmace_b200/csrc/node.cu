@@ -338,8 +338,10 @@ int symcon_backward_launch(int n_rows, int n_groups, const float* coef, const in
                            const float* msg, const float* d_basis, float* d_msg, cudaStream_t stream) {
     if (n_groups <= kFewGroups)
         return launch_backward_group<LOUT, 2, 64, 1>(n_rows, n_groups, coef, species, groups, msg, d_basis, d_msg, stream);
-    if (LOUT == 2) return launch_backward_group<LOUT, 1, 128, 1>(n_rows, n_groups, coef, species, groups, msg, d_basis, d_msg, stream);
-    return launch_backward_group<LOUT, 1, 32, 12>(n_rows, n_groups, coef, species, groups, msg, d_basis, d_msg, stream);
+    if constexpr (LOUT == 2)
+        return launch_backward_group<LOUT, 1, 128, 1>(n_rows, n_groups, coef, species, groups, msg, d_basis, d_msg, stream);
+    else
+        return launch_backward_group<LOUT, 1, 32, 12>(n_rows, n_groups, coef, species, groups, msg, d_basis, d_msg, stream);
 }
 
 }  // namespace

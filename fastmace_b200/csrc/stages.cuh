@@ -33,8 +33,7 @@ struct TpArgs {
     float* atom_virial;
     int first_layer_of_pass;
     uint32_t* error_word;  // device status word for bounded-wait failures of the staged kernels
-    const int32_t* mirror; // with `slot`: the weights of edge e are row slot[min(e, mirror[e])] of tp_w (one row per pair)
-    const int32_t* slot;
+    const int32_t* slot;   // or null: the weights of edge e are row slot[e] of tp_w (one row per pair of opposite edges)
 };
 int tp_forward_launch(const TpArgs& t, cudaStream_t stream);
 int tp_backward_launch(const TpArgs& t, cudaStream_t stream);
@@ -92,7 +91,7 @@ struct EdgeAdjointArgs {
     float* qe;                     // [edges][4]
     float* d_x;                    // [n_rows][(lin + 1)^2][C]
     uint32_t* error_word;
-    const int32_t* slot;           // or null: the weights of edge e are row slot[min(e, mirror[e])] of tp_w
+    const int32_t* slot;           // or null: the weights of edge e are row slot[e] of tp_w
 };
 // `slot`, `list`, `list_count` (or null): the edges below *listed_below that stand for their pair
 int mirror_map(const fmb_nl_t* nl, int32_t* mirror, uint32_t* status, const long long* listed_below, int32_t* slot,
