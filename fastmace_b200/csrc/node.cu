@@ -1,158 +1,13 @@
-// Per-atom stages: symmetric contraction (correlation 3) as a species-dependent polynomial in the 16 message
-// components, readouts with their gradient, the float64 energy / virial reductions.
+// Per-atom stages: readouts with their gradient, the float64 energy / virial reductions.
 //
-// Reference: EquivariantProductBasisBlock / SymmetricContraction of mace-torch, in the polynomial form the reference's
-// generated kernels evaluate (fastmace/kernels/cuda/sc_generated.py:1-20: one block per atom, one thread per
-// channel, y_C = sum_a w_a sum coef * monomial); energy contract fastmace/model/energy.py:92-99 (per-atom terms in
-// model precision, reduced in float64, E0 in float64).
+// Reference: energy contract fastmace/model/energy.py:92-99 (per-atom terms in model precision, reduced in float64, E0
+// in float64).
 
 #include "stages.cuh"
-#include "generated/symcon_generated.cuh"
 
 namespace fmb {
 
 namespace {
-
-// One thread per (atom, channel); the polynomial is generated straight-line code (generated/symcon_generated.cuh):
-// 16 inputs and the outputs live in registers, each coefficient is one coalesced load from the [species][term][C] table.
-template <int LOUT>
-__global__ void __launch_bounds__(kC)
-k_symcon_forward(int n_atoms, int n_terms, const float* __restrict__ coef, const int32_t* __restrict__ species,
-                 const float* __restrict__ msg, float* __restrict__ basis) {
-    constexpr int OUT = SymconShape<LOUT>::kOut;
-    const int a = blockIdx.x, c = threadIdx.x;
-    if (a >= n_atoms) return;
-    float x[kNSH], y[OUT];
-#pragma unroll
-    for (int k = 0; k < kNSH; ++k) x[k] = msg[((long long)a * kNSH + k) * kC + c];
-#pragma unroll
-    for (int k = 0; k < OUT; ++k) y[k] = 0.0f;
-    symcon_forward_body<LOUT>(x, coef + (long long)species[a] * n_terms * kC + c, y);
-#pragma unroll
-    for (int k = 0; k < OUT; ++k) basis[((long long)a * OUT + k) * kC + c] = y[k];
-}
-
-template <int LOUT>
-__global__ void __launch_bounds__(kC)
-k_symcon_backward(int n_atoms, int n_terms, const float* __restrict__ coef, const int32_t* __restrict__ species,
-                  const float* __restrict__ msg, const float* __restrict__ d_basis, float* __restrict__ d_msg) {
-    constexpr int OUT = SymconShape<LOUT>::kOut;
-    const int a = blockIdx.x, c = threadIdx.x;
-    if (a >= n_atoms) return;
-    float x[kNSH], dx[kNSH], g[OUT];
-#pragma unroll
-    for (int k = 0; k < kNSH; ++k) {
-        x[k] = msg[((long long)a * kNSH + k) * kC + c];
-        dx[k] = 0.0f;
-    }
-#pragma unroll
-    for (int k = 0; k < OUT; ++k) g[k] = d_basis[((long long)a * OUT + k) * kC + c];
-    symcon_backward_body<LOUT>(x, coef + (long long)species[a] * n_terms * kC + c, g, dx);
-#pragma unroll
-    for (int k = 0; k < kNSH; ++k) d_msg[((long long)a * kNSH + k) * kC + c] = dx[k];
-}
-
-// The same for the four atoms of a group (one species; -1 = empty slot; atoms at or beyond n_rows are skipped): a
-// coefficient is loaded once and used for two pairs of atoms on the packed FP32 pipe. A CTA takes CH of the 128 channels;
-// PARTS sets of CH threads share them, each with a run of the monomials, and their sums meet in shared memory.
-//
-// Bound: the coefficient table that a group streams from L2 (48, 210 or 454 KB for outputs up to l = 0, 1, 2), and with few
-// groups the chain of a thread's terms. Two atoms at a time on scalar instructions, as before: 1,944 atoms 41 -> 31 us
-// forward (both layers), 10,368 atoms 117 -> 83 and 170 -> 148 us, 13,824 atoms of the large model 445 -> 183 and
-// 364 -> 294 us.
-__device__ __forceinline__ int group_member(const int32_t* __restrict__ groups, int group, int slot, int n_rows) {
-    const int atom = groups[4 * group + slot];
-    return atom < n_rows ? atom : -1;
-}
-
-template <int K>
-__device__ __forceinline__ void load_pairs(const float* __restrict__ rows, const int (&atom)[4], int c, float2 (&v)[2][K]) {
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            v[r][k].x = atom[2 * r] >= 0 ? rows[((long long)atom[2 * r] * K + k) * kC + c] : 0.0f;
-            v[r][k].y = atom[2 * r + 1] >= 0 ? rows[((long long)atom[2 * r + 1] * K + k) * kC + c] : 0.0f;
-        }
-}
-
-// adds the parts' values into those of part 0 (pairwise: half of the parts hand over at a time)
-template <int K, int PARTS, int CH>
-__device__ __forceinline__ void add_parts(float2 (&v)[2][K], int part, int c, float2* shared) {
-#pragma unroll
-    for (int half = PARTS / 2; half >= 1; half >>= 1) {
-        float2* const slot = shared + (part & (half - 1)) * 2 * K * CH + c;
-        if (part >= half && part < 2 * half) {
-#pragma unroll
-            for (int q = 0; q < 2 * K; ++q) slot[q * CH] = v[q / K][q % K];
-        }
-        __syncthreads();
-        if (part < half) {
-#pragma unroll
-            for (int q = 0; q < 2 * K; ++q) {
-                const float2 o = slot[q * CH];
-                v[q / K][q % K].x += o.x;
-                v[q / K][q % K].y += o.y;
-            }
-        }
-        if (half > 1) __syncthreads();
-    }
-}
-
-template <int K>
-__device__ __forceinline__ void store_pairs(float* __restrict__ rows, const int (&atom)[4], int c, const float2 (&v)[2][K]) {
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            if (atom[2 * r] >= 0) rows[((long long)atom[2 * r] * K + k) * kC + c] = v[r][k].x;
-            if (atom[2 * r + 1] >= 0) rows[((long long)atom[2 * r + 1] * K + k) * kC + c] = v[r][k].y;
-        }
-}
-
-template <int LOUT, int PARTS, int CH, int MINB>
-__global__ void __launch_bounds__(CH * PARTS, MINB)
-k_symcon_forward_group(int n_rows, const float* __restrict__ coef, const int32_t* __restrict__ species,
-                       const int32_t* __restrict__ groups, const float* __restrict__ msg, float* __restrict__ basis) {
-    constexpr int OUT = SymconShape<LOUT>::kOut;
-    extern __shared__ float2 shared[];
-    const int group = blockIdx.x / (kC / CH), t = threadIdx.x % CH, part = threadIdx.x / CH;
-    const int c = t + CH * (blockIdx.x % (kC / CH));
-    const int atom[4] = {group_member(groups, group, 0, n_rows), group_member(groups, group, 1, n_rows),
-                         group_member(groups, group, 2, n_rows), group_member(groups, group, 3, n_rows)};
-    const int lead = max(max(atom[0], atom[1]), max(atom[2], atom[3]));
-    if (lead < 0) return;
-    float2 x[2][kNSH], y[2][OUT];
-    load_pairs(msg, atom, c, x);
-#pragma unroll
-    for (int q = 0; q < 2 * OUT; ++q) y[q / OUT][q % OUT] = make_float2(0.0f, 0.0f);
-    symcon_forward_group<LOUT, PARTS>(part, x, coef + (long long)species[lead] * SymconShape<LOUT>::kTerms * kC + c, y);
-    add_parts<OUT, PARTS, CH>(y, part, t, shared);
-    if (part == 0) store_pairs(basis, atom, c, y);
-}
-
-template <int LOUT, int PARTS, int CH, int MINB>
-__global__ void __launch_bounds__(CH * PARTS, MINB)
-k_symcon_backward_group(int n_rows, const float* __restrict__ coef, const int32_t* __restrict__ species,
-                        const int32_t* __restrict__ groups, const float* __restrict__ msg, const float* __restrict__ d_basis,
-                        float* __restrict__ d_msg) {
-    constexpr int OUT = SymconShape<LOUT>::kOut;
-    extern __shared__ float2 shared[];
-    const int group = blockIdx.x / (kC / CH), t = threadIdx.x % CH, part = threadIdx.x / CH;
-    const int c = t + CH * (blockIdx.x % (kC / CH));
-    const int atom[4] = {group_member(groups, group, 0, n_rows), group_member(groups, group, 1, n_rows),
-                         group_member(groups, group, 2, n_rows), group_member(groups, group, 3, n_rows)};
-    const int lead = max(max(atom[0], atom[1]), max(atom[2], atom[3]));
-    if (lead < 0) return;
-    float2 x[2][kNSH], dx[2][kNSH], g[2][OUT];
-    load_pairs(msg, atom, c, x);
-    load_pairs(d_basis, atom, c, g);
-#pragma unroll
-    for (int q = 0; q < 2 * kNSH; ++q) dx[q / kNSH][q % kNSH] = make_float2(0.0f, 0.0f);
-    symcon_backward_group<LOUT, PARTS>(part, x, coef + (long long)species[lead] * SymconShape<LOUT>::kTerms * kC + c, g, dx);
-    add_parts<kNSH, PARTS, CH>(dx, part, t, shared);
-    if (part == 0) store_pairs(d_msg, atom, c, dx);
-}
 
 // h[a][k][c] = table[species[a]][k][c]  (layer 0's species-only skip connection)
 __global__ void k_fill_from_species(int n_atoms, int row, const int32_t* __restrict__ species,
@@ -296,103 +151,6 @@ __global__ void k_commit(int n3, const float* __restrict__ forces, const double*
 }
 
 }  // namespace
-
-namespace {
-
-template <int LOUT, int PARTS, int CH, int MINB>
-int launch_forward_group(int n_rows, int n_groups, const float* coef, const int32_t* species, const int32_t* groups,
-                         const float* msg, float* basis, cudaStream_t stream) {
-    constexpr int smem = (PARTS / 2) * 2 * SymconShape<LOUT>::kOut * CH * (int)sizeof(float2);
-    auto kernel = k_symcon_forward_group<LOUT, PARTS, CH, MINB>;
-    kernel<<<n_groups * (kC / CH), CH * PARTS, smem, stream>>>(n_rows, coef, species, groups, msg, basis);
-    return FMB_OK;
-}
-
-template <int LOUT, int PARTS, int CH, int MINB>
-int launch_backward_group(int n_rows, int n_groups, const float* coef, const int32_t* species, const int32_t* groups,
-                          const float* msg, const float* d_basis, float* d_msg, cudaStream_t stream) {
-    constexpr int smem = (PARTS / 2) * 2 * kNSH * CH * (int)sizeof(float2);
-    auto kernel = k_symcon_backward_group<LOUT, PARTS, CH, MINB>;
-    kernel<<<n_groups * (kC / CH), CH * PARTS, smem, stream>>>(n_rows, coef, species, groups, msg, d_basis, d_msg);
-    return FMB_OK;
-}
-
-// Few groups leave SMs without work and each thread with a chain of 94, 410 or 887 terms: two sets of threads share the
-// monomials (249 atoms, both layers: 28 -> 18 us forward, 36 -> 23 us adjoint). With more groups one set does, since the
-// second one's inputs and sums cost more than the shorter chain gives (10,368 atoms: 83 against 99 us forward).
-constexpr int kFewGroups = 148;
-
-template <int LOUT>
-int symcon_forward_launch(int n_rows, int n_groups, const float* coef, const int32_t* species, const int32_t* groups,
-                          const float* msg, float* basis, cudaStream_t stream) {
-    if (n_groups <= kFewGroups) return launch_forward_group<LOUT, 2, 64, 1>(n_rows, n_groups, coef, species, groups, msg, basis, stream);
-    return launch_forward_group<LOUT, 1, 64, 1>(n_rows, n_groups, coef, species, groups, msg, basis, stream);
-}
-
-// The adjoint holds the messages of four atoms and their gradients (170 registers, 234 for outputs up to l = 2): CTAs of
-// one warp fill the registers of an SM evenly (486 groups of the 1,944-atom cell in CTAs of four are a wave and a tenth:
-// 55 us, 48 with single warps, 148 against 168 us at 10,368 atoms); for l = 2 whole CTAs read the coefficients together
-// (13,824 atoms: 294 us, 384 with single warps).
-template <int LOUT>
-int symcon_backward_launch(int n_rows, int n_groups, const float* coef, const int32_t* species, const int32_t* groups,
-                           const float* msg, const float* d_basis, float* d_msg, cudaStream_t stream) {
-    if (n_groups <= kFewGroups)
-        return launch_backward_group<LOUT, 2, 64, 1>(n_rows, n_groups, coef, species, groups, msg, d_basis, d_msg, stream);
-    if constexpr (LOUT == 2)
-        return launch_backward_group<LOUT, 1, 128, 1>(n_rows, n_groups, coef, species, groups, msg, d_basis, d_msg, stream);
-    else
-        return launch_backward_group<LOUT, 1, 32, 12>(n_rows, n_groups, coef, species, groups, msg, d_basis, d_msg, stream);
-}
-
-}  // namespace
-
-#define FMB_TRY_SYM(expr)        \
-    {                            \
-        const int rc__ = (expr); \
-        if (rc__) return rc__;   \
-    }
-
-int symcon_forward(int n_atoms, int n_terms, int out_dim, const int32_t* terms, const float* coef,
-                   const int32_t* species, const float* msg, float* basis, const int32_t* groups, int n_groups,
-                   cudaStream_t stream) {
-    (void)terms;
-    if (n_atoms <= 0) return FMB_OK;
-#define FMB_SYM(L_)                                                                                              \
-    {                                                                                                            \
-        FMB_REQUIRE(n_terms == SymconShape<L_>::kTerms, "symcon: coefficient table does not match the kernel"); \
-        if (groups && n_groups > 0)                                                                              \
-            FMB_TRY_SYM((symcon_forward_launch<L_>(n_atoms, n_groups, coef, species, groups, msg, basis, stream)))  \
-        else                                                                                                     \
-            k_symcon_forward<L_><<<n_atoms, kC, 0, stream>>>(n_atoms, n_terms, coef, species, msg, basis);       \
-    }
-    if (out_dim == 1) FMB_SYM(0) else if (out_dim == 4) FMB_SYM(1) else if (out_dim == 9) FMB_SYM(2) else {
-        FMB_REQUIRE(false, "symcon: unsupported output irreps");
-    }
-#undef FMB_SYM
-    FMB_LAUNCH_CHECK();
-    return FMB_OK;
-}
-
-int symcon_backward(int n_atoms, int n_terms, int out_dim, const int32_t* terms, const float* coef,
-                    const int32_t* species, const float* msg, const float* d_basis, float* d_msg, const int32_t* groups,
-                    int n_groups, cudaStream_t stream) {
-    (void)terms;
-    if (n_atoms <= 0) return FMB_OK;
-#define FMB_SYM(L_)                                                                                                  \
-    {                                                                                                                \
-        FMB_REQUIRE(n_terms == SymconShape<L_>::kTerms, "symcon: coefficient table does not match the kernel");     \
-        if (groups && n_groups > 0)                                                                                  \
-            FMB_TRY_SYM((symcon_backward_launch<L_>(n_atoms, n_groups, coef, species, groups, msg, d_basis, d_msg, stream))) \
-        else                                                                                                         \
-            k_symcon_backward<L_><<<n_atoms, kC, 0, stream>>>(n_atoms, n_terms, coef, species, msg, d_basis, d_msg); \
-    }
-    if (out_dim == 1) FMB_SYM(0) else if (out_dim == 4) FMB_SYM(1) else if (out_dim == 9) FMB_SYM(2) else {
-        FMB_REQUIRE(false, "symcon: unsupported output irreps");
-    }
-#undef FMB_SYM
-    FMB_LAUNCH_CHECK();
-    return FMB_OK;
-}
 
 int fill_from_species(int n_atoms, int row, const int32_t* species, const float* table, float* out, cudaStream_t stream) {
     const long long total = (long long)n_atoms * row;
