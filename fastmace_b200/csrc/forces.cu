@@ -461,6 +461,7 @@ int backward_layer(const Ctx& c, int layer, const float* d_h_out, float* d_h_in,
         t.n_gather = c.exchange ? c.n : c.n0;      // halo atoms collect their shares too: they go back to their owners
         t.row_ptr = c.nl->edge_row_ptr; t.senders = c.nl->edge_index; t.mirror = c.w->mirror; t.x = c.w->x;
         t.receivers = c.nl->edge_index + c.count_cap;
+        t.dx_rows = dx_rows(c);
         t.edge_sh = c.w->edge_sh; t.edge_vec = c.w->edge_vec; t.tp_w = c.w->tp_w;
         t.tangent_offset = weight_rows(c) * L.n_paths * kC; t.d_mid = c.w->d_mid; t.dxe = c.w->edge_dx; t.qe = c.w->edge_q;
         t.d_x = c.w->d_x; t.error_word = c.w->status;

@@ -87,7 +87,7 @@ struct EdgeAdjointArgs {
     long long tangent_offset;
     const float* d_mid;
     float* dxe;                    // [edges from dx_e0 on][(lin + 1)^2][C]
-    long long dx_e0;
+    long long dx_e0, dx_rows;      // first edge and rows of dxe
     float* qe;                     // [edges][4]
     float* d_x;                    // [n_rows][(lin + 1)^2][C]
     uint32_t* error_word;
