@@ -174,12 +174,13 @@ def _table_is_accurate(table, per: int, function, r_cut: float) -> bool:
     value, tangent = function(r)
     largest = [torch.zeros(windows, dtype=torch.float64).scatter_reduce(0, window, f.abs().amax(1) * inside, "amax")
                for f in (value, tangent)]
-    c = table.double()
-    for u, at in ((-1.0, slice(0, n)), (1.0, slice(1, n + 1)), (0.5, slice(n + 1, 2 * n + 1))):
-        powers = torch.tensor([u ** k for k in range(c.shape[1])], dtype=torch.float64)
-        slopes = torch.tensor([k * u ** max(k - 1, 0) for k in range(c.shape[1])], dtype=torch.float64) * (2 * per)
-        for weights, exact, bound, top in ((powers, value, 2e-7, largest[0]), (slopes, tangent, 4e-7, largest[1])):
-            error = (torch.einsum("k,nkf->nf", weights, c) - exact[at]).abs().amax(1) * inside[at]
+    n_c, probes = table.shape[1], ((-1.0, slice(0, n)), (1.0, slice(1, n + 1)), (0.5, slice(n + 1, 2 * n + 1)))
+    powers = [[u ** k for k in range(n_c)] for u, _ in probes]
+    slopes = [[2.0 * per * k * u ** max(k - 1, 0) for k in range(n_c)] for u, _ in probes]
+    got = torch.tensor(powers + slopes, dtype=torch.float64) @ table.double()                       # [n, 6, features]
+    for q, (_, at) in enumerate(probes):
+        for row, exact, bound, top in ((q, value, 2e-7, largest[0]), (q + 3, tangent, 4e-7, largest[1])):
+            error = (got[:, row] - exact[at]).abs().amax(1) * inside[at]
             if not bool((error <= bound * top[window[at]]).all()):
                 return False
     return True
