@@ -160,12 +160,14 @@ def test_medium_216_atoms():
     assert df <= 5e-4 * fscale + 1e-7
 
 
-def test_pair_rows_hold_the_radial_weights_of_both_edges_of_a_pair():
+@pytest.mark.parametrize("name", ["small", "medium216", "large"])
+def test_pair_rows_hold_the_radial_weights_of_both_edges_of_a_pair(name):
     """With the whole list as one chunk an edge and its opposite edge share one row of radial weights (they have the
-    same length). After a force call: every pair is listed once, the slots are the rows 0 .. pairs - 1, and the row an
-    edge reads -- slot[min(e, mirror e)] -- holds hidden(e) x (last radial layer) for values and for d/dr."""
+    same length). After a force call: every pair is listed once, the slots are the rows 0 .. pairs - 1, both edges of a pair
+    have the same one, and the row an edge reads -- slot[e] -- holds hidden(e) x (last radial layer) for values and for
+    d/dr."""
     from fastmace_b200.forcefield import B200ForceField
-    spec, weights, s = _case("medium216")
+    spec, weights, s = _case(name)
     ff = B200ForceField(spec, weights, s.numbers, s.cell, compute_stress=True)
     ff.evaluate(s, stress=True)
     torch.cuda.synchronize()
@@ -180,7 +182,8 @@ def test_pair_rows_hold_the_radial_weights_of_both_edges_of_a_pair():
     slots = ff.buf["edge_slot"][:count].long()
     assert torch.equal(torch.sort(slots[listed]).values, torch.arange(pairs, device=ff.device))
     assert torch.equal(ff.buf["canon_list"][:pairs].long()[slots[listed]], edges[listed])
-    row = slots[torch.minimum(edges, mirror)]
+    assert torch.equal(slots[mirror], slots)
+    row = slots
     last = spec.num_interactions - 1
     rad = ff.packed.tensors[f"l{last}.rad.3"].double()                        # [64][paths * C], scaled
     rows_per_half = ff.buf["tp_w"].shape[0] // 2
@@ -221,8 +224,8 @@ def test_gemm_kernels_against_torch():
 
 
 def test_warp_specialised_gemm_against_torch():
-    """The kernel behind the node linears, called alone through its weight image: launches below one wave use
-    128 x 128 tiles, larger ones pair column tiles (128 x 256), with an odd 128-wide tile left where N / 128 is odd."""
+    """The kernel behind the node linears, called alone through its weight image: launches of few tiles use tiles of 32 or 64
+    columns, larger ones 128 columns, and beyond one tile per SM persistent CTAs walk the tiles."""
     from fastmace_b200 import _lib
     from fastmace_b200.packing import tensor_core_image
     lib = _lib.load()
@@ -246,21 +249,29 @@ def test_warp_specialised_gemm_against_torch():
     assert int(status.item()) == 0
 
 
-@pytest.mark.parametrize("name,chunk,edge_adjoint", [
-    ("medium", 1 << 19, False),      # mirror-evaluation adjoint (the path of lists too large for the per-edge
-    ("large", 4096, False),          # hand-over buffers), one chunk and several, node l_max 1 and 2
-    ("large", 4096, None),           # several chunks: fused forward (weights only in tensor memory), per-edge adjoint
-    ("silica", 2048, None),          # the same on the amorphous cell's long rows
+@pytest.mark.parametrize("name,chunk,edge_adjoint,hand_over", [
+    ("medium", 1 << 19, False, True),     # sender gradients of one chunk at a time (lists too long for the hand-over
+    ("large", 4096, False, True),         # buffers of all their edges), one chunk and several, node l_max 1 and 2
+    ("large", 4096, None, True),          # several chunks, hand-over buffers for the whole list
+    ("silica", 2048, None, True),         # the same on the amorphous cell's long rows
+    ("small", 500, False, False),         # no hand-over buffers at all: every edge evaluated from both ends, in several
+    ("medium", 1 << 19, False, False),    # chunks and in one, node l_max 0, 1 and 2
+    ("silica", 2048, False, False),
+    ("large", 4096, False, False),
 ])
-def test_paths_of_other_size_regimes_against_oracle(name, chunk, edge_adjoint):
-    """The kernels that large systems select by themselves (chunked edge lists, the mirror adjoint), reached here on
-    small cells through the constructor arguments that size them, against the oracle like the default path."""
+def test_paths_of_other_size_regimes_against_oracle(name, chunk, edge_adjoint, hand_over):
+    """The kernels that large systems select by themselves (chunked edge lists, hand-over by chunk, evaluation from both
+    ends), reached here on small cells through the constructor arguments that size them, against the oracle like the
+    default path."""
     from fastmace_b200.forcefield import B200ForceField
     spec, weights, s = _case(name)
     ff = B200ForceField(spec, weights, s.numbers, s.cell, compute_stress=True, chunk_edges=chunk,
                         edge_adjoint=edge_adjoint)
+    if not hand_over:
+        ff.rebuild(torch.tensor(s.positions, device="cuda"))
+        ff.work.mirror, ff.work.edge_q, ff.work.edge_dx = None, None, None
     e, f, st = ff.evaluate(s, stress=True)
-    assert ff.edge_local == (edge_adjoint is None)
+    assert ff.edge_local == (edge_adjoint is None) and bool(ff.work.edge_dx) == hand_over
     e_ref, f_ref, s_ref = _oracle(spec, weights, s)
     de, df, ds, fscale = _report(f"{name} chunk {chunk} edge_adjoint {edge_adjoint}", e, f, st, e_ref, f_ref, s_ref,
                                  s.natoms)
