@@ -163,13 +163,13 @@ def compulsory_bytes(spec, n_atoms: int, n_edges: int, n_species: int = 2) -> di
 
 def design_bytes(spec, n_atoms: int, n_edges: int, n_species: int = 2) -> dict:
     """Bytes the kernels as built move per force call: the compulsory ones plus the per-edge radial weights in HBM
-    (values and d/dr, 4 P C bytes each, written once and read by the tensor-product kernels) and the per-edge
-    hand-over of the sender gradient (written by the adjoint, read back by the gather)."""
+    (values and d/dr, 4 P C bytes each, written once per pair of opposite edges and read by the tensor-product kernels
+    for both) and the per-edge hand-over of the sender gradient (written by the adjoint, read back by the gather)."""
     c = spec.channels
     hid = (spec.hidden_lmax + 1) ** 2
     p1 = len(spec.paths(1))
     out = dict(compulsory_bytes(spec, n_atoms, n_edges, n_species))
-    out["radial_gemm"] += n_edges * 2 * p1 * c * 4
+    out["radial_gemm"] += n_edges * p1 * c * 4            # one row of each per pair of opposite edges
     out["tp_forward_l1"] += n_edges * p1 * c * 4
     out["tp_backward_l0"] += n_edges * 16 * 64 * 4
     out["tp_backward_l1"] += n_edges * (2 * p1 * c * 4 + 2 * hid * c * 4)
