@@ -50,18 +50,20 @@ def test_evaluation_from_both_ends_without_hand_over_buffers(model):
 
 @pytest.mark.parametrize("model", ["small", "medium", "large"])
 @pytest.mark.parametrize("chunk", [37, 200, 1000, 4096])
-def test_sender_gradients_of_one_chunk_at_a_time_are_the_bits_of_the_whole_list(model, chunk):
-    """A row's terms come in the same order whether they are collected behind each chunk or at the end."""
+@pytest.mark.parametrize("n_owned,n_inner", [(-1, -1), (40, 91)])
+def test_sender_gradients_of_one_chunk_at_a_time_are_the_bits_of_the_whole_list(model, chunk, n_owned, n_inner):
+    """A row's terms come in the same order whether they are collected behind each chunk or at the end; with an inner halo
+    the rows behind it hand over nothing."""
     from fastmace_b200.forcefield import B200ForceField
     spec, weights, x, numbers, cell = _case(model)
     outputs = []
     for edge_adjoint in (None, False):
         ff = B200ForceField(spec, weights, numbers, cell, positions=x, compute_stress=True, chunk_edges=chunk,
-                            edge_adjoint=edge_adjoint)
+                            edge_adjoint=edge_adjoint, n_owned=n_owned, n_inner=n_inner)
         assert int(ff.work.dx_edges) == (0 if edge_adjoint is None else min(chunk, ff.edge_capacity))
         ff(x)
         ff.buf["d_x"].fill_(float("nan"))                # every row is written anew
         out = ff(x)
-        outputs.append([t.clone() for t in out] + [ff.buf["d_x"][:len(numbers)].clone()])
+        outputs.append([t.clone() for t in out] + [ff.buf["d_x"][:n_inner if n_inner > 0 else len(numbers)].clone()])
         ff.check_status()
     assert all(torch.equal(a, b) for a, b in zip(*outputs))
