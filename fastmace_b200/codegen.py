@@ -312,8 +312,6 @@ def _write(path: str, text: str) -> None:
 
 # --------------------------------------------------------------------------------------------- coupled bodies
 COUPLED_OUT = os.path.join(HERE, "csrc", "generated", "tp_coupled_generated.cuh")
-COUPLE_PARTS = {0: (4,), 1: (4, 8), 2: (8, 16)}      # threads an edge's couplings are spread over
-
 
 def coupled_layout(paths):
     """Where the couplings of an edge stand: T[path][m_out][m_in] = sum_me coef * Y[me], structural zeros left out, every
@@ -341,18 +339,19 @@ def _emit_coupled(lin: int) -> str:
     slots, _ = message_slots(paths)
     in_dim, mid = (lin + 1) ** 2, so3.mid_dim(paths)
     offset, sums, stride = coupled_layout(paths)
-    out = [f"// ---- node l_max = {lin}",
-           f"template <> struct TpCoupled<{lin}> {{ static constexpr int kFloats = {stride}; }};", ""]
+    out = [f"// ---- node l_max = {lin}"]
+    # how each coupling is made, for a thread per coupling: c0 Y[at & 15] + c1 Y[at >> 8 & 15], stored at at >> 16
     order = sorted(sums)
-    for parts in COUPLE_PARTS[lin]:
-        # thread `part` of `parts` computes a run of the couplings of one edge
-        out.append(f"template <> __device__ __forceinline__ void tp_couple<{lin}, {parts}>(int part, const float* Y, float* T) {{")
-        per = -(-len(order) // parts)
-        for q in range(parts):
-            body = " ".join(f"T[{k}] = " + " + ".join(f"{_lit(c)} * Y[{e}]" for e, c in sums[k]) + ";"
-                            for k in order[q * per:(q + 1) * per])
-            out.append(f"    {'else ' if q else ''}if (part == {q}) {{ {body} }}")
-        out += ["}", ""]
+    assert all(len(sums[k]) <= 2 for k in order)
+    rows = []
+    for k in order:
+        (e0, c0), (e1, c1) = (*sums[k], (0, 0.0))[:2]
+        rows.append(f"{{{_lit(c0)}, {_lit(c1)}, {k << 16 | e1 << 8 | e0}, 0}}")
+    out += [f"__device__ const CoupleTerm kCouple{lin}[{len(order)}] = {{" + ", ".join(rows) + "};",
+            f"template <> struct TpCoupled<{lin}> {{",
+            f"    static constexpr int kFloats = {stride}, kEntries = {len(order)};",
+            f"    static __device__ __forceinline__ const CoupleTerm* terms() {{ return kCouple{lin}; }}",
+            "};", ""]
 
     def t_loads(p):
         ks = [k for (pp, _, _), k in offset.items() if pp == p]
@@ -435,7 +434,7 @@ def render_coupled() -> str:
             "",
             "__device__ __forceinline__ float2 pair_of(float v) { return make_float2(v, v); }",
             "template <int LIN> struct TpCoupled;",
-            "template <int LIN, int PARTS> __device__ __forceinline__ void tp_couple(int part, const float* Y, float* T);",
+            "struct alignas(16) CoupleTerm { float c0, c1; int at, unused; };",
             "template <int LIN> __device__ __forceinline__ void tp_forward_coupled(const float2* x, const float4* T, const float2* w, "
             "float2 (&acc)[LIN == 0 ? 16 : LIN == 1 ? 40 : 71]);",
             "template <int LIN> __device__ __forceinline__ void tp_backward_coupled(const float2* xp, const float4* T, "

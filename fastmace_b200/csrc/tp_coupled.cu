@@ -3,13 +3,13 @@
 // the packed FP32 pipe (fma.rn.f32x2), the harmonics coupled once per edge.
 //
 // An edge's harmonics enter every channel in the same few combinations, T[path][m_out][m_in] = sum_me C Y[me]. The
-// threads of a CTA compute them for a batch of edges at a time (a sixteenth to a quarter of an edge per thread, from
-// harmonics that a bulk copy brought) and read them back as broadcasts: per channel pair the forward pass is then 110
+// threads of a CTA compute them for a batch of edges at a time (a lane per coupling, from harmonics that a bulk copy
+// brought) and read them back as broadcasts: per channel pair the forward pass is then 110
 // packed FMAs for node l_max 1 and the adjoint 330, where coupling inside each thread took 126 + 86 scalar products and
 // 456. In the adjoint the gradient of the weighted sender features serves dE/dx and the derivative of the weights, and
 // the products of weighted features and message gradient are formed once for all the harmonics they couple to.
 //
-// Streaming: a group of 64 threads walks a contiguous range of edges; one thread keeps STAGES - 1 edges ahead of the
+// Streaming: a group of 64 threads walks a contiguous range of edges; its first warp keeps STAGES - 1 edges ahead of the
 // group with bulk copies that complete on mbarriers (weights, in the adjoint their d/dr, the sender's feature rows), a
 // stage is handed back by one arrival per warp. Weights and rows are read from the stage where a path needs them and
 // not copied to registers first, which is what lets node l_max 2 (71 message components) run in this form.
@@ -19,11 +19,17 @@
 // chain of a row's edges. Forward / adjoint with its gather, before (scalar or in-thread coupling) and after: 62 k
 // edges of l_max 1 118 -> 75 and 250 -> 188 us; 748 k edges of l_max 2 2.29 -> 1.41 and 7.21 -> 4.43 ms; 88 k edges of
 // l_max 0 92 -> 64 and 205 -> 135 us.
+//
+// On small and middle lists the chain of an edge counts (IPC 0.46 with the weights in L2 as well): requests by an elected
+// lane of a uniform warp, couplings without divergence and one fold for all 17 sums took the adjoint / forward kernels of
+// l_max 0 (88 k edges) from 105 to 90 and 59 to 47 us, of l_max 2 (98 k edges) from 491 to 454 and 181 to 178, the adjoint
+// of l_max 1 (62 k edges) from 153 to 145; at 615 k edges of l_max 1 both are at the HBM (5.5 TB/s).
 
 #include "stages.cuh"
 #include "generated/tp_generated.cuh"
 #include "generated/tp_coupled_generated.cuh"
 #include "edge_gradient.cuh"
+#include "fold.cuh"
 #include "tc_common.cuh"
 
 namespace fmb {
@@ -42,7 +48,7 @@ template <int LIN, int BATCH>
 struct Ahead {
     static constexpr int kT = TpCoupled<LIN>::kFloats;
     static constexpr int kFloats = 2 * BATCH * (kT + 16) + 8 * BATCH;
-    static constexpr int kParts = kGroup / BATCH;
+    static constexpr int kWarpEdges = BATCH / (kGroup / 32);         // a warp's share of a batch
     float* t;                                  // [2][BATCH][kT]
     float* y;                                  // [2][BATCH][16]
     int32_t* index;                            // [4][senders BATCH, weight rows BATCH]
@@ -50,50 +56,64 @@ struct Ahead {
     const float* edge_sh;
     const int32_t* senders;
     const int32_t* slot;
-    long long w0;                              // the edge whose weights are row 0 of tp_w
-    long long eb, ee;
+    int w0;                                    // the edge whose weights are row 0 of tp_w
+    int eb, ee;
     int c, sync_id;
     volatile int* abort_flag;
 
     __device__ __forceinline__ Ahead(float* memory, uint32_t bar_, const float* edge_sh_, const int32_t* senders_,
-                                     const int32_t* slot_, long long w0_, long long eb_, long long ee_, int c_, int sync_id_,
+                                     const int32_t* slot_, int w0_, int eb_, int ee_, int c_, int sync_id_,
                                      volatile int* abort_)
         : t(memory), y(memory + 2 * BATCH * kT), index(reinterpret_cast<int32_t*>(memory + 2 * BATCH * (kT + 16))), bar(bar_),
           edge_sh(edge_sh_), senders(senders_), slot(slot_), w0(w0_), eb(eb_), ee(ee_), c(c_), sync_id(sync_id_), abort_flag(abort_) {}
 
     // thread c < BATCH: the indices of its edge of batch b
     __device__ __forceinline__ void look_up(int b) const {
-        const long long e = eb + (long long)b * BATCH + c;
+        const int e = eb + b * BATCH + c;
         if (c < BATCH && e < ee) {
             const uint32_t dst = tc::smem_u32(index + (b & 3) * 2 * BATCH + c);
             asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(dst), "l"(senders + e) : "memory");
             if (slot) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(dst + 4 * BATCH), "l"(slot + e) : "memory");
         }
     }
-    __device__ __forceinline__ int sender(long long e) const {
-        const int k = (int)(e - eb);
+    __device__ __forceinline__ int sender(int e) const {
+        const int k = e - eb;
         return index[((k / BATCH) & 3) * 2 * BATCH + k % BATCH];
     }
     // the row of tp_w that holds an edge's weights: its own, or with one row per pair of opposite edges the pair's
-    __device__ __forceinline__ long long weight_row(long long e) const {
-        const int k = (int)(e - eb);
-        return slot ? (long long)index[((k / BATCH) & 3) * 2 * BATCH + BATCH + k % BATCH] : e - w0;
+    __device__ __forceinline__ int weight_row(int e) const {
+        const int k = e - eb;
+        return slot ? index[((k / BATCH) & 3) * 2 * BATCH + BATCH + k % BATCH] : e - w0;
     }
 
     __device__ __forceinline__ void request(int b) const {
-        const long long first = eb + (long long)b * BATCH;
+        const int first = eb + b * BATCH;
         if (c == 0 && first < ee) {
-            const uint32_t bytes = (uint32_t)min((long long)BATCH, ee - first) * 64u, full = bar + 8u * (b & 1);
+            const uint32_t bytes = (uint32_t)min(BATCH, ee - first) * 64u, full = bar + 8u * (b & 1);
             tc::mbar_expect_tx(full, bytes);
-            tc::bulk_load(tc::smem_u32(y + (b & 1) * BATCH * 16), edge_sh + 16 * first, bytes, full);
+            tc::bulk_load(tc::smem_u32(y + (b & 1) * BATCH * 16), edge_sh + 16 * (long long)first, bytes, full);
         }
     }
+    // the couplings of batch b: a lane per coupling, each warp half of the edges (with a run of couplings per thread the four
+    // runs of a warp went one after the other: 350 cycles an edge of the 3,200 its chain takes)
     __device__ __forceinline__ void compute(int b) const {
-        if (eb + (long long)b * BATCH >= ee) return;
+        if (eb + b * BATCH >= ee) return;
         tc::mbar_wait(bar + 8u * (b & 1), (uint32_t)(b >> 1) & 1u, abort_flag, kSpin);
-        const int el = c % BATCH;
-        if (eb + (long long)b * BATCH + el < ee)
-            tp_couple<LIN, kParts>(c / BATCH, y + ((b & 1) * BATCH + el) * 16, t + ((b & 1) * BATCH + el) * kT);
+        const int first = (c >> 5) * kWarpEdges;
+        const float* const from = y + ((b & 1) * BATCH + first) * 16;
+        float* const to = t + ((b & 1) * BATCH + first) * kT;
+#pragma unroll
+        for (int k0 = 0; k0 < TpCoupled<LIN>::kEntries; k0 += 32) {
+            const int k = k0 + (c & 31);
+            if (k >= TpCoupled<LIN>::kEntries) break;
+            const int4 term = __ldg(reinterpret_cast<const int4*>(TpCoupled<LIN>::terms()) + k);
+            const float c0 = __int_as_float(term.x), c1 = __int_as_float(term.y);
+            const float* const y0 = from + (term.z & 15);
+            const float* const y1 = from + (term.z >> 8 & 15);
+            float* const place = to + (term.z >> 16);
+#pragma unroll
+            for (int e = 0; e < kWarpEdges; ++e) place[e * kT] = fmaf(c1, y1[16 * e], c0 * y0[16 * e]);
+        }
     }
     __device__ __forceinline__ void start() const {
         look_up(0);
@@ -117,7 +137,9 @@ struct Ahead {
     }
 };
 
-// One thread's requests for the edges' rows.
+// One warp's requests for the edges' rows: all lanes wait and look the indices up, an elected one issues, so that the
+// copies' operands stay in uniform registers (requests by a single thread took 850 cycles an edge, with the other warp
+// waiting for it).
 template <int LIN, int STAGES, bool TANGENT>
 struct Rows {
     static constexpr int P = TpShape<LIN>::kPaths, IN = TpShape<LIN>::kInDim;
@@ -129,7 +151,7 @@ struct Rows {
     const float* tp_w;
     long long tangent_offset;
     const float* x;
-    long long ee, issued;
+    int ee, issued;
     volatile int* abort_flag;
     int stage = 0;
     uint32_t parity = 1;
@@ -137,12 +159,16 @@ struct Rows {
     template <typename AheadT>
     __device__ __forceinline__ void issue(const AheadT& ahead) {
         tc::mbar_wait(bar + 8u * (STAGES + stage), parity, abort_flag, kSpin);
-        const uint32_t full = bar + 8u * stage, dst = tc::smem_u32(ring + stage * kStage);
-        const long long weight_row = ahead.weight_row(issued);
-        tc::mbar_expect_tx(full, kStage * 4);
-        tc::bulk_load(dst, tp_w + weight_row * kW, kW * 4, full);
-        if (TANGENT) tc::bulk_load(dst + kW * 4, tp_w + tangent_offset + weight_row * kW, kW * 4, full);
-        tc::bulk_load(dst + kX * 4, x + (long long)ahead.sender(issued) * (IN * kC), IN * kC * 4, full);
+        const uint32_t full = bar + 8u * stage, dst = tc::smem_u32(ring) + stage * kStage * 4;
+        const int weight_row = __shfl_sync(0xffffffffu, ahead.weight_row(issued), 0), sender = __shfl_sync(0xffffffffu, ahead.sender(issued), 0);
+        const float* const w = tp_w + (long long)weight_row * kW;
+        if (tc::elect_one()) {
+            tc::mbar_expect_tx(full, kStage * 4);
+            tc::bulk_load(dst, w, kW * 4, full);
+            if (TANGENT) tc::bulk_load(dst + kW * 4, w + tangent_offset, kW * 4, full);
+            tc::bulk_load(dst + kX * 4, x + (long long)sender * (IN * kC), IN * kC * 4, full);
+        }
+        __syncwarp();
         ++issued;
         if (++stage == STAGES) { stage = 0; parity ^= 1u; }
     }
@@ -189,25 +215,26 @@ k_tp_forward_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
     extern __shared__ __align__(128) float smem[];
     __shared__ uint64_t bars[GROUPS * (2 * STAGES + 2)];
     __shared__ int abort_sh;
-    const int group = threadIdx.x / kGroup, c = threadIdx.x % kGroup, lane = c & 31;
-    int first = 0, last = n_rows;
-    long long e1 = 0;
+    const int uniform = tc::uniform_warp(), group = GROUPS > 1 ? uniform / (kGroup / 32) : 0, warp = uniform - group * (kGroup / 32);
+    const int c = threadIdx.x - group * kGroup, lane = c & 31;
+    int first = 0, last = n_rows, begin = 0, e1 = 0;
     if (RANGE) {
-        const long long total = row_ptr[n_rows];
-        e1 = min(total, e0 + e_span);
+        const int total = row_ptr[n_rows];
+        e1 = (int)min((long long)total, e0 + e_span);
         if (e0 > 0 && e0 >= total) return;
+        begin = (int)e0;
         rows_of_range(row_ptr, n_rows, e0, e1, total, first, last);
     }
     const int r0 = first + (int)((long long)blockIdx.x * (last - first) / gridDim.x),
               r1 = first + (int)((long long)(blockIdx.x + 1) * (last - first) / gridDim.x);
     if (r0 >= r1) return;
-    long long eb = row_ptr[r0], ee = row_ptr[r1];
+    int eb = row_ptr[r0], ee = row_ptr[r1];
     if (RANGE) {
-        eb = max(eb, e0);
+        eb = max(eb, begin);
         ee = min(ee, e1);
     }
     if (GROUPS > 1) {
-        const long long len = ee - eb;
+        const int len = ee - eb;
         ee = eb + len * (group + 1) / GROUPS;
         eb = eb + len * group / GROUPS;
     }
@@ -225,20 +252,20 @@ k_tp_forward_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
     __syncthreads();
     float* const own = smem + group * forward_group_floats<LIN, STAGES, BATCH>();
     float* const tail = own + STAGES * Rows<LIN, STAGES, false>::kStage;
-    const Ahead<LIN, BATCH> ahead(tail, bar + 8 * (2 * STAGES), edge_sh, senders, slot, RANGE ? e0 : 0, eb, ee, c, 1 + group, &abort_sh);
+    const Ahead<LIN, BATCH> ahead(tail, bar + 8 * (2 * STAGES), edge_sh, senders, slot, begin, eb, ee, c, 1 + group, &abort_sh);
     Rows<LIN, STAGES, false> rows{own, bar, tp_w, 0, x, ee, eb, &abort_sh};
     ahead.start();
-    if (c == 0)
+    if (warp == 0)
         while (rows.issued < ee && rows.issued < eb + STAGES - 1) rows.issue(ahead);
     ahead.compute(0);
     int stage = 0, batch = -1, el = BATCH;
     uint32_t parity = 0;
-    long long e = eb;
+    int e = eb;
     for (int i = r0; i < r1; ++i) {
-        long long re = GROUPS > 1 ? ee : (long long)row_ptr[i + 1];
+        int re = GROUPS > 1 ? ee : row_ptr[i + 1];
         if (RANGE) re = min(re, e1);
         float2* const out = reinterpret_cast<float2*>(mid + ((long long)i * MID) * kC) + c;
-        const bool begun = RANGE && row_ptr[i] < e0;                  // the range before holds the row's first edges
+        const bool begun = RANGE && row_ptr[i] < begin;                  // the range before holds the row's first edges
         float2 acc[MID];
 #pragma unroll
         for (int k = 0; k < MID; ++k) acc[k] = begun ? out[(long long)k * (kC / 2)] : make_float2(0.0f, 0.0f);
@@ -248,7 +275,7 @@ k_tp_forward_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
                 ahead.enter(++batch);
                 el = 0;
             }
-            if (c == 0 && rows.issued < ee && rows.issued < e + STAGES) rows.issue(ahead);
+            if (warp == 0 && rows.issued < ee && rows.issued < e + STAGES) rows.issue(ahead);
             tc::mbar_wait(bar + 8 * stage, parity, &abort_sh, kSpin);
             const float* st = own + stage * Rows<LIN, STAGES, false>::kStage;
             tp_forward_coupled<LIN>(reinterpret_cast<const float2*>(st + Rows<LIN, STAGES, false>::kX) + c, ahead.row(batch, el),
@@ -307,11 +334,11 @@ k_tp_adjoint_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
     __shared__ uint64_t bars[2 * STAGES + 2];
     __shared__ int abort_sh, first_row_sh;
     __shared__ float red[2][BATCH][2][18];
-    const int c = threadIdx.x, warp = c >> 5, lane = c & 31;
-    const long long e1 = min((long long)row_ptr[n_rows], e0 + e_span);
-    if (e0 >= e1) return;
-    const long long per_cta = (e1 - e0 + gridDim.x - 1) / gridDim.x;
-    const long long eb = e0 + (long long)blockIdx.x * per_cta, ee = min(e1, eb + per_cta);
+    const int c = threadIdx.x, warp = tc::uniform_warp(), lane = c & 31;
+    const long long total = min((long long)row_ptr[n_rows], e0 + e_span);
+    if (e0 >= total) return;
+    const int begin = (int)e0, e1 = (int)total, per_cta = (e1 - begin + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int eb = (int)min(total, begin + (long long)blockIdx.x * per_cta), ee = eb + min(e1 - eb, per_cta);
     if (eb >= ee) return;
     const uint32_t bar = tc::smem_u32(bars);
     if (c == 0) {
@@ -326,27 +353,27 @@ k_tp_adjoint_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
     }
     __syncthreads();
     float* const tail = smem + STAGES * RowsT::kStage;
-    const Ahead<LIN, BATCH> ahead(tail, bar + 8 * (2 * STAGES), edge_sh, senders, slot, e0, eb, ee, c, 1, &abort_sh);
+    const Ahead<LIN, BATCH> ahead(tail, bar + 8 * (2 * STAGES), edge_sh, senders, slot, begin, eb, ee, c, 1, &abort_sh);
     RowsT rows{smem, bar, tp_w, tangent_offset, x, ee, eb, &abort_sh};
     ahead.start();
-    if (c == 0) {
+    if (warp == 0) {
         while (rows.issued < ee && rows.issued < eb + STAGES - 1) rows.issue(ahead);
         int lo = 0, hi = n_rows - 1;
         while (lo < hi) {
             const int at = (lo + hi + 1) >> 1;
             if (row_ptr[at] <= eb) lo = at; else hi = at - 1;
         }
-        first_row_sh = lo;
+        if (lane == 0) first_row_sh = lo;
     }
     __syncthreads();
     int a = first_row_sh;
-    long long row_end = row_ptr[a + 1];
+    int row_end = row_ptr[a + 1];
     float2 g[MID];
 #pragma unroll
     for (int k = 0; k < MID; ++k) g[k] = __ldg(reinterpret_cast<const float2*>(d_mid + ((long long)a * MID + k) * kC) + c);
     ahead.compute(0);
     auto finish = [&](int b) {
-        const long long e = eb + (long long)b * BATCH + c;
+        const int e = eb + b * BATCH + c;
         if (c >= BATCH || e >= ee) return;
         const float (&r)[2][18] = red[b & 1][c];
         float gy[16];
@@ -357,10 +384,18 @@ k_tp_adjoint_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
         edge_vector_gradient(gy, r[0][16] + r[1][16], uv.x, uv.y, uv.z, uv.w, q3);
         qe[e] = make_float4(q3[0], q3[1], q3[2], 0.0f);
     };
+    int place;                                 // the sum that `fold` leaves in this lane
+    {
+        int id[17];
+#pragma unroll
+        for (int q = 0; q < 17; ++q) id[q] = q;
+        fold_ids<17, 16>(id, lane);
+        place = id[0];
+    }
     int stage = 0, batch = -1, el = BATCH;
     uint32_t parity = 0;
 #pragma unroll 1
-    for (long long e = eb; e < ee; ++e) {
+    for (int e = eb; e < ee; ++e) {
         if (el == BATCH) {
             ahead.enter(++batch);
             el = 0;
@@ -371,7 +406,7 @@ k_tp_adjoint_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
 #pragma unroll
             for (int k = 0; k < MID; ++k) g[k] = __ldg(reinterpret_cast<const float2*>(d_mid + ((long long)a * MID + k) * kC) + c);
         }
-        if (c == 0 && rows.issued < ee && rows.issued < e + STAGES) rows.issue(ahead);
+        if (warp == 0 && rows.issued < ee && rows.issued < e + STAGES) rows.issue(ahead);
         float2 dY2[16], dx[IN], dr2 = make_float2(0.0f, 0.0f);
 #pragma unroll
         for (int q = 0; q < 16; ++q) dY2[q] = make_float2(0.0f, 0.0f);
@@ -387,24 +422,13 @@ k_tp_adjoint_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
         if (++stage == STAGES) { stage = 0; parity ^= 1u; }
 #pragma unroll
         for (int q = 0; q < IN; ++q) reinterpret_cast<float2*>(dxe + ((e - dx0) * IN + q) * kC)[c] = dx[q];
-        // 16 + 1 sums over the channels: transpose-reduce inside the warp, the two warps meet in shared memory
-        float dY[16];
+        // 16 + 1 sums over the channels: inside the warp here, the two warps meet in shared memory
+        float sums[17];
 #pragma unroll
-        for (int q = 0; q < 16; ++q) dY[q] = dY2[q].x + dY2[q].y;
-#pragma unroll
-        for (int half = 8, bit = 16; half >= 1; half >>= 1, bit >>= 1) {
-            const bool upper = (lane & bit) != 0;
-#pragma unroll
-            for (int i = 0; i < half; ++i) {
-                const float keep = upper ? dY[i + half] : dY[i];
-                const float send = upper ? dY[i] : dY[i + half];
-                dY[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
-            }
-        }
-        dY[0] += __shfl_xor_sync(0xffffffffu, dY[0], 1);
-        const float dr = warp_sum(dr2.x + dr2.y);
-        if ((lane & 1) == 0) red[batch & 1][el][warp][lane >> 1] = dY[0];
-        if (lane == 0) red[batch & 1][el][warp][16] = dr;
+        for (int q = 0; q < 16; ++q) sums[q] = dY2[q].x + dY2[q].y;
+        sums[16] = dr2.x + dr2.y;
+        fold<17, 16>(sums, lane);
+        red[batch & 1][el][warp][place] = sums[0];
         ++el;
     }
     __syncthreads();
