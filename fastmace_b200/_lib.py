@@ -16,6 +16,7 @@ LIB_PATH = os.path.join(HERE, "libfmb200.so")
 MAX_ROW = 1024
 MAX_LAYERS = 2
 MAX_SPECIES = 8
+IMAGE_ONCHIP = 1                     # bits of LayerStruct.extra_images
 
 STATUS_CAND_OVERFLOW = 1
 STATUS_ROW_OVERFLOW = 2
@@ -55,7 +56,7 @@ class NlStruct(ctypes.Structure):
 class LayerStruct(ctypes.Structure):
     _fields_ = [
         ("l_in_max", c_int32), ("l_out_max", c_int32), ("n_paths", c_int32), ("mid_dim", c_int32),
-        ("n_sc_terms", c_int32), ("skip_lmax", c_int32), ("is_last", c_int32), ("pad_", c_int32),
+        ("n_sc_terms", c_int32), ("skip_lmax", c_int32), ("is_last", c_int32), ("extra_images", c_int32),
         ("rad_w", c_void_p * 4), ("x_species", c_void_p), ("sc_species", c_void_p), ("w_up", c_void_p),
         ("w_up_t", c_void_p), ("w_skip", c_void_p), ("w_skip_t", c_void_p), ("w_lin", c_void_p),
         ("w_lin_t", c_void_p), ("w_prod", c_void_p), ("w_prod_t", c_void_p), ("sc_terms", c_void_p),

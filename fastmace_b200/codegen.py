@@ -359,75 +359,77 @@ def _emit_coupled(lin: int) -> str:
         lines = [f"const float4 t{k} = T[{k}];" for k in range(first, last + 1)]
         return lines, lambda mo, mi: f"t{offset[p, mo, mi] // 4}.{'xyzw'[offset[p, mo, mi] % 4]}"
 
-    fwd = [f"template <> __device__ __forceinline__ void tp_forward_coupled<{lin}>(const float2* x, const float4* T, "
-           f"const float2* w, float2 (&acc)[{mid}]) {{"]
-    fwd += [f"    const float2 x{k} = x[{k * 64}];" for k in range(in_dim)]
-    for p, path in enumerate(paths):
-        l_in, l_out, off = path["l_in"], path["l_out"], path["in_off"]
-        n_in, n_out = 2 * l_in + 1, 2 * l_out + 1
-        loads, t = t_loads(p)
-        fwd.append(f"    {{  // path {p}: {l_in} x {path['l_edge']} -> {l_out}")
-        fwd.append(f"        const float2 wp = w[{p * 64}]; {' '.join(loads)}")
-        if n_in <= n_out:
-            fwd.append("        " + " ".join(f"const float2 a{mi} = __fmul2_rn(wp, x{off + mi});" for mi in range(n_in)))
-        for mo in range(n_out):
-            ins = [mi for mi in range(n_in) if (p, mo, mi) in offset]
-            slot = slots[p, mo]
+    for ld in (64, 32) if lin < 2 else (64,):           # all channels, or half of them (tp_onchip.cu)
+        fwd = [f"template <> __device__ __forceinline__ void tp_forward_coupled<{lin}, {ld}>(const float2* x, const float4* T, "
+               f"const float2* w, float2 (&acc)[{mid}]) {{"]
+        fwd += [f"    const float2 x{k} = x[{k * ld}];" for k in range(in_dim)]
+        for p, path in enumerate(paths):
+            l_in, l_out, off = path["l_in"], path["l_out"], path["in_off"]
+            n_in, n_out = 2 * l_in + 1, 2 * l_out + 1
+            loads, t = t_loads(p)
+            fwd.append(f"    {{  // path {p}: {l_in} x {path['l_edge']} -> {l_out}")
+            fwd.append(f"        const float2 wp = w[{p * ld}]; {' '.join(loads)}")
             if n_in <= n_out:
-                fwd += [f"        acc[{slot}] = __ffma2_rn(a{mi}, pair_of({t(mo, mi)}), acc[{slot}]);" for mi in ins]
-            else:
-                lines = [f"float2 s = __fmul2_rn(x{off + ins[0]}, pair_of({t(mo, ins[0])}));"]
-                lines += [f"s = __ffma2_rn(x{off + mi}, pair_of({t(mo, mi)}), s);" for mi in ins[1:]]
-                fwd.append(f"        {{ {' '.join(lines)} acc[{slot}] = __ffma2_rn(wp, s, acc[{slot}]); }}")
-        fwd.append("    }")
-    fwd += ["}", ""]
+                fwd.append("        " + " ".join(f"const float2 a{mi} = __fmul2_rn(wp, x{off + mi});" for mi in range(n_in)))
+            for mo in range(n_out):
+                ins = [mi for mi in range(n_in) if (p, mo, mi) in offset]
+                slot = slots[p, mo]
+                if n_in <= n_out:
+                    fwd += [f"        acc[{slot}] = __ffma2_rn(a{mi}, pair_of({t(mo, mi)}), acc[{slot}]);" for mi in ins]
+                else:
+                    lines = [f"float2 s = __fmul2_rn(x{off + ins[0]}, pair_of({t(mo, ins[0])}));"]
+                    lines += [f"s = __ffma2_rn(x{off + mi}, pair_of({t(mo, mi)}), s);" for mi in ins[1:]]
+                    fwd.append(f"        {{ {' '.join(lines)} acc[{slot}] = __ffma2_rn(wp, s, acc[{slot}]); }}")
+            fwd.append("    }")
+        fwd += ["}", ""]
 
-    bwd = [f"template <> __device__ __forceinline__ void tp_backward_coupled<{lin}>(const float2* xp, const float4* T, "
-           f"const float2* w, const float2* wd, const float2 (&g)[{mid}], float2 (&dY)[16], float2& dr, float2 (&dx)[{in_dim}]) {{"]
-    bwd += [f"    const float2 x{k} = xp[{k * 64}];" for k in range(in_dim)]
-    for p, path in enumerate(paths):
-        l_in, l_out, off = path["l_in"], path["l_out"], path["in_off"]
-        n_in, n_out = 2 * l_in + 1, 2 * l_out + 1
-        loads, t = t_loads(p)
-        bwd.append(f"    {{  // path {p}: {l_in} x {path['l_edge']} -> {l_out}")
-        bwd.append(f"        const float2 wp = w[{p * 64}]; {' '.join(loads)}")
-        # gradient of the weighted sender features, shared by dx and by the derivative of the weight
-        for mi in range(n_in):
-            outs = [mo for mo in range(n_out) if (p, mo, mi) in offset]
-            lines = [f"float2 u{mi} = __fmul2_rn(g[{slots[p, outs[0]]}], pair_of({t(outs[0], mi)}));"]
-            lines += [f"u{mi} = __ffma2_rn(g[{slots[p, mo]}], pair_of({t(mo, mi)}), u{mi});" for mo in outs[1:]]
-            bwd.append("        " + " ".join(lines))
-        bwd.append("        float2 dw = __fmul2_rn(" + f"x{off}, u0); "
-                   + " ".join(f"dw = __ffma2_rn(x{off + mi}, u{mi}, dw);" for mi in range(1, n_in))
-                   + f" dr = __ffma2_rn(wd[{p * 64}], dw, dr);")
-        bwd.append("        " + " ".join(f"dx[{off + mi}] = __ffma2_rn(wp, u{mi}, dx[{off + mi}]);" for mi in range(n_in)))
-        # products of weighted features and message gradient, coupled into the harmonics' gradient
-        by_pair: dict[tuple, list] = {}
-        for mi, me, mo, c in path["terms"]:
-            by_pair.setdefault((mi, mo), []).append((path["edge_off"] + me, c))
-        weigh_in = n_in <= n_out
-        if weigh_in:
-            bwd.append("        " + " ".join(f"const float2 a{mi} = __fmul2_rn(wp, x{off + mi});" for mi in range(n_in)))
-        else:
-            bwd.append("        " + " ".join(f"const float2 a{mo} = __fmul2_rn(wp, g[{slots[p, mo]}]);" for mo in range(n_out)))
-        for (mi, mo), terms in sorted(by_pair.items()):
-            prod = (f"a{mi}, g[{slots[p, mo]}]" if weigh_in else f"x{off + mi}, a{mo}")
-            if len(terms) == 1 and abs(terms[0][1] - 1.0) < 1e-12:
-                e = terms[0][0]
-                bwd.append(f"        dY[{e}] = __ffma2_rn({prod}, dY[{e}]);")
+        bwd = [f"template <> __device__ __forceinline__ void tp_backward_coupled<{lin}, {ld}>(const float2* xp, const float4* T, "
+               f"const float2* w, const float2* wd, const float2 (&g)[{mid}], float2 (&dY)[16], float2& dr, float2 (&dx)[{in_dim}]) {{"]
+        bwd += [f"    const float2 x{k} = xp[{k * ld}];" for k in range(in_dim)]
+        for p, path in enumerate(paths):
+            l_in, l_out, off = path["l_in"], path["l_out"], path["in_off"]
+            n_in, n_out = 2 * l_in + 1, 2 * l_out + 1
+            loads, t = t_loads(p)
+            bwd.append(f"    {{  // path {p}: {l_in} x {path['l_edge']} -> {l_out}")
+            bwd.append(f"        const float2 wp = w[{p * ld}]; {' '.join(loads)}")
+            # gradient of the weighted sender features, shared by dx and by the derivative of the weight
+            for mi in range(n_in):
+                outs = [mo for mo in range(n_out) if (p, mo, mi) in offset]
+                lines = [f"float2 u{mi} = __fmul2_rn(g[{slots[p, outs[0]]}], pair_of({t(outs[0], mi)}));"]
+                lines += [f"u{mi} = __ffma2_rn(g[{slots[p, mo]}], pair_of({t(mo, mi)}), u{mi});" for mo in outs[1:]]
+                bwd.append("        " + " ".join(lines))
+            bwd.append("        float2 dw = __fmul2_rn(" + f"x{off}, u0); "
+                       + " ".join(f"dw = __ffma2_rn(x{off + mi}, u{mi}, dw);" for mi in range(1, n_in))
+                       + f" dr = __ffma2_rn(wd[{p * ld}], dw, dr);")
+            bwd.append("        " + " ".join(f"dx[{off + mi}] = __ffma2_rn(wp, u{mi}, dx[{off + mi}]);" for mi in range(n_in)))
+            # products of weighted features and message gradient, coupled into the harmonics' gradient
+            by_pair: dict[tuple, list] = {}
+            for mi, me, mo, c in path["terms"]:
+                by_pair.setdefault((mi, mo), []).append((path["edge_off"] + me, c))
+            weigh_in = n_in <= n_out
+            if weigh_in:
+                bwd.append("        " + " ".join(f"const float2 a{mi} = __fmul2_rn(wp, x{off + mi});" for mi in range(n_in)))
             else:
-                bwd.append(f"        {{ const float2 s = __fmul2_rn({prod}); "
-                           + " ".join(f"dY[{e}] = __ffma2_rn(s, pair_of({_lit(c)}), dY[{e}]);" for e, c in terms) + " }")
-        bwd.append("    }")
-    bwd += ["}", ""]
-    return "\n".join(out + fwd + bwd)
+                bwd.append("        " + " ".join(f"const float2 a{mo} = __fmul2_rn(wp, g[{slots[p, mo]}]);" for mo in range(n_out)))
+            for (mi, mo), terms in sorted(by_pair.items()):
+                prod = (f"a{mi}, g[{slots[p, mo]}]" if weigh_in else f"x{off + mi}, a{mo}")
+                if len(terms) == 1 and abs(terms[0][1] - 1.0) < 1e-12:
+                    e = terms[0][0]
+                    bwd.append(f"        dY[{e}] = __ffma2_rn({prod}, dY[{e}]);")
+                else:
+                    bwd.append(f"        {{ const float2 s = __fmul2_rn({prod}); "
+                               + " ".join(f"dY[{e}] = __ffma2_rn(s, pair_of({_lit(c)}), dY[{e}]);" for e, c in terms) + " }")
+            bwd.append("    }")
+        bwd += ["}", ""]
+        out += fwd + bwd
+    return "\n".join(out)
 
 
 def render_coupled() -> str:
     head = ["// GENERATED by fastmace_b200/codegen.py from fastmace_b200/so3.py -- do not edit.",
             "// The channelwise tensor product for two channels per thread on harmonics coupled once per edge (same",
             "// coefficients and message layout as tp_generated.cuh). x, w, wd: this thread's channel pair of the rows in",
-            "// shared memory, 64 pairs from one component or path to the next; T: the edge's couplings, 16-byte aligned.",
+            "// shared memory, LD pairs from one component or path to the next; T: the edge's couplings, 16-byte aligned.",
             "#pragma once",
             "",
             "namespace fmb {",
@@ -435,9 +437,10 @@ def render_coupled() -> str:
             "__device__ __forceinline__ float2 pair_of(float v) { return make_float2(v, v); }",
             "template <int LIN> struct TpCoupled;",
             "struct alignas(16) CoupleTerm { float c0, c1; int at, unused; };",
-            "template <int LIN> __device__ __forceinline__ void tp_forward_coupled(const float2* x, const float4* T, const float2* w, "
+            "// LD: channel pairs from one row to the next",
+            "template <int LIN, int LD> __device__ __forceinline__ void tp_forward_coupled(const float2* x, const float4* T, const float2* w, "
             "float2 (&acc)[LIN == 0 ? 16 : LIN == 1 ? 40 : 71]);",
-            "template <int LIN> __device__ __forceinline__ void tp_backward_coupled(const float2* xp, const float4* T, "
+            "template <int LIN, int LD> __device__ __forceinline__ void tp_backward_coupled(const float2* xp, const float4* T, "
             "const float2* w, const float2* wd, const float2 (&g)[LIN == 0 ? 16 : LIN == 1 ? 40 : 71], float2 (&dY)[16], "
             "float2& dr, float2 (&dx)[(LIN + 1) * (LIN + 1)]);",
             ""]

@@ -333,7 +333,7 @@ k_first_adjoint_rows(int n_rows, int n_valid, int n_add, int n_species, const in
                      const int32_t* __restrict__ senders, const int32_t* __restrict__ species,
                      const float* __restrict__ edge_sh, const float* __restrict__ edge_vec,
                      const float* __restrict__ hidden, const float* __restrict__ hidden_tangent,
-                     const float* __restrict__ d_s, float4* __restrict__ qe) {
+                     const float* __restrict__ d_s, float4* __restrict__ qe, const float* __restrict__ parts, long long part_stride) {
     extern __shared__ __align__(16) float staged[];       // [2 buffers][values, tangents][kFaPass][kFaLd]
     float* const own = staged + 4 * kFaPass * kFaLd;      // [4 groups][4][n_species][kFaLd]
     const int c = threadIdx.x, slot = c >> 2, grp = c & 3, lane = c & 31;
@@ -398,6 +398,15 @@ k_first_adjoint_rows(int n_rows, int n_valid, int n_add, int n_species, const in
                     term(h.w, hp.w, d0.w, d1.w, d2.w, d3.w);
                 }
             }
+            if (live && parts && a < n_add) {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const float* const from = parts + (half * part_stride + e) * 20;
+                    const float4 more = __ldg(reinterpret_cast<const float4*>(from) + grp);
+                    g[0] += more.x; g[1] += more.y; g[2] += more.z; g[3] += more.w;
+                    if (grp == 0) dr += __ldg(from + 16);
+                }
+            }
             // the four threads of an edge exchange their harmonics' gradients and add up the radial one
             float all[16];
             const int base = lane & ~3;
@@ -412,7 +421,7 @@ k_first_adjoint_rows(int n_rows, int n_valid, int n_add, int n_species, const in
                 float q3[3];
                 edge_vector_gradient(all, dr, uv.x, uv.y, uv.z, uv.w, q3);
                 float4 out = make_float4(q3[0], q3[1], q3[2], 0.0f);
-                if (a < n_add) {
+                if (a < n_add && !parts) {
                     const float4 old = qe[e];
                     out.x += old.x; out.y += old.y; out.z += old.z;
                 }
@@ -534,7 +543,7 @@ int gather_sender_gradient(const EdgeAdjointArgs& t, bool chunk, cudaStream_t st
     return FMB_ERR_UNSUPPORTED;
 }
 
-int first_adjoint_edges(const FirstArgs& f, int n_add, float* qe, cudaStream_t stream) {
+int first_adjoint_edges(const FirstArgs& f, int n_add, float* qe, const float* parts, long long part_stride, cudaStream_t stream) {
     if (f.n_rows <= 0) return FMB_OK;
     const size_t smem = (size_t)(4 * fa_group(f.n_species) + 4 * kFaPass * kFaLd) * sizeof(float);
     FMB_CUDA_CHECK(opt_in_shared_memory((const void*)k_first_adjoint_rows,
@@ -542,7 +551,7 @@ int first_adjoint_edges(const FirstArgs& f, int n_add, float* qe, cudaStream_t s
     const int grid_cap = grid_for((const void*)k_first_adjoint_rows, 1 << 30, kFaThreads, smem);
     k_first_adjoint_rows<<<f.n_rows < grid_cap ? f.n_rows : grid_cap, kFaThreads, smem, stream>>>(
         f.n_rows, f.n_valid, n_add, f.n_species, f.row_ptr, f.senders, f.species, f.edge_sh, f.edge_vec, f.hidden,
-        f.hidden_tangent, f.d_s, reinterpret_cast<float4*>(qe));
+        f.hidden_tangent, f.d_s, reinterpret_cast<float4*>(qe), parts, part_stride);
     FMB_LAUNCH_CHECK();
     return FMB_OK;
 }

@@ -170,17 +170,28 @@ const long long* edge_limit(const Ctx& c, int which) {
     return plain_rows(c) ? (const long long*)c.nl->count : edge_limits(c) + which;
 }
 
+// rows of each half of tp_w (values, then d/dr)
+long long weight_rows(const Ctx& c) { return c.w->pair_capacity > 0 ? (long long)c.w->pair_capacity : c.chunk; }
+
+// The last interaction with its last radial layer inside the kernels (tp_onchip.cu): the layer is packed for them, every row
+// carries a gradient, and tp_w, which then holds no weights, has room for their scratch. Not where rows are few: the kernels
+// load 160 KB of weights per CTA first and give every warp a range of edges, where the others cut a receiver's row in four.
+constexpr int kOnChipRows = 300;
+bool radial_on_chip(const Ctx& c) {
+    const fmb_layer_t& L = c.m->layer[c.m->n_layers - 1];
+    if (c.m->n_layers < 2 || !L.rad_img || !(L.extra_images & FMB_IMAGE_ONCHIP) || !tensor_cores_enabled() || !edge_local_adjoint(c)) return false;
+    const long long scratch = tp_onchip_scratch_floats(L.l_in_max, c.count_cap);
+    return c.n0 == c.n1 && c.n0 > kOnChipRows && scratch >= 0 && 2 * weight_rows(c) * L.n_paths * kC >= scratch;
+}
+
 // One row of radial weights per pair of opposite edges (they have the same length): the whole list is one chunk whose
 // weights are kept, the per-edge adjoint's mirror map exists, and the tensor-core producer applies (the kernels of a
 // whole list read the rows by slot).
 bool pair_rows(const Ctx& c) {
     const int last = c.m->n_layers - 1;
-    return last > 0 && keeps_forward_weights(c, last) && edge_local_adjoint(c) && c.w->edge_slot && c.w->canon_list &&
+    return last > 0 && !radial_on_chip(c) && keeps_forward_weights(c, last) && edge_local_adjoint(c) && c.w->edge_slot && c.w->canon_list &&
            c.w->canon_count && c.m->layer[last].rad_img != nullptr;
 }
-
-// rows of each half of tp_w (values, then d/dr)
-long long weight_rows(const Ctx& c) { return c.w->pair_capacity > 0 ? (long long)c.w->pair_capacity : c.chunk; }
 
 // first .. last: 0 = values, 1 = their d/dr (second half of tp_w)
 // `stream` / `max_ctas`: the producer can run on the side stream with fewer CTAs than SMs (it is one persistent CTA per
@@ -303,6 +314,17 @@ void queue_linear_up(LinearBatch& lb, const Ctx& c, int layer) {
                      (long long)l * kC * kC, c.w->x, (long long)in_dim * kC, (long long)l * l * kC, kC, l, 0);
 }
 
+TpOnChipArgs onchip_args(const Ctx& c, int layer) {
+    const fmb_layer_t& L = c.m->layer[layer];
+    TpOnChipArgs t{};
+    t.lin = L.l_in_max; t.n_rows = c.n1; t.row_ptr = c.nl->edge_row_ptr; t.senders = c.nl->edge_index; t.x = c.w->x;
+    t.edge_sh = c.w->edge_sh; t.hidden = hidden_of(c, layer, 0); t.tangent = hidden_of(c, layer, 1);
+    t.image = L.rad_img + (long long)L.n_paths * 4 * 4096;
+    t.mid = c.w->mid; t.d_mid = c.w->d_mid; t.e_span = c.count_cap; t.dxe = c.w->edge_dx; t.scratch = c.w->tp_w;
+    t.part_stride = c.count_cap; t.error_word = c.w->status;
+    return t;
+}
+
 int forward_layer(const Ctx& c, int layer, bool with_up = true) {
     const fmb_layer_t& L = c.m->layer[layer];
     const MidLayout ml = mid_layout(L.l_in_max);
@@ -348,6 +370,10 @@ int forward_layer(const Ctx& c, int layer, bool with_up = true) {
                          (long long)l * l * kC, kC, l, 0);
         FMB_TRY(run_linears(c, lb));
     } else {
+    if (layer > 0 && radial_on_chip(c)) {
+        StageScope scope(c.stream, kStTpFwd1);
+        FMB_TRY(tp_forward_onchip(onchip_args(c, layer), c.stream));
+    } else {
     // a list in several chunks: the forward pass has no use for the d/dr half of tp_w and fills both with values, which
     // halves its launches. A producer launch takes 44 us however few rows it has: force call of 562 k edges in chunks of
     // 8,192 18.3 -> 15.8 ms, of 16,384 11.6 -> 10.3, of 2^19 the same
@@ -366,6 +392,7 @@ int forward_layer(const Ctx& c, int layer, bool with_up = true) {
         if (layer == c.m->n_layers - 1 && pair_rows(c)) t.slot = c.w->edge_slot;
         StageScope scope(c.stream, layer == 0 ? kStTpFwd0 : kStTpFwd1);
         FMB_TRY(tp_forward_launch(t, c.stream));
+    }
     }
     for (int l = 0; l <= 3; ++l)
         block_linear(lb, c, rows, c.w->mid, (long long)ml.mid_dim * kC, (long long)ml.base[l] * kC, ml.segs[l] * kC, L.w_lin,
@@ -442,7 +469,9 @@ int backward_layer(const Ctx& c, int layer, const float* d_h_out, float* d_h_in,
         if (edge_local_adjoint(c)) {
             // the later interaction has written the edge-vector gradients of the rows below n0; add this one's and
             // turn the per-edge gradients into forces and virials
-            FMB_TRY(first_adjoint_edges(f, first_layer_of_pass ? 0 : c.n0, c.w->edge_q, c.stream));
+            const bool parts = !first_layer_of_pass && radial_on_chip(c);
+            FMB_TRY(first_adjoint_edges(f, first_layer_of_pass ? 0 : c.n0, c.w->edge_q, parts ? c.w->tp_w : nullptr, c.count_cap,
+                                        c.stream));
             FMB_TRY(force_gather(c.n, c.exchange ? rows : c.n, c.nl->edge_row_ptr, c.nl->edge_index, c.w->mirror,
                                  c.w->edge_q, c.w->edge_vec, c.w->force_acc, c.w->atom_virial, c.stream));
             return FMB_OK;
@@ -466,9 +495,12 @@ int backward_layer(const Ctx& c, int layer, const float* d_h_out, float* d_h_in,
         t.tangent_offset = weight_rows(c) * L.n_paths * kC; t.d_mid = c.w->d_mid; t.dxe = c.w->edge_dx; t.qe = c.w->edge_q;
         t.d_x = c.w->d_x; t.error_word = c.w->status;
         if (layer == c.m->n_layers - 1 && pair_rows(c)) t.slot = c.w->edge_slot;
+        const bool on_chip = radial_on_chip(c);
         for (int k = 0; k < c.n_chunks; ++k) {
             const long long e0 = (long long)k * c.chunk;
-            if (c.radial_ready) {
+            if (on_chip) {
+                // no weights to produce
+            } else if (c.radial_ready) {
                 FMB_CUDA_CHECK(cudaStreamWaitEvent(c.stream, c.radial_ready, 0));
             } else {
                 FMB_TRY(radial_weights(c, layer, e0, keeps_forward_weights(c, layer) ? 1 : 0, 1, edge_limit(c, 0)));
@@ -478,7 +510,13 @@ int backward_layer(const Ctx& c, int layer, const float* d_h_out, float* d_h_in,
             const bool by_chunk = dx_rows(c) < c.count_cap;
             t.dx_e0 = by_chunk ? e0 : 0;
             StageScope scope(c.stream, kStTpBwd1);
-            FMB_TRY(tp_adjoint_edges(t, c.stream));
+            if (on_chip) {
+                TpOnChipArgs q = onchip_args(c, layer);
+                q.e0 = e0; q.e_span = c.chunk; q.dx0 = t.dx_e0;
+                FMB_TRY(tp_adjoint_onchip(q, c.stream));
+            } else {
+                FMB_TRY(tp_adjoint_edges(t, c.stream));
+            }
             if (by_chunk || k == c.n_chunks - 1) FMB_TRY(gather_sender_gradient(t, by_chunk, c.stream));
         }
         if (with_up) FMB_TRY(backward_linear_up(c, layer, d_h_in));
@@ -585,7 +623,7 @@ extern "C" FMB_API int fmb_edge_features(const fmb_model_t* model, const fmb_nl_
 // little, beside the adjoint's node kernels it took 120 of their SMs.
 int fork_radial(Ctx& c, int which, bool tangent_too = false, cudaEvent_t* tangent_ready = nullptr) {
     const int layer = c.m->n_layers - 1;
-    if (!overlap_enabled() || !keeps_forward_weights(c, layer) || !c.m->layer[layer].rad_img || !tensor_cores_enabled())
+    if (!overlap_enabled() || radial_on_chip(c) || !keeps_forward_weights(c, layer) || !c.m->layer[layer].rad_img || !tensor_cores_enabled())
         return FMB_OK;
     SideStream* side = side_stream(c.stream);
     if (!side) return FMB_OK;

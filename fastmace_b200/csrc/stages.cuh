@@ -93,6 +93,32 @@ struct EdgeAdjointArgs {
     uint32_t* error_word;
     const int32_t* slot;           // or null: the weights of edge e are row slot[e] of tp_w
 };
+// Interactions after the first with the last radial layer inside the kernel (tp_onchip.cu; node l_max 0 and 1)
+struct TpOnChipArgs {
+    int lin, n_rows;
+    const int32_t* row_ptr;
+    const int32_t* senders;
+    const float* x;
+    const float* edge_sh;
+    const float* hidden;           // [edges][64]
+    const float* tangent;
+    const float* image;            // the last radial layer, behind the producer's image in fmb_layer_t.rad_img
+    float* mid;                    // forward output
+    const float* d_mid;            // adjoint input
+    long long e0, e_span;          // adjoint: the edges [e0, e0 + e_span) below the count
+    float* dxe;                    // [edges from dx0 on][(lin + 1)^2][C]
+    long long dx0;
+    // forward: sums of rows that lie in several ranges of edges; adjoint output: per half of the channels and edge the
+    // gradients of the 16 harmonics and of the length, [2][part_stride][20], to be added up
+    float* scratch;
+    long long part_stride;
+    uint32_t* error_word;
+};
+// floats of `scratch` for a list of `edges` edges (negative: no kernel for this node l_max)
+long long tp_onchip_scratch_floats(int lin, long long edges);
+int tp_forward_onchip(const TpOnChipArgs& t, cudaStream_t stream);
+int tp_adjoint_onchip(const TpOnChipArgs& t, cudaStream_t stream);
+
 // `slot`, `list`, `list_count` (or null): the edges below *listed_below that stand for their pair
 int mirror_map(const fmb_nl_t* nl, int32_t* mirror, uint32_t* status, const long long* listed_below, int32_t* slot,
                int32_t* list, long long* list_count, int list_capacity, cudaStream_t stream);
@@ -103,8 +129,10 @@ int tp_adjoint_coupled_launch(const EdgeAdjointArgs& t, cudaStream_t stream);
 // the gather of the sender-side gradients into d_x: of the whole list after its last chunk, or (`chunk`: dxe holds one
 // chunk) behind every chunk, the first of which starts d_x from zero
 int gather_sender_gradient(const EdgeAdjointArgs& t, bool chunk, cudaStream_t stream);
-// first interaction: adds its edge-vector gradients to qe (rows below n_add) or stores them
-int first_adjoint_edges(const FirstArgs& f, int n_add, float* qe, cudaStream_t stream);
+// first interaction: adds its edge-vector gradients to qe (rows below n_add) or stores them; with `parts` it adds the later
+// interaction's gradients of harmonics and length, parts[2][part_stride][20], to its own before they become one of the edge
+// vector, and what qe holds is not read
+int first_adjoint_edges(const FirstArgs& f, int n_add, float* qe, const float* parts, long long part_stride, cudaStream_t stream);
 // forces (as gradients) and per-atom virials from the per-edge gradients; only the edges into atoms [0, n_valid) carry
 // a gradient (the others are read as zero, whatever qe holds for them)
 int force_gather(int n_atoms, int n_valid, const int32_t* row_ptr, const int32_t* senders, const int32_t* mirror,

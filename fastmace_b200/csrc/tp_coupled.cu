@@ -278,7 +278,7 @@ k_tp_forward_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
             if (warp == 0 && rows.issued < ee && rows.issued < e + STAGES) rows.issue(ahead);
             tc::mbar_wait(bar + 8 * stage, parity, &abort_sh, kSpin);
             const float* st = own + stage * Rows<LIN, STAGES, false>::kStage;
-            tp_forward_coupled<LIN>(reinterpret_cast<const float2*>(st + Rows<LIN, STAGES, false>::kX) + c, ahead.row(batch, el),
+            tp_forward_coupled<LIN, kC / 2>(reinterpret_cast<const float2*>(st + Rows<LIN, STAGES, false>::kX) + c, ahead.row(batch, el),
                                     reinterpret_cast<const float2*>(st) + c, acc);
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(bar + 8 * (STAGES + stage));
@@ -414,7 +414,7 @@ k_tp_adjoint_coupled(int n_rows, const int32_t* __restrict__ row_ptr, const int3
         for (int q = 0; q < IN; ++q) dx[q] = make_float2(0.0f, 0.0f);
         tc::mbar_wait(bar + 8 * stage, parity, &abort_sh, kSpin);
         const float* st = smem + stage * RowsT::kStage;
-        tp_backward_coupled<LIN>(reinterpret_cast<const float2*>(st + RowsT::kX) + c, ahead.row(batch, el),
+        tp_backward_coupled<LIN, kC / 2>(reinterpret_cast<const float2*>(st + RowsT::kX) + c, ahead.row(batch, el),
                                  reinterpret_cast<const float2*>(st) + c, reinterpret_cast<const float2*>(st + RowsT::kW) + c, g, dY2,
                                  dr2, dx);
         __syncwarp();

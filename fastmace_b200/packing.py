@@ -17,7 +17,7 @@ import numpy as np
 import torch
 
 from . import so3
-from ._lib import MAX_SPECIES, LayerStruct, ModelStruct
+from ._lib import IMAGE_ONCHIP, MAX_SPECIES, LayerStruct, ModelStruct
 from .codegen import message_slots
 from .model import SILU_NORM, MaceSpec, e0_table
 
@@ -129,6 +129,28 @@ def mlp_image(w0: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor) -> torch.Ten
                 base = 4096 + layer * 8192 + part * 4096 + half * 2048
                 image[base + index] = source[:, half * 32:half * 32 + 32].reshape(-1)
     return image
+
+
+ONCHIP_HEADER = 4                      # floats before the image: three scales, one unused
+
+
+def onchip_image(w4: torch.Tensor, largest: float, largest_tangent: float) -> torch.Tensor:
+    """The last radial layer [64][paths * 128] (fp32, already scaled) as the kernels that evaluate the tensor product
+    beside it keep it in tensor memory, fp32 words: a header (scale of the hidden features, scale of their d/dr, inverse of
+    the product's scale; powers of two that put the ``largest`` magnitudes half way up the fp16 range), then per half of the
+    channels and pair of paths the values and the remainders of 128 rows (path, channel of the half) of 64 weights as fp16
+    pairs, [8][128 rows][4 words] each."""
+    k, n = w4.shape
+    paths = n // 128
+    w = w4.to(torch.float64).t().reshape(paths, 2, 64, k)                       # [path][half][channel][64]
+    scale = [2.0 ** min(math.floor(math.log2(32768.0 / max(float(v), 1e-30))), 40) for v in (largest, largest_tangent, w.abs().max())]
+    rows = (w * scale[2]).transpose(0, 1).reshape(2, paths // 2, 128, k)
+    value = rows.to(torch.float16)
+    rest = (rows - value.to(torch.float64)).to(torch.float16)
+    image = torch.stack([value, rest], dim=2)                                   # [half][pair][part][128][64]
+    image = image.reshape(2, paths // 2, 2, 128, 8, 8).transpose(3, 4).contiguous()
+    header = torch.tensor([scale[0], scale[1], 1.0 / (scale[0] * scale[2]), 0.0], dtype=torch.float64)
+    return torch.cat([header.to(torch.float32), image.reshape(-1).view(torch.float32)])
 
 
 RADIAL_DEGREE = 5
@@ -303,6 +325,16 @@ class PackedModel:
                     if found is not None:
                         layer.rad_tab = self._put(f"l{t}.rad.table", found[0])
                         layer.rad_tab_intervals, layer.rad_tab_per_angstrom = int(found[0].shape[0]), float(found[1])
+                        if t > 0 and c == 128 and len(paths) % 2 == 0:
+                            # behind the producer's image the one of the kernels that keep the layer on the SM
+                            table, power = found[0].double(), torch.arange(1, RADIAL_DEGREE + 1, dtype=torch.float64)
+                            largest = table.abs().sum(1).max()
+                            largest_tangent = (table[:, 1:].abs() * power[None, :, None]).sum(1).max() * 2.0 * found[1]
+                            w4 = self.tensors[f"l{t}.rad.3"].cpu()
+                            if bool(torch.isfinite(w4).all()) and largest > 0 and largest_tangent > 0:
+                                layer.rad_img = self._put(f"l{t}.rad.img", torch.cat(
+                                    [radial_image(w4, c), onchip_image(w4, largest, largest_tangent)]))
+                                layer.extra_images |= IMAGE_ONCHIP
             if t == 0:
                 x_species = h0 @ (w["l0.up.0"] / math.sqrt(c))
                 sc = torch.zeros(len(idx), spec.out_dim(0), c, dtype=torch.float64)

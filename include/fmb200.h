@@ -38,6 +38,10 @@ extern "C" {
 #define FMB_STATUS_NO_MIRROR 32u      /* an edge has no opposite edge: the neighbour list is not a full list */
 #define FMB_STATUS_PAIR_OVERFLOW 64u  /* more pairs of opposite edges than tp_w has rows (pair_capacity) */
 
+/* bits of fmb_layer_t.extra_images */
+#define FMB_IMAGE_ONCHIP 1            /* rad_img is followed by the image of the kernels that keep the last radial layer on the
+                                         SM; without it they are not used */
+
 #define FMB_MAX_ROW 1024              /* candidates per receiver the in-kernel sort can hold */
 #define FMB_MAX_LAYERS 2
 #define FMB_MAX_SPECIES 8
@@ -126,7 +130,7 @@ typedef struct {
     int32_t n_sc_terms;               /* polynomial terms of the symmetric contraction */
     int32_t skip_lmax;
     int32_t is_last;
-    int32_t pad_;
+    int32_t extra_images;             /* FMB_IMAGE_* bits: what the images below hold beyond what every host packs */
     const float* rad_w[4];            /* radial MLP, [in][out], 1/sqrt(fan_in) folded */
     const float* x_species;           /* layer 0: linear_up(embedding) per species [n_species][C] */
     const float* sc_species;          /* layer 0: skip connection per species [n_species][out_dim][C] */
@@ -155,7 +159,11 @@ typedef struct {
     /* Last radial layer as the radial-weight producer streams it into shared memory: for path p, K half h (32 of
      * the 64 hidden features) and part (0 = tf32 remainder, 1 = tf32 value) a 16 KB tile [128 channels][32] of
      * W4^T in the K-major 128-byte-swizzled operand layout, at float offset ((p * 2 + h) * 2 + part) * 4096.
-     * Null = materialise the per-edge weights with a GEMM. */
+     * Null = materialise the per-edge weights with a GEMM. With FMB_IMAGE_ONCHIP (l_in_max 0 and 1), from float offset
+     * n_paths * 16384 on: four floats (the powers of two s and s' by which the hidden features and their d/dr are
+     * multiplied to fill the fp16 range, the inverse of s times the weights' own scale, one unused), then per half of the
+     * channels and pair of paths the scaled weights as fp16 values and then as fp16 remainders, [8][128 rows][8] each (row =
+     * path of the pair, channel of the half). */
     const float* rad_img;
     /* The tensor-core twins again, packed for bulk copies into shared memory (warp-specialised GEMM): for a [K][N]
      * block at float offset o the image starts at 2 o and holds, for column tile nt (128 columns) and K chunk kc
@@ -208,7 +216,8 @@ typedef struct {
     float* edge_sh;                   /* [edge_capacity][16] */
     float* edge_hidden;               /* [n_layers][2][edge_capacity][64]: last hidden layer and its d/dr */
     float* tp_w;                      /* [2 * chunk_edges][max_paths * C]: weights, then their d/dr (both halves weights in the
-                                         forward pass of a list in several chunks) */
+                                         forward pass of a list in several chunks); scratch of the kernels that keep the
+                                         last radial layer on the SM */
     float* x;                         /* [n_atoms][in_dim(1)][C] linear_up output of layer 1 */
     float* mid;                       /* [n_atoms][max mid_dim][C] scattered message (reused by both layers) */
     float* msg;                       /* [n_layers][n_atoms][16][C] */
