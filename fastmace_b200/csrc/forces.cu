@@ -453,10 +453,16 @@ int backward_layer(const Ctx& c, int layer, const float* d_h_out, float* d_h_in,
         // reassociated first layer: gradient of the outer-product sums, then the per-edge kernel
         const int nz = c.m->n_species;
         const long long s_atom = (long long)kNSH * nz * kRadial;
-        for (int l = 0; l <= 3; ++l)
+        for (int l = 0; l <= 3; ++l) {
             block_linear(lb, c, rows, c.w->d_msg, (long long)kNSH * kC, (long long)l * l * kC, kC, L.first[1], L.first[3], L.first_img[1],
                          (long long)l * nz * kRadial * kC, c.w->d_mid, s_atom, (long long)l * l * nz * kRadial,
                          nz * kRadial, l, 0);
+            if (L.extra_images & FMB_IMAGE_FIRST_PADDED) {
+                GemmArgs& g = lb.list[lb.count - 1];
+                g.img_n = (g.n + 127) / 128 * 128;
+                g.b_img = L.first_img[1] + 2ll * l * kC * g.img_n;
+            }
+        }
         FMB_TRY(run_linears(c, lb));
         FirstArgs f{};
         // halo-exchange mode: the halo rows' edges belong to other ranks and are skipped altogether

@@ -16,6 +16,7 @@ struct GemmArgs {
     const float* bt_lo = nullptr;
     // optional: the same parts packed per (128 columns, 32 K) piece in the shared-memory operand layout (gemm_ws.cu)
     const float* b_img = nullptr;
+    int img_n = 0;                    // columns of b_img where it is padded: n rounded up to a multiple of 128
     uint32_t* error_word = nullptr;   // device status word for bounded-wait failures
     float* c = nullptr;
     int m = 0, n = 0, k = 0;

@@ -1,5 +1,6 @@
 // Warp-specialised tcgen05 / TMEM GEMM (3xTF32) for the per-irrep linears, the species skip and the first-layer
-// fold: C[r, :] (+)= A[r, :] * W with strided rows (GemmArgs), N a multiple of 128, K a multiple of 32.
+// fold: C[r, :] (+)= A[r, :] * W with strided rows (GemmArgs), N a multiple of 128 (of 64 where the image is padded), K a
+// multiple of 32.
 //
 //   * The weights never pass through registers: their tf32 value / remainder parts are packed at load time into the
 //     K-major 128-byte-swizzled operand layout and one thread brings the pieces in with bulk copies that complete on
@@ -118,7 +119,7 @@ k_gemm_ws(const __grid_constant__ WsBatch batch) {
     const float* __restrict__ a = pr.a;
     float* const c_out = pr.c;
     const WsRowMap amap = pr.amap, cmap = pr.cmap;
-    const int accumulate = pr.accumulate, select = pr.select, k = pr.k, nm = pr.nm, batch_limit = pr.batch_limit;
+    const int accumulate = pr.accumulate, select = pr.select, k = pr.k, n = pr.n, nm = pr.nm, batch_limit = pr.batch_limit;
     const uint32_t nm_magic = pr.nm_magic;
     const int32_t* const batch_species = pr.batch_species;
     const int32_t* const batch_list = pr.batch_list;
@@ -302,11 +303,12 @@ k_gemm_ws(const __grid_constant__ WsBatch batch) {
         constexpr int kRowsPerStore = 32 / kSlots;
         const int slot = lane % kSlots;
         float* const c_tile = c_out + col0 + half * kCols + 4 * slot;
+        const bool live = col0 + half * kCols < n;                    // the second half of the last tile may be padding
 #pragma unroll 4
         for (int rr = lane / kSlots; rr < 32; rr += kRowsPerStore) {
             const float4 v = turn[rr * kSlots + (slot ^ (rr & (kSlots - 1)))];
             const long long row = __shfl_sync(0xffffffffu, my_row, rr);
-            if (row >= 0) {
+            if (row >= 0 && live) {
                 float* dst = c_tile + row;
                 // accumulate: the add happens at the memory side (every element has one writer, so the sum is the
                 // same old + new as a load and a store would give, without the round trip for the old values)
@@ -549,6 +551,7 @@ k_gemm_walk(const __grid_constant__ WsBatch batch, int total) {
             }
             const int accumulate = cur.pr->accumulate;
             float* const c_tile = cur.pr->c + cur.col0 + half * 64 + 4 * (lane & 7);
+            const bool live = cur.col0 + half * 64 < cur.pr->n;       // the second half of the last tile may be padding
             mbar_wait(bar(kWpAccFull + (turn & 1)), (turn >> 1) & 1, abort_flag, kWsSpin);
             fence_after_sync();
             const uint32_t acc = tmem_base + (uint32_t)(turn & 1) * 256u + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 64);
@@ -573,7 +576,7 @@ k_gemm_walk(const __grid_constant__ WsBatch batch, int total) {
                 for (int rr = lane >> 3; rr < 32; rr += 4) {
                     const float4 v = turn_buf[rr * 8 + ((lane & 7) ^ (rr & 7))];
                     const long long at = __shfl_sync(0xffffffffu, my_row, rr);
-                    if (at >= 0) {
+                    if (at >= 0 && live) {
                         float* dst = c_tile + at + part * 32;
                         if (accumulate) add_to_global(dst, v);
                         else *reinterpret_cast<float4*>(dst) = v;
@@ -619,10 +622,12 @@ int gemm_ws_batch(const GemmArgs* list, int count, cudaStream_t stream) {
     int tiles128 = 0;
     for (int q = 0; q < count; ++q) {
         const GemmArgs& g = list[q];
-        if (!g.b_img || g.n % 128 != 0 || g.k % kWsTK != 0 || g.k < kWsTK) return FMB_ERR_UNSUPPORTED;
+        const int columns = g.img_n > 0 ? g.img_n : g.n;             // whole column tiles of the image
+        if (!g.b_img || columns % 128 != 0 || columns - g.n >= 128 || g.n % 64 != 0 || g.n > columns || g.k % kWsTK != 0 || g.k < kWsTK)
+            return FMB_ERR_UNSUPPORTED;
         FMB_REQUIRE(g.a && g.c, "gemm_ws: null operand");
         FMB_REQUIRE(g.a_nm == g.c_nm, "gemm_ws: rows of A and C belong to the same batches");
-        tiles128 += ceil_div(std::max(g.m, 0), 128) * (g.n / 128);
+        tiles128 += ceil_div(std::max(g.m, 0), 128) * (columns / 128);
     }
     // the widest tile that still gives every SM no more than one CTA when cut in four or two
     const int tn = tiles128 * 4 <= sm_count ? 32 : tiles128 * 2 <= sm_count ? 64 : 128;
@@ -641,9 +646,9 @@ int gemm_ws_batch(const GemmArgs* list, int count, cudaStream_t stream) {
         p.batch_species = g.batch_species; p.select = g.select;
         p.batch_list = g.batch_list; p.batch_limit = g.batch_limit;
         p.tile_begin = tiles;
-        p.column_tiles = g.n / tn;
+        p.column_tiles = ceil_div(g.n, tn);
         p.column_magic = p.column_tiles > 1 ? magic_of(p.column_tiles) : 0;
-        tiles += ceil_div(p.m, 128) * (g.n / tn);
+        tiles += ceil_div(p.m, 128) * p.column_tiles;
     }
     if (tiles == 0) return FMB_OK;
     if (tn == 32) return launch_ws<32, 4>(batch, tiles, stream);

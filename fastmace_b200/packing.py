@@ -17,7 +17,7 @@ import numpy as np
 import torch
 
 from . import so3
-from ._lib import IMAGE_ONCHIP, MAX_SPECIES, LayerStruct, ModelStruct
+from ._lib import IMAGE_FIRST_PADDED, IMAGE_ONCHIP, MAX_SPECIES, LayerStruct, ModelStruct
 from .codegen import message_slots
 from .model import SILU_NORM, MaceSpec, e0_table
 
@@ -357,7 +357,13 @@ class PackedModel:
                 layer.first[2] = self._twin("l0.first", blocks)
                 layer.first_img[0] = self._image_of("l0.first")
                 layer.first[3] = self._twin("l0.first_t", [b.t().contiguous() for b in blocks])
-                layer.first_img[1] = self._image_of("l0.first_t")
+                if len(idx) % 2:
+                    # N = 64 for every species: an odd number of them leaves half a column tile
+                    padded = [torch.nn.functional.pad(b.t(), (0, 64)) for b in blocks]
+                    layer.first_img[1] = self._put("l0.first_t.img", tensor_core_image(padded))
+                    layer.extra_images |= IMAGE_FIRST_PADDED
+                else:
+                    layer.first_img[1] = self._image_of("l0.first_t")
             else:
                 up = torch.stack([w[f"l{t}.up.{l}"] / math.sqrt(c) for l in range(spec.l_in_max(t) + 1)])
                 layer.w_up = self._put(f"l{t}.w_up", up)

@@ -41,6 +41,8 @@ extern "C" {
 /* bits of fmb_layer_t.extra_images */
 #define FMB_IMAGE_ONCHIP 1            /* rad_img is followed by the image of the kernels that keep the last radial layer on the
                                          SM; without it they are not used */
+#define FMB_IMAGE_FIRST_PADDED 2      /* first_img[1]: blocks whose N is an odd multiple of 64 are padded with zero columns to a
+                                         multiple of 128, one block's image behind the other's */
 
 #define FMB_MAX_ROW 1024              /* candidates per receiver the in-kernel sort can hold */
 #define FMB_MAX_LAYERS 2
