@@ -359,7 +359,7 @@ def _emit_coupled(lin: int) -> str:
         lines = [f"const float4 t{k} = T[{k}];" for k in range(first, last + 1)]
         return lines, lambda mo, mi: f"t{offset[p, mo, mi] // 4}.{'xyzw'[offset[p, mo, mi] % 4]}"
 
-    for ld in (64, 32) if lin < 2 else (64,):           # all channels, or half of them (tp_onchip.cu)
+    for ld in (64, 32) if lin == 1 else (64,):          # all channels, or half of them (tp_onchip.cu)
         fwd = [f"template <> __device__ __forceinline__ void tp_forward_coupled<{lin}, {ld}>(const float2* x, const float4* T, "
                f"const float2* w, float2 (&acc)[{mid}]) {{"]
         fwd += [f"    const float2 x{k} = x[{k * ld}];" for k in range(in_dim)]

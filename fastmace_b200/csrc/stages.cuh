@@ -93,7 +93,7 @@ struct EdgeAdjointArgs {
     uint32_t* error_word;
     const int32_t* slot;           // or null: the weights of edge e are row slot[e] of tp_w
 };
-// Interactions after the first with the last radial layer inside the kernel (tp_onchip.cu; node l_max 0 and 1)
+// Interactions after the first with the last radial layer inside the kernel (tp_onchip.cu; node l_max 1)
 struct TpOnChipArgs {
     int lin, n_rows;
     const int32_t* row_ptr;

@@ -1,10 +1,10 @@
-// Channelwise tensor product of the interactions after the first with the last radial layer inside the kernel (node l_max 0 and
+// Channelwise tensor product of the interactions after the first with the last radial layer inside the kernel (node l_max
 // 1): the per-edge radial weights and their d/dr are products of the tensor cores that never leave the SM, where the kernels of
 // tp_coupled.cu read them from memory (20 P C bytes written and read per pair of edges and force call).
 //
 // The last radial layer stays in tensor memory. As fp16 values and remainders (22 bits, as many as the tf32 pair holds) the
-// columns of half the channels, 64 P of them, take 128 (P = 4) or 320 (P = 10) of 512 TMEM columns as the first operand of
-// the MMAs, K along the columns; two CTAs share a range of edges, one per half. An MMA whose first operand is in TMEM
+// columns of half the channels, 640 of them, take 320 of 512 TMEM columns as the first operand of the MMAs, K along the
+// columns; two CTAs share a range of edges, one per half. An MMA whose first operand is in TMEM
 // takes 12 cycles at N = 16 where one that reads 128 rows from shared memory takes 40 whatever its N. The second operand is the
 // hidden radial features of a tile, split in the kernel: 16 edges, or 8 edges and their d/dr.
 //
@@ -47,9 +47,9 @@ struct Shape {
     // an edge's block of a stage (floats): weights, in the adjoint their d/dr, the sender's features, the couplings
     static constexpr int kW = P * kCh, kX = (ADJOINT ? 2 : 1) * kW, kCoupled = kX + IN * kCh, kBlock = kCoupled + kT;
     static constexpr int kStageBytes = kEdges * kBlock * 4;
-    static constexpr int kStages = LIN == 0 ? 6 : ADJOINT ? 4 : 3;
+    static constexpr int kStages = ADJOINT ? 4 : 3;
     static constexpr int kY = kEdges * 64;
-    static constexpr int kWorkerRegisters = LIN == 0 ? 136 : 168;      // of 256 for a worker's and a feeding warp's thread together
+    static constexpr int kWorkerRegisters = 168;                       // of 256 for a worker's and a feeding warp's thread together
     static constexpr int kB = 0, kStage0 = kBSlots * kBSlotBytes, kY0 = kStage0 + kStages * kStageBytes, kBytes = kY0 + kY + 1024;
     static constexpr int kBFull = 0, kBEmpty = kBSlots, kDFull = 2 * kBSlots, kDEmpty = kDFull + kAccumulators,
                          kFull = kDEmpty + kAccumulators, kEmpty = kFull + kStages, kBars = kEmpty + kStages;
@@ -270,7 +270,7 @@ __device__ __forceinline__ void bring_rows(const Cta<LIN, ADJOINT>& c, int part)
         at[j] = term.z;
     }
     float* const y = reinterpret_cast<float*>(c.smem + S::kY0) + q0 * 16;
-    const float* const from = c.a.x + c.slice * kCh + (S::IN > 1 ? (lane >> 4) * kC : 0) + 4 * (lane & 15);
+    const float* const from = c.a.x + c.slice * kCh + (lane >> 4) * kC + 4 * (lane & 15);
     int sender = 0;
     float4 harmonics = make_float4(0.f, 0.f, 0.f, 0.f);
     auto fetch = [&](int k) {
@@ -294,11 +294,10 @@ __device__ __forceinline__ void bring_rows(const Cta<LIN, ADJOINT>& c, int part)
         const uint32_t dst = smem_u32(first + S::kX) + 16 * lane;
 #pragma unroll
         for (int j = 0; j < N * S::IN / 2; ++j) {
-            const int q = 2 * j / S::IN;                                     // edge (one component: the lower half-warp's)
-            const int s = __shfl_sync(0xffffffffu, sender, S::IN > 1 ? q : 2 * j + (lane >> 4));
-            const float* src = from + (long long)s * (S::IN * kC) + (S::IN > 1 ? 2 * j % S::IN * kC : 0);
-            const uint32_t to = S::IN > 1 ? dst + (q * S::kBlock + 2 * j % S::IN * kCh) * 4
-                                          : dst + (2 * j * S::kBlock) * 4 + (lane >> 4) * (S::kBlock - kCh) * 4;
+            const int q = 2 * j / S::IN, component = 2 * j % S::IN;
+            const int s = __shfl_sync(0xffffffffu, sender, q);
+            const float* src = from + (long long)s * (S::IN * kC) + component * kC;
+            const uint32_t to = dst + (q * S::kBlock + component * kCh) * 4;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(to), "l"(src) : "memory");
         }
         asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" :: "r"(c.bar(S::kFull + st)) : "memory");
@@ -550,32 +549,30 @@ int launch(const OnChipArgs& a, cudaStream_t stream) {
 }  // namespace
 
 long long tp_onchip_scratch_floats(int lin, long long edges) {
-    if (lin != 0 && lin != 1) return -1;
+    // node l_max 0 has four paths of one component and too little to do per edge: 142 + 75 us for the adjoint and the forward
+    // kernel of 88 k edges, 90 + 47 in tp_coupled.cu
+    if (lin != 1) return -1;
     const long long ranges = device_sms() / kSlices * kWorkers;
-    const long long forward = ranges * ((lin == 0 ? TpShape<0>::kMidDim : TpShape<1>::kMidDim) * kC + 1);
-    const long long adjoint = kSlices * edges * kPartFloats;
+    const long long forward = ranges * (TpShape<1>::kMidDim * kC + 1), adjoint = kSlices * edges * kPartFloats;
     return forward > adjoint ? forward : adjoint;
 }
 
 int tp_forward_onchip(const TpOnChipArgs& t, cudaStream_t stream) {
+    if (t.lin != 1) return FMB_ERR_UNSUPPORTED;
     OnChipArgs a{};
     a.n_rows = t.n_rows; a.row_ptr = t.row_ptr; a.senders = t.senders; a.x = t.x; a.edge_sh = t.edge_sh; a.hidden = t.hidden;
     a.image = t.image; a.mid = t.mid; a.heads = t.scratch; a.error_word = t.error_word;
-    const long long ranges = device_sms() / kSlices * kWorkers;
-    a.head_row = reinterpret_cast<int32_t*>(t.scratch + ranges * ((t.lin == 0 ? TpShape<0>::kMidDim : TpShape<1>::kMidDim) * kC));
-    if (t.lin == 0) return launch<0, false>(a, stream);
-    if (t.lin == 1) return launch<1, false>(a, stream);
-    return FMB_ERR_UNSUPPORTED;
+    a.head_row = reinterpret_cast<int32_t*>(t.scratch + (long long)(device_sms() / kSlices * kWorkers) * TpShape<1>::kMidDim * kC);
+    return launch<1, false>(a, stream);
 }
 
 int tp_adjoint_onchip(const TpOnChipArgs& t, cudaStream_t stream) {
+    if (t.lin != 1) return FMB_ERR_UNSUPPORTED;
     OnChipArgs a{};
     a.n_rows = t.n_rows; a.row_ptr = t.row_ptr; a.senders = t.senders; a.x = t.x; a.edge_sh = t.edge_sh; a.hidden = t.hidden;
     a.tangent = t.tangent; a.image = t.image; a.d_mid = t.d_mid; a.dxe = t.dxe; a.parts = t.scratch; a.part_stride = t.part_stride;
     a.e0 = t.e0; a.e_span = t.e_span; a.dx0 = t.dx0; a.error_word = t.error_word;
-    if (t.lin == 0) return launch<0, true>(a, stream);
-    if (t.lin == 1) return launch<1, true>(a, stream);
-    return FMB_ERR_UNSUPPORTED;
+    return launch<1, true>(a, stream);
 }
 
 }  // namespace fmb

@@ -325,7 +325,7 @@ class PackedModel:
                     if found is not None:
                         layer.rad_tab = self._put(f"l{t}.rad.table", found[0])
                         layer.rad_tab_intervals, layer.rad_tab_per_angstrom = int(found[0].shape[0]), float(found[1])
-                        if t > 0 and c == 128 and len(paths) % 2 == 0:
+                        if t > 0 and c == 128 and spec.l_in_max(t) == 1:
                             # behind the producer's image the one of the kernels that keep the layer on the SM
                             table, power = found[0].double(), torch.arange(1, RADIAL_DEGREE + 1, dtype=torch.float64)
                             largest = table.abs().sum(1).max()

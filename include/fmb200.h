@@ -161,7 +161,7 @@ typedef struct {
     /* Last radial layer as the radial-weight producer streams it into shared memory: for path p, K half h (32 of
      * the 64 hidden features) and part (0 = tf32 remainder, 1 = tf32 value) a 16 KB tile [128 channels][32] of
      * W4^T in the K-major 128-byte-swizzled operand layout, at float offset ((p * 2 + h) * 2 + part) * 4096.
-     * Null = materialise the per-edge weights with a GEMM. With FMB_IMAGE_ONCHIP (l_in_max 0 and 1), from float offset
+     * Null = materialise the per-edge weights with a GEMM. With FMB_IMAGE_ONCHIP (l_in_max 1), from float offset
      * n_paths * 16384 on: four floats (the powers of two s and s' by which the hidden features and their d/dr are
      * multiplied to fill the fp16 range, the inverse of s times the weights' own scale, one unused), then per half of the
      * channels and pair of paths the scaled weights as fp16 values and then as fp16 remainders, [8][128 rows][8] each (row =
