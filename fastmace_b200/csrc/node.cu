@@ -4,6 +4,7 @@
 // in float64).
 
 #include "stages.cuh"
+#include "fold.cuh"
 
 namespace fmb {
 
@@ -18,65 +19,65 @@ __global__ void k_fill_from_species(int n_atoms, int row, const int32_t* __restr
     out[i] = table[(long long)species[a] * row + k];
 }
 
-// One warp per atom. Non-last layers: e += h[a][0][:] . w, gradient w. Last layer: 128 -> 16 -> SiLU -> 1 with its
-// gradient. The energy scale is folded in here. mode bit 0: add to node_energy instead of overwriting.
-__global__ void __launch_bounds__(128)
-k_readout(int n_atoms, int n_energy, int dim_first, int dim_last, int mlp_hidden, float scale, float shift, float silu_norm,
+// A warp per atom, four channels per lane, the weights of both readouts in registers for all the atoms it visits. Non-last
+// layers: e += h[a][0][:] . w, gradient w. Last layer: 128 -> 16 -> SiLU -> 1 with its gradient. The energy scale is folded
+// in here. Bound by the rows it writes (the gradient of the first layer's features, zeros but for the scalars), on small
+// systems by its chain. With the weights read again for every atom (64 strided loads, twice) and every sum a butterfly of its
+// own 62 -> 13 us for 10,368 atoms of the middle model, 14.5 -> 8.5 for 1,944.
+constexpr int kReadoutWarps = 4;
+__global__ void __launch_bounds__(32 * kReadoutWarps)
+k_readout(int n_atoms, int n_energy, int dim_first, int dim_last, float scale, float shift, float silu_norm,
           const float* __restrict__ h_first, const float* __restrict__ h_last, const float* __restrict__ w_first,
           const float* __restrict__ w_last0, const float* __restrict__ w_last1, float* __restrict__ node_energy,
           float* __restrict__ d_h_first, float* __restrict__ d_h_last) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int a = blockIdx.x * 4 + warp;
-    if (a >= n_atoms) return;
-    if (a >= n_energy) {
-        // an atom whose energy belongs to another domain: it contributes no energy and seeds no gradient
-        float* df = d_h_first + (long long)a * dim_first * kC;
-        for (int k = lane; k < dim_first * kC; k += 32) df[k] = 0.0f;
-        if (lane == 0) node_energy[a] = 0.0f;
-        return;
-    }
-    // first readout (linear) and the gradient it leaves on h_first's scalars; other components start at zero
-    float e = 0.0f;
-    const float* hf = h_first + (long long)a * dim_first * kC;
-    float* df = d_h_first + (long long)a * dim_first * kC;
+    const int lane = threadIdx.x & 31, warps = gridDim.x * kReadoutWarps;
+    const bool wide = ((reinterpret_cast<uintptr_t>(w_first) | reinterpret_cast<uintptr_t>(w_last0)) & 15) == 0;
+    auto weights = [wide](const float* from) {
+        return wide ? __ldg(reinterpret_cast<const float4*>(from)) : make_float4(__ldg(from), __ldg(from + 1), __ldg(from + 2), __ldg(from + 3));
+    };
+    const float4 wf = weights(w_first + 4 * lane);
+    float w[4][16];                            // of channels 4 lane .. 4 lane + 3
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int c = lane + 32 * q;
-        e = fmaf(hf[c], w_first[c], e);
-        df[c] = scale * w_first[c];
-    }
-    for (int k = kC + lane; k < dim_first * kC; k += 32) df[k] = 0.0f;
-    // last readout
-    const float* hl = h_last + (long long)a * dim_last * kC;
-    float z[16];
+    for (int c = 0; c < 4; ++c)
 #pragma unroll
-    for (int j = 0; j < 16; ++j) z[j] = 0.0f;
-    float hv[4];
+        for (int j = 0; j < 16; j += 4) {
+            const float4 v = weights(w_last0 + (4 * lane + c) * 16 + j);
+            w[c][j] = v.x; w[c][j + 1] = v.y; w[c][j + 2] = v.z; w[c][j + 3] = v.w;
+        }
+    const float w1 = __ldg(w_last1 + (lane >> 1));         // `fold` leaves sum j of 16 in the lanes 2 j and 2 j + 1
+    for (int a = blockIdx.x * kReadoutWarps + (threadIdx.x >> 5); a < n_atoms; a += warps) {
+        float4* const df = reinterpret_cast<float4*>(d_h_first + (long long)a * dim_first * kC) + lane;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 1; k < dim_first; ++k) df[k * (kC / 4)] = zero;
+        if (a >= n_energy) {
+            // an atom whose energy belongs to another domain: it contributes no energy and seeds no gradient
+            df[0] = zero;
+            if (lane == 0) node_energy[a] = 0.0f;
+            continue;
+        }
+        // first readout (linear) and the gradient it leaves on h_first's scalars; other components start at zero
+        const float4 hf = __ldg(reinterpret_cast<const float4*>(h_first + (long long)a * dim_first * kC) + lane);
+        const float4 hl = __ldg(reinterpret_cast<const float4*>(h_last + (long long)a * dim_last * kC) + lane);
+        float e = fmaf(hf.x, wf.x, fmaf(hf.y, wf.y, fmaf(hf.z, wf.z, hf.w * wf.w)));
+        df[0] = make_float4(scale * wf.x, scale * wf.y, scale * wf.z, scale * wf.w);
+        // last readout
+        float z[16];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int c = lane + 32 * q;
-        hv[q] = hl[c];
+        for (int j = 0; j < 16; ++j) z[j] = fmaf(hl.x, w[0][j], fmaf(hl.y, w[1][j], fmaf(hl.z, w[2][j], hl.w * w[3][j])));
+        fold<16, 16>(z, lane);
+        const float zz = z[0], sig = 1.0f / (1.0f + expf(-zz));
+        if ((lane & 1) == 0) e += silu_norm * zz * sig * w1;          // two lanes hold every sum
+        const float dz = scale * w1 * silu_norm * sig * (1.0f + zz * (1.0f - sig));
+        e = warp_sum(e);
+        if (lane == 0) node_energy[a] = scale * e + shift;
+        float g[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int j = 0; j < 16; ++j) z[j] = fmaf(hv[q], w_last0[c * 16 + j], z[j]);
-    }
-    float dz[16];
+        for (int j = 0; j < 16; ++j) {
+            const float d = __shfl_sync(0xffffffffu, dz, 2 * j);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        const float zz = warp_sum(z[j]);
-        const float sig = 1.0f / (1.0f + expf(-zz));
-        e += (lane == 0) ? silu_norm * zz * sig * w_last1[j] : 0.0f;
-        dz[j] = scale * w_last1[j] * silu_norm * sig * (1.0f + zz * (1.0f - sig));
-    }
-    e = warp_sum(e);
-    if (lane == 0) node_energy[a] = scale * e + shift;
-    float* dl = d_h_last + (long long)a * dim_last * kC;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int c = lane + 32 * q;
-        float g = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) g = fmaf(w_last0[c * 16 + j], dz[j], g);
-        dl[c] = g;
+            for (int c = 0; c < 4; ++c) g[c] = fmaf(w[c][j], d, g[c]);
+        }
+        reinterpret_cast<float4*>(d_h_last + (long long)a * dim_last * kC)[lane] = make_float4(g[0], g[1], g[2], g[3]);
     }
 }
 
@@ -164,9 +165,10 @@ int readout(const fmb_model_t* m, int n_atoms, int n_energy, const float* h_firs
     const int dim_first = (m->layer[0].l_out_max + 1) * (m->layer[0].l_out_max + 1);
     const int dim_last = 1;
     const float* w_last = m->layer[m->n_layers - 1].w_readout;
-    k_readout<<<ceil_div(n_atoms, 4), 128, 0, stream>>>(n_atoms, n_energy, dim_first, dim_last, m->mlp_hidden, m->scale, m->shift,
-                                                        m->silu_norm, h_first, h_last, m->layer[0].w_readout, w_last,
-                                                        w_last + kC * 16, node_energy, d_h_first, d_h_last);
+    const int blocks = ceil_div(n_atoms, kReadoutWarps);
+    k_readout<<<blocks < 592 ? blocks : 592, 32 * kReadoutWarps, 0, stream>>>(
+        n_atoms, n_energy, dim_first, dim_last, m->scale, m->shift, m->silu_norm, h_first, h_last, m->layer[0].w_readout, w_last,
+        w_last + kC * 16, node_energy, d_h_first, d_h_last);
     FMB_LAUNCH_CHECK();
     return FMB_OK;
 }
