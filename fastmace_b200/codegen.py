@@ -314,8 +314,7 @@ def _write(path: str, text: str) -> None:
 COUPLED_OUT = os.path.join(HERE, "csrc", "generated", "tp_coupled_generated.cuh")
 
 def coupled_layout(paths):
-    """Where the couplings of an edge stand: T[path][m_out][m_in] = sum_me coef * Y[me], structural zeros left out, every
-    path on a 16-byte boundary. Returns ({(path, m_out, m_in): offset}, {offset: [(edge component, coef)]}, floats); the
+    """Where the couplings of an edge stand: T[path][m_out][m_in] = sum_me coef * Y[me], structural zeros left out. Returns ({(path, m_out, m_in): offset}, {offset: [(edge component, coef)]}, floats); the
     row stride is 4 mod 32 floats so that the rows of neighbouring edges start in different banks."""
     offset, sums, at = {}, {}, 0
     for p, path in enumerate(paths):
@@ -325,8 +324,7 @@ def coupled_layout(paths):
                 sums[at] = []
                 at += 1
             sums[offset[p, mo, mi]].append((path["edge_off"] + me, c))
-        at = -(-at // 4) * 4
-    stride = at
+    stride = -(-at // 4) * 4
     while stride % 32 != 4:
         stride += 4
     return offset, sums, stride
@@ -354,8 +352,9 @@ def _emit_coupled(lin: int) -> str:
             "};", ""]
 
     def t_loads(p):
+        # the groups of four that start with path p (paths are not padded: a group may have begun with the path before)
         ks = [k for (pp, _, _), k in offset.items() if pp == p]
-        first, last = min(ks) // 4, max(ks) // 4
+        first, last = -(-min(ks) // 4), max(ks) // 4
         lines = [f"const float4 t{k} = T[{k}];" for k in range(first, last + 1)]
         return lines, lambda mo, mi: f"t{offset[p, mo, mi] // 4}.{'xyzw'[offset[p, mo, mi] % 4]}"
 
@@ -367,8 +366,8 @@ def _emit_coupled(lin: int) -> str:
             l_in, l_out, off = path["l_in"], path["l_out"], path["in_off"]
             n_in, n_out = 2 * l_in + 1, 2 * l_out + 1
             loads, t = t_loads(p)
-            fwd.append(f"    {{  // path {p}: {l_in} x {path['l_edge']} -> {l_out}")
-            fwd.append(f"        const float2 wp = w[{p * ld}]; {' '.join(loads)}")
+            fwd.append(f"    {' '.join(loads)}\n    {{  // path {p}: {l_in} x {path['l_edge']} -> {l_out}")
+            fwd.append(f"        const float2 wp = w[{p * ld}];")
             if n_in <= n_out:
                 fwd.append("        " + " ".join(f"const float2 a{mi} = __fmul2_rn(wp, x{off + mi});" for mi in range(n_in)))
             for mo in range(n_out):
@@ -390,8 +389,8 @@ def _emit_coupled(lin: int) -> str:
             l_in, l_out, off = path["l_in"], path["l_out"], path["in_off"]
             n_in, n_out = 2 * l_in + 1, 2 * l_out + 1
             loads, t = t_loads(p)
-            bwd.append(f"    {{  // path {p}: {l_in} x {path['l_edge']} -> {l_out}")
-            bwd.append(f"        const float2 wp = w[{p * ld}]; {' '.join(loads)}")
+            bwd.append(f"    {' '.join(loads)}\n    {{  // path {p}: {l_in} x {path['l_edge']} -> {l_out}")
+            bwd.append(f"        const float2 wp = w[{p * ld}];")
             # gradient of the weighted sender features, shared by dx and by the derivative of the weight
             for mi in range(n_in):
                 outs = [mo for mo in range(n_out) if (p, mo, mi) in offset]
