@@ -14,6 +14,11 @@
 // rows (16-byte asynchronous copies) and couple the harmonics. A tile is one edge (forward: two) of each of the eight
 // ranges, so that a warp meets the edges of its rows one after the other. Registers are dealt again after the start.
 // Every wait is bounded (tc::mbar_wait).
+//
+// Bound by the evaluating warps: two per scheduler, FP32 pipe 52 %, shared memory 58 % and issue slots 53 % busy in the adjoint.
+// Adjoint / forward kernel, streamed and here: 62 k edges 145 -> 160 and 72 -> 90 us, 615 k edges 1,378 -> 1,374 and 650 -> 775,
+// and no producers (2 x 43 us and 2 x 360 us on the second stream, which slowed what ran beside them): a step of 1,944 atoms
+// 742 -> 683 us, a force call of 10,368 atoms 4,679 -> 3,956, one in chunks 6,190 -> 4,159.
 
 #include "stages.cuh"
 #include "generated/tp_generated.cuh"
