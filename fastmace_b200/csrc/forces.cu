@@ -475,7 +475,7 @@ int backward_layer(const Ctx& c, int layer, const float* d_h_out, float* d_h_in,
         if (edge_local_adjoint(c)) {
             // the later interaction has written the edge-vector gradients of the rows below n0; add this one's and
             // turn the per-edge gradients into forces and virials
-            const bool parts = !first_layer_of_pass && radial_on_chip(c);
+            const bool parts = !first_layer_of_pass && !c.exchange && radial_on_chip(c);
             FMB_TRY(first_adjoint_edges(f, first_layer_of_pass ? 0 : c.n0, c.w->edge_q, parts ? c.w->tp_w : nullptr, c.count_cap,
                                         c.stream));
             FMB_TRY(force_gather(c.n, c.exchange ? rows : c.n, c.nl->edge_row_ptr, c.nl->edge_index, c.w->mirror,
@@ -524,6 +524,11 @@ int backward_layer(const Ctx& c, int layer, const float* d_h_out, float* d_h_in,
                 FMB_TRY(tp_adjoint_edges(t, c.stream));
             }
             if (by_chunk || k == c.n_chunks - 1) FMB_TRY(gather_sender_gradient(t, by_chunk, c.stream));
+        }
+        if (on_chip && c.exchange) {
+            // the caller's turn comes before the first interaction's adjoint: nothing waits in tp_w for that
+            StageScope scope(c.stream, kStTpBwd1);
+            FMB_TRY(join_halves(c.n0, c.count_cap, c.nl->edge_row_ptr, c.w->edge_vec, c.w->tp_w, c.count_cap, c.w->edge_q, c.stream));
         }
         if (with_up) FMB_TRY(backward_linear_up(c, layer, d_h_in));
         return FMB_OK;

@@ -219,7 +219,7 @@ typedef struct {
     float* edge_hidden;               /* [n_layers][2][edge_capacity][64]: last hidden layer and its d/dr */
     float* tp_w;                      /* [2 * chunk_edges][max_paths * C]: weights, then their d/dr (both halves weights in the
                                          forward pass of a list in several chunks); scratch of the kernels that keep the
-                                         last radial layer on the SM */
+                                         last radial layer on the SM. Nothing in it is read after phase 1 of a phased call */
     float* x;                         /* [n_atoms][in_dim(1)][C] linear_up output of layer 1 */
     float* mid;                       /* [n_atoms][max mid_dim][C] scattered message (reused by both layers) */
     float* msg;                       /* [n_layers][n_atoms][16][C] */
