@@ -16,7 +16,7 @@ LIB_PATH = os.path.join(HERE, "libfmb200.so")
 MAX_ROW = 1024
 MAX_LAYERS = 2
 MAX_SPECIES = 8
-IMAGE_ONCHIP, IMAGE_FIRST_PADDED = 1, 2   # bits of LayerStruct.extra_images
+IMAGES, IMAGE_ONCHIP, IMAGE_FIRST_PADDED = 0x464d4200, 1, 2   # LayerStruct.extra_images: mark and bits
 
 STATUS_CAND_OVERFLOW = 1
 STATUS_ROW_OVERFLOW = 2

@@ -173,13 +173,15 @@ const long long* edge_limit(const Ctx& c, int which) {
 // rows of each half of tp_w (values, then d/dr)
 long long weight_rows(const Ctx& c) { return c.w->pair_capacity > 0 ? (long long)c.w->pair_capacity : c.chunk; }
 
+bool has_image(const fmb_layer_t& L, int bit) { return (L.extra_images & ~0xff) == FMB_IMAGES && (L.extra_images & bit) != 0; }
+
 // The last interaction with its last radial layer inside the kernels (tp_onchip.cu): the layer is packed for them, every row
 // carries a gradient, and tp_w, which then holds no weights, has room for their scratch. Not where rows are few: the kernels
 // load 160 KB of weights per CTA first and give every warp a range of edges, where the others cut a receiver's row in four.
 constexpr int kOnChipRows = 300;
 bool radial_on_chip(const Ctx& c) {
     const fmb_layer_t& L = c.m->layer[c.m->n_layers - 1];
-    if (c.m->n_layers < 2 || !L.rad_img || !(L.extra_images & FMB_IMAGE_ONCHIP) || !tensor_cores_enabled() || !edge_local_adjoint(c)) return false;
+    if (c.m->n_layers < 2 || !L.rad_img || !has_image(L, FMB_IMAGE_ONCHIP) || !tensor_cores_enabled() || !edge_local_adjoint(c)) return false;
     const long long scratch = tp_onchip_scratch_floats(L.l_in_max, c.count_cap);
     return c.n0 == c.n1 && c.n0 > kOnChipRows && scratch >= 0 && 2 * weight_rows(c) * L.n_paths * kC >= scratch;
 }
@@ -457,7 +459,7 @@ int backward_layer(const Ctx& c, int layer, const float* d_h_out, float* d_h_in,
             block_linear(lb, c, rows, c.w->d_msg, (long long)kNSH * kC, (long long)l * l * kC, kC, L.first[1], L.first[3], L.first_img[1],
                          (long long)l * nz * kRadial * kC, c.w->d_mid, s_atom, (long long)l * l * nz * kRadial,
                          nz * kRadial, l, 0);
-            if (L.extra_images & FMB_IMAGE_FIRST_PADDED) {
+            if (has_image(L, FMB_IMAGE_FIRST_PADDED)) {
                 GemmArgs& g = lb.list[lb.count - 1];
                 g.img_n = (g.n + 127) / 128 * 128;
                 g.b_img = L.first_img[1] + 2ll * l * kC * g.img_n;

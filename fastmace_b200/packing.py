@@ -17,7 +17,7 @@ import numpy as np
 import torch
 
 from . import so3
-from ._lib import IMAGE_FIRST_PADDED, IMAGE_ONCHIP, MAX_SPECIES, LayerStruct, ModelStruct
+from ._lib import IMAGE_FIRST_PADDED, IMAGE_ONCHIP, IMAGES, MAX_SPECIES, LayerStruct, ModelStruct
 from .codegen import message_slots
 from .model import SILU_NORM, MaceSpec, e0_table
 
@@ -334,7 +334,7 @@ class PackedModel:
                             if bool(torch.isfinite(w4).all()) and largest > 0 and largest_tangent > 0:
                                 layer.rad_img = self._put(f"l{t}.rad.img", torch.cat(
                                     [radial_image(w4, c), onchip_image(w4, largest, largest_tangent)]))
-                                layer.extra_images |= IMAGE_ONCHIP
+                                layer.extra_images |= IMAGES | IMAGE_ONCHIP
             if t == 0:
                 x_species = h0 @ (w["l0.up.0"] / math.sqrt(c))
                 sc = torch.zeros(len(idx), spec.out_dim(0), c, dtype=torch.float64)
@@ -361,7 +361,7 @@ class PackedModel:
                     # N = 64 for every species: an odd number of them leaves half a column tile
                     padded = [torch.nn.functional.pad(b.t(), (0, 64)) for b in blocks]
                     layer.first_img[1] = self._put("l0.first_t.img", tensor_core_image(padded))
-                    layer.extra_images |= IMAGE_FIRST_PADDED
+                    layer.extra_images |= IMAGES | IMAGE_FIRST_PADDED
                 else:
                     layer.first_img[1] = self._image_of("l0.first_t")
             else:

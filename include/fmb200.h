@@ -38,7 +38,9 @@ extern "C" {
 #define FMB_STATUS_NO_MIRROR 32u      /* an edge has no opposite edge: the neighbour list is not a full list */
 #define FMB_STATUS_PAIR_OVERFLOW 64u  /* more pairs of opposite edges than tp_w has rows (pair_capacity) */
 
-/* bits of fmb_layer_t.extra_images */
+/* fmb_layer_t.extra_images is FMB_IMAGES with bits below it; any other value, such as what a host left there that knows the
+ * field as padding, stands for no bits */
+#define FMB_IMAGES 0x464d4200
 #define FMB_IMAGE_ONCHIP 1            /* rad_img is followed by the image of the kernels that keep the last radial layer on the
                                          SM; without it they are not used */
 #define FMB_IMAGE_FIRST_PADDED 2      /* first_img[1]: blocks whose N is an odd multiple of 64 are padded with zero columns to a
@@ -132,7 +134,7 @@ typedef struct {
     int32_t n_sc_terms;               /* polynomial terms of the symmetric contraction */
     int32_t skip_lmax;
     int32_t is_last;
-    int32_t extra_images;             /* FMB_IMAGE_* bits: what the images below hold beyond what every host packs */
+    int32_t extra_images;             /* FMB_IMAGES | FMB_IMAGE_* bits: what the images below hold beyond what every host packs */
     const float* rad_w[4];            /* radial MLP, [in][out], 1/sqrt(fan_in) folded */
     const float* x_species;           /* layer 0: linear_up(embedding) per species [n_species][C] */
     const float* sc_species;          /* layer 0: skip connection per species [n_species][out_dim][C] */
