@@ -124,7 +124,7 @@ struct Cta {
     uint32_t bar0, tmem;
     volatile int* abort_flag;
     int slice, lane;
-    int begin, until, share, range0, ranges;   // edges of the launch, edges of a range, the first worker's range
+    int begin, until, share, range0;           // edges of the launch, edges of a range, the first worker's range
 
     __device__ __forceinline__ uint32_t bar(int slot) const { return bar0 + 8u * (uint32_t)slot; }
     __device__ __forceinline__ void wait(int slot, uint32_t parity) const { mbar_wait(bar(slot), parity, abort_flag, kSpin); }
@@ -325,19 +325,25 @@ __device__ __forceinline__ void bring_rows(const Cta<LIN, ADJOINT>& c, int part)
 
 // ------------------------------------------------------------------------------------------------ evaluating warps
 
-// The rows that begin in this warp's range, and first the rest of one that began in an earlier one (whose sum goes to `heads` and
-// is added to the row afterwards).
+// The rows with edges in this warp's range: the first may have begun in an earlier one (its sum goes to `heads` and is added to
+// the row afterwards). Rows without edges are passed over by a search: k_finish_rows writes them, spread over the GPU. (With
+// them written here 20,000 isolated atoms behind a crystal of 2,744 were one warp's: 7,660 us a force call.)
 template <int LIN>
 __device__ __forceinline__ void forward_range(const Cta<LIN, false>& c, int worker) {
     using S = Shape<LIN, false>;
     const int lane = c.lane, range = c.range0 + worker, first = c.first(worker), end = c.first(worker + 1), tiles = c.tiles();
-    const int r0 = lower_row(c.a.row_ptr, c.a.n_rows, first, lane);
-    const int r1 = range + 1 == c.ranges ? c.a.n_rows : lower_row(c.a.row_ptr, c.a.n_rows, end, lane);
-    const bool head = first < end && __ldg(c.a.row_ptr + r0) > first;
-    if (c.slice == 0 && lane == 0) c.a.head_row[range] = head ? r0 - 1 : -1;
-    int e = first, k = 0;
-    for (int row = head ? r0 - 1 : r0; row < r1 || (head && row < r0); ++row) {
-        const int re = min(__ldg(c.a.row_ptr + row + 1), end);
+    int row = first < end ? lower_row(c.a.row_ptr, c.a.n_rows, first + 1, lane) - 1 : 0, row_end = 0, k = 0;
+    const bool head = first < end && __ldg(c.a.row_ptr + row) < first;
+    if (c.slice == 0 && lane == 0) c.a.head_row[range] = head ? row : -1;
+    float* to = c.a.heads + (long long)range * S::MID * kC;
+    for (int e = first; e < end; ++row) {
+        row_end = __ldg(c.a.row_ptr + row + 1);
+        if (row_end <= e) {
+            row = lower_row(c.a.row_ptr, c.a.n_rows, e + 1, lane) - 1;
+            row_end = __ldg(c.a.row_ptr + row + 1);
+        }
+        if (!head || e > first) to = c.a.mid + (long long)row * S::MID * kC;
+        const int re = min(row_end, end);
         float2 acc[S::MID];
 #pragma unroll
         for (int q = 0; q < S::MID; ++q) acc[q] = make_float2(0.0f, 0.0f);
@@ -354,7 +360,6 @@ __device__ __forceinline__ void forward_range(const Cta<LIN, false>& c, int work
                 ++k;
             }
         }
-        float* const to = head && row < r0 ? c.a.heads + (long long)range * S::MID * kC : c.a.mid + (long long)row * S::MID * kC;
         float2* const out = reinterpret_cast<float2*>(to + c.slice * kCh) + lane;
 #pragma unroll
         for (int q = 0; q < S::MID; ++q) out[q * (kC / 2)] = acc[q];
@@ -472,7 +477,7 @@ k_tp_onchip(const __grid_constant__ OnChipArgs a) {
     __syncthreads();
     fence_after_sync();
     const Cta<LIN, ADJOINT> c{a, smem, smem_u32(bars), __shfl_sync(0xffffffffu, tmem_slot, 0), &abort_sh, (int)(blockIdx.x % kSlices), lane,
-                              begin, until, (until - begin + ranges - 1) / ranges, (int)(blockIdx.x / kSlices) * kWorkers, ranges};
+                              begin, until, (until - begin + ranges - 1) / ranges, (int)(blockIdx.x / kSlices) * kWorkers};
     if (warp < 8) {
         // this half of the last radial layer into tensor memory: lane = row, 32 words of value pairs, 32 of remainders
         const uint4* const image = reinterpret_cast<const uint4*>(a.image + 4) + (size_t)c.slice * S::kTiles * 2 * 1024 + (warp & 3) * 32 + lane;
@@ -511,13 +516,24 @@ k_tp_onchip(const __grid_constant__ OnChipArgs a) {
     }
 }
 
-// Adds the sums of the ranges behind a row's first to the row, in order: one CTA per range, the first of a row does it.
-constexpr int kHeadThreads = 512;
-__global__ void __launch_bounds__(kHeadThreads)
-k_add_heads(int ranges, int row_floats, const float* __restrict__ heads, const int32_t* __restrict__ head_row, float* __restrict__ mid) {
+// Zeroes the rows without edges (a lane looks at a row, a warp writes) and adds the sums of the ranges behind a row's first to the
+// row, in order: one CTA per range, the first of a row does it.
+constexpr int kFinishThreads = 512;
+__global__ void __launch_bounds__(kFinishThreads)
+k_finish_rows(int n_rows, int ranges, int row_floats, const int32_t* __restrict__ row_ptr, const float* __restrict__ heads,
+              const int32_t* __restrict__ head_row, float* __restrict__ mid) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int base = (warp * gridDim.x + blockIdx.x) * 32; base < n_rows; base += gridDim.x * kFinishThreads) {
+        const int mine = base + lane;
+        unsigned empty = __ballot_sync(0xffffffffu, mine < n_rows && __ldg(row_ptr + mine) == __ldg(row_ptr + mine + 1));
+        for (; empty; empty &= empty - 1) {
+            float4* const to = reinterpret_cast<float4*>(mid + (long long)(base + __ffs(empty) - 1) * row_floats);
+            for (int q = lane; q < row_floats / 4; q += 32) to[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    }
     const int range = blockIdx.x, row = head_row[range];
     if (row < 0 || (range > 0 && head_row[range - 1] == row)) return;
-    for (int q = threadIdx.x; q < row_floats / 4; q += kHeadThreads) {
+    for (int q = threadIdx.x; q < row_floats / 4; q += kFinishThreads) {
         float4* const to = reinterpret_cast<float4*>(mid + (long long)row * row_floats) + q;
         float4 sum = *to;
         for (int r = range; r < ranges && head_row[r] == row; ++r) {
@@ -545,7 +561,7 @@ int launch(const OnChipArgs& a, cudaStream_t stream) {
     k_tp_onchip<LIN, ADJOINT><<<grid, kThreads, S::kBytes, stream>>>(a);
     FMB_LAUNCH_CHECK();
     if (!ADJOINT) {
-        k_add_heads<<<ranges, kHeadThreads, 0, stream>>>(ranges, S::MID * kC, a.heads, a.head_row, a.mid);
+        k_finish_rows<<<ranges, kFinishThreads, 0, stream>>>(a.n_rows, ranges, S::MID * kC, a.row_ptr, a.heads, a.head_row, a.mid);
         FMB_LAUNCH_CHECK();
     }
     return FMB_OK;
