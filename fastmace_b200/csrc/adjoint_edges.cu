@@ -494,29 +494,6 @@ int grid_for(const void* kernel, int rows, int threads, size_t smem) {
     return rows < cap ? rows : cap;
 }
 
-// The second interaction's gradients of harmonics and length (two halves of the channels, tp_onchip.cu) as gradients of the
-// edge vector: a thread per edge. Bound by the 160 bytes an edge has there; the first interaction's adjoint adds them up
-// itself where nothing of the caller's comes between the two.
-constexpr int kJoinThreads = 256;
-__global__ void __launch_bounds__(kJoinThreads)
-k_join_halves(int n_rows, long long capacity, const int32_t* __restrict__ row_ptr, const float* __restrict__ edge_vec,
-              const float* __restrict__ parts, long long part_stride, float4* __restrict__ qe) {
-    const int edges = (int)min((long long)row_ptr[n_rows], capacity);
-    for (int e = blockIdx.x * kJoinThreads + threadIdx.x; e < edges; e += gridDim.x * kJoinThreads) {
-        const float* const a = parts + (long long)e * 20;
-        const float* const b = a + part_stride * 20;
-        float g[16], q[3];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float4 va = __ldg(reinterpret_cast<const float4*>(a) + k), vb = __ldg(reinterpret_cast<const float4*>(b) + k);
-            g[4 * k] = va.x + vb.x; g[4 * k + 1] = va.y + vb.y; g[4 * k + 2] = va.z + vb.z; g[4 * k + 3] = va.w + vb.w;
-        }
-        const float4 uv = __ldg(reinterpret_cast<const float4*>(edge_vec) + e);
-        edge_vector_gradient(g, __ldg(a + 16) + __ldg(b + 16), uv.x, uv.y, uv.z, uv.w, q);
-        qe[e] = make_float4(q[0], q[1], q[2], 0.0f);
-    }
-}
-
 }  // namespace
 
 int mirror_map(const fmb_nl_t* nl, int32_t* mirror, uint32_t* status, const long long* listed_below, int32_t* slot,
@@ -575,17 +552,6 @@ int first_adjoint_edges(const FirstArgs& f, int n_add, float* qe, const float* p
     k_first_adjoint_rows<<<f.n_rows < grid_cap ? f.n_rows : grid_cap, kFaThreads, smem, stream>>>(
         f.n_rows, f.n_valid, n_add, f.n_species, f.row_ptr, f.senders, f.species, f.edge_sh, f.edge_vec, f.hidden,
         f.hidden_tangent, f.d_s, reinterpret_cast<float4*>(qe), parts, part_stride);
-    FMB_LAUNCH_CHECK();
-    return FMB_OK;
-}
-
-int join_halves(int n_rows, long long capacity, const int32_t* row_ptr, const float* edge_vec, const float* parts,
-                long long part_stride, float* qe, cudaStream_t stream) {
-    static const int grid_cap = grid_for((const void*)k_join_halves, 1 << 30, kJoinThreads, 0);
-    const long long blocks = (capacity + kJoinThreads - 1) / kJoinThreads;
-    k_join_halves<<<blocks < grid_cap ? (int)blocks : grid_cap, kJoinThreads, 0, stream>>>(n_rows, capacity, row_ptr, edge_vec,
-                                                                                          parts, part_stride,
-                                                                                          reinterpret_cast<float4*>(qe));
     FMB_LAUNCH_CHECK();
     return FMB_OK;
 }

@@ -186,6 +186,12 @@ bool radial_on_chip(const Ctx& c) {
     return c.n0 == c.n1 && c.n0 > kOnChipRows && scratch >= 0 && 2 * weight_rows(c) * L.n_paths * kC >= scratch;
 }
 
+// where the adjoint's partial gradients of harmonics and length are when the first interaction's adjoint adds them up
+static_assert(tp_onchip_part_floats(1) <= 2 * kRadial, "an edge's partial gradients fit in its hidden features and their d/dr");
+float* onchip_parts(const Ctx& c) {
+    return c.exchange ? c.w->edge_hidden + 2ll * (c.m->n_layers - 1) * c.count_cap * kRadial : c.w->tp_w;
+}
+
 // One row of radial weights per pair of opposite edges (they have the same length): the whole list is one chunk whose
 // weights are kept, the per-edge adjoint's mirror map exists, and the tensor-core producer applies (the kernels of a
 // whole list read the rows by slot).
@@ -477,8 +483,8 @@ int backward_layer(const Ctx& c, int layer, const float* d_h_out, float* d_h_in,
         if (edge_local_adjoint(c)) {
             // the later interaction has written the edge-vector gradients of the rows below n0; add this one's and
             // turn the per-edge gradients into forces and virials
-            const bool parts = !first_layer_of_pass && !c.exchange && radial_on_chip(c);
-            FMB_TRY(first_adjoint_edges(f, first_layer_of_pass ? 0 : c.n0, c.w->edge_q, parts ? c.w->tp_w : nullptr, c.count_cap,
+            const bool parts = !first_layer_of_pass && radial_on_chip(c);
+            FMB_TRY(first_adjoint_edges(f, first_layer_of_pass ? 0 : c.n0, c.w->edge_q, parts ? onchip_parts(c) : nullptr, c.count_cap,
                                         c.stream));
             FMB_TRY(force_gather(c.n, c.exchange ? rows : c.n, c.nl->edge_row_ptr, c.nl->edge_index, c.w->mirror,
                                  c.w->edge_q, c.w->edge_vec, c.w->force_acc, c.w->atom_virial, c.stream));
@@ -528,9 +534,11 @@ int backward_layer(const Ctx& c, int layer, const float* d_h_out, float* d_h_in,
             if (by_chunk || k == c.n_chunks - 1) FMB_TRY(gather_sender_gradient(t, by_chunk, c.stream));
         }
         if (on_chip && c.exchange) {
-            // the caller's turn comes before the first interaction's adjoint: nothing waits in tp_w for that
+            // the caller's turn comes before the first interaction's adjoint, and tp_w is theirs from here on: what waits for
+            // that adjoint moves to this layer's hidden features, which nothing reads any more (1 % of a step of two bricks of 3,456 atoms)
             StageScope scope(c.stream, kStTpBwd1);
-            FMB_TRY(join_halves(c.n0, c.count_cap, c.nl->edge_row_ptr, c.w->edge_vec, c.w->tp_w, c.count_cap, c.w->edge_q, c.stream));
+            FMB_CUDA_CHECK(cudaMemcpyAsync(onchip_parts(c), c.w->tp_w, (size_t)tp_onchip_part_floats(c.count_cap) * sizeof(float),
+                                           cudaMemcpyDeviceToDevice, c.stream));
         }
         if (with_up) FMB_TRY(backward_linear_up(c, layer, d_h_in));
         return FMB_OK;

@@ -116,6 +116,8 @@ struct TpOnChipArgs {
 };
 // floats of `scratch` for a list of `edges` edges (negative: no kernel for this node l_max)
 long long tp_onchip_scratch_floats(int lin, long long edges);
+// of them the adjoint's output
+constexpr long long tp_onchip_part_floats(long long edges) { return 2 * edges * 20; }
 int tp_forward_onchip(const TpOnChipArgs& t, cudaStream_t stream);
 int tp_adjoint_onchip(const TpOnChipArgs& t, cudaStream_t stream);
 
@@ -133,9 +135,6 @@ int gather_sender_gradient(const EdgeAdjointArgs& t, bool chunk, cudaStream_t st
 // interaction's gradients of harmonics and length, parts[2][part_stride][20], to its own before they become one of the edge
 // vector, and what qe holds is not read
 int first_adjoint_edges(const FirstArgs& f, int n_add, float* qe, const float* parts, long long part_stride, cudaStream_t stream);
-// `parts` as gradients of the edge vector in qe, for the edges of the rows below n_rows
-int join_halves(int n_rows, long long capacity, const int32_t* row_ptr, const float* edge_vec, const float* parts,
-                long long part_stride, float* qe, cudaStream_t stream);
 // forces (as gradients) and per-atom virials from the per-edge gradients; only the edges into atoms [0, n_valid) carry
 // a gradient (the others are read as zero, whatever qe holds for them)
 int force_gather(int n_atoms, int n_valid, const int32_t* row_ptr, const int32_t* senders, const int32_t* mirror,

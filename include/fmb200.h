@@ -218,7 +218,8 @@ typedef struct {
     const int32_t* species;           /* [n_atoms] index into the present species */
     float* edge_vec;                  /* [edge_capacity][4] unit vector and length */
     float* edge_sh;                   /* [edge_capacity][16] */
-    float* edge_hidden;               /* [n_layers][2][edge_capacity][64]: last hidden layer and its d/dr */
+    float* edge_hidden;               /* [n_layers][2][edge_capacity][64]: last hidden layer and its d/dr; the last layer's holds
+                                         other things from phase 1 to phase 2 of a phased call */
     float* tp_w;                      /* [2 * chunk_edges][max_paths * C]: weights, then their d/dr (both halves weights in the
                                          forward pass of a list in several chunks); scratch of the kernels that keep the
                                          last radial layer on the SM. Nothing in it is read after phase 1 of a phased call */
