@@ -326,7 +326,7 @@ TpOnChipArgs onchip_args(const Ctx& c, int layer) {
     const fmb_layer_t& L = c.m->layer[layer];
     TpOnChipArgs t{};
     t.lin = L.l_in_max; t.n_rows = c.n1; t.row_ptr = c.nl->edge_row_ptr; t.senders = c.nl->edge_index; t.x = c.w->x;
-    t.edge_sh = c.w->edge_sh; t.hidden = hidden_of(c, layer, 0); t.tangent = hidden_of(c, layer, 1);
+    t.edge_sh = c.w->edge_sh; t.edge_vec = c.w->edge_vec; t.hidden = hidden_of(c, layer, 0); t.tangent = hidden_of(c, layer, 1);
     t.image = L.rad_img + (long long)L.n_paths * 4 * 4096;
     t.mid = c.w->mid; t.d_mid = c.w->d_mid; t.e_span = c.count_cap; t.dxe = c.w->edge_dx; t.scratch = c.w->tp_w;
     t.part_stride = c.count_cap; t.error_word = c.w->status;

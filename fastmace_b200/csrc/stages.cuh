@@ -100,6 +100,7 @@ struct TpOnChipArgs {
     const int32_t* senders;
     const float* x;
     const float* edge_sh;
+    const float* edge_vec;
     const float* hidden;           // [edges][64]
     const float* tangent;
     const float* image;            // the last radial layer, behind the producer's image in fmb_layer_t.rad_img

@@ -2,15 +2,21 @@
 // 1): the per-edge radial weights and their d/dr are products of the tensor cores that never leave the SM, where the kernels of
 // tp_coupled.cu read them from memory (20 P C bytes written and read per pair of edges and force call).
 //
-// The last radial layer stays in tensor memory. As fp16 values and remainders (22 bits, as many as the tf32 pair holds) the
-// columns of half the channels, 640 of them, take 320 of 512 TMEM columns as the first operand of the MMAs, K along the
+// The last radial layer stays in tensor memory. As fp16 values and remainders the columns of half the channels, 640 of them,
+// take 320 of 512 TMEM columns as the first operand of the MMAs, K along the
 // columns; two CTAs share a range of edges, one per half. An MMA whose first operand is in TMEM
 // takes 12 cycles at N = 16 where one that reads 128 rows from shared memory takes 40 whatever its N. The second operand is the
 // hidden radial features of a tile, split in the kernel: 16 edges, or 8 edges and their d/dr.
 //
+// A pair of fp16 numbers holds the 22 bits of a tf32 pair down to 2^-17 of the top of its scale. The features of an edge near
+// the cutoff have a scale of their own (Splitter); the layer has one, and only layers whose products come out as the tf32
+// pairs give them are packed (packing.onchip_is_accurate). Message and adjoint of single pairs against float64, relative
+// to their norm: 1.2e-7 to 1.9e-7 at any length, 4e-7 with the weights of the tf32 pairs; with one scale for all lengths
+// 8e-7 at 5.9 A, 1e-5 at 5.95 and 7e-3 at 5.99.
+//
 // Warps: eight that evaluate edges, each a contiguous range of its own, a lane two channels on the packed FP32 pipe (the
 // bodies of tp_coupled.cu); four that carry a tile's weights from TMEM, where a lane is a channel of one path, to the
-// edges' blocks in shared memory; one that issues the MMAs, one that splits hidden features, two that bring the senders'
+// edges' blocks in shared memory; two that split hidden features, one of which issues the MMAs; two that bring the senders'
 // rows (16-byte asynchronous copies) and couple the harmonics. A tile is one edge (forward: two) of each of the eight
 // ranges, so that a warp meets the edges of its rows one after the other. Registers are dealt again after the start.
 // Every wait is bounded (tc::mbar_wait).
@@ -41,6 +47,9 @@ constexpr int kThreads = 512;
 constexpr int kBSlots = 2;                     // tiles of hidden features between the split and the MMAs
 constexpr int kBSlotBytes = 4096;              // [16 rows][64] fp16 values, then remainders
 constexpr int kAccumulators = 2;
+constexpr int kScaleSlots = 8;                 // tiles whose rows' scales are kept: tile k's are written while tile k - 4's may be read
+constexpr float kNearest = 0.001953125f;       // A from the cutoff: closer edges are scaled like one there
+constexpr int kHeader = 8;                     // floats before the weights
 constexpr int kPartFloats = 20;                // of an edge's sums: 16 harmonics, the length, 3 unused
 
 template <int LIN, bool ADJOINT>
@@ -55,7 +64,8 @@ struct Shape {
     static constexpr int kStages = ADJOINT ? 4 : 3;
     static constexpr int kY = kEdges * 64;
     static constexpr int kWorkerRegisters = 168;                       // of 256 for a worker's and a feeding warp's thread together
-    static constexpr int kB = 0, kStage0 = kBSlots * kBSlotBytes, kY0 = kStage0 + kStages * kStageBytes, kBytes = kY0 + kY + 1024;
+    static constexpr int kB = 0, kStage0 = kBSlots * kBSlotBytes, kY0 = kStage0 + kStages * kStageBytes,
+                         kScale0 = kY0 + kY, kBytes = kScale0 + kScaleSlots * 72 + 1024;
     static constexpr int kBFull = 0, kBEmpty = kBSlots, kDFull = 2 * kBSlots, kDEmpty = kDFull + kAccumulators,
                          kFull = kDEmpty + kAccumulators, kEmpty = kFull + kStages, kBars = kEmpty + kStages;
     static_assert(P % 2 == 0 && kWColumns + kAccumulators * kDColumns <= 512 && kBytes <= 226 * 1024 && kBlock % 4 == 0, "fits an SM");
@@ -67,9 +77,10 @@ struct OnChipArgs {
     const int32_t* senders;
     const float* x;
     const float* edge_sh;
+    const float* edge_vec;
     const float* hidden;
     const float* tangent;
-    const float* image;            // [4] scales, then [slice][tile][value, remainder][8][128][4] words
+    const float* image;            // [kHeader] (packing.onchip_image), then [slice][tile][value, remainder][8][128][4] words
     float* mid;
     float* heads;                  // forward: [range][MID][C] sums of rows that begin in an earlier range
     int32_t* head_row;             // forward: [range] that row, or -1
@@ -142,6 +153,13 @@ struct Cta {
         return at < share && e < until ? (int)e : -1;
     }
     __device__ __forceinline__ int tiles() const { return (first(1) - first(0) + S::kPerWorker - 1) / S::kPerWorker; }
+    __device__ __forceinline__ float* scales(int k) const {
+        return reinterpret_cast<float*>(smem + S::kScale0) + (k % kScaleSlots) * 16;
+    }
+    // per part of the split: whether a row of tile k may have a scale that is not 1
+    __device__ __forceinline__ int* scaled(int k) const {
+        return reinterpret_cast<int*>(smem + S::kScale0 + kScaleSlots * 64) + (k % kScaleSlots) * 2;
+    }
     __device__ __forceinline__ float* block(int k, int q) const {
         return reinterpret_cast<float*>(smem + S::kStage0 + (k % S::kStages) * S::kStageBytes) + q * S::kBlock;
     }
@@ -149,13 +167,119 @@ struct Cta {
 
 // ------------------------------------------------------------------------------------------------ feeding warps
 
+// exponent field of the power of two that brings v >= 0 to [1, 2), or as near as powers of two go
+__device__ __forceinline__ unsigned power_below(float v) { return min(254u - (__float_as_uint(v) >> 23), 253u); }
+
+// Hidden radial features into the second operand (16 rows of 64 fp16, K-major, 128-byte swizzle; values, then remainders): the
+// 16 edges of a tile, or its 8 edges and then their d/dr. Two warps split 8 rows each, those of the next tile on their way
+// meanwhile: a warp shares its scheduler with two that evaluate, and one for all 16 rows was what the adjoint waited for (615 k
+// edges with the gather behind it, the scales below included: 1,788 -> 1,620 us).
+//
+// Features of an edge near the cutoff are a million times smaller than those of a bond: they vanish with the fourth power of
+// its distance from the cutoff (envelope and Bessel functions), their d/dr with the third. fp16 numbers below 2^-14 are
+// spaced 2^-24: a row whose largest magnitude is below 1/4 at the scale that all share would be held less exactly than by
+// tf32 pairs (2^-23 of the largest). By those laws rows of edges of a certain length or more are brought up by a power
+// of two, and what takes their products back is left in `scales`. (Looking for the largest magnitude of every row instead
+// cost twice as much.)
+template <int LIN, bool ADJOINT>
+struct Splitter {
+    using S = Shape<LIN, ADJOINT>;
+    const Cta<LIN, ADJOINT>& c;
+    const int part, col, half;                 // of the rows; of a row's 16 pieces of four; row of a pair
+    const float* const from;
+    const float scale, reach, cutoff, size;
+    int apart, at, my_at;
+    float length;
+    float4 held[4];
+
+    __device__ __forceinline__ Splitter(const Cta<LIN, ADJOINT>& c_, int part_)
+        : c(c_), part(part_), col(c_.lane & 15), half(c_.lane >> 4), from((ADJOINT && part_ ? c_.a.tangent : c_.a.hidden) + 4 * (c_.lane & 15)),
+          scale(__ldg(c_.a.image + (ADJOINT ? part_ : 0))), reach(__ldg(c_.a.image + 3)), cutoff(__ldg(c_.a.image + 4)),
+          size(__ldg(c_.a.image + (ADJOINT && part_ ? 6 : 5))) {
+        // row 2 i + half of this part is the edge at + i * apart; lane q < 8 looks at the length of its edge q
+        const int range = c.range0 + (ADJOINT ? 0 : 4 * part), lane = c.lane;
+        apart = (ADJOINT ? 2 : 1) * c.share;
+        at = c.begin + c.share * (range + (ADJOINT ? half : 0)) + (ADJOINT ? 0 : half);
+        my_at = c.begin + c.share * (range + (ADJOINT ? lane : lane >> 1)) + (ADJOINT ? 0 : lane & 1);
+        fetch(0);
+    }
+
+    __device__ __forceinline__ void fetch(int k) {
+        const int left = c.share - k * S::kPerWorker;          // edges of a range from this tile on
+        const bool inside = ADJOINT || half < left;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int e = at + i * apart;
+            held[i] = inside && (unsigned)e < (unsigned)c.until ? __ldg(reinterpret_cast<const float4*>(from + (long long)e * kRadial))
+                                                                : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        length = c.lane < 8 && (ADJOINT || (c.lane & 1) < left) && (unsigned)my_at < (unsigned)c.until
+                     ? __ldg(c.a.edge_vec + 4ll * my_at + 3) : 0.0f;
+        at += S::kPerWorker;
+        my_at += S::kPerWorker;
+    }
+
+    __device__ __forceinline__ void put(int k, int tiles) {
+        const bool small = !(length < reach);
+        const unsigned near = __ballot_sync(0xffffffffu, small);
+        if (near) {
+            // power of two, as exponent field, for the row of this lane's edge if its largest is below 1/4 (4 law at most):
+            // to [1, 8], so that features that are far above the law, by the rounding of what made them, still fit
+            const float d = fmaxf(cutoff - length, kNearest), law = (ADJOINT && part ? d * d : d * d * d) * d * size;
+            const unsigned field = small && law < 0.0625f ? power_below(law) : 127u;
+            if (c.lane < 8) c.scales(k)[8 * part + c.lane] = __uint_as_float((254u - field) << 23);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if ((near >> 2 * i & 3u) == 0) continue;
+                const float up = __uint_as_float(__shfl_sync(0xffffffffu, field, 2 * i + half) << 23);
+                held[i].x *= up; held[i].y *= up; held[i].z *= up; held[i].w *= up;
+            }
+        }
+        if (c.lane == 0) c.scaled(k)[part] = near != 0;
+        uint2 value[4], rest[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 lo = make_float2(held[i].x * scale, held[i].y * scale), hi = make_float2(held[i].z * scale, held[i].w * scale);
+            const __half2 vl = __float22half2_rn(lo), vh = __float22half2_rn(hi);
+            const float2 bl = __half22float2(vl), bh = __half22float2(vh);
+            const __half2 rl = __float22half2_rn(make_float2(lo.x - bl.x, lo.y - bl.y)),
+                          rh = __float22half2_rn(make_float2(hi.x - bh.x, hi.y - bh.y));
+            value[i] = make_uint2(reinterpret_cast<const uint32_t&>(vl), reinterpret_cast<const uint32_t&>(vh));
+            rest[i] = make_uint2(reinterpret_cast<const uint32_t&>(rl), reinterpret_cast<const uint32_t&>(rh));
+        }
+        if (k + 1 < tiles) fetch(k + 1);
+        const int slot = k % kBSlots;
+        c.wait(S::kBEmpty + slot, ((uint32_t)(k / kBSlots) & 1u) ^ 1u);
+        uint8_t* const tile = c.smem + S::kB + slot * kBSlotBytes + part * 1024;       // 8 rows
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = 2 * i + half, to = row * 128 + (((col >> 1) ^ row) << 4) + (col & 1) * 8;
+            *reinterpret_cast<uint2*>(tile + to) = value[i];
+            *reinterpret_cast<uint2*>(tile + 2048 + to) = rest[i];
+        }
+        fence_async_smem();
+        c.arrive(S::kBFull + slot);
+    }
+};
+
+// The first part of the split.
+template <int LIN, bool ADJOINT>
+__device__ __forceinline__ void split_features(const Cta<LIN, ADJOINT>& c) {
+    const int tiles = c.tiles();
+    Splitter<LIN, ADJOINT> split(c, 0);
+#pragma unroll 1
+    for (int k = 0; k < tiles; ++k) split.put(k, tiles);
+}
+
 // The MMAs of the tiles: remainder x value, value x remainder, value x value over K = 64, the small products first (the
-// tensor core truncates its accumulator at every instruction).
+// tensor core truncates its accumulator at every instruction); the second part of the next tile's split while they run.
 template <int LIN, bool ADJOINT>
 __device__ __forceinline__ void issue_products(const Cta<LIN, ADJOINT>& c) {
     using S = Shape<LIN, ADJOINT>;
     constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(16 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);   // D fp32, A and B fp16
     const int tiles = c.tiles();
+    Splitter<LIN, ADJOINT> split(c, 1);
+    if (tiles > 0) split.put(0, tiles);
 #pragma unroll 1
     for (int k = 0; k < tiles; ++k) {
         const int slot = k % kBSlots, acc = k % kAccumulators;
@@ -177,59 +301,25 @@ __device__ __forceinline__ void issue_products(const Cta<LIN, ADJOINT>& c) {
             }
             mma_commit(c.bar(S::kBEmpty + slot));
             mma_commit(c.bar(S::kDFull + acc));
+            mbar_arrive(c.bar(S::kDFull + acc));                      // hands on what the split left in `scales`
         }
         __syncwarp();
+        if (k + 1 < tiles) split.put(k + 1, tiles);
     }
 }
 
-// Hidden radial features into the second operand (16 rows of 64 fp16, K-major, 128-byte swizzle; values, then remainders): the
-// 16 edges of a tile, or its 8 edges and then their d/dr. The rows of the next tile are on their way meanwhile.
-template <int LIN, bool ADJOINT>
-__device__ __forceinline__ void split_features(const Cta<LIN, ADJOINT>& c) {
-    using S = Shape<LIN, ADJOINT>;
-    const int lane = c.lane, col = lane & 15, half = lane >> 4, tiles = c.tiles();
-    const float scale = __ldg(c.a.image), tangent_scale = __ldg(c.a.image + 1);
-    float4 held[8];
-    auto fetch = [&](int k) {
+// eight columns of the accumulator back to the common scale
+template <int FIRST>
+__device__ __forceinline__ void unscale(float (&v)[16], const float* scales) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int e = c.edge(k, ADJOINT ? 2 * (i & 3) + half : 2 * i + half);
-            const float* const from = (ADJOINT && i >= 4 ? c.a.tangent : c.a.hidden) + 4 * col;
-            held[i] = e >= 0 ? __ldg(reinterpret_cast<const float4*>(from + (long long)e * kRadial)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    };
-    fetch(0);
-#pragma unroll 1
-    for (int k = 0; k < tiles; ++k) {
-        uint2 value[8], rest[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float s = ADJOINT && i >= 4 ? tangent_scale : scale;
-            const float2 lo = make_float2(held[i].x * s, held[i].y * s), hi = make_float2(held[i].z * s, held[i].w * s);
-            const __half2 vl = __float22half2_rn(lo), vh = __float22half2_rn(hi);
-            const float2 bl = __half22float2(vl), bh = __half22float2(vh);
-            const __half2 rl = __float22half2_rn(make_float2(lo.x - bl.x, lo.y - bl.y)),
-                          rh = __float22half2_rn(make_float2(hi.x - bh.x, hi.y - bh.y));
-            value[i] = make_uint2(reinterpret_cast<const uint32_t&>(vl), reinterpret_cast<const uint32_t&>(vh));
-            rest[i] = make_uint2(reinterpret_cast<const uint32_t&>(rl), reinterpret_cast<const uint32_t&>(rh));
-        }
-        if (k + 1 < tiles) fetch(k + 1);
-        const int slot = k % kBSlots;
-        c.wait(S::kBEmpty + slot, ((uint32_t)(k / kBSlots) & 1u) ^ 1u);
-        uint8_t* const tile = c.smem + S::kB + slot * kBSlotBytes;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int row = 2 * i + half;
-            const int at = (row >> 3) * 1024 + (row & 7) * 128 + (((col >> 1) ^ (row & 7)) << 4) + (col & 1) * 8;
-            *reinterpret_cast<uint2*>(tile + at) = value[i];
-            *reinterpret_cast<uint2*>(tile + 2048 + at) = rest[i];
-        }
-        fence_async_smem();
-        c.arrive(S::kBFull + slot);
+    for (int q = FIRST; q < FIRST + 8; q += 2) {
+        const float2 w = __fmul2_rn(make_float2(v[q], v[q + 1]), *reinterpret_cast<const float2*>(scales + q));
+        v[q] = w.x;
+        v[q + 1] = w.y;
     }
 }
 
-// Weights of a tile from the accumulator (lane = channel of a path, column = edge) to the edges' blocks.
+// Weights of a tile from the accumulator (lane = channel of a path, column = edge) to the edges' blocks, at the common scale.
 template <int LIN, bool ADJOINT>
 __device__ __forceinline__ void carry_weights(const Cta<LIN, ADJOINT>& c, int quadrant) {
     using S = Shape<LIN, ADJOINT>;
@@ -241,11 +331,14 @@ __device__ __forceinline__ void carry_weights(const Cta<LIN, ADJOINT>& c, int qu
         c.wait(S::kEmpty + st, ((uint32_t)(k / S::kStages) & 1u) ^ 1u);
         c.wait(S::kDFull + acc, (uint32_t)(k / kAccumulators) & 1u);
         fence_after_sync();
+        const int2 scaled = *reinterpret_cast<const int2*>(c.scaled(k));
         float* const to = c.block(k, 0) + at;
 #pragma unroll
         for (int j = 0; j < S::kTiles; ++j) {
             float v[16];
             tmem_load_16(base + acc * S::kDColumns + 16 * j, v);
+            if (scaled.x) unscale<0>(v, c.scales(k));
+            if (scaled.y) unscale<8>(v, c.scales(k));
             if (j == S::kTiles - 1) {
                 fence_before_sync();
                 c.arrive(S::kDEmpty + acc);
@@ -456,11 +549,11 @@ k_tp_onchip(const __grid_constant__ OnChipArgs a) {
     if (warp == 12) {
         if (elect_one()) {
             for (int q = 0; q < kBSlots; ++q) {
-                mbar_init(smem_u32(bars + S::kBFull + q), 1);
+                mbar_init(smem_u32(bars + S::kBFull + q), 2);             // the two parts of the split
                 mbar_init(smem_u32(bars + S::kBEmpty + q), 1);
             }
             for (int q = 0; q < kAccumulators; ++q) {
-                mbar_init(smem_u32(bars + S::kDFull + q), 1);
+                mbar_init(smem_u32(bars + S::kDFull + q), 2);             // the products, and their issuer
                 mbar_init(smem_u32(bars + S::kDEmpty + q), 4);
             }
             for (int q = 0; q < S::kStages; ++q) {
@@ -480,7 +573,7 @@ k_tp_onchip(const __grid_constant__ OnChipArgs a) {
                               begin, until, (until - begin + ranges - 1) / ranges, (int)(blockIdx.x / kSlices) * kWorkers};
     if (warp < 8) {
         // this half of the last radial layer into tensor memory: lane = row, 32 words of value pairs, 32 of remainders
-        const uint4* const image = reinterpret_cast<const uint4*>(a.image + 4) + (size_t)c.slice * S::kTiles * 2 * 1024 + (warp & 3) * 32 + lane;
+        const uint4* const image = reinterpret_cast<const uint4*>(a.image + kHeader) + (size_t)c.slice * S::kTiles * 2 * 1024 + (warp & 3) * 32 + lane;
         for (int part = warp >> 2; part < 2 * S::kTiles; part += 2) {
             uint32_t v[32];
 #pragma unroll
@@ -581,7 +674,7 @@ long long tp_onchip_scratch_floats(int lin, long long edges) {
 int tp_forward_onchip(const TpOnChipArgs& t, cudaStream_t stream) {
     if (t.lin != 1) return FMB_ERR_UNSUPPORTED;
     OnChipArgs a{};
-    a.n_rows = t.n_rows; a.row_ptr = t.row_ptr; a.senders = t.senders; a.x = t.x; a.edge_sh = t.edge_sh; a.hidden = t.hidden;
+    a.n_rows = t.n_rows; a.row_ptr = t.row_ptr; a.senders = t.senders; a.x = t.x; a.edge_sh = t.edge_sh; a.edge_vec = t.edge_vec; a.hidden = t.hidden;
     a.image = t.image; a.mid = t.mid; a.heads = t.scratch; a.error_word = t.error_word;
     a.head_row = reinterpret_cast<int32_t*>(t.scratch + (long long)(device_sms() / kSlices * kWorkers) * TpShape<1>::kMidDim * kC);
     return launch<1, false>(a, stream);
@@ -590,7 +683,7 @@ int tp_forward_onchip(const TpOnChipArgs& t, cudaStream_t stream) {
 int tp_adjoint_onchip(const TpOnChipArgs& t, cudaStream_t stream) {
     if (t.lin != 1) return FMB_ERR_UNSUPPORTED;
     OnChipArgs a{};
-    a.n_rows = t.n_rows; a.row_ptr = t.row_ptr; a.senders = t.senders; a.x = t.x; a.edge_sh = t.edge_sh; a.hidden = t.hidden;
+    a.n_rows = t.n_rows; a.row_ptr = t.row_ptr; a.senders = t.senders; a.x = t.x; a.edge_sh = t.edge_sh; a.edge_vec = t.edge_vec; a.hidden = t.hidden;
     a.tangent = t.tangent; a.image = t.image; a.d_mid = t.d_mid; a.dxe = t.dxe; a.parts = t.scratch; a.part_stride = t.part_stride;
     a.e0 = t.e0; a.e_span = t.e_span; a.dx0 = t.dx0; a.error_word = t.error_word;
     return launch<1, true>(a, stream);

@@ -131,26 +131,86 @@ def mlp_image(w0: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor) -> torch.Ten
     return image
 
 
-ONCHIP_HEADER = 4                      # floats before the image: three scales, one unused
+ONCHIP_HEADER = 8                      # floats before the image
+ONCHIP_NEAREST = 2.0 ** -9             # distance from the cutoff below which the kernels' scales no longer grow
 
 
-def onchip_image(w4: torch.Tensor, largest: float, largest_tangent: float) -> torch.Tensor:
+def onchip_image(w4: torch.Tensor, largest: float, largest_tangent: float, long=(math.inf, math.inf, 0.0, 0.0)) -> torch.Tensor:
     """The last radial layer [64][paths * 128] (fp32, already scaled) as the kernels that evaluate the tensor product
     beside it keep it in tensor memory, fp32 words: a header (scale of the hidden features, scale of their d/dr, inverse of
-    the product's scale; powers of two that put the ``largest`` magnitudes half way up the fp16 range), then per half of the
+    the product's scale; powers of two that put the ``largest`` magnitudes half way up the fp16 range; then ``onchip_long``'s
+    four numbers, one unused), then per half of the
     channels and pair of paths the values and the remainders of 128 rows (path, channel of the half) of 64 weights as fp16
     pairs, [8][128 rows][4 words] each."""
     k, n = w4.shape
     paths = n // 128
     w = w4.to(torch.float64).t().reshape(paths, 2, 64, k)                       # [path][half][channel][64]
-    scale = [2.0 ** min(math.floor(math.log2(32768.0 / max(float(v), 1e-30))), 40) for v in (largest, largest_tangent, w.abs().max())]
+    scale = [onchip_scale(v) for v in (largest, largest_tangent, w.abs().max())]
     rows = (w * scale[2]).transpose(0, 1).reshape(2, paths // 2, 128, k)
     value = rows.to(torch.float16)
     rest = (rows - value.to(torch.float64)).to(torch.float16)
     image = torch.stack([value, rest], dim=2)                                   # [half][pair][part][128][64]
     image = image.reshape(2, paths // 2, 2, 128, 8, 8).transpose(3, 4).contiguous()
-    header = torch.tensor([scale[0], scale[1], 1.0 / (scale[0] * scale[2]), 0.0], dtype=torch.float64)
+    header = torch.tensor([scale[0], scale[1], 1.0 / (scale[0] * scale[2]), *long, 0.0], dtype=torch.float64)
     return torch.cat([header.to(torch.float32), image.reshape(-1).view(torch.float32)])
+
+
+def onchip_scale(largest: float) -> float:
+    return 2.0 ** min(math.floor(math.log2(32768.0 / max(float(largest), 1e-30))), 40)
+
+
+def table_rows(table: torch.Tensor, per: int, first: int = 0):
+    """Hidden features and their d/dr from the intervals of a table from ``first`` on, in nine places of each: lengths
+    [intervals, 9] and [intervals, 9, 64] each, float64."""
+    u = torch.linspace(-1, 1, 9, dtype=torch.float64)
+    powers = torch.stack([u ** k for k in range(table.shape[1])])
+    slopes = torch.stack([2.0 * per * k * u ** max(k - 1, 0) for k in range(table.shape[1])])
+    r = (torch.arange(first, len(table), dtype=torch.float64)[:, None] + 0.5 + 0.5 * u) / per
+    return r, *(torch.einsum("nkf,ku->nuf", table[first:].double(), p) for p in (powers, slopes))
+
+
+def onchip_long(table: torch.Tensor, per: int, scale: float, tangent_scale: float, r_cut: float):
+    """How the kernels scale the features of long edges: (length from which on they look at them, cutoff, factor a, factor b).
+    Near the cutoff the largest value is at most 4 a (cutoff - r)^4 and the largest d/dr 4 b (cutoff - r)^3 under the scales;
+    beyond the length one of these is below 1/4, and rows of which that holds are scaled by the inverse of the law."""
+    r, value, slope = table_rows(table, per)
+    tops = value.abs().amax(2) * scale, slope.abs().amax(2) * tangent_scale
+    least = torch.minimum(*tops)
+    least[0, 0] = least[0, 1]
+    small = torch.nonzero(least.amin(1) < 1.0)
+    first = int(small[0]) if len(small) else len(table)
+    d = (r_cut - r).clamp_min(ONCHIP_NEAREST)
+    inside = (r >= first / per) & (r <= r_cut)
+    law = [0.25 * float((top * inside / d ** k).max()) for top, k in zip(tops, (4, 3))]
+    reach = r_cut - max((0.0625 / max(a, 1e-30)) ** (1 / k) for a, k in zip(law, (4, 3)))
+    return max(reach, first / per), r_cut, *law
+
+
+def onchip_is_accurate(w4: torch.Tensor, image: torch.Tensor, r: torch.Tensor, features: torch.Tensor, tangents: torch.Tensor) -> bool:
+    """Does the image (``onchip_image``) of the layer give products with the hidden ``features`` and their d/dr [n, 64] at the
+    lengths ``r`` that are off by no more than those of tf32 pairs can be: 2^-23 of every term for the remainder of each operand
+    and 2^-22 for the product of remainders that is left out? fp16 pairs have fewer bits where a weight is below 2^-17 of the
+    layer's largest, or a feature below 2^-2 under its row's scale."""
+    n_out = w4.shape[1]
+    weights = w4.to(torch.float64)
+    parts = image[ONCHIP_HEADER:].view(torch.float16).double().reshape(2, n_out // 256, 2, 8, 128, 8) * float(image[0]) * float(image[2])
+    parts = parts.permute(2, 1, 4, 0, 3, 5).reshape(2, n_out // 256, 2, 64, 2, 64)     # [part][pair][path][channel][half][k]
+    parts = parts.transpose(3, 4).reshape(2, n_out, 64).transpose(1, 2)
+    d = (float(image[4]) - r).clamp_min(ONCHIP_NEAREST)
+    for scale, rows, law in ((image[0], features, d ** 4 * float(image[5])), (image[1], tangents, d ** 3 * float(image[6]))):
+        h = rows.to(torch.float32).to(torch.float64)
+        up = torch.where((r < float(image[3])) | (law >= 0.0625), torch.ones_like(r),
+                         torch.exp2(-torch.floor(torch.log2(law.clamp_min(2.0 ** -126)))))
+        power = float(scale) * up[:, None]
+        if not bool((h * power).abs().max() < 65504.0):
+            return False
+        value = (h * power).to(torch.float16).double()
+        rest = (h * power - value).to(torch.float16).double()
+        off = ((h - (value + rest) / power).abs() @ weights.abs() + h.abs() @ (weights - parts.sum(0)).abs()
+               + (rest / power).abs() @ parts[1].abs())
+        if not bool((off <= 2.0 ** -21 * (h.abs() @ weights.abs())).all()):
+            return False
+    return True
 
 
 RADIAL_DEGREE = 5
@@ -332,9 +392,17 @@ class PackedModel:
                             largest_tangent = (table[:, 1:].abs() * power[None, :, None]).sum(1).max() * 2.0 * found[1]
                             w4 = self.tensors[f"l{t}.rad.3"].cpu()
                             if bool(torch.isfinite(w4).all()) and largest > 0 and largest_tangent > 0:
-                                layer.rad_img = self._put(f"l{t}.rad.img", torch.cat(
-                                    [radial_image(w4, c), onchip_image(w4, largest, largest_tangent)]))
-                                layer.extra_images |= IMAGES | IMAGE_ONCHIP
+                                long = onchip_long(*found, onchip_scale(largest), onchip_scale(largest_tangent), spec.r_cut)
+                                image = onchip_image(w4, largest, largest_tangent, long)
+                                # accurate at every eighth interval and, where the scales begin to grow, at all
+                                r, value, slope = table_rows(*found)
+                                some = torch.arange(len(r)) % 8 == 0
+                                some |= r[:, 0] >= long[0] - 0.25
+                                picked = [q[some][:, ::4].reshape(-1, *q.shape[2:]) for q in (r, value, slope)]
+                                within = (picked[0] > 0) & (picked[0] < spec.r_cut - ONCHIP_NEAREST)
+                                if onchip_is_accurate(w4, image, *(q[within] for q in picked)):
+                                    layer.rad_img = self._put(f"l{t}.rad.img", torch.cat([radial_image(w4, c), image]))
+                                    layer.extra_images |= IMAGES | IMAGE_ONCHIP
             if t == 0:
                 x_species = h0 @ (w["l0.up.0"] / math.sqrt(c))
                 sc = torch.zeros(len(idx), spec.out_dim(0), c, dtype=torch.float64)

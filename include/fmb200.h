@@ -164,8 +164,11 @@ typedef struct {
      * the 64 hidden features) and part (0 = tf32 remainder, 1 = tf32 value) a 16 KB tile [128 channels][32] of
      * W4^T in the K-major 128-byte-swizzled operand layout, at float offset ((p * 2 + h) * 2 + part) * 4096.
      * Null = materialise the per-edge weights with a GEMM. With FMB_IMAGE_ONCHIP (l_in_max 1), from float offset
-     * n_paths * 16384 on: four floats (the powers of two s and s' by which the hidden features and their d/dr are
-     * multiplied to fill the fp16 range, the inverse of s times the weights' own scale, one unused), then per half of the
+     * n_paths * 16384 on: eight floats (powers of two s and s' that bring the largest hidden features and d/dr of any
+     * length half way up the fp16 range, the inverse of s times the weights' own scale; a length, the cutoff, and two
+     * numbers a and b such that the largest feature of an edge of that length or more is at most 4 a (cutoff - r)^4 and the
+     * largest d/dr 4 b (cutoff - r)^3 under s and s': where that is below 1/4 they are split under a power of two made from
+     * it; one unused), then per half of the
      * channels and pair of paths the scaled weights as fp16 values and then as fp16 remainders, [8][128 rows][8] each (row =
      * path of the pair, channel of the half). */
     const float* rad_img;
