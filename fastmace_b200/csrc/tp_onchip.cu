@@ -306,6 +306,11 @@ __device__ __forceinline__ void issue_products(const Cta<LIN, ADJOINT>& c) {
         __syncwarp();
         if (k + 1 < tiles) split.put(k + 1, tiles);
     }
+    // after a wait that ran out nobody may have waited for the last products: they end before tensor memory is given back
+    if (*c.abort_flag && tiles > 0) {
+        const int k = tiles - 1;
+        for (unsigned spin = 0; spin < kSpin && !mbar_try(c.bar(S::kBEmpty + k % kBSlots), (uint32_t)(k / kBSlots) & 1u); ++spin) {}
+    }
 }
 
 // eight columns of the accumulator back to the common scale
@@ -414,6 +419,7 @@ __device__ __forceinline__ void bring_rows(const Cta<LIN, ADJOINT>& c, int part)
         }
         c.arrive(S::kFull + st);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");                  // in flight still only after a wait that ran out
 }
 
 // ------------------------------------------------------------------------------------------------ evaluating warps
