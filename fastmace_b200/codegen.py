@@ -313,9 +313,11 @@ def _write(path: str, text: str) -> None:
 # --------------------------------------------------------------------------------------------- coupled bodies
 COUPLED_OUT = os.path.join(HERE, "csrc", "generated", "tp_coupled_generated.cuh")
 
+
 def coupled_layout(paths):
-    """Where the couplings of an edge stand: T[path][m_out][m_in] = sum_me coef * Y[me], structural zeros left out. Returns ({(path, m_out, m_in): offset}, {offset: [(edge component, coef)]}, floats); the
-    row stride is 4 mod 32 floats so that the rows of neighbouring edges start in different banks."""
+    """Where the couplings of an edge stand: T[path][m_out][m_in] = sum_me coef * Y[me], structural zeros left out. Returns
+    ({(path, m_out, m_in): offset}, {offset: [(edge component, coef)]}, floats); the row stride is 4 mod 32 floats so that
+    the rows of neighbouring edges start in different banks."""
     offset, sums, at = {}, {}, 0
     for p, path in enumerate(paths):
         for mi, me, mo, c in sorted(path["terms"], key=lambda t: (t[2], t[0], t[1])):

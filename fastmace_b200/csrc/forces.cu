@@ -3,7 +3,8 @@
 // autograd force/virial path it runs (fastmace/rewrites/engine.py:122-192). Everything is stream-ordered and reads
 // the edge count from the device, so the whole call can be captured in a CUDA graph.
 //
-// Tensor-product weights are materialised per chunk of `chunk_edges` edges (values in the first half of tp_w,
+// The second interaction of node l_max 1 makes its radial weights where it uses them (radial_on_chip). Elsewhere they are
+// materialised per chunk of `chunk_edges` edges (values in the first half of tp_w,
 // d/dr in the second half; of twice as many edges in the forward pass, which needs the values only); the backward pass
 // recomputes them chunk by chunk instead of keeping them, unless the whole list is one chunk.
 
@@ -176,8 +177,12 @@ long long weight_rows(const Ctx& c) { return c.w->pair_capacity > 0 ? (long long
 bool has_image(const fmb_layer_t& L, int bit) { return (L.extra_images & ~0xff) == FMB_IMAGES && (L.extra_images & bit) != 0; }
 
 // The last interaction with its last radial layer inside the kernels (tp_onchip.cu): the layer is packed for them, every row
-// carries a gradient, and tp_w, which then holds no weights, has room for their scratch. Not where rows are few: the kernels
-// load 160 KB of weights per CTA first and give every warp a range of edges, where the others cut a receiver's row in four.
+// carries a gradient, and tp_w, which then holds no weights, has room for their scratch: 12 MB, and 160 bytes for every entry
+// of the whole list. A list in more than 64 chunks (beyond 33.5 M entries, where tp_w is sized for one of them) has not, and
+// keeps the kernels that read the weights from memory. Nor are lists of up to 300 rows moved: their results stay those of
+// the other kernels. By time the line could lie lower: a force call, weights in memory / on the SM, takes 203 / 197 us for 129
+// atoms of silica, 250 / 233 for 249, 276 / 250 for 303, 400 / 364 for 600; for 256 atoms of NaCl 199 / 183, for 384
+// 224 / 209; for gases of 3 to 12 neighbours and 150 to 640 atoms they are within 6 %.
 constexpr int kOnChipRows = 300;
 bool radial_on_chip(const Ctx& c) {
     const fmb_layer_t& L = c.m->layer[c.m->n_layers - 1];
@@ -333,6 +338,31 @@ TpOnChipArgs onchip_args(const Ctx& c, int layer) {
     return t;
 }
 
+// The message of a layer from radial weights in memory, chunk by chunk.
+int forward_streamed(const Ctx& c, int layer, int rows, const float* x) {
+    const fmb_layer_t& L = c.m->layer[layer];
+    // a list in several chunks: the forward pass has no use for the d/dr half of tp_w and fills both with values, which
+    // halves its launches. A producer launch takes 44 us however few rows it has: force call of 562 k edges in chunks of
+    // 8,192 18.3 -> 15.8 ms, of 16,384 11.6 -> 10.3, of 2^19 the same
+    const long long chunk = c.n_chunks > 1 ? std::min(2 * c.chunk, c.count_cap) : c.chunk;
+    for (long long e0 = 0; e0 < c.count_cap; e0 += chunk) {
+        if (c.radial_ready && layer > 0) {
+            FMB_CUDA_CHECK(cudaStreamWaitEvent(c.stream, c.radial_ready, 0));     // produced beside the first interaction
+        } else {
+            FMB_TRY(radial_weights(c, layer, e0, 0, 0, edge_limit(c, layer == 0 ? 0 : 1), nullptr, 0, chunk));
+        }
+        TpArgs t{};
+        t.lin = L.l_in_max; t.species_x = layer == 0; t.n_atoms = c.n; t.n_rows = rows;
+        t.chunk_e0 = e0; t.chunk_edges = chunk; t.whole_list = chunk >= c.count_cap; t.error_word = c.w->status;
+        t.count = (const long long*)c.nl->count; t.row_ptr = c.nl->edge_row_ptr; t.senders = c.nl->edge_index;
+        t.species = c.w->species; t.x = x; t.edge_sh = c.w->edge_sh; t.tp_w = c.w->tp_w; t.mid = c.w->mid;
+        if (layer == c.m->n_layers - 1 && pair_rows(c)) t.slot = c.w->edge_slot;
+        StageScope scope(c.stream, layer == 0 ? kStTpFwd0 : kStTpFwd1);
+        FMB_TRY(tp_forward_launch(t, c.stream));
+    }
+    return FMB_OK;
+}
+
 int forward_layer(const Ctx& c, int layer, bool with_up = true) {
     const fmb_layer_t& L = c.m->layer[layer];
     const MidLayout ml = mid_layout(L.l_in_max);
@@ -378,34 +408,16 @@ int forward_layer(const Ctx& c, int layer, bool with_up = true) {
                          (long long)l * l * kC, kC, l, 0);
         FMB_TRY(run_linears(c, lb));
     } else {
-    if (layer > 0 && radial_on_chip(c)) {
-        StageScope scope(c.stream, kStTpFwd1);
-        FMB_TRY(tp_forward_onchip(onchip_args(c, layer), c.stream));
-    } else {
-    // a list in several chunks: the forward pass has no use for the d/dr half of tp_w and fills both with values, which
-    // halves its launches. A producer launch takes 44 us however few rows it has: force call of 562 k edges in chunks of
-    // 8,192 18.3 -> 15.8 ms, of 16,384 11.6 -> 10.3, of 2^19 the same
-    const long long chunk = c.n_chunks > 1 ? std::min(2 * c.chunk, c.count_cap) : c.chunk;
-    for (long long e0 = 0; e0 < c.count_cap; e0 += chunk) {
-        if (c.radial_ready && layer > 0) {
-            FMB_CUDA_CHECK(cudaStreamWaitEvent(c.stream, c.radial_ready, 0));     // produced beside the first interaction
+        if (layer > 0 && radial_on_chip(c)) {
+            StageScope scope(c.stream, kStTpFwd1);
+            FMB_TRY(tp_forward_onchip(onchip_args(c, layer), c.stream));
         } else {
-            FMB_TRY(radial_weights(c, layer, e0, 0, 0, edge_limit(c, layer == 0 ? 0 : 1), nullptr, 0, chunk));
+            FMB_TRY(forward_streamed(c, layer, rows, x));
         }
-        TpArgs t{};
-        t.lin = L.l_in_max; t.species_x = layer == 0; t.n_atoms = c.n; t.n_rows = rows;
-        t.chunk_e0 = e0; t.chunk_edges = chunk; t.whole_list = chunk >= c.count_cap; t.error_word = c.w->status;
-        t.count = (const long long*)c.nl->count; t.row_ptr = c.nl->edge_row_ptr; t.senders = c.nl->edge_index;
-        t.species = c.w->species; t.x = x; t.edge_sh = c.w->edge_sh; t.tp_w = c.w->tp_w; t.mid = c.w->mid;
-        if (layer == c.m->n_layers - 1 && pair_rows(c)) t.slot = c.w->edge_slot;
-        StageScope scope(c.stream, layer == 0 ? kStTpFwd0 : kStTpFwd1);
-        FMB_TRY(tp_forward_launch(t, c.stream));
-    }
-    }
-    for (int l = 0; l <= 3; ++l)
-        block_linear(lb, c, rows, c.w->mid, (long long)ml.mid_dim * kC, (long long)ml.base[l] * kC, ml.segs[l] * kC, L.w_lin,
-                     L.tc[5], L.tc_img[5], lin_weight_offset(ml, l), msg, (long long)kNSH * kC, (long long)l * l * kC, kC, l, 0);
-    FMB_TRY(run_linears(c, lb));
+        for (int l = 0; l <= 3; ++l)
+            block_linear(lb, c, rows, c.w->mid, (long long)ml.mid_dim * kC, (long long)ml.base[l] * kC, ml.segs[l] * kC, L.w_lin,
+                         L.tc[5], L.tc_img[5], lin_weight_offset(ml, l), msg, (long long)kNSH * kC, (long long)l * l * kC, kC, l, 0);
+        FMB_TRY(run_linears(c, lb));
     }
     {
         StageScope scope(c.stream, kStSymFwd);

@@ -12,6 +12,9 @@
 // rows, accumulate, species mask -- the same GemmArgs contract as the SIMT kernel). Two CTAs of 8 warps fit per SM
 // (96 KB shared memory, 128 TMEM columns each).
 //
+// The weights as this package packs them all have images for gemm_ws.cu, which is faster: this kernel serves fmb_gemm and hosts
+// that pack the twins without the images (gemm_batch in gemm.cu takes whichever is there).
+//
 // Every wait is bounded: if the mbarrier does not flip within the spin limit the CTA raises the error word, skips the
 // remaining work, frees its TMEM and returns.
 

@@ -165,8 +165,13 @@ int readout(const fmb_model_t* m, int n_atoms, int n_energy, const float* h_firs
     const int dim_first = (m->layer[0].l_out_max + 1) * (m->layer[0].l_out_max + 1);
     const int dim_last = 1;
     const float* w_last = m->layer[m->n_layers - 1].w_readout;
+    static const int cap = [] {                // four CTAs per SM
+        int device = 0, sms = 148;
+        if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        return 4 * sms;
+    }();
     const int blocks = ceil_div(n_atoms, kReadoutWarps);
-    k_readout<<<blocks < 592 ? blocks : 592, 32 * kReadoutWarps, 0, stream>>>(
+    k_readout<<<blocks < cap ? blocks : cap, 32 * kReadoutWarps, 0, stream>>>(
         n_atoms, n_energy, dim_first, dim_last, m->scale, m->shift, m->silu_norm, h_first, h_last, m->layer[0].w_readout, w_last,
         w_last + kC * 16, node_energy, d_h_first, d_h_last);
     FMB_LAUNCH_CHECK();

@@ -1,6 +1,6 @@
 // Channelwise tensor product of the interactions after the first with the last radial layer inside the kernel (node l_max
 // 1): the per-edge radial weights and their d/dr are products of the tensor cores that never leave the SM, where the kernels of
-// tp_coupled.cu read them from memory (20 P C bytes written and read per pair of edges and force call).
+// tp_coupled.cu read them from memory (per pair of edges and force call 8 P C bytes written and 24 P C read).
 //
 // The last radial layer stays in tensor memory. As fp16 values and remainders the columns of half the channels, 640 of them,
 // take 320 of 512 TMEM columns as the first operand of the MMAs, K along the
@@ -21,10 +21,12 @@
 // ranges, so that a warp meets the edges of its rows one after the other. Registers are dealt again after the start.
 // Every wait is bounded (tc::mbar_wait).
 //
-// Bound by the evaluating warps: two per scheduler, FP32 pipe 52 %, shared memory 58 % and issue slots 53 % busy in the adjoint.
-// Adjoint / forward kernel, streamed and here: 62 k edges 145 -> 160 and 72 -> 90 us, 615 k edges 1,378 -> 1,374 and 650 -> 775,
-// and no producers (2 x 43 us and 2 x 360 us on the second stream, which slowed what ran beside them): a step of 1,944 atoms
-// 742 -> 683 us, a force call of 10,368 atoms 4,679 -> 3,956, one in chunks 6,190 -> 4,159.
+// Bound inside the SM, two evaluating warps per scheduler: adjoint / forward, 62 k edges, shared memory 68 / 63 %, FP32 pipe 57 /
+// 33, issue slots 59 / 39, tensor pipe 19 / 16, HBM 14 / 4 % busy.
+// Adjoint / forward kernel, streamed and here: 62 k edges 145 -> 162 and 72 -> 96 us, 615 k edges (the adjoint's with the gather
+// behind it) 1,620 either way and 650 -> 800, and no producers (2 x 43 us and 2 x 360 us on the second stream, which slowed
+// what ran beside them): a step of 1,944 atoms 742 -> 665 us, a force call of 10,368 atoms 4,679 -> 3,856, one in chunks
+// 6,190 -> 4,006.
 
 #include "stages.cuh"
 #include "generated/tp_generated.cuh"
