@@ -161,18 +161,27 @@ def compulsory_bytes(spec, n_atoms: int, n_edges: int, n_species: int = 2) -> di
     return out
 
 
-def design_bytes(spec, n_atoms: int, n_edges: int, n_species: int = 2) -> dict:
-    """Bytes the kernels as built move per force call: the compulsory ones plus the per-edge radial weights in HBM
-    (values and d/dr, 4 P C bytes each, written once per pair of opposite edges and read by the tensor-product kernels
-    for both) and the per-edge hand-over of the sender gradient (written by the adjoint, read back by the gather)."""
+def design_bytes(spec, n_atoms: int, n_edges: int, n_species: int = 2, on_chip: bool = False) -> dict:
+    """Bytes the kernels as built move per force call: the compulsory ones, the per-edge hand-over of the sender gradient
+    (written by the adjoint, read back by the gather), and either the per-edge radial weights in HBM (values and d/dr, 4 P C
+    bytes each, written once per pair of opposite edges and read by the tensor-product kernels for both) or, with the last
+    radial layer on the SM (``on_chip``), the edges' rows read by both halves of the channels and 80 bytes of partial
+    gradients that each half writes and the first interaction's adjoint reads."""
     c = spec.channels
     hid = (spec.hidden_lmax + 1) ** 2
     p1 = len(spec.paths(1))
     out = dict(compulsory_bytes(spec, n_atoms, n_edges, n_species))
-    out["radial_gemm"] += n_edges * p1 * c * 4            # one row of each per pair of opposite edges
-    out["tp_forward_l1"] += n_edges * p1 * c * 4
     out["tp_backward_l0"] += n_edges * 16 * 64 * 4
-    out["tp_backward_l1"] += n_edges * (2 * p1 * c * 4 + 2 * hid * c * 4)
+    out["tp_backward_l1"] += n_edges * 2 * hid * c * 4
+    if on_chip:
+        out["radial_gemm"] = 0
+        out["tp_forward_l1"] += n_edges * (64 * 4 + 64 + 4)
+        out["tp_backward_l0"] += n_edges * 2 * 80
+        out["tp_backward_l1"] += n_edges * (2 * 64 * 4 + 64 + 4 + 2 * 80)
+    else:
+        out["radial_gemm"] += n_edges * p1 * c * 4        # one row of each per pair of opposite edges
+        out["tp_forward_l1"] += n_edges * p1 * c * 4
+        out["tp_backward_l1"] += n_edges * 2 * p1 * c * 4
     return out
 
 
@@ -612,8 +621,12 @@ def main():
     force_ms = sum(stage_ms.values())
     n_species = len(set(int(z) for z in structure.numbers))
     algo = compulsory_bytes(spec, n_atoms, n_edges, n_species)
-    design = design_bytes(spec, n_atoms, n_edges, n_species)
+    design = design_bytes(spec, n_atoms, n_edges, n_species, on_chip=stages["radial_gemm"][1] == 0)   # no producer ran
     top = max((k for k in stage_ms if k in algo), key=lambda k: stage_ms[k])
+    # every step writes or reads all of these: per edge hidden features with d/dr and sender gradients, per atom the node rows
+    per_edge = ff.buf["edge_hidden"].numel() // ff.edge_capacity + (ff.buf["edge_dx"][0].numel() if "edge_dx" in ff.buf else 0)
+    per_atom = sum(ff.buf[name].numel() // ff.atom_capacity for name in ("mid", "d_mid", "msg", "d_msg", "h"))
+    working_set = 4 * (n_edges * per_edge + n_atoms * per_atom)
     pk = peaks()
     achieved = algo[top] / (stage_ms[top] * 1e-3) / 1e9
     traffic = measured_traffic(top, n_edges) if args.workload == DEFAULT_WORKLOAD else None
@@ -632,7 +645,8 @@ def main():
                 scaling="weak", vs_baseline=None, dtype="f32", data="synthetic",
                 config=dict(workload=args.workload, atoms=n_atoms, edges=n_edges, model=WORKLOADS[args.workload]["model"],
                             integrator="langevin_nvt_1fs_0.01perfs", parallelism=f"replicas{world}" if world > 1 else "1gpu",
-                            l2="per-step working set (radial weight tensors, > 600 MB) exceeds the 126 MB L2; no flush",
+                            l2=f"per-step working set ({working_set / 1e6:.0f} MB of hidden features, sender gradients and node "
+                               "rows) exceeds the 126 MB L2; no flush",
                             neighbour_rebuilds=ff.neighbours.rebuilds),
                 clocks=clocks,
                 e2e=dict(value=e2e_value, unit="atom-steps/s", h2d_bytes_per_step=2 * n_atoms * 3 * 8,
