@@ -23,10 +23,10 @@
 //
 // Bound inside the SM, two evaluating warps per scheduler: adjoint / forward, 62 k edges, shared memory 68 / 63 %, FP32 pipe 57 /
 // 33, issue slots 59 / 39, tensor pipe 19 / 16, HBM 14 / 4 % busy.
-// Adjoint / forward kernel, streamed and here: 62 k edges 145 -> 162 and 72 -> 96 us, 615 k edges (the adjoint's with the gather
-// behind it) 1,620 either way and 650 -> 800, and no producers (2 x 43 us and 2 x 360 us on the second stream, which slowed
-// what ran beside them): a step of 1,944 atoms 742 -> 665 us, a force call of 10,368 atoms 4,679 -> 3,856, one in chunks
-// 6,190 -> 4,006.
+// Adjoint / forward kernel, streamed and here: 62 k edges 145 -> 160 and 72 -> 96 us, 615 k edges 1,378 -> 1,350 (1,595 with the
+// gather behind it) and 650 -> 800, and no producers (2 x 43 us and 2 x 360 us on the second stream, which slowed what ran
+// beside them): a step of 1,944 atoms 742 -> 666 us, a force call of 10,368 atoms 4,679 -> 3,825, one in chunks
+// 6,190 -> 4,010.
 
 #include "stages.cuh"
 #include "generated/tp_generated.cuh"
@@ -317,12 +317,13 @@ __device__ __forceinline__ void issue_products(const Cta<LIN, ADJOINT>& c) {
 
 // eight columns of the accumulator back to the common scale
 template <int FIRST>
-__device__ __forceinline__ void unscale(float (&v)[16], const float* scales) {
+__device__ __forceinline__ void unscale(float (&v)[16], const float4* scale) {
 #pragma unroll
-    for (int q = FIRST; q < FIRST + 8; q += 2) {
-        const float2 w = __fmul2_rn(make_float2(v[q], v[q + 1]), *reinterpret_cast<const float2*>(scales + q));
-        v[q] = w.x;
-        v[q + 1] = w.y;
+    for (int q = FIRST; q < FIRST + 8; q += 4) {
+        const float4 s = scale[q / 4];
+        const float2 a = __fmul2_rn(make_float2(v[q], v[q + 1]), make_float2(s.x, s.y)),
+                     b = __fmul2_rn(make_float2(v[q + 2], v[q + 3]), make_float2(s.z, s.w));
+        v[q] = a.x; v[q + 1] = a.y; v[q + 2] = b.x; v[q + 3] = b.y;
     }
 }
 
@@ -338,14 +339,20 @@ __device__ __forceinline__ void carry_weights(const Cta<LIN, ADJOINT>& c, int qu
         c.wait(S::kEmpty + st, ((uint32_t)(k / S::kStages) & 1u) ^ 1u);
         c.wait(S::kDFull + acc, (uint32_t)(k / kAccumulators) & 1u);
         fence_after_sync();
+        // the scales of a part wait in registers in the adjoint (615 k edges 1,629 -> 1,595 us), in the forward pass in shared
+        // memory (808 us, 821 in registers)
         const int2 scaled = *reinterpret_cast<const int2*>(c.scaled(k));
+        const float4* const scales = reinterpret_cast<const float4*>(c.scales(k));
+        float4 scale[4];
+        if (ADJOINT && scaled.x) { scale[0] = scales[0]; scale[1] = scales[1]; }
+        if (ADJOINT && scaled.y) { scale[2] = scales[2]; scale[3] = scales[3]; }
         float* const to = c.block(k, 0) + at;
 #pragma unroll
         for (int j = 0; j < S::kTiles; ++j) {
             float v[16];
             tmem_load_16(base + acc * S::kDColumns + 16 * j, v);
-            if (scaled.x) unscale<0>(v, c.scales(k));
-            if (scaled.y) unscale<8>(v, c.scales(k));
+            if (scaled.x) unscale<0>(v, ADJOINT ? scale : scales);
+            if (scaled.y) unscale<8>(v, ADJOINT ? scale : scales);
             if (j == S::kTiles - 1) {
                 fence_before_sync();
                 c.arrive(S::kDEmpty + acc);

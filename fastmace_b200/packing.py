@@ -159,31 +159,30 @@ def onchip_scale(largest: float) -> float:
     return 2.0 ** min(math.floor(math.log2(32768.0 / max(float(largest), 1e-30))), 40)
 
 
-def table_rows(table: torch.Tensor, per: int, first: int = 0):
-    """Hidden features and their d/dr from the intervals of a table from ``first`` on, in nine places of each: lengths
-    [intervals, 9] and [intervals, 9, 64] each, float64."""
+def table_rows(table: torch.Tensor, per: int):
+    """Hidden features and their d/dr from a table, in nine places of every interval: lengths [intervals, 9] and
+    [intervals, 9, 64] each, float64."""
     u = torch.linspace(-1, 1, 9, dtype=torch.float64)
     powers = torch.stack([u ** k for k in range(table.shape[1])])
     slopes = torch.stack([2.0 * per * k * u ** max(k - 1, 0) for k in range(table.shape[1])])
-    r = (torch.arange(first, len(table), dtype=torch.float64)[:, None] + 0.5 + 0.5 * u) / per
-    return r, *(torch.einsum("nkf,ku->nuf", table[first:].double(), p) for p in (powers, slopes))
+    r = (torch.arange(len(table), dtype=torch.float64)[:, None] + 0.5 + 0.5 * u) / per
+    return r, *(torch.einsum("nkf,ku->nuf", table.double(), p) for p in (powers, slopes))
 
 
-def onchip_long(table: torch.Tensor, per: int, scale: float, tangent_scale: float, r_cut: float):
-    """How the kernels scale the features of long edges: (length from which on they look at them, cutoff, factor a, factor b).
+def onchip_long(r: torch.Tensor, value: torch.Tensor, slope: torch.Tensor, scale: float, tangent_scale: float, r_cut: float):
+    """How the kernels scale the features of long edges (``table_rows``): (length from which on they look at them, cutoff, factor a, factor b).
     Near the cutoff the largest value is at most 4 a (cutoff - r)^4 and the largest d/dr 4 b (cutoff - r)^3 under the scales;
     beyond the length one of these is below 1/4, and rows of which that holds are scaled by the inverse of the law."""
-    r, value, slope = table_rows(table, per)
     tops = value.abs().amax(2) * scale, slope.abs().amax(2) * tangent_scale
     least = torch.minimum(*tops)
     least[0, 0] = least[0, 1]
     small = torch.nonzero(least.amin(1) < 1.0)
-    first = int(small[0]) if len(small) else len(table)
+    first = float(r[int(small[0]), 0]) if len(small) else r_cut
     d = (r_cut - r).clamp_min(ONCHIP_NEAREST)
-    inside = (r >= first / per) & (r <= r_cut)
+    inside = (r >= first) & (r <= r_cut)
     law = [0.25 * float((top * inside / d ** k).max()) for top, k in zip(tops, (4, 3))]
     reach = r_cut - max((0.0625 / max(a, 1e-30)) ** (1 / k) for a, k in zip(law, (4, 3)))
-    return max(reach, first / per), r_cut, *law
+    return max(reach, first), r_cut, *law
 
 
 def onchip_is_accurate(w4: torch.Tensor, image: torch.Tensor, r: torch.Tensor, features: torch.Tensor, tangents: torch.Tensor) -> bool:
@@ -392,15 +391,13 @@ class PackedModel:
                             largest_tangent = (table[:, 1:].abs() * power[None, :, None]).sum(1).max() * 2.0 * found[1]
                             w4 = self.tensors[f"l{t}.rad.3"].cpu()
                             if bool(torch.isfinite(w4).all()) and largest > 0 and largest_tangent > 0:
-                                long = onchip_long(*found, onchip_scale(largest), onchip_scale(largest_tangent), spec.r_cut)
+                                rows = table_rows(*found)
+                                long = onchip_long(*rows, onchip_scale(largest), onchip_scale(largest_tangent), spec.r_cut)
                                 image = onchip_image(w4, largest, largest_tangent, long)
-                                # accurate at every eighth interval and, where the scales begin to grow, at all
-                                r, value, slope = table_rows(*found)
-                                some = torch.arange(len(r)) % 8 == 0
-                                some |= r[:, 0] >= long[0] - 0.25
-                                picked = [q[some][:, ::4].reshape(-1, *q.shape[2:]) for q in (r, value, slope)]
-                                within = (picked[0] > 0) & (picked[0] < spec.r_cut - ONCHIP_NEAREST)
-                                if onchip_is_accurate(w4, image, *(q[within] for q in picked)):
+                                # accurate in the middle of every 16th interval and, where the scales begin to grow, of all?
+                                some = (torch.arange(len(rows[0])) % 16 == 0) | (rows[0][:, 0] >= long[0] - 0.1)
+                                some &= rows[0][:, 4] < spec.r_cut - ONCHIP_NEAREST
+                                if onchip_is_accurate(w4, image, *(q[some, 4] for q in rows)):
                                     layer.rad_img = self._put(f"l{t}.rad.img", torch.cat([radial_image(w4, c), image]))
                                     layer.extra_images |= IMAGES | IMAGE_ONCHIP
             if t == 0:
