@@ -21,7 +21,7 @@
 // ranges, so that a warp meets the edges of its rows one after the other. Registers are dealt again after the start.
 // Every wait is bounded (tc::mbar_wait).
 //
-// Bound inside the SM, two evaluating warps per scheduler: adjoint / forward, 62 k edges, shared memory 68 / 63 %, FP32 pipe 57 /
+// Bound inside the SM, two evaluating warps per scheduler: adjoint / forward, 62 k edges, shared memory 66 / 63 %, FP32 pipe 58 /
 // 33, issue slots 59 / 39, tensor pipe 19 / 16, HBM 14 / 4 % busy.
 // Adjoint / forward kernel, streamed and here: 62 k edges 145 -> 160 and 72 -> 96 us, 615 k edges 1,378 -> 1,350 (1,595 with the
 // gather behind it) and 650 -> 800, and no producers (2 x 43 us and 2 x 360 us on the second stream, which slowed what ran
